@@ -1,568 +1,356 @@
-// Streamwise (x) line operators of lip.f90 (interpxx, difvisxx), one thread
-// per line. A line is a fixed (j, kr) of the plane layout; its nx values are
-// read with the plane stride, so the reference's chp2x transpose is replaced
-// by these strided, warp-coalesced loads (its REAL4 rounding is applied at
-// the same points when OTBL_XPOSE_FP32 is set).
-#include <cudaTypedefs.h>
-
-#include <type_traits>
+// Streamwise (x) line operators of lip.f90 (interpxx, difvisxx). A line is a
+// fixed (j, kr) of the plane layout; its nx values are read with the plane
+// stride, so the reference's chp2x transpose is replaced by these strided
+// loads (its REAL4 rounding is applied at the same points when
+// OTBL_XPOSE_FP32 is set). The tridiagonal solves are the chunked ones of
+// lines.cuh: a CTA holds L pairs of neighbouring lines, a thread K planes of
+// one pair.
+#include <algorithm>
 
 #include "devcommon.cuh"
+#include "lines.cuh"
 #include "otbl_internal.cuh"
-#include "tma.cuh"
 
 namespace otbl {
 
-// ---------------------------------------------------------------------------
-// x-lines streamed through registers: one thread per line (pencil), the
-// threads of a warp on consecutive (j, kr), so every row access is a
-// coalesced 256-byte request and every coefficient a broadcast. The forward
-// sweep y_i = b_i + l_i y_{i-1} (b the explicit stencil) leaves a checkpoint
-// of y every K rows in scratch; the backward sweep x_i = (y_i - u_i x_{i+1})
-// d_i walks the segments from the last one, recomputing each segment's y in
-// registers from its checkpoint. This is the serial Thomas of lip.f90 in the
-// reference's order; the traffic is about 1.5x the minimum (inputs read
-// twice) with no shared memory and no scan.
-//
 // T is the arithmetic and output type: double, or float on the mixed path
-// (the FP64 state is read and rounded on load, the FP32 coefficient copy is
-// used). Element types of the buffers: interpx reads the state (double),
-// difvisx reads the products (T) and the state; outputs and checkpoints T.
-// ---------------------------------------------------------------------------
-struct XStream {
+// (the FP64 state is read and rounded on load, the FP32 coefficients are
+// used). interpx reads the state (double), difvisx the products (T) and the
+// state; outputs T.
+struct XArgs {
   const void *in[3];
-  const double *in2[3];  // in2: the second input of difvisxx (velocity)
+  const double *in2[3];  // the second input of difvisxx (velocity)
   void *out[3];
-  double *ck[3];         // checkpoint scratch of each line set
-  int which[3], np[3];
+  int np[3];             // lines of each field
+  int tiles[3];          // CTA tiles of each field
+  const void *tab;       // coefficient tables (T): u-type, then v-type
+  int C, lgL;
 };
 
-// Segment lengths and occupancy per arithmetic type, measured on B200 at
-// 1025x193x512 over segments of 8-32 rows and 4-8 CTAs of 128 threads per
-// SM: interpxx 16 rows (FP64) / 8 rows (FP32) at >= 8 CTAs per SM; difvisxx
-// 8 rows at >= 6 CTAs per SM (3.16 ms per substep in FP64 against 3.46 for
-// 16 rows at 4 CTAs; 1.78 against 2.50 in FP32). FP32 interpxx runs
-// unbounded (56 registers).
-template <typename T>
-struct XTune;
-// tma: the TMA-fed kernels (k_xline_t) instead of the register streams,
-// with segments of kti (interpxx) and ktd (difvisxx) planes; at 1025x193x512
-// with the coefficient rows staged in the ring, FP64 RK3 step: 42.2 ms at
-// kti 8, 42.5 at 4; ktd 6 against 4 and 8: 42.5, 42.7, 42.7 (FP32 ktd 8
-// against 12: 30.8, 30.9). Before the staging: FP64 interpxx 1.17 ms (4
-// planes; 1.49 register-streamed), difvisxx 3.02 (6 planes; 3.18); FP32
-// interpxx 0.87, difvisxx 1.70.
-#ifndef OTBL_XT_DI
-#define OTBL_XT_DI 8
-#endif
-#ifndef OTBL_XT_DD
-#define OTBL_XT_DD 6
-#endif
-#ifndef OTBL_XT_FI
-#define OTBL_XT_FI 8
-#endif
-#ifndef OTBL_XT_FD
-#define OTBL_XT_FD 8
-#endif
-template <>
-struct XTune<double> {
-  static constexpr int kxi = 16, kxd = 8, minb_i = 8, kti = OTBL_XT_DI, ktd = OTBL_XT_DD;
-  static constexpr bool tma = true;
-};
-template <>
-struct XTune<float> {
-  // minb_i: 0.88 ms unbounded, 1.19 at >= 8
-  static constexpr int kxi = 8, kxd = 8, minb_i = 1, kti = OTBL_XT_FI, ktd = OTBL_XT_FD;
-  static constexpr bool tma = true;
-};
-
-
-template <typename T>
-__global__ void __launch_bounds__(128, XTune<T>::minb_i) k_interpx(DCoefT<T> c, XStream a) {
-  constexpr int KXI = XTune<T>::kxi;
-  const int f = blockIdx.y, np = pick3(a.np, f);
-  const int mp = blockIdx.x * blockDim.x + threadIdx.x;
-  if (mp >= np) return;
-  const int nx = c.nx, xr = c.xround, which = pick3(a.which, f);
-  const double *in = static_cast<const double *>(pick3(a.in, f)) + mp;
-  T *out = static_cast<T *>(pick3(a.out, f)) + mp;
-  T *ck = reinterpret_cast<T *>(pick3(a.ck, f)) + mp;
-  const T *icon = which == 0 ? c.inxu : c.inxv;
-  const T *econ = which == 0 ? c.cofiux : c.cofivx;
-  const int chi = which == 0 ? 2 : 1, chi2 = which == 0 ? 3 : 4;
-  const T *ib = c.inbx;
-  auto G = [&](int i) { return (T)rnd(__ldg(in + (size_t)i * np), xr); };
-  const T b0 = M4(ib, chi2, 1) * G(0) + M4(ib, chi2, 2) * G(1) + M4(ib, chi2, 3) * G(2) + M4(ib, chi2, 4) * G(3);
-  const T bN = M4(ib, chi, 1) * G(nx - 1) + M4(ib, chi, 2) * G(nx - 2) + M4(ib, chi, 3) * G(nx - 3) +
-               M4(ib, chi, 4) * G(nx - 4);
-  // right-hand side of row i from g_i, g_{i+1} (interior: lip.f90 stencil)
-  auto rhs = [&](int i, T gi, T gi1) {
-    return i == 0 ? b0 : (i == nx - 1 ? bN : __ldg(econ + 2 * i) * gi + __ldg(econ + 2 * i + 1) * gi1);
-  };
-  const int nseg = (nx + KXI - 1) / KXI;
-  T y = T(0);
-  for (int sg = 0; sg < nseg; ++sg) {
-    const int s = sg * KXI;
-    ck[(size_t)sg * np] = y;  // y of row s-1
-    T gv[KXI + 1];
-#pragma unroll
-    for (int b = 0; b <= KXI; ++b) gv[b] = G(min(s + b, nx - 1));
-#pragma unroll
-    for (int b = 0; b < KXI; ++b) {
-      const int i = s + b;
-      if (i < nx) y = rhs(i, gv[b], gv[b + 1]) + (i > 0 ? __ldg(icon + 3 * i) : T(0)) * y;
-    }
-  }
-  T xn = T(0);
-  for (int sg = nseg - 1; sg >= 0; --sg) {
-    const int s = sg * KXI;
-    T gv[KXI + 1], yv[KXI];
-#pragma unroll
-    for (int b = 0; b <= KXI; ++b) gv[b] = G(min(s + b, nx - 1));
-    T yy = ck[(size_t)sg * np];
-#pragma unroll
-    for (int b = 0; b < KXI; ++b) {
-      const int i = s + b;
-      if (i < nx) yy = rhs(i, gv[b], gv[b + 1]) + (i > 0 ? __ldg(icon + 3 * i) : T(0)) * yy;
-      yv[b] = yy;
-    }
-#pragma unroll
-    for (int b = KXI - 1; b >= 0; --b) {
-      const int i = s + b;
-      if (i < nx) {
-        xn = (yv[b] - __ldg(icon + 3 * i + 2) * xn) * __ldg(icon + 3 * i + 1);
-        out[(size_t)i * np] = (T)rnd(xn, xr);
-      }
-    }
-  }
+// coefficients of a table: interpxx w0, w1, l, d, e; difvisxx the same for
+// the convective system, then f1, f2, f3, l, d, e of the viscous one; after
+// the C chunks' values, the chunk products P, Q of each system
+constexpr int xcoefs(bool dv) { return dv ? 11 : 5; }
+// Tables of lines longer than 1152 planes (K > 9) stay in global memory:
+// with the tiles they exceed the shared memory of an SM.
+constexpr bool x_table_global(int K) { return K > 9; }
+static size_t xtab_elems(int K, int C, bool dv) {  // rounded up to a 16-byte multiple in either type
+  return ((size_t)C * (xcoefs(dv) * K + (dv ? 4 : 2)) + 3) / 4 * 4;
 }
 
-template <typename T>
-__global__ void __launch_bounds__(128, 6) k_difvisx(DCoefT<T> c, XStream a) {
-  constexpr int KXD = XTune<T>::kxd;
-  const int f = blockIdx.y, np = pick3(a.np, f);
-  const int mp = blockIdx.x * blockDim.x + threadIdx.x;
-  if (mp >= np) return;
-  const int nx = c.nx, xr = c.xround, which = pick3(a.which, f);
-  const T *gin = static_cast<const T *>(pick3(a.in, f)) + mp;
-  const double *uin = pick3(a.in2, f) + mp;
-  T *out = static_cast<T *>(pick3(a.out, f)) + mp;
-  T *ck = reinterpret_cast<T *>(pick3(a.ck, f)) + mp;
-  const T *icon = which == 0 ? c.dcxu : c.dcxv;
-  const T *iconv = which == 0 ? c.vixu : c.vixv;
-  const T *econ = which == 0 ? c.cofcxu : c.cofcxv;
-  const T *econv = which == 0 ? c.cofvxu : c.cofvxv;
-  const int chv = which == 0 ? 1 : 2, chv1 = chv + 2, ic = which == 0 ? 3 : 1;
-  const T *db = c.dcbx, *vb = c.cofvbx;
-  const T rex = c.S[OTBL_S_REX], idx = c.S[OTBL_S_IDX], uinf = c.S[OTBL_S_UINF];
-  auto G = [&](int i) { return (T)rnd(__ldg(gin + (size_t)i * np), xr); };
-  auto U = [&](int i) { return (T)rnd(__ldg(uin + (size_t)i * np), xr); };
-  const T gb0 = M5(db, chv, 1) * G(0) + M5(db, chv, 2) * G(1) + M5(db, chv, 3) * G(2) + M5(db, chv, 4) * G(3);
-  const T ub0 = M4(vb, ic, 1) * U(0) + M4(vb, ic, 2) * U(1) + M4(vb, ic, 3) * U(2) + M4(vb, ic, 4) * U(3);
-  const T gbN = M5(db, chv1, 1) * G(nx - 1) + M5(db, chv1, 2) * G(nx - 2) + M5(db, chv1, 3) * G(nx - 3) +
-                M5(db, chv1, 4) * G(nx - 4);
-  const T uN = U(nx - 1), uN1 = U(nx - 2);
-  const T ubN = M4(vb, ic + 1, 1) * uN + M4(vb, ic + 1, 2) * uN1 + M4(vb, ic + 1, 3) * U(nx - 3) +
-                M4(vb, ic + 1, 4) * U(nx - 4);
-  // right-hand sides of row i: convective e1 g_{i-1} + e2 g_i, viscous
-  // f1 u_{i+1} + f2 u_i + f3 u_{i-1} (lip.f90:52-142)
-  auto rg = [&](int i, T gm, T g0) {
-    return i == 0 ? gb0 : (i == nx - 1 ? gbN : __ldg(econ + 2 * i) * gm + __ldg(econ + 2 * i + 1) * g0);
-  };
-  auto ru = [&](int i, T um, T u0, T up) {
-    return i == 0 ? ub0
-                  : (i == nx - 1 ? ubN
-                                 : __ldg(econv + 3 * i) * up + __ldg(econv + 3 * i + 1) * u0 +
-                                       __ldg(econv + 3 * i + 2) * um);
-  };
-  const int nseg = (nx + KXD - 1) / KXD;
-  T yg = T(0), yu = T(0);
-  for (int sg = 0; sg < nseg; ++sg) {
-    const int s = sg * KXD;
-    ck[(size_t)(2 * sg) * np] = yg;
-    ck[(size_t)(2 * sg + 1) * np] = yu;
-    T gv[KXD + 1], uv[KXD + 2];  // rows s-1 .. s+K-1 (g), s-1 .. s+K (u)
-#pragma unroll
-    for (int b = 0; b <= KXD; ++b) gv[b] = G(min(max(s + b - 1, 0), nx - 1));
-#pragma unroll
-    for (int b = 0; b <= KXD + 1; ++b) uv[b] = U(min(max(s + b - 1, 0), nx - 1));
-#pragma unroll
-    for (int b = 0; b < KXD; ++b) {
-      const int i = s + b;
-      if (i < nx) {
-        yg = rg(i, gv[b], gv[b + 1]) + (i > 0 ? __ldg(icon + 3 * i) : T(0)) * yg;
-        yu = ru(i, uv[b], uv[b + 1], uv[b + 2]) + (i > 0 ? __ldg(iconv + 3 * i) : T(0)) * yu;
-      }
-    }
-  }
-  T xg = T(0), xu = T(0);
-  for (int sg = nseg - 1; sg >= 0; --sg) {
-    const int s = sg * KXD;
-    T gv[KXD + 1], uv[KXD + 2], ygv[KXD], yuv[KXD];
-#pragma unroll
-    for (int b = 0; b <= KXD; ++b) gv[b] = G(min(max(s + b - 1, 0), nx - 1));
-#pragma unroll
-    for (int b = 0; b <= KXD + 1; ++b) uv[b] = U(min(max(s + b - 1, 0), nx - 1));
-    T a1 = ck[(size_t)(2 * sg) * np], a2 = ck[(size_t)(2 * sg + 1) * np];
-#pragma unroll
-    for (int b = 0; b < KXD; ++b) {
-      const int i = s + b;
-      if (i < nx) {
-        a1 = rg(i, gv[b], gv[b + 1]) + (i > 0 ? __ldg(icon + 3 * i) : T(0)) * a1;
-        a2 = ru(i, uv[b], uv[b + 1], uv[b + 2]) + (i > 0 ? __ldg(iconv + 3 * i) : T(0)) * a2;
-      }
-      ygv[b] = a1;
-      yuv[b] = a2;
-    }
-#pragma unroll
-    for (int b = KXD - 1; b >= 0; --b) {
-      const int i = s + b;
-      if (i < nx) {
-        xg = (ygv[b] - __ldg(icon + 3 * i + 2) * xg) * __ldg(icon + 3 * i + 1);
-        xu = (yuv[b] - __ldg(iconv + 3 * i + 2) * xu) * __ldg(iconv + 3 * i + 1);
-        const T v = i == nx - 1 ? uinf * (uN - uN1) * idx + rex * T(0) : xg + rex * xu;
-        out[(size_t)i * np] = (T)rnd(v, xr);
-      }
-    }
-  }
-}
-
-// ---------------------------------------------------------------------------
-// The same x-line operators fed by TMA: a CTA owns TB consecutive lines of
-// one field; thread 0 loads, for the next segment of K planes, boxes of 32
-// lines x K+1 (K+2) planes of each input into a two-stage shared-memory ring
-// counted on mbarriers (bounded waits), while every thread runs its line's
-// serial sweeps from shared memory. The sequence of segments is the forward
-// sweep (0..nseg-1) then the backward one (nseg-1..0). DV: difvisxx (inputs:
-// the product, FP32 on the mixed path, and the FP64 velocity) or interpxx
-// (input: the FP64 velocity). The arithmetic is k_interpx / k_difvisx's,
-// with segments of K planes (XTune kti, ktd).
-// ---------------------------------------------------------------------------
-template <typename T, bool DV>
-constexpr int xseg() {
-  return DV ? XTune<T>::ktd : XTune<T>::kti;
-}
-
-template <typename T, bool DV, int TB>
-__global__ void __launch_bounds__(TB) k_xline_t(DCoefT<T> c, XStream a, int *err, const __grid_constant__ XMaps maps) {
-  constexpr int K = xseg<T, DV>(), NB = TB / 32;
+// A persistent CTA walks tiles of L pairs of lines (neighbouring CTAs on
+// neighbouring tiles, so the CTAs at work read contiguous rows). Each input
+// tile is copied to shared memory by cp.async while the tile before it is
+// being solved; its buffer is free as soon as every thread holds its rows in
+// registers. Five CTA barriers per difvisxx tile, three per interpxx tile.
+template <typename T, int K, bool DV, bool XR>
+__global__ void __launch_bounds__(K > 9 ? 256 : 512, 1) k_xline(DCoefT<T> c, XArgs a) {
+  using V = V2<T>;
   using TG = typename std::conditional<DV, T, double>::type;
-  constexpr int GR = K + 1, UR = K + 2;
-  constexpr int GBYTES = NB * GR * 32 * (int)sizeof(TG);
-  constexpr int GB = (GBYTES + 127) / 128 * 128;
-  constexpr int UBYTES = DV ? NB * UR * 32 * 8 : 0;
-  constexpr int RCB = K * 16 * (int)sizeof(T);  // the segment's coefficient rows
-  constexpr int STG = GB + UBYTES + RCB;
-  constexpr unsigned TX = (unsigned)(GBYTES + UBYTES + RCB);
-  extern __shared__ __align__(128) unsigned char smraw[];
-  uint64_t *bar = reinterpret_cast<uint64_t *>(smraw + 2 * STG);
-  const int f = blockIdx.y, np = pick3(a.np, f);
-  const int t = threadIdx.x, mp0 = blockIdx.x * TB;
-  if (mp0 >= np) return;  // the whole CTA lies past this field's lines
-  const int mp = mp0 + t;
-  const bool active = mp < np;
-  const int mpc = active ? mp : np - 1;
-  const CUtensorMap *mg = f == 0 ? &maps.g[0] : (f == 1 ? &maps.g[1] : &maps.g[2]);
-  const CUtensorMap *mu = f == 0 ? &maps.u[0] : (f == 1 ? &maps.u[1] : &maps.u[2]);
-  const CUtensorMap *mr = f == 0 ? &maps.r[0] : (f == 1 ? &maps.r[1] : &maps.r[2]);
-  const int nx = c.nx, xr = c.xround, which = pick3(a.which, f);
-  const int nseg = (nx + K - 1) / K;
-  auto seg_of = [&](int it) { return it < nseg ? it : 2 * nseg - 1 - it; };
-  auto issue = [&](int stg, int sg) {
-    unsigned char *b = smraw + stg * STG;
-    const int s0 = sg * K;
-    mbar_arrive_expect_tx(&bar[stg], TX);
-#pragma unroll
-    for (int j = 0; j < NB; ++j) {
-      tma_load_2d(b + j * GR * 32 * (int)sizeof(TG), mg, mp0 + 32 * j, DV ? s0 - 1 : s0, &bar[stg]);
-      if (DV) tma_load_2d(b + GB + j * UR * 32 * 8, mu, mp0 + 32 * j, s0 - 1, &bar[stg]);
-    }
-    tma_load_2d(b + GB + UBYTES, mr, 0, s0, &bar[stg]);
-  };
-  if (t == 0) {
-    mbar_init(&bar[0], 1);
-    mbar_init(&bar[1], 1);
-    mbar_init_fence();
-  }
-  __syncthreads();
-  if (t == 0) issue(0, 0);
-  T *out = static_cast<T *>(pick3(a.out, f)) + mpc;
-  T *ck = reinterpret_cast<T *>(pick3(a.ck, f)) + mpc;
-  const int gofs = ((t >> 5) * GR) * 32 + (t & 31), uofs = ((t >> 5) * UR) * 32 + (t & 31);
-  // ---- operator setup (boundary stencils from global memory)
-  T gb0, gbN, ub0 = T(0), ubN = T(0), uN = T(0), uN1 = T(0);
-  const T rex = c.S[OTBL_S_REX], idx = c.S[OTBL_S_IDX], uinf = c.S[OTBL_S_UINF];
-  if constexpr (DV) {
-    const TG *gin = static_cast<const TG *>(pick3(a.in, f)) + mpc;
-    const double *uin = pick3(a.in2, f) + mpc;
-    const int chv = which == 0 ? 1 : 2, chv1 = chv + 2, ic = which == 0 ? 3 : 1;
-    const T *db = c.dcbx, *vb = c.cofvbx;
-    auto G = [&](int i) { return (T)rnd(__ldg(gin + (size_t)i * np), xr); };
-    auto U = [&](int i) { return (T)rnd(__ldg(uin + (size_t)i * np), xr); };
-    gb0 = M5(db, chv, 1) * G(0) + M5(db, chv, 2) * G(1) + M5(db, chv, 3) * G(2) + M5(db, chv, 4) * G(3);
-    ub0 = M4(vb, ic, 1) * U(0) + M4(vb, ic, 2) * U(1) + M4(vb, ic, 3) * U(2) + M4(vb, ic, 4) * U(3);
-    gbN = M5(db, chv1, 1) * G(nx - 1) + M5(db, chv1, 2) * G(nx - 2) + M5(db, chv1, 3) * G(nx - 3) +
-          M5(db, chv1, 4) * G(nx - 4);
-    uN = U(nx - 1);
-    uN1 = U(nx - 2);
-    ubN = M4(vb, ic + 1, 1) * uN + M4(vb, ic + 1, 2) * uN1 + M4(vb, ic + 1, 3) * U(nx - 3) +
-          M4(vb, ic + 1, 4) * U(nx - 4);
-  } else {
-    const double *gin = static_cast<const double *>(pick3(a.in, f)) + mpc;
-    const int chi = which == 0 ? 2 : 1, chi2 = which == 0 ? 3 : 4;
-    const T *ib = c.inbx;
-    auto G = [&](int i) { return (T)rnd(__ldg(gin + (size_t)i * np), xr); };
-    gb0 = M4(ib, chi2, 1) * G(0) + M4(ib, chi2, 2) * G(1) + M4(ib, chi2, 3) * G(2) + M4(ib, chi2, 4) * G(3);
-    gbN = M4(ib, chi, 1) * G(nx - 1) + M4(ib, chi, 2) * G(nx - 2) + M4(ib, chi, 3) * G(nx - 3) +
-          M4(ib, chi, 4) * G(nx - 4);
-  }
-  // right-hand sides: interpxx e1 g_i + e2 g_{i+1}; difvisxx convective
-  // e1 g_{i-1} + e2 g_i and viscous f1 u_{i+1} + f2 u_i + f3 u_{i-1}; q is
-  // the plane's coefficient row in shared memory (k_x_rows' layout)
-  auto rg = [&](int i, const T *q, T ga, T gb) { return i == 0 ? gb0 : (i == nx - 1 ? gbN : q[0] * ga + q[1] * gb); };
-  auto ru = [&](int i, const T *q, T um, T u0, T up) {
-    return i == 0 ? ub0 : (i == nx - 1 ? ubN : q[5] * up + q[6] * u0 + q[7] * um);
-  };
-  T yg = T(0), yu = T(0), xg = T(0), xu = T(0);
-  for (int it = 0; it < 2 * nseg; ++it) {
-    const int stg = it & 1;
-    const bool ok = mbar_wait_bounded(&bar[stg], (it >> 1) & 1, 2000000000ull);
-    if (__syncthreads_or(!ok)) {
-      if (t == 0) atomicExch(err, OTBL_ERR_TIMEOUT);
-      return;
-    }
-    if (t == 0 && it + 1 < 2 * nseg) issue(stg ^ 1, seg_of(it + 1));
-    if (!active) continue;
-    const int sg = seg_of(it), s0 = sg * K;
-    const unsigned char *bs = smraw + stg * STG;
-    const TG *gs = reinterpret_cast<const TG *>(bs) + gofs;
-    const double *us = reinterpret_cast<const double *>(bs + GB) + uofs;
-    const T *rcs = reinterpret_cast<const T *>(bs + GB + UBYTES);
-    auto g = [&](int b) { return (T)rnd(gs[b * 32], xr); };
-    auto u = [&](int b) { return (T)rnd(us[b * 32], xr); };
-    if (it < nseg) {  // forward sweep, checkpoint at the segment start
-      ck[(size_t)((DV ? 2 : 1) * sg) * np] = yg;
-      if (DV) ck[(size_t)(2 * sg + 1) * np] = yu;
-#pragma unroll
-      for (int b = 0; b < K; ++b) {
-        const int i = s0 + b;
-        const T *q = rcs + 16 * b;
-        if (i < nx) {
-          yg = rg(i, q, g(b), g(b + 1)) + (i > 0 ? q[2] : T(0)) * yg;
-          if (DV) yu = ru(i, q, u(b), u(b + 1), u(b + 2)) + (i > 0 ? q[8] : T(0)) * yu;
-        }
-      }
-    } else {  // backward sweep: recompute the segment, then substitute
-      T a1 = ck[(size_t)((DV ? 2 : 1) * sg) * np], a2 = DV ? ck[(size_t)(2 * sg + 1) * np] : T(0);
-      T y1[K], y2[K];
-#pragma unroll
-      for (int b = 0; b < K; ++b) {
-        const int i = s0 + b;
-        const T *q = rcs + 16 * b;
-        if (i < nx) {
-          a1 = rg(i, q, g(b), g(b + 1)) + (i > 0 ? q[2] : T(0)) * a1;
-          if (DV) a2 = ru(i, q, u(b), u(b + 1), u(b + 2)) + (i > 0 ? q[8] : T(0)) * a2;
-        }
-        y1[b] = a1;
-        y2[b] = a2;
-      }
-#pragma unroll
-      for (int b = K - 1; b >= 0; --b) {
-        const int i = s0 + b;
-        const T *q = rcs + 16 * b;
-        if (i < nx) {
-          xg = (y1[b] - q[4] * xg) * q[3];
-          T v = xg;
-          if (DV) {
-            xu = (y2[b] - q[10] * xu) * q[9];
-            v = i == nx - 1 ? uinf * (uN - uN1) * idx + rex * T(0) : xg + rex * xu;
-          }
-          out[(size_t)i * np] = (T)rnd(v, xr);
-        }
-      }
-    }
-  }
-}
-
-template <typename T, bool DV>
-static void xline_t_launch(otbl_ctx *c, const DCoefT<T> &dc, const XStream &a, const XMaps &m, int npmax) {
-  constexpr int K = xseg<T, DV>();
-  using TG = typename std::conditional<DV, T, double>::type;
-  auto smem = [&](int tb) {
-    const int nb = tb / 32;
-    const int gb = (nb * (K + 1) * 32 * (int)sizeof(TG) + 127) / 128 * 128;
-    return 2 * (gb + (DV ? nb * (K + 2) * 32 * 8 : 0) + K * 16 * (int)sizeof(T)) + 128;
-  };
-  const int bs = c->tune_bs[DV ? 1 : 0];
-  int *err = &c->st->err;
-  if (bs <= 32) {
-    cudaFuncSetAttribute(k_xline_t<T, DV, 32>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem(32));
-    k_xline_t<T, DV, 32><<<dim3((npmax + 31) / 32, 3), 32, smem(32), c->stream>>>(dc, a, err, m);
-  } else if (bs <= 64) {
-    cudaFuncSetAttribute(k_xline_t<T, DV, 64>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem(64));
-    k_xline_t<T, DV, 64><<<dim3((npmax + 63) / 64, 3), 64, smem(64), c->stream>>>(dc, a, err, m);
-  } else {
-    cudaFuncSetAttribute(k_xline_t<T, DV, 128>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem(128));
-    k_xline_t<T, DV, 128><<<dim3((npmax + 127) / 128, 3), 128, smem(128), c->stream>>>(dc, a, err, m);
-  }
-}
-
-// One row of 16 T per plane i of each table (dv, which), dv 0 interpxx and
-// 1 difvisxx, which 0 u-type and 1 v-type coefficients: the right-hand-side
-// weights econ[2i], econ[2i+1] and the LU coefficients icon[3i..3i+2], then
-// for difvisxx the viscous operator's econv[3i..3i+2] and iconv[3i..3i+2].
-// k_xline_t's ring stages a segment's rows with its line boxes. Entries a
-// plane does not use are 0.
-template <typename T>
-__global__ void __launch_bounds__(128) k_x_rows(DCoefT<T> c, T *tab) {
+  using VG = V2<TG>;
+  constexpr int NCF = xcoefs(DV), S = NCF * K;
+  constexpr bool GT = x_table_global(K);
+  extern __shared__ __align__(16) unsigned char smraw[];
+  const int L = 1 << a.lgL, C = a.C, NT = blockDim.x, t = threadIdx.x, lane = t & (L - 1);
   const int nx = c.nx;
-  const int e = blockIdx.x * blockDim.x + threadIdx.x;
-  if (e >= 4 * nx) return;
-  const int dv = e / (2 * nx), which = (e / nx) & 1, i = e % nx;
-  T *q = tab + (size_t)e * 16;
-  for (int k = 0; k < 16; ++k) q[k] = T(0);
-  const T *icon = dv ? (which == 0 ? c.dcxu : c.dcxv) : (which == 0 ? c.inxu : c.inxv);
-  const T *econ = dv ? (which == 0 ? c.cofcxu : c.cofcxv) : (which == 0 ? c.cofiux : c.cofivx);
-  const bool inner = i > 0 && i < nx - 1;
-  if (inner) {
-    q[0] = econ[2 * i];
-    q[1] = econ[2 * i + 1];
-  }
-  for (int k = 0; k < 3; ++k) q[2 + k] = icon[3 * i + k];
-  if (dv) {
-    const T *iconv = which == 0 ? c.vixu : c.vixv, *econv = which == 0 ? c.cofvxu : c.cofvxv;
-    for (int k = 0; k < 3; ++k) {
-      if (inner) q[5 + k] = econv[3 * i + k];
-      q[8 + k] = iconv[3 * i + k];
+  const int telems = (C * (S + (DV ? 4 : 2)) + 3) & ~3;
+  T *tabs = reinterpret_cast<T *>(smraw);
+  VG *gb = reinterpret_cast<VG *>(tabs + (GT ? 0 : telems));              // [nx][L]
+  double2 *ub = reinterpret_cast<double2 *>(gb + (size_t)((nx * L + 1) & ~1));  // [nx][L], difvisxx
+  V *ex = DV ? reinterpret_cast<V *>(ub + (size_t)nx * L) : reinterpret_cast<V *>(gb + (size_t)((nx * L + 1) & ~1));
+  const int q = min(t >> a.lgL, C - 1);       // spare threads repeat the last chunk
+  const int s = q * K, left = nx - s;         // first plane, planes from there on
+  const int bl = q == C - 1 ? left - 1 : -1;  // the last plane's place in the chunk
+  const T *tab = tabs + q * S, *P = tabs + C * S;
+  const V zero = cmake<V>(T(0), T(0));
+  auto cv = [&](auto g) {
+    if constexpr (XR) return cmake<V>((T)rnd(g.x, 1), (T)rnd(g.y, 1));
+    return cmake<V>((T)g.x, (T)g.y);
+  };
+  const int n0 = a.tiles[0], n1 = n0 + a.tiles[1], ntile = n1 + a.tiles[2];
+  auto field = [&](int tile) { return tile < n0 ? 0 : (tile < n1 ? 1 : 2); };
+  auto first_pair = [&](int tile, int f) { return (tile - (f == 0 ? 0 : (f == 1 ? n0 : n1))) << a.lgL; };
+  // copies a tile of a field (base in, npp pairs per plane) into buf
+  auto stage = [&](auto *buf, const auto *in, int p0, int npp) {
+    const bool ok = p0 + lane < npp;
+    const auto *g = in + (size_t)(t >> a.lgL) * npp + (ok ? p0 + lane : 0);
+    const size_t step = (size_t)(NT >> a.lgL) * npp;
+    for (int e = t; e < nx * L; e += NT) {
+      cp_async_v(buf + e, g, ok);
+      g += step;
+    }
+    cp_async_commit();
+  };
+  auto stage_u = [&](int tile) {
+    if constexpr (DV) {
+      if (tile < ntile) {
+        const int f = field(tile);
+        stage(ub, reinterpret_cast<const double2 *>(pick3(a.in2, f)), first_pair(tile, f), pick3(a.np, f) >> 1);
+      } else {
+        cp_async_commit();
+      }
+    }
+  };
+  auto stage_g = [&](int tile) {
+    if (tile < ntile) {
+      const int f = field(tile);
+      stage(gb, static_cast<const VG *>(pick3(a.in, f)), first_pair(tile, f), pick3(a.np, f) >> 1);
+    } else {
+      cp_async_commit();
+    }
+  };
+  stage_u(blockIdx.x);
+  stage_g(blockIdx.x);
+  const T rex = c.S[OTBL_S_REX], idx = c.S[OTBL_S_IDX], uinf = c.S[OTBL_S_UINF];
+  int have = -1;  // the table in shared memory
+  for (int tile = blockIdx.x; tile < ntile; tile += gridDim.x) {
+    const int f = field(tile), which = f == 0 ? 0 : 1, npp = pick3(a.np, f) >> 1;
+    const int pm = first_pair(tile, f) + lane;
+    if (which != have) {  // (every thread is past the barrier after its last use of the old table)
+      const T *src = static_cast<const T *>(a.tab) + (size_t)which * telems;
+      if constexpr (GT) {
+        tab = src + q * S;
+        P = src + C * S;
+      } else {
+        __syncthreads();
+        for (int e = t; e < telems; e += NT) tabs[e] = src[e];
+      }
+      have = which;
+    }
+    V xu[DV ? K : 1];
+    V uN = zero, uN1 = zero;
+    if constexpr (DV) {
+      cp_async_wait<1>();
+      __syncthreads();
+      const double2 *u = ub + (size_t)s * L + lane;
+      const int ic = which == 0 ? 3 : 1;
+      const T *vb = c.cofvbx;
+      V um = q > 0 ? cv(u[-L]) : zero, u0 = cv(u[0]);
+#pragma unroll
+      for (int b = 0; b < K; ++b) {
+        const V up = b + 1 < left ? cv(u[(b + 1) * L]) : zero;
+        V r = zero;
+        fma2(r, tab[5 * K + b], up);
+        fma2(r, tab[6 * K + b], u0);
+        fma2(r, tab[7 * K + b], um);
+        xu[b] = r;
+        um = u0;
+        u0 = up;
+      }
+      if (q == 0) {
+#pragma unroll
+        for (int m = 1; m <= 4; ++m) fma2(xu[0], M4(vb, ic, m), cv(u[(m - 1) * L]));
+      }
+      if (q == C - 1) {
+        const double2 *ul = ub + (size_t)(nx - 1) * L + lane;
+        uN = cv(ul[0]);
+        uN1 = cv(ul[-L]);
+        V r = zero;
+        fma2(r, M4(vb, ic + 1, 1), uN);
+        fma2(r, M4(vb, ic + 1, 2), uN1);
+        fma2(r, M4(vb, ic + 1, 3), cv(ul[-2 * L]));
+        fma2(r, M4(vb, ic + 1, 4), cv(ul[-3 * L]));
+#pragma unroll
+        for (int b = 0; b < K; ++b)
+          xu[b] = select2(b == bl, r, xu[b]);
+      }
+      chunk_forward<K, 1, T>(xu, tab + 8 * K, P + 2 * C, ex, q, t, L);
+      stage_u(tile + gridDim.x);  // every thread holds its planes
+      cp_async_wait<1>();         // this tile's g, made visible by the next barrier
+      chunk_backward<K, 1, T>(xu, tab + 9 * K, tab + 10 * K, P + 3 * C, ex + NT, q, C, t, L);
+    } else {
+      cp_async_wait<0>();
+      __syncthreads();
+    }
+    V y[K];
+    {
+      // difvisxx: w0 g_{i-1} + w1 g_i; interpxx: w0 g_i + w1 g_{i+1}
+      const VG *g = gb + (size_t)s * L + lane;
+      V g0 = DV ? (q > 0 ? cv(g[-L]) : zero) : cv(g[0]);
+#pragma unroll
+      for (int b = 0; b < K; ++b) {
+        const int o = DV ? b : b + 1;
+        const V g1 = o < left ? cv(g[o * L]) : zero;
+        V r = zero;
+        fma2(r, tab[b], g0);
+        fma2(r, tab[K + b], g1);
+        y[b] = r;
+        g0 = g1;
+      }
+      const VG *gl = gb + (size_t)(nx - 1) * L + lane;
+      const int cf = DV ? (which == 0 ? 1 : 2) : (which == 0 ? 3 : 4), cl = DV ? cf + 2 : (which == 0 ? 2 : 1);
+      if (q == 0) {
+#pragma unroll
+        for (int m = 1; m <= 4; ++m) fma2(y[0], DV ? M5(c.dcbx, cf, m) : M4(c.inbx, cf, m), cv(g[(m - 1) * L]));
+      }
+      if (q == C - 1) {
+        V r = zero;
+#pragma unroll
+        for (int m = 1; m <= 4; ++m) fma2(r, DV ? M5(c.dcbx, cl, m) : M4(c.inbx, cl, m), cv(gl[(1 - m) * L]));
+#pragma unroll
+        for (int b = 0; b < K; ++b)
+          y[b] = select2(b == bl, r, y[b]);
+      }
+    }
+    chunk_forward<K, 1, T>(y, tab + 2 * K, P, ex, q, t, L);
+    stage_g(tile + gridDim.x);
+    chunk_backward<K, 1, T>(y, tab + 3 * K, tab + 4 * K, P + C, ex + NT, q, C, t, L);
+    if (pm < npp && t < C * L) {
+      V *out = static_cast<V *>(pick3(a.out, f)) + (size_t)s * npp + pm;
+#pragma unroll
+      for (int b = 0; b < K; ++b) {
+        if (b < left) {
+          V v = y[b];
+          if constexpr (DV) {
+            fma2(v, rex, xu[b]);
+            if (b == bl) {  // outflow: lip.f90:105,132
+              v.x = uinf * (uN.x - uN1.x) * idx;
+              v.y = uinf * (uN.y - uN1.y) * idx;
+            }
+          }
+          if constexpr (XR) v = cmake<V>((T)rnd(v.x, 1), (T)rnd(v.y, 1));
+          *out = v;
+          out += npp;
+        }
+      }
     }
   }
+  cp_async_wait<0>();
 }
 
-cudaError_t launch_x_rows(otbl_ctx *c) {
-  const int n = 4 * c->cfg.nx;
-  if (c->mixed)
-    k_x_rows<float><<<(n + 127) / 128, 128, 0, c->stream>>>(c->dcf, static_cast<float *>(c->w.xrowc));
-  else
-    k_x_rows<double><<<(n + 127) / 128, 128, 0, c->stream>>>(c->dc, static_cast<double *>(c->w.xrowc));
-  c->launches += 1;
+// ---------------------------------------------------------------------------
+// launches and tables
+// ---------------------------------------------------------------------------
+// Planes per chunk: the shortest of 5, 9, 17, 33 whose chunks leave a CTA at
+// least four pairs of lines (64-byte rows in FP64), so that short lines get
+// short serial chains and long ones full sectors.
+static int x_chunk(int nx) {
+  if (nx <= 160) return 5;
+  for (int K : {9, 17})
+    if ((nx + K - 1) / K <= 128) return K;
+  return 33;
+}
+
+size_t xline_table_bytes(int nx, bool mixed) {
+  const int K = x_chunk(nx), C = (nx + K - 1) / K;
+  return 2 * (xtab_elems(K, C, false) + xtab_elems(K, C, true)) * (mixed ? sizeof(float) : sizeof(double));
+}
+
+template <typename T>
+static cudaError_t x_tables(otbl_ctx *c) {
+  const int nx = c->cfg.nx, K = x_chunk(nx), C = (nx + K - 1) / K;
+  otbl_coef_offsets o;
+  otbl_coef_layout(nx, c->cfg.ny, c->cfg.nz, &o);
+  std::vector<T> cf(c->coef_host.begin(), c->coef_host.end());
+  auto A = [&](int id) { return cf.data() + o.off[id]; };
+  std::vector<T> all;
+  for (int dv = 0; dv < 2; ++dv)
+    for (int wh = 0; wh < 2; ++wh) {
+      const int S = xcoefs(dv) * K;
+      std::vector<T> tab(xtab_elems(K, C, dv), T(0));
+      T *P = tab.data() + (size_t)C * S;
+      auto put = [&](int i, int r, T v) { tab[(size_t)(r / K) * S + i * K + r % K] = v; };
+      const T *icon = dv ? A(wh ? OTBL_C_DCXV : OTBL_C_DCXU) : A(wh ? OTBL_C_INXV : OTBL_C_INXU);
+      const T *econ = dv ? A(wh ? OTBL_C_COFCXV : OTBL_C_COFCXU) : A(wh ? OTBL_C_COFIVX : OTBL_C_COFIUX);
+      for (int i = 1; i < nx - 1; ++i) {
+        put(0, i, econ[2 * i]);
+        put(1, i, econ[2 * i + 1]);
+      }
+      auto lde = [&](int at) { return [&put, at](int i, int r, T v) { put(at + i, r, v); }; };
+      chunk_factors<T>(lde(2), K, nx, icon, 0, P, P + C);
+      if (dv) {
+        const T *ev = A(wh ? OTBL_C_COFVXV : OTBL_C_COFVXU);
+        for (int i = 1; i < nx - 1; ++i)
+          for (int k = 0; k < 3; ++k) put(5 + k, i, ev[3 * i + k]);
+        chunk_factors<T>(lde(8), K, nx, A(wh ? OTBL_C_VIXV : OTBL_C_VIXU), 0, P + 2 * C, P + 3 * C);
+      }
+      all.insert(all.end(), tab.begin(), tab.end());
+    }
+  const cudaError_t e =
+      cudaMemcpyAsync(c->w.xtab, all.data(), all.size() * sizeof(T), cudaMemcpyHostToDevice, c->stream);
+  return e == cudaSuccess ? cudaStreamSynchronize(c->stream) : e;
+}
+
+cudaError_t prepare_xlines(otbl_ctx *c) { return c->mixed ? x_tables<float>(c) : x_tables<double>(c); }
+
+template <typename T, bool DV>
+static cudaError_t xline_launch(otbl_ctx *c, const DCoefT<T> &dc, XArgs &a) {
+  const int nx = c->cfg.nx, K = x_chunk(nx), C = (nx + K - 1) / K;
+  // threads per CTA: 256 (512 for lines of more than 64 chunks), or a half or
+  // a quarter of that when the autotuner found narrower CTAs faster (tune_bs
+  // 128, 64, 32), and what shared memory holds
+  const int most = std::max((C > 64 && K <= 9 ? 4 : 2) * c->tune_bs[DV ? 1 : 0], C);
+  auto bytes = [&](int lg) {
+    const size_t n = ((size_t)nx << lg) + 1, nt = ((C << lg) + 31) / 32 * 32;
+    return (x_table_global(K) ? 0 : xtab_elems(K, C, DV) * sizeof(T)) + n * (DV ? 16 + sizeof(V2<T>) : 16) +
+           2 * nt * sizeof(V2<T>) + 16;
+  };
+  const size_t room = 232448;
+  int lg = 0;
+  while ((C << (lg + 1)) <= most && lg < 4 && bytes(lg + 1) <= room) ++lg;
+  const size_t smem = bytes(lg);
+  if (smem > room) return cudaErrorInvalidConfiguration;
+  a.C = C;
+  a.lgL = lg;
+  a.tab = static_cast<const T *>(c->w.xtab) + (DV ? 2 * xtab_elems(K, C, false) : 0);
+  int ntile = 0;
+  for (int f = 0; f < 3; ++f) {
+    a.tiles[f] = (a.np[f] / 2 + (1 << lg) - 1) >> lg;
+    ntile += a.tiles[f];
+  }
+  const int NT = ((C << lg) + 31) / 32 * 32;
+  auto go = [&](auto kern) {
+    if (smem > 48 * 1024) cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    const int regs = K > 9 ? 256 : 128;  // per thread, by the launch bounds
+    const int per = std::max(1, std::min((int)(233472 / (smem + 1024)), 65536 / (regs * NT)));
+    kern<<<std::min(ntile, per * sm_count()), NT, smem, c->stream>>>(dc, a);
+  };
+  auto byk = [&](auto xr) {
+    constexpr bool XR = decltype(xr)::value;
+    switch (K) {
+      case 5: go(k_xline<T, 5, DV, XR>); break;
+      case 9: go(k_xline<T, 9, DV, XR>); break;
+      case 17: go(k_xline<T, 17, DV, XR>); break;
+      default: go(k_xline<T, 33, DV, XR>);
+    }
+  };
+  if constexpr (sizeof(T) == 8) {
+    if (c->dc.xround)
+      byk(std::true_type{});
+    else
+      byk(std::false_type{});
+  } else {
+    byk(std::false_type{});
+  }
   return cudaGetLastError();
 }
 
-// 2D map of one table of Work::xrowc: [nx planes][16 T], boxes of K planes
-static bool encode_xrows(CUtensorMap *m, const void *base, size_t esz, int nx, int k) {
-  auto fn = reinterpret_cast<PFN_cuTensorMapEncodeTiled_v12000>(tensor_map_encoder());
-  if (!fn || ((uintptr_t)base) % 16 != 0) return false;
-  const cuuint64_t dims[2] = {16, (cuuint64_t)nx};
-  const cuuint64_t strides[1] = {16 * esz};
-  const cuuint32_t box[2] = {16, (cuuint32_t)k};
-  const cuuint32_t es[2] = {1, 1};
-  const CUtensorMapDataType dt = esz == 8 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT64 : CU_TENSOR_MAP_DATA_TYPE_FLOAT32;
-  return fn(m, dt, 2, const_cast<void *>(base), dims, strides, box, es, CU_TENSOR_MAP_INTERLEAVE_NONE,
-            CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
-            CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
-}
-
-// ---- TMA descriptors (host): field [nx][np], boxes of 32 lines x rows
-static bool encode_lines(CUtensorMap *m, const void *base, size_t esz, int nx, int np, int rows) {
-  auto fn = reinterpret_cast<PFN_cuTensorMapEncodeTiled_v12000>(tensor_map_encoder());
-  if (!fn || (np * esz) % 16 != 0 || ((uintptr_t)base) % 16 != 0) return false;
-  const cuuint64_t dims[2] = {(cuuint64_t)np, (cuuint64_t)nx};
-  const cuuint64_t strides[1] = {(cuuint64_t)np * esz};
-  const cuuint32_t box[2] = {32, (cuuint32_t)rows};
-  const cuuint32_t es[2] = {1, 1};
-  const CUtensorMapDataType dt = esz == 8 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT64 : CU_TENSOR_MAP_DATA_TYPE_FLOAT32;
-  return fn(m, dt, 2, const_cast<void *>(base), dims, strides, box, es, CU_TENSOR_MAP_INTERLEAVE_NONE,
-            CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
-            CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
-}
-
-bool build_x_maps(otbl_ctx *c) {
-  const int KI = c->mixed ? xseg<float, false>() : xseg<double, false>();
-  const int KD = c->mixed ? xseg<float, true>() : xseg<double, true>();
-  const int nx = c->cfg.nx, nz1 = c->dc.nz1, ny = c->cfg.ny;
-  const int np[3] = {nz1 * (ny + 1), nz1 * ny, nz1 * (ny + 1)};
+template <bool DV>
+static cudaError_t xlines(otbl_ctx *c, const void *const (&in)[3], void *const (&out)[3]) {
+  const int nz1 = c->dc.nz1, ny = c->cfg.ny;
   const double *st[3] = {c->f[OTBL_F_U], c->f[OTBL_F_V], c->f[OTBL_F_W]};
-  const void *pr[3] = {c->w.uu, c->w.uv, c->w.uw};
-  const size_t ew = c->mixed ? sizeof(float) : sizeof(double);
-  bool ok = true;
-  const int which[3] = {0, 1, 1};  // u-type or v-type operator of each field
-  const char *tab = static_cast<const char *>(c->w.xrowc);
-  auto table = [&](int dv, int wh) { return tab + (size_t)(2 * dv + wh) * nx * 16 * ew; };
-  for (int f = 0; f < 3 && ok; ++f) {
-    ok = ok && encode_lines(&c->xmi.g[f], st[f], 8, nx, np[f], KI + 1);
-    c->xmi.u[f] = c->xmi.g[f];  // unused by interpxx
-    ok = ok && encode_xrows(&c->xmi.r[f], table(0, which[f]), ew, nx, KI);
-    ok = ok && encode_lines(&c->xmd.g[f], pr[f], ew, nx, np[f], KD + 1);
-    ok = ok && encode_lines(&c->xmd.u[f], st[f], 8, nx, np[f], KD + 2);
-    ok = ok && encode_xrows(&c->xmd.r[f], table(1, which[f]), ew, nx, KD);
+  XArgs a;
+  for (int f = 0; f < 3; ++f) {
+    a.in[f] = in[f];
+    a.in2[f] = st[f];
+    a.out[f] = out[f];
+    a.np[f] = nz1 * (f == 1 ? ny : ny + 1);
   }
-  c->xmaps_ok = ok;
-  return ok;
+  prof_begin(c, DV ? PK_DIFVISX : PK_INTERPX);
+  const cudaError_t e = stream_xlines(c, DV) ? launch_xlines_stream(c, DV)
+                        : c->mixed           ? xline_launch<float, DV>(c, c->dcf, a)
+                                             : xline_launch<double, DV>(c, c->dc, a);
+  prof_end(c);
+  c->launches += 1;
+  return e;
 }
 
 cudaError_t launch_interpx(otbl_ctx *c) {
-  const int nz1 = c->dc.nz1, ny = c->cfg.ny;
-  const int npu = nz1 * (ny + 1), npv = nz1 * ny;
-  XStream a;
-  const double *ins[3] = {c->f[OTBL_F_U], c->f[OTBL_F_V], c->f[OTBL_F_W]};
-  void *outs[3] = {c->w.ux, c->w.vx, c->w.wx};
-  double *cks[3] = {c->w.s1, c->w.s2, c->w.s3};
-  const int which[3] = {0, 1, 1}, np[3] = {npu, npv, npu};
-  for (int f = 0; f < 3; ++f) {
-    a.in[f] = ins[f];
-    a.in2[f] = nullptr;
-    a.out[f] = outs[f];
-    a.ck[f] = cks[f];
-    a.which[f] = which[f];
-    a.np[f] = np[f];
-  }
-  const int bs = c->tune_bs[0];
-  prof_begin(c, PK_INTERPX);
-  if (c->xmaps_ok && (c->mixed ? XTune<float>::tma : XTune<double>::tma)) {
-    if (c->mixed)
-      xline_t_launch<float, false>(c, c->dcf, a, c->xmi, npu);
-    else
-      xline_t_launch<double, false>(c, c->dc, a, c->xmi, npu);
-  } else if (c->mixed)
-    k_interpx<float><<<dim3((npu + bs - 1) / bs, 3), bs, 0, c->stream>>>(c->dcf, a);
-  else
-    k_interpx<double><<<dim3((npu + bs - 1) / bs, 3), bs, 0, c->stream>>>(c->dc, a);
-  prof_end(c);
-  c->launches += 1;
-  return cudaGetLastError();
+  return xlines<false>(c, {c->f[OTBL_F_U], c->f[OTBL_F_V], c->f[OTBL_F_W]}, {c->w.ux, c->w.vx, c->w.wx});
 }
 
 cudaError_t launch_difvisx(otbl_ctx *c) {
-  const int nz1 = c->dc.nz1, ny = c->cfg.ny;
-  const int npu = nz1 * (ny + 1), npv = nz1 * ny;
-  XStream a;
-  const void *gins[3] = {c->w.uu, c->w.uv, c->w.uw};
-  const double *uins[3] = {c->f[OTBL_F_U], c->f[OTBL_F_V], c->f[OTBL_F_W]};
-  void *outs[3] = {c->w.cu, c->w.cv, c->w.cw};
-  double *cks[3] = {c->w.s1, c->w.s2, c->w.s3};
-  const int which[3] = {0, 1, 1}, np[3] = {npu, npv, npu};
-  for (int f = 0; f < 3; ++f) {
-    a.in[f] = gins[f];
-    a.in2[f] = uins[f];
-    a.out[f] = outs[f];
-    a.ck[f] = cks[f];
-    a.which[f] = which[f];
-    a.np[f] = np[f];
-  }
-  const int bs = c->tune_bs[1];
-  prof_begin(c, PK_DIFVISX);
-  if (c->xmaps_ok && (c->mixed ? XTune<float>::tma : XTune<double>::tma)) {
-    if (c->mixed)
-      xline_t_launch<float, true>(c, c->dcf, a, c->xmd, npu);
-    else
-      xline_t_launch<double, true>(c, c->dc, a, c->xmd, npu);
-  } else if (c->mixed)
-    k_difvisx<float><<<dim3((npu + bs - 1) / bs, 3), bs, 0, c->stream>>>(c->dcf, a);
-  else
-    k_difvisx<double><<<dim3((npu + bs - 1) / bs, 3), bs, 0, c->stream>>>(c->dc, a);
-  prof_end(c);
-  c->launches += 1;
-  return cudaGetLastError();
+  return xlines<true>(c, {c->w.uu, c->w.uv, c->w.uw}, {c->w.cu, c->w.cv, c->w.cw});
 }
 
 }  // namespace otbl

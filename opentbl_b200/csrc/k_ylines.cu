@@ -1,904 +1,490 @@
-// Wall-normal (y) line operators of the substep, one thread per column
-// (i, kr) of the plane layout: consecutive threads take consecutive kr, so
-// every row access is a coalesced request and every per-row coefficient a
-// broadcast, and there are far more columns (nx*nz1) than resident threads.
-// A column's compact operators are the serial Thomas sweeps of lip.f90 in
-// the reference's order: the forward sweep keeps a checkpoint every KY rows
-// in scratch, the backward sweep recomputes each KY-row segment from its
-// checkpoint in registers.
+// Wall-normal (y) line operators of the substep on the plane layout, as the
+// chunked solves of lines.cuh: a thread holds K rows of one spanwise mode
+// (its real and imaginary column), the chunks of L neighbouring modes make a
+// CTA, so every row access is a segment of L x 16 (8) bytes.
 //   k_interpy    interpyy (lip.f90:359-440) of u, w and v in Fourier space
-//   k_final_s1/2 the tail of rhsp (rhsp.F90:291-484)
+//   k_tail       the tail of rhsp (rhsp.F90:291-484)
 //   k_pois_lu    pivots of the (x-mode, kz) y-systems of pois (once)
 //   k_pois_solve their solution every substep (pois.f90:106-117, soltriy)
 #include <cudaTypedefs.h>
 
+#include <algorithm>
 #include <type_traits>
 
 #include "devcommon.cuh"
+#include "lines.cuh"
 #include "otbl_internal.cuh"
-#include "tma.cuh"
 
 namespace otbl {
 
-constexpr int KY = 8;  // rows per checkpointed segment
-// Segment length and occupancy of the rhsp tail (k_final_s1), per
-// element type of its FP32-capable inputs; measured on B200 at
-// 1025x193x512 over KF in {4, 6, 8} x CTAs/SM in {3..6}: FP64 4 rows at 4
-// CTAs of 128 threads per SM (7.2 ms per substep, 7.8 at 8 rows), mixed 6
-// rows at 5 CTAs (7.0 ms, 8.4 at 8 rows at 4).
-template <typename W>
-struct FinalTune;
-#ifndef OTBL_FT_DK
-#define OTBL_FT_DK 4
-#define OTBL_FT_DM 4
-#endif
-#ifndef OTBL_FT_FK
-#define OTBL_FT_FK 6
-#define OTBL_FT_FM 5
-#endif
-// split: pass A in a kernel of its own (FP32 inputs: 6.69 against 7.09 ms;
-// FP64: 7.18 against 6.84 ms fused)
-// kf_tma: segment of the TMA-fed pass (k_final_tb) and its pass A. With the
-// coefficient rows staged in the ring, 4 rows: rhsp tail 3.47 ms per FP64
-// substep against 3.73 at 3, 3.90 at 2, 3.71 at 5 and 3.82 at 6 (mixed 2.62,
-// 2.77, 2.87, 2.74, 2.72), and 3.99 with a three-stage ring; before the
-// staging 2 rows were best (6.38 against 6.49 at 4).
-#ifndef OTBL_FT_TK
-#define OTBL_FT_TK 4
-#endif
-#ifndef OTBL_FT_NS
-#define OTBL_FT_NS 2
-#endif
-// tma_a: pass A fed by TMA too (k_final_ta). With the per-row coefficients
-// staged in its ring: FP64 4.00 against 4.76 ms per substep for the
-// register-streamed pass A (before the staging, 6.50 against 5.94); FP32
-// inputs 2.97 ms.
-template <>
-struct FinalTune<double> {
-  static constexpr int kf = OTBL_FT_DK, minb = OTBL_FT_DM, kf_tma = OTBL_FT_TK, ns_tma = OTBL_FT_NS;
-  static constexpr bool split = false, tma_a = true;
-};
-template <>
-struct FinalTune<float> {
-  static constexpr int kf = OTBL_FT_FK, minb = OTBL_FT_FM, kf_tma = OTBL_FT_TK, ns_tma = OTBL_FT_NS;
-  static constexpr bool split = true, tma_a = true;
+// two neighbouring columns' values at p, not kept in L1
+__device__ __forceinline__ double2 ld_stream(const double2 *p) {
+  double2 v;
+  asm volatile("ld.global.L1::no_allocate.v2.f64 {%0, %1}, [%2];" : "=d"(v.x), "=d"(v.y) : "l"(p) : "memory");
+  return v;
+}
+__device__ __forceinline__ float2 ld_stream(const float2 *p) {
+  float2 v;
+  asm volatile("ld.global.L1::no_allocate.v2.f32 {%0, %1}, [%2];" : "=f"(v.x), "=f"(v.y) : "l"(p) : "memory");
+  return v;
+}
+template <typename V>
+__device__ __forceinline__ V ld_row(const V *p, bool ok) {
+  return ok ? ld_stream(p) : cmake<V>(0, 0);
+}
+
+// Rows per chunk: 7 rows keep the tail's three solves in 168 registers; boxes
+// taller than 447 rows take longer chunks.
+static int y_chunk(int ny) { return ny < 7 * 64 ? 7 : 15; }
+constexpr bool y_table_global(int K) { return K > 7; }
+// The tail's tables: coefficient i of row s + b of chunk q at tab[q S + i K +
+// b], S = ncf K, the chunk products after the C chunks, rounded up to 16 bytes.
+// Its persistent CTAs copy them to shared memory once (read through L1 they
+// were evicted: 257x193x256, two thirds of their sectors from L2, a warp
+// waited 12-18 cycles per instruction); boxes taller than 447 rows read them
+// from global memory.
+static size_t ytab_elems(int K, int C, int ncf, int nprod) { return ((size_t)C * (ncf * K + nprod) + 2 + 3) / 4 * 4; }
+// lanes of a CTA of C chunks: what NT threads hold, at most 32, at least 1
+static int y_lanes(int C, int NT) { return std::max(1, std::min(32, NT / C)); }
+static int y_threads(int C, int L) { return (C * L + 31) / 32 * 32; }
+
+// a thread's place: chunk q of mode mc (of ncm, in storage order), rows s..
+struct YPlace {
+  int L, C, t, NT, q, s, mc;
+  bool active;
+  __device__ YPlace(int L_, int C_, int K)
+      : L(L_), C(C_), t(threadIdx.x), NT(blockDim.x), q(min(t / L_, C_ - 1)), s(q * K) {}
+  __device__ void tile(int n, int ncm) {
+    const int m = n * L + t % L;
+    active = m < ncm && t < C * L;  // the others repeat a valid place and store nothing
+    mc = min(m, ncm - 1);
+  }
 };
 
 // interpyy, which 0: u, w (in rows ny+1), which 1: v (in rows ny); out rows
 // 1..ny. blockIdx.y = field (u, w, v). T: arithmetic and output type (float
-// on the mixed path, with the FP32 coefficient copy); the state is FP64.
+// on the mixed path, with the FP32 coefficient copy); the state is FP64. Its
+// table is small enough to be read through L1 (coefficient i of row s + b of
+// chunk q at [(i K + b) QS + q], one line per row): staged in shared memory by
+// persistent CTAs, with the next tile's rows fetched ahead, it took 37.4
+// against 33.3 us at 257x97x128 and 193 against 161 at 513x129x256.
 struct InterpyArgs {
   const double *in[3];
   void *out[3];
-  double *ck[3];
+  const void *tab[2];  // wA, wB, l, d, e, then P, Q, per which
   int which[3];
+  int C, L;
+};
+constexpr int kYInterp = 5;
+
+// a table read through L1
+template <typename T>
+struct LdgTab {
+  const T *p;
+  __device__ T operator[](int i) const { return __ldg(p + i); }
+  __device__ T operator*() const { return __ldg(p); }
+  __device__ LdgTab operator+(int i) const { return {p + i}; }
+  __device__ LdgTab &operator+=(int i) {
+    p += i;
+    return *this;
+  }
 };
 
-template <typename T>
-__global__ void __launch_bounds__(128) k_interpy(DCoefT<T> c, InterpyArgs a) {
-  const int f = blockIdx.y;
-  const int ny = c.ny, nz1 = c.nz1, ncol = c.nx * nz1;
-  const int col = blockIdx.x * blockDim.x + threadIdx.x;
-  if (col >= ncol) return;
-  const int which = pick3(a.which, f), jin = which == 0 ? ny + 1 : ny;
-  const int i = col / nz1 + 1, kr = col - (i - 1) * nz1;
-  const size_t S = nz1;
-  const double *g = pick3(a.in, f) + (size_t)(i - 1) * jin * nz1 + kr;
-  T *o = static_cast<T *>(pick3(a.out, f)) + (size_t)(i - 1) * ny * nz1 + kr;
-  T *ck = reinterpret_cast<T *>(pick3(a.ck, f)) + col;
-  const T *iny = which == 0 ? c.inyu : c.inyv;
-  const T *econ = which == 0 ? c.cofiuy : c.cofivy;
-  const T *ib = c.inby;
-  auto G = [&](int r) { return (T)__ldg(g + (size_t)min(max(r, 0), jin - 1) * S); };
-  T b0 = T(0), bN;
-  if (which == 0) {
-    bN = M4(ib, 1, 1) * G(ny) + M4(ib, 1, 2) * G(ny - 1) + M4(ib, 1, 3) * G(ny - 2) + M4(ib, 1, 4) * G(ny - 3);
-  } else {
-    b0 = M4(ib, 3, 1) * G(0) + M4(ib, 3, 2) * G(1) + M4(ib, 3, 3) * G(2) + M4(ib, 3, 4) * G(3);
-    bN = M4(ib, 4, 1) * G(ny - 1) + M4(ib, 4, 2) * G(ny - 2) + M4(ib, 4, 3) * G(ny - 3) + M4(ib, 4, 4) * G(ny - 4);
+template <typename T, int K, int QS>
+__global__ void __launch_bounds__(256, K > 7 ? 1 : 2) k_interpy(DCoefT<T> c, InterpyArgs a) {
+  using V = V2<T>;
+  extern __shared__ __align__(16) unsigned char smraw[];
+  const int f = blockIdx.y, ny = c.ny, nk = c.nz1 >> 1;
+  YPlace w(a.L, a.C, K);
+  w.tile(blockIdx.x, c.nx * nk);
+  const int which = pick3(a.which, f), jin = which == 0 ? ny + 1 : ny, left = ny - w.s;
+  const int i = w.mc / nk, k = w.mc - i * nk;
+  const double2 *in = reinterpret_cast<const double2 *>(pick3(a.in, f)) + (size_t)i * jin * nk + k;
+  const LdgTab<T> all{static_cast<const T *>(which == 0 ? a.tab[0] : a.tab[1])};
+  const LdgTab<T> P = all + kYInterp * K * QS, tab = all + w.q;
+  // u, w: e1 g(r) + e2 g(r+1), wall row 0; v: e1 g(r-1) + e2 g(r)
+  const int off = which == 0 ? 0 : -1;
+  double2 g[K + 1];
+  const double2 *p = in + (ptrdiff_t)(w.s + off) * nk;
+#pragma unroll
+  for (int b = 0; b <= K; ++b) {
+    const int r = w.s + off + b;
+    g[b] = ld_row(p, r >= 0 && r < jin);
+    p += nk;
   }
-  // right-hand side of output row r from input rows r-1, r, r+1:
-  // u,w: e1 g(r) + e2 g(r+1), wall row 0; v: e2 g(r) + e1 g(r-1)
-  auto rhs = [&](int r, T gm, T g0, T gp) {
-    const T e1 = __ldg(econ + 2 * r), e2 = __ldg(econ + 2 * r + 1);
-    const T in = which == 0 ? e1 * g0 + e2 * gp : e2 * g0 + e1 * gm;
-    return r == 0 ? b0 : (r == ny - 1 ? bN : in);
-  };
-  const int nseg = (ny + KY - 1) / KY;
-  T y = T(0);
-  for (int sg = 0; sg < nseg; ++sg) {
-    const int s0 = sg * KY;
-    ck[(size_t)sg * ncol] = y;
-    T gv[KY + 2];
+  V y[K], g0 = cmake<V>((T)g[0].x, (T)g[0].y);
 #pragma unroll
-    for (int b = 0; b < KY + 2; ++b) gv[b] = G(s0 + b - 1);
-#pragma unroll
-    for (int b = 0; b < KY; ++b) {
-      const int r = s0 + b;
-      if (r < ny) y = rhs(r, gv[b], gv[b + 1], gv[b + 2]) + (r > 0 ? __ldg(iny + 3 * r) : T(0)) * y;
-    }
+  for (int b = 0; b < K; ++b) {
+    const V g1 = cmake<V>((T)g[b + 1].x, (T)g[b + 1].y);
+    V r = cmake<V>(T(0), T(0));
+    fma2(r, tab[b * QS], g0);
+    fma2(r, tab[(K + b) * QS], g1);
+    y[b] = r;
+    g0 = g1;
   }
-  T x = T(0);
-  for (int sg = nseg - 1; sg >= 0; --sg) {
-    const int s0 = sg * KY;
-    T gv[KY + 2], yv[KY];
+  if (w.q == 0 && which == 1) {
 #pragma unroll
-    for (int b = 0; b < KY + 2; ++b) gv[b] = G(s0 + b - 1);
-    T yy = ck[(size_t)sg * ncol];
+    for (int m = 1; m <= 4; ++m) fma2(y[0], M4(c.inby, 3, m), cmake<V>((T)g[m].x, (T)g[m].y));
+  }
+  if (w.q == a.C - 1) {
+    V r = cmake<V>(T(0), T(0));
 #pragma unroll
-    for (int b = 0; b < KY; ++b) {
-      const int r = s0 + b;
-      if (r < ny) yy = rhs(r, gv[b], gv[b + 1], gv[b + 2]) + (r > 0 ? __ldg(iny + 3 * r) : T(0)) * yy;
-      yv[b] = yy;
+    for (int m = 1; m <= 4; ++m) {
+      const double2 v = ld_stream(in + (size_t)(jin - m) * nk);
+      fma2(r, M4(c.inby, (which == 0 ? 1 : 4), m), cmake<V>((T)v.x, (T)v.y));
     }
 #pragma unroll
-    for (int b = KY - 1; b >= 0; --b) {
-      const int r = s0 + b;
-      if (r < ny) {
-        x = (yv[b] - __ldg(iny + 3 * r + 2) * x) * __ldg(iny + 3 * r + 1);
-        o[(size_t)r * S] = x;
-      }
-    }
+    for (int b = 0; b < K; ++b) y[b] = select2(b == left - 1, r, y[b]);
   }
-}
-
-// interpyy fed by TMA: a CTA owns 128 consecutive kr of one plane of one
-// field; thread 0 loads, for the next segment of KYT rows, a box of 128 kr x
-// KYT+2 rows of the input into a two-stage shared-memory ring on mbarriers
-// (bounded waits); the segments run forward (0..nseg-1), then backward. The
-// arithmetic is k_interpy's with segments of KYT rows.
-template <typename T>
-struct YTune;
-#ifndef OTBL_YT
-#define OTBL_YT 8
-#endif
-template <>
-struct YTune<double> {
-  static constexpr int kt = OTBL_YT;
-};
-template <>
-struct YTune<float> {
-  static constexpr int kt = OTBL_YT;
-};
-
-template <typename T>
-__global__ void __launch_bounds__(128) k_interpy_t(DCoefT<T> c, InterpyArgs a, int *err,
-                                                   const __grid_constant__ YMaps maps) {
-  constexpr int K = YTune<T>::kt, TB = 128, R = K + 2;
-  constexpr int RC = K * 8 * (int)sizeof(T);  // the segment's coefficient rows
-  constexpr int STG = R * TB * 8 + RC;
-  constexpr unsigned TX = (unsigned)STG;
-  extern __shared__ __align__(128) unsigned char smraw[];
-  uint64_t *bar = reinterpret_cast<uint64_t *>(smraw + 2 * STG);
-  const int f = blockIdx.z;
-  const int ny = c.ny, nz1 = c.nz1, ncol = c.nx * nz1;
-  const int t = threadIdx.x, kr0 = blockIdx.x * TB, kr = kr0 + t, i = blockIdx.y + 1;
-  const bool active = kr < nz1;
-  const int krc = active ? kr : 0;
-  const int which = pick3(a.which, f), jin = which == 0 ? ny + 1 : ny;
-  const CUtensorMap *mg = f == 0 ? &maps.g[0] : (f == 1 ? &maps.g[1] : &maps.g[2]);
-  const CUtensorMap *mr = f == 0 ? &maps.r[0] : (f == 1 ? &maps.r[1] : &maps.r[2]);
-  const int nseg = (ny + K - 1) / K;
-  auto seg_of = [&](int it) { return it < nseg ? it : 2 * nseg - 1 - it; };
-  auto issue = [&](int stg, int sg) {
-    mbar_arrive_expect_tx(&bar[stg], TX);
-    tma_load_3d(smraw + stg * STG, mg, kr0, sg * K - 1, i - 1, &bar[stg]);
-    tma_load_2d(smraw + stg * STG + R * TB * 8, mr, 0, sg * K, &bar[stg]);
-  };
-  if (t == 0) {
-    mbar_init(&bar[0], 1);
-    mbar_init(&bar[1], 1);
-    mbar_init_fence();
-  }
-  __syncthreads();
-  if (t == 0) issue(0, 0);
-  const size_t S = nz1;
-  const int col = (i - 1) * nz1 + krc;
-  const double *g = pick3(a.in, f) + (size_t)(i - 1) * jin * nz1 + krc;
-  T *o = static_cast<T *>(pick3(a.out, f)) + (size_t)(i - 1) * ny * nz1 + krc;
-  T *ck = reinterpret_cast<T *>(pick3(a.ck, f)) + col;
-  const T *ib = c.inby;
-  auto G = [&](int r) { return (T)__ldg(g + (size_t)min(max(r, 0), jin - 1) * S); };
-  T b0 = T(0), bN;
-  if (which == 0) {
-    bN = M4(ib, 1, 1) * G(ny) + M4(ib, 1, 2) * G(ny - 1) + M4(ib, 1, 3) * G(ny - 2) + M4(ib, 1, 4) * G(ny - 3);
-  } else {
-    b0 = M4(ib, 3, 1) * G(0) + M4(ib, 3, 2) * G(1) + M4(ib, 3, 3) * G(2) + M4(ib, 3, 4) * G(3);
-    bN = M4(ib, 4, 1) * G(ny - 1) + M4(ib, 4, 2) * G(ny - 2) + M4(ib, 4, 3) * G(ny - 3) + M4(ib, 4, 4) * G(ny - 4);
-  }
-  // q: the row's coefficients in shared memory (k_y_rows' layout)
-  auto rhs = [&](int r, const T *q, T gm, T g0, T gp) {
-    const T e1 = q[0], e2 = q[1];
-    const T in = which == 0 ? e1 * g0 + e2 * gp : e2 * g0 + e1 * gm;
-    return r == 0 ? b0 : (r == ny - 1 ? bN : in);
-  };
-  T y = T(0), x = T(0);
-  for (int it = 0; it < 2 * nseg; ++it) {
-    const int stg = it & 1;
-    const bool ok = mbar_wait_bounded(&bar[stg], (it >> 1) & 1, 2000000000ull);
-    if (__syncthreads_or(!ok)) {
-      if (t == 0) atomicExch(err, OTBL_ERR_TIMEOUT);
-      return;
-    }
-    if (t == 0 && it + 1 < 2 * nseg) issue(stg ^ 1, seg_of(it + 1));
-    if (!active) continue;
-    const int sg = seg_of(it), s0 = sg * K;
-    const double *gs = reinterpret_cast<const double *>(smraw + stg * STG) + t;
-    const T *rcs = reinterpret_cast<const T *>(smraw + stg * STG + R * TB * 8);
-    auto gv = [&](int b) { return (T)gs[b * TB]; };  // row s0 - 1 + b
-    if (it < nseg) {
-      ck[(size_t)sg * ncol] = y;
+  V *ex = reinterpret_cast<V *>(smraw);
+  chunk_forward<K, QS, T>(y, tab + 2 * K * QS, P, ex, w.q, w.t, w.L);
+  chunk_backward<K, QS, T>(y, tab + 3 * K * QS, tab + 4 * K * QS, P + QS, ex + w.NT, w.q, a.C, w.t, w.L);
+  if (!w.active) return;
+  V *o = static_cast<V *>(pick3(a.out, f)) + ((size_t)i * ny + w.s) * nk + k;
 #pragma unroll
-      for (int b = 0; b < K; ++b) {
-        const int r = s0 + b;
-        const T *q = rcs + 8 * b;
-        if (r < ny) y = rhs(r, q, gv(b), gv(b + 1), gv(b + 2)) + (r > 0 ? q[2] : T(0)) * y;
-      }
-    } else {
-      T yy = ck[(size_t)sg * ncol], yv[K];
-#pragma unroll
-      for (int b = 0; b < K; ++b) {
-        const int r = s0 + b;
-        const T *q = rcs + 8 * b;
-        if (r < ny) yy = rhs(r, q, gv(b), gv(b + 1), gv(b + 2)) + (r > 0 ? q[2] : T(0)) * yy;
-        yv[b] = yy;
-      }
-#pragma unroll
-      for (int b = K - 1; b >= 0; --b) {
-        const int r = s0 + b;
-        const T *q = rcs + 8 * b;
-        if (r < ny) {
-          x = (yv[b] - q[4] * x) * q[3];
-          o[(size_t)r * S] = x;
-        }
-      }
-    }
+  for (int b = 0; b < K; ++b) {
+    if (b < left) *o = y[b];
+    o += nk;
   }
 }
 
 // ---------------------------------------------------------------------------
 // tail of rhsp (rhsp.F90:291-484) for planes 2..nx, one velocity component
-// per launch pair: RHS assembly, pressure gradient, boun, vistyy, RK3
-// combination, rhs history, implzy.
+// per blockIdx.y, in one pass: each thread reads its K rows of the product,
+// the velocity, the difvisxx output, the kz product, the pressure and the RHS
+// history once, solves differzy (of the product) and vistyy (of the old
+// velocity), assembles the RHS (convective, viscous, pressure gradient),
+// applies boun, forms the RK3 combination and the new RHS history, and solves
+// implzy for the new velocity. W: element type of the intermediate fields, the
+// pressure and the RHS history and of differzy's and vistyy's arithmetic
+// (float on the mixed path); everything else is FP64.
+// Bound: the fields' bytes in flight. The fields that the row-wise part needs
+// are fetched by cp.async to the thread's own slots in shared memory, the
+// next tile's as soon as this tile's are used, so they arrive during the
+// solves; product and velocity are loaded to registers. FP64: two CTAs of 128
+// threads per SM at 255 registers (at 128 and 168 registers the three solves
+// spilled or the velocity had to be read twice: 257x97x128 219 and 209 us
+// against 156), FP32: three at 168.
 // ---------------------------------------------------------------------------
-// W: element type of the difvisxx outputs, the products, the pressure and
-// the RHS history (float on the mixed path); the arithmetic is FP64
-// throughout.
 template <typename W>
-struct FinalArgs {
+struct TailArgs {
   double *u, *v, *w;                 // state: old on entry, new on exit
-  const W *p;                        // p and the RHS history: W as well
+  const W *p;
   W *rhsupa, *rhsvpa, *rhswpa;       // old on entry, new on exit
   const W *cu, *cv, *cw;             // difvisxx outputs
   const W *uv, *uw, *vw, *vv, *ww;
-  const double *fac_u, *fac_v;
+  const W *tw[2];                    // differzy wA, wB, l, d, e; vistyy f1, f2, f3, l, d, e; P, Q of each
+  const double *td[2];               // vyi (3), l, d, e of implzy, idyy; P, Q; A_2, C_{jee-1}
   const DState *st;
+  int comp[3];
+  int C[2], L[2], nw[2], nd[2];      // chunks, lanes, elements of the tables
 };
+constexpr int kTailW = 11, kTailD = 7;
 
-// ---------------------------------------------------------------------------
-// The rhsp tail streamed through registers, one thread per column (i, kr),
-// consecutive threads on consecutive kr: every row access is a coalesced
-// request, every coefficient a broadcast, and there are far more columns
-// (nx*nz1) than a GPU has threads, so latency is hidden by occupancy.
-//   k_final_s1<.., 1>, pass A (rows ascending): the forward sweeps of
-//     differzy (of the product) and vistyy (of the old velocity), with a
-//     checkpoint every KF rows (FinalTune); a light kernel of its own, at
-//     high occupancy.
-//   k_final_s1<.., 2>, pass B (segments descending): both forward sweeps recomputed
-//     from the checkpoints into registers, both back-substitutions, the RHS
-//     assembly, the RK3 combination, the new RHS history, the right-hand
-//     side of implzy (rows q..q+2 of the combination) and, in the same
-//     descending order, its elimination with the top-down factors of k_dt
-//     (implzy_factor), written to scratch.
-//   k_final_s2 (rows ascending): implzy's substitution and the new
-//     velocity, with the boundary values ub1, ubt; a light kernel, so that
-//     this serial sweep runs at high occupancy.
-// differzy and vistyy are the serial Thomas sweeps of lip.f90 in the
-// reference's order; implzy is eliminated from the top row down.
-// ---------------------------------------------------------------------------
-template <typename W>
-struct FinalStream {
-  FinalArgs<W> a;
-  double *ck;   // checkpoints: [2*seg + op][column]
-  double *yq;   // implzy right-hand side after the descending elimination: [q][column]
-  double *ub;   // ub1, ubt: [2][column]
-};
-
-// PASSES: 1 pass A only (k_final_sA, a light kernel at high occupancy),
-// 2 pass B only, 3 both
-template <int COMP, typename W, int PASSES, int KF = FinalTune<W>::kf>
-__global__ void __launch_bounds__(128, PASSES == 1 ? 6 : FinalTune<W>::minb)
-    k_final_s1(DCoef c, FinalStream<W> fs) {
-  const FinalArgs<W> &a = fs.a;
-  const int nx = c.nx, ny = c.ny, nz1 = c.nz1;
-  const int ncol = (nx - 1) * nz1;
-  const int col = blockIdx.x * blockDim.x + threadIdx.x;
-  if (col >= ncol) return;
-  const int i = col / nz1 + 2, kr = col - (i - 2) * nz1;
-  const int k = kr >> 1, odd = kr & 1, pof = odd ? -1 : 1;
-  const bool last = i == nx;
-  const int jee = COMP == 1 ? ny : ny + 1, n = jee - 2;
-  const int krows = COMP == 0 ? ny + 1 : ny;
-  const size_t PU = (size_t)(ny + 1) * nz1, PV = (size_t)ny * nz1;
-  const size_t pl = (size_t)(i - 1) * (COMP == 1 ? PV : PU), plv = (size_t)(i - 1) * PV;
-  const size_t S = nz1;  // row stride
-  const W *prod = (COMP == 0 ? a.uv : (COMP == 1 ? a.vv : a.vw)) + plv + kr;
-  const W *kp = (COMP == 0 ? a.uw : (COMP == 1 ? a.vw : a.ww)) + (COMP == 0 ? pl : plv) + kr + pof;
-  double *vel = (COMP == 0 ? a.u : (COMP == 1 ? a.v : a.w)) + pl + kr;
-  const W *cX = (COMP == 0 ? a.cu : (COMP == 1 ? a.cv : a.cw)) + pl + kr;
-  W *hp = (COMP == 0 ? a.rhsupa : (COMP == 1 ? a.rhsvpa : a.rhswpa)) + pl + kr;
-  const W *pc = a.p + plv + kr;
-  const double kz = c.kaz[k], kv = c.kvis[k];
-  const double var1 = a.st->var1, var3 = a.st->var3, var4 = a.st->var4;
-  const double v2 = last ? 0.0 : a.st->var2;
-  const double idxx = c.S[OTBL_S_IDXX];
-  const double *ib = c.inby, *cc = c.ccon;
-  const double sgn = odd ? 1.0 : -1.0;
-  const int which = COMP == 1 ? 1 : 0;
-  const double *dcy = which == 0 ? c.dcyu : c.dcyv, *ecd = which == 0 ? c.cofcyu : c.cofcyv;
-  const double *viy = which == 0 ? c.viyu : c.viyv, *ecv = which == 0 ? c.cofvyu : c.cofvyv;
-  const double *vyi = which == 0 ? c.vyui : c.vyvi;
-  const double *fac = COMP == 1 ? a.fac_v : a.fac_u;
-  auto Pg = [&](int r) { return (double)__ldg(prod + (size_t)min(max(r, 0), ny - 1) * S); };
-  auto Vg = [&](int r) { return __ldg(vel + (size_t)min(max(r, 0), jee - 1) * S); };
-  // velocity after the pressure gradient (rhsp.F90:291-339) at row r
-  auto star = [&](int r, double o) -> double {
-    const int rp = min(r, ny - 1);
-    if (COMP == 0)
-      return last ? o
-                  : o - var1 * idxx * ((double)__ldg(pc + PV + (size_t)rp * S) - (double)__ldg(pc + (size_t)rp * S));
-    if (COMP == 1)
-      return o - var1 * c.idyy[r] *
-                     ((double)__ldg(pc + (size_t)min(r + 1, ny - 1) * S) - (double)__ldg(pc + (size_t)rp * S));
-    const double pp = (double)__ldg(pc + (size_t)rp * S + pof);
-    const double av = var1 * kz;
-    return o - (odd ? av * pp : -av * pp);
-  };
-  // boundary stencils of differzy (prod) and vistyy (velocity), boun values
-  const int chv = which == 0 ? 3 : 1, cha = chv + 1, ic = which == 0 ? 3 : 1;
-  const double *db = c.dcby, *vb = c.cofvby;
-  double bot = 0.0, top = 0.0;
-  if (!last) {
-    bot = M4(db, chv, 1) * Pg(0) + M4(db, chv, 2) * Pg(1) + M4(db, chv, 3) * Pg(2) + M4(db, chv, 4) * Pg(3);
-    top = M4(db, cha, 1) * Pg(ny - 1) + M4(db, cha, 2) * Pg(ny - 2) + M4(db, cha, 3) * Pg(ny - 3) +
-          M4(db, cha, 4) * Pg(ny - 4);
-  }
-  const double b0 = M4(vb, ic, 1) * Vg(0) + M4(vb, ic, 2) * Vg(1) + M4(vb, ic, 3) * Vg(2) + M4(vb, ic, 4) * Vg(3);
-  const double bN = M4(vb, ic + 1, 1) * Vg(jee - 1) + M4(vb, ic + 1, 2) * Vg(jee - 2) +
-                    M4(vb, ic + 1, 3) * Vg(jee - 3) + M4(vb, ic + 1, 4) * Vg(jee - 4);
-  double ub1 = 0.0, ubt = 0.0;
-  if (COMP == 1) {
-    ubt = kr == 0 ? c.vmagic[i - 1] : 0.0;
-  } else {
-    const double s2 = star(1, Vg(1)), s3 = star(2, Vg(2)), s4 = star(3, Vg(3));
-    const double sn = star(ny - 1, Vg(ny - 1)), sn1 = star(ny - 2, Vg(ny - 2)), sn2 = star(ny - 3, Vg(ny - 3));
-    ub1 = -1.0 / M4(ib, 2, 1) * (M4(ib, 2, 2) * s2 + M4(ib, 2, 3) * s3 + M4(ib, 2, 4) * s4);
-    ubt = -1.0 / M2(cc, 1, 1) * (M2(cc, 1, 2) * sn + M2(cc, 1, 3) * sn1 + M2(cc, 1, 4) * sn2);
-  }
-  // right-hand sides of row r from rows r-1, r, r+1 of the product (g) and
-  // the old velocity (u)
-  auto rd = [&](int r, double gm, double g0, double gp) {
-    const double in = which == 0 ? __ldg(ecd + 2 * r + 1) * g0 + __ldg(ecd + 2 * r) * gm
-                                 : __ldg(ecd + 2 * r + 1) * gp + __ldg(ecd + 2 * r) * g0;
-    return r == 0 ? bot : (r == jee - 1 ? top : in);
-  };
-  auto rv = [&](int r, double um, double u0, double up) {
-    const double in = __ldg(ecv + 3 * r) * up + __ldg(ecv + 3 * r + 1) * u0 + __ldg(ecv + 3 * r + 2) * um;
-    return r == 0 ? b0 : (r == jee - 1 ? bN : in);
-  };
-  const int nseg = (jee + KF - 1) / KF;
-  double *ck = fs.ck + col;
-  // ---- pass A: forward sweeps, checkpoints every KF rows; the loads go in
-  // batches of KA >= KF rows (a multiple of KF), so that short checkpoint
-  // segments still keep many loads in flight
-  if constexpr ((PASSES & 1) != 0) {
-  constexpr int KA = KF >= 8 ? KF : (8 / KF) * KF;
-  double yd = 0.0, yv = 0.0;
-  for (int s0 = 0; s0 < jee; s0 += KA) {
-    double gv[KA + 2], uv[KA + 2];  // rows s0-1 .. s0+KA
-#pragma unroll
-    for (int b = 0; b < KA + 2; ++b) {
-      gv[b] = last ? 0.0 : Pg(s0 + b - 1);
-      uv[b] = Vg(s0 + b - 1);
-    }
-#pragma unroll
-    for (int b = 0; b < KA; ++b) {
-      const int r = s0 + b;
-      if (r % KF == 0 && r < jee) {  // y of row r-1 at the start of segment r/KF
-        ck[(size_t)(2 * (r / KF)) * ncol] = yd;
-        ck[(size_t)(2 * (r / KF) + 1) * ncol] = yv;
-      }
-      if (r < jee) {
-        if (!last) yd = rd(r, gv[b], gv[b + 1], gv[b + 2]) + (r > 0 ? __ldg(dcy + 3 * r) : 0.0) * yd;
-        yv = rv(r, uv[b], uv[b + 1], uv[b + 2]) + (r > 0 ? __ldg(viy + 3 * r) : 0.0) * yv;
-      }
-    }
-  }
-  }
-  if constexpr ((PASSES & 2) == 0) return;
-  // ---- pass B: back-substitutions and everything row-local, rows descending
-  const double a1raw = fac[3 * (jee + 1)], a3raw = fac[3 * (jee + 1) + 1];
-  double xd = 0.0, xv = 0.0;
-  double R1 = 0.0, R2 = 0.0, R3 = 0.0;       // RHS rows 1..3 (wall row of u,w)
-  double res1 = 0.0, res2 = 0.0;             // combination of rows r+1, r+2
-  double *yq = fs.yq + col;
-  double yel = 0.0;  // implzy right-hand side of row q+1 after elimination
-  for (int sg = nseg - 1; sg >= 0; --sg) {
-    const int s0 = sg * KF;
-    double gv[KF + 2], uv[KF + 2], ydv[KF], yvv[KF];
-#pragma unroll
-    for (int b = 0; b < KF + 2; ++b) {
-      gv[b] = last ? 0.0 : Pg(s0 + b - 1);
-      uv[b] = Vg(s0 + b - 1);
-    }
-    double ad = ck[(size_t)(2 * sg) * ncol], av = ck[(size_t)(2 * sg + 1) * ncol];
-#pragma unroll
-    for (int b = 0; b < KF; ++b) {
-      const int r = s0 + b;
-      if (r < jee) {
-        if (!last) ad = rd(r, gv[b], gv[b + 1], gv[b + 2]) + (r > 0 ? __ldg(dcy + 3 * r) : 0.0) * ad;
-        av = rv(r, uv[b], uv[b + 1], uv[b + 2]) + (r > 0 ? __ldg(viy + 3 * r) : 0.0) * av;
-      }
-      ydv[b] = ad;
-      yvv[b] = av;
-    }
-    double cxv[KF], kpv[KF], hv[KF];
-#pragma unroll
-    for (int b = 0; b < KF; ++b) {
-      const int rr = min(s0 + b, jee - 1);
-      cxv[b] = (double)__ldg(cX + (size_t)rr * S);
-      kpv[b] = last ? 0.0 : (double)__ldg(kp + (size_t)min(rr, krows - 1) * S);
-      hv[b] = (double)__ldg(hp + (size_t)rr * S);
-    }
-#pragma unroll
-    for (int b = KF - 1; b >= 0; --b) {
-      const int r = s0 + b, j = r + 1;
-      if (r >= jee) continue;
-      if (!last) xd = (ydv[b] - __ldg(dcy + 3 * r + 2) * xd) * __ldg(dcy + 3 * r + 1);
-      xv = (yvv[b] - __ldg(viy + 3 * r + 2) * xv) * __ldg(viy + 3 * r + 1);
-      // RHS assembly (rhsp.F90:164-169, 181-204, 351-418, 423-445)
-      const double d1 = last ? 0.0 : xd;
-      const double u0 = uv[b + 1];
-      double R = cxv[b];
-      const double kzt = sgn * kz * ((!last && (COMP != 2 || r < ny)) ? kpv[b] : 0.0);
-      if (COMP == 0) {
-        if (!last) {
-          R = (d1 + kzt) + R;
-          if (j >= 2 && j <= ny) R = R - u0 * kv;
-        }
-      } else if (COMP == 1) {
-        if (!last) {
-          if (j >= 2 && j <= ny - 1) R = R - u0 * kv;
-          R = R + kzt;
-          R = R + d1;
-        }
-        if (j == 1 || j == ny) R = 0.0;
-      } else {
-        if (!last) {
-          if (j >= 2 && j <= ny) R = R - u0 * kv;
-          R = R + d1;
-          if (j <= ny) R = R + kzt;
-        }
-      }
-      if (COMP != 1) {  // wall and top rows of the u,w RHS (rhsp.F90:438-442)
-        if (r == jee - 1) R = 0.0;
-        if (r == 0) R = -1.0 / M4(ib, 2, 1) * (M4(ib, 2, 2) * R1 + M4(ib, 2, 3) * R2 + M4(ib, 2, 4) * R3);
-        if (r == 3) R3 = R;
-        if (r == 2) R2 = R;
-        if (r == 1) R1 = R;
-      }
-      // RK3 combination and the new RHS history (rhsp.F90:448-475)
-      const double st = r == 0 ? ub1 : (r == jee - 1 ? ubt : star(r, u0));
-      const double res = st - (var3 * R + v2 * xv + var4 * hv[b]);
-      hp[(size_t)r * S] = (W)R;
-      // implzy right-hand side of row q = r from rows r..r+2 (lip.f90:528-597)
-      if (r < n) {
-        double v = __ldg(vyi + 3 * (r + 1)) * res + __ldg(vyi + 3 * (r + 1) + 1) * res1 +
-                   __ldg(vyi + 3 * (r + 1) + 2) * res2;
-        if (r == 0) v = v - a1raw * ub1;
-        if (r == n - 1) v = v - a3raw * ubt;
-        yel = v + fac[3 * (r + 2) + 2] * yel;
-        yq[(size_t)r * ncol] = yel;
-      }
-      res2 = res1;
-      res1 = res;
-    }
-  }
-  fs.ub[col] = ub1;
-  fs.ub[(size_t)ncol + col] = ubt;
+// copies a coefficient table to shared memory (visible after a CTA barrier)
+template <typename T>
+__device__ __forceinline__ const T *stage_table(T *dst, const T *src, int n) {
+  for (int e = threadIdx.x; e < n; e += blockDim.x) dst[e] = __ldg(src + e);
+  return dst;
 }
 
-// implzy substitution x_q = (y_q - A_q x_{q-1}) / B'_q on the eliminated
-// right-hand side of k_final_s1 (rows q = 0..n-1 are velocity rows q+1),
-// then the boundary rows ub1, ubt
-template <int COMP>
-__global__ void __launch_bounds__(128) k_final_s2(DCoef c, double *u, double *v, double *w, const double *fac_u,
-                                                  const double *fac_v, const double *__restrict__ yqb,
-                                                  const double *__restrict__ ub) {
-  const int nx = c.nx, ny = c.ny, nz1 = c.nz1;
-  const int ncol = (nx - 1) * nz1;
-  const int col = blockIdx.x * blockDim.x + threadIdx.x;
-  if (col >= ncol) return;
-  const int i = col / nz1 + 2, kr = col - (i - 2) * nz1;
-  const int jee = COMP == 1 ? ny : ny + 1, n = jee - 2;
-  const size_t PU = (size_t)(ny + 1) * nz1, PV = (size_t)ny * nz1;
-  double *vel = (COMP == 0 ? u : (COMP == 1 ? v : w)) + (size_t)(i - 1) * (COMP == 1 ? PV : PU) + kr;
-  const double *fac = COMP == 1 ? fac_v : fac_u;
-  const double *yq = yqb + col;
-  constexpr int K = 8;
-  double x = 0.0;
-  for (int q0 = 0; q0 < n; q0 += K) {
-    double yv[K];
-#pragma unroll
-    for (int b = 0; b < K; ++b) yv[b] = yq[(size_t)min(q0 + b, n - 1) * ncol];
+template <int COMP, typename W, int K>
+__device__ __forceinline__ void tail_body(const DCoef &c, const DCoefT<W> &cw, const TailArgs<W> &a,
+                                          unsigned char *smraw) {
+  using VW = V2<W>;
+  constexpr int WH = COMP == 1 ? 1 : 0;
+  const int nx = c.nx, ny = c.ny, nk = c.nz1 >> 1, C = a.C[WH];
+  const int ncm = (nx - 1) * nk;
+  YPlace w(a.L[WH], C, K);
+  const int q = w.q, s = w.s, t = w.t, L = w.L, NT = w.NT;
+  const int jee = COMP == 1 ? ny : ny + 1, krows = COMP == 0 ? ny + 1 : ny, left = jee - s;
+  double2 *ex = reinterpret_cast<double2 *>(smraw);
+  VW *st = reinterpret_cast<VW *>(ex + 4 * NT) + t;
+  const double *td = a.td[WH];
+  const W *tw = a.tw[WH];
+  if constexpr (!y_table_global(K)) {
+    double *sd = reinterpret_cast<double *>(st - t + 5 * K * NT);
+    td = stage_table(sd, td, a.nd[WH]);
+    tw = stage_table(reinterpret_cast<W *>(sd + a.nd[WH]), tw, a.nw[WH]);
+  }
+  constexpr bool SLOTS = !y_table_global(K);  // else the rows are read when they are needed
+  const double *PD = td + C * kTailD * K;
+  const W *PW = tw + C * kTailW * K;
+  td += q * kTailD * K;
+  tw += q * kTailW * K;
+  // the fields that the row-wise part needs, to the thread's slots: cx, kp,
+  // p, history, p of the next plane
+  auto stage = [&](int tile) {
+    w.tile(tile, ncm);
+    const int i = w.mc / nk + 2, k = w.mc - (i - 2) * nk;
+    const bool last = i == nx;
+    const size_t PU = (size_t)(ny + 1) * nk, PV = (size_t)ny * nk, o0 = (size_t)s * nk + k;
+    const size_t pl = (size_t)(i - 1) * (COMP == 1 ? PV : PU) + o0, plv = (size_t)(i - 1) * PV + o0;
+    const VW *kp = reinterpret_cast<const VW *>(COMP == 0 ? a.uw : (COMP == 1 ? a.vw : a.ww)) + (COMP == 0 ? pl : plv);
+    const VW *cx = reinterpret_cast<const VW *>(COMP == 0 ? a.cu : (COMP == 1 ? a.cv : a.cw)) + pl;
+    const VW *hp = reinterpret_cast<const VW *>(COMP == 0 ? a.rhsupa : (COMP == 1 ? a.rhsvpa : a.rhswpa)) + pl;
+    const VW *pc = reinterpret_cast<const VW *>(a.p) + plv;
 #pragma unroll
     for (int b = 0; b < K; ++b) {
-      const int q = q0 + b;
-      if (q < n) {
-        x = (yv[b] - __ldg(fac + 3 * (q + 2)) * x) * __ldg(fac + 3 * (q + 2) + 1);
-        vel[(size_t)(q + 1) * nz1] = x;
-      }
+      const int r = s + b;
+      const size_t o = (size_t)b * nk;
+      cp_async_v(st + b * NT, cx + o, r < jee);
+      cp_async_v(st + (K + b) * NT, kp + o, !last && r < krows);
+      cp_async_v(st + (2 * K + b) * NT, pc + o, r < ny);
+      cp_async_v(st + (3 * K + b) * NT, hp + o, r < jee);
+      if (COMP == 0) cp_async_v(st + (4 * K + b) * NT, pc + PV + o, !last && r < ny);
     }
-  }
-  vel[0] = ub[col];
-  vel[(size_t)(jee - 1) * nz1] = ub[(size_t)ncol + col];
-}
-
-// ---------------------------------------------------------------------------
-// Pass B of the rhsp tail fed by TMA. A CTA owns 128 consecutive kr of one
-// plane i (one column per thread); thread 0 loads, for the next segment of
-// KF rows (descending), one box per field (the product and the velocity on
-// rows s0-1..s0+KF, the difvisxx output, the kz product and the RHS history
-// on rows s0..s0+KF-1, the pressure rows that component's pressure
-// gradient needs)
-// into a two-stage shared-memory ring, counted on one mbarrier per stage,
-// while all threads work on the current segment from shared memory. Element
-// (row b, column t) of a box is at b*128 + t, so each thread's reads are
-// conflict-free. Rows outside the field read as 0 and are not used. The
-// arithmetic is k_final_s1's pass B, operation for operation.
-// ---------------------------------------------------------------------------
-template <typename W, int COMP>
-struct FinalBox {
-  static constexpr int KF = FinalTune<W>::kf_tma, T = 128, E = (int)sizeof(W);
-  // pressure box: u needs planes i, i+1 on rows s0..s0+KF-1, v rows
-  // s0..s0+KF of plane i, w rows s0..s0+KF-1 of plane i
-  static constexpr int PR = COMP == 1 ? KF + 1 : KF, PP = COMP == 0 ? 2 : 1;
-  static constexpr int r128(int b) { return (b + 127) / 128 * 128; }
-  static constexpr int prod = 0;                              // W (KF+2) rows
-  static constexpr int vel = prod + r128((KF + 2) * T * E);   // double (KF+2) rows
-  static constexpr int cx = vel + (KF + 2) * T * 8;           // W KF rows
-  static constexpr int kp = cx + r128(KF * T * E);            // W KF rows
-  static constexpr int hp = kp + r128(KF * T * E);            // W KF rows
-  static constexpr int p = hp + r128(KF * T * E);             // W PR x PP
-  static constexpr int rc = p + r128(PR * PP * T * E);         // KF coefficient rows
-  static constexpr int stage = rc + KF * 128;
-  static constexpr unsigned tx =
-      (unsigned)((KF + 2) * T * E + (KF + 2) * T * 8 + 3 * KF * T * E + PR * PP * T * E + KF * 128);
-  static constexpr int NS = FinalTune<W>::ns_tma;  // ring stages
-  static constexpr int smem = NS * stage + 128;    // the stages and the barriers
-};
-
-template <int COMP, typename W>
-__global__ void __launch_bounds__(128) k_final_tb(DCoef c, DCoefT<W> cw, FinalStream<W> fs, int *err,
-                                                  const __grid_constant__ FinalMaps maps) {
-  using B = FinalBox<W, COMP>;
-  constexpr int KF = B::KF, TB = B::T;
-  extern __shared__ __align__(128) unsigned char smraw[];
-  constexpr int NS = B::NS;
-  uint64_t *full = reinterpret_cast<uint64_t *>(smraw + NS * B::stage);
-  const FinalArgs<W> &a = fs.a;
-  const int nx = c.nx, ny = c.ny, nz1 = c.nz1;
-  const int ncol = (nx - 1) * nz1;
-  const int t = threadIdx.x;
-  const int i = blockIdx.y + 2, kr0 = blockIdx.x * TB, kr = kr0 + t;
-  const bool active = kr < nz1;
-  const int col = (i - 2) * nz1 + kr;
-  const int k = kr >> 1, odd = kr & 1;
-  const bool last = i == nx;
-  const int jee = COMP == 1 ? ny : ny + 1, n = jee - 2;
-  const int nseg = (jee + KF - 1) / KF;
-  // ---- the ring: thread 0 initialises the barriers and loads segment nseg-1
-  auto issue = [&](int stg, int sg) {
-    unsigned char *b = smraw + stg * B::stage;
-    const int s0 = sg * KF;
-    mbar_arrive_expect_tx(&full[stg], B::tx);
-    tma_load_3d(b + B::prod, &maps.prod, kr0, s0 - 1, i - 1, &full[stg]);
-    tma_load_3d(b + B::vel, &maps.vel, kr0, s0 - 1, i - 1, &full[stg]);
-    tma_load_3d(b + B::cx, &maps.cx, kr0, s0, i - 1, &full[stg]);
-    tma_load_3d(b + B::kp, &maps.kp, kr0, s0, i - 1, &full[stg]);
-    tma_load_3d(b + B::hp, &maps.hp, kr0, s0, i - 1, &full[stg]);
-    tma_load_3d(b + B::p, &maps.p, kr0, s0, i - 1, &full[stg]);
-    tma_load_2d(b + B::rc, &maps.rc, 0, s0, &full[stg]);
+    cp_async_commit();
   };
-  if (t == 0) {
-    for (int q = 0; q < NS; ++q) mbar_init(&full[q], 1);
-    mbar_init_fence();
-  }
-  __syncthreads();
-  if (t == 0)  // the first NS-1 segments (descending)
-    for (int q = 0; q < NS - 1 && q < nseg; ++q) issue(q, nseg - 1 - q);
-  // ---- per-column setup (as k_final_s1)
-  const int pof = odd ? -1 : 1;
-  const size_t PU = (size_t)(ny + 1) * nz1, PV = (size_t)ny * nz1;
-  const size_t pl = (size_t)(i - 1) * (COMP == 1 ? PV : PU), plv = (size_t)(i - 1) * PV;
-  const size_t S = nz1;
-  const int krc = active ? kr : 0;  // inactive threads read a valid column and write nothing
-  const W *prod = (COMP == 0 ? a.uv : (COMP == 1 ? a.vv : a.vw)) + plv + krc;
-  const double *vel = (COMP == 0 ? a.u : (COMP == 1 ? a.v : a.w)) + pl + krc;
-  W *hp = (COMP == 0 ? a.rhsupa : (COMP == 1 ? a.rhsvpa : a.rhswpa)) + pl + krc;
-  const W *pc = a.p + plv + krc;
-  const double kz = c.kaz[k], kv = c.kvis[k];
-  const double var1 = a.st->var1, var3 = a.st->var3, var4 = a.st->var4;
-  const double v2 = last ? 0.0 : a.st->var2;
-  const double idxx = c.S[OTBL_S_IDXX];
-  const double *ib = c.inby, *cc = c.ccon;
-  const double sgn = odd ? 1.0 : -1.0;
-  const int which = COMP == 1 ? 1 : 0;
-  // differzy and vistyy run in W on the coefficient copy cw (FP32 on the
-  // mixed path); the RHS assembly, RK3 combination and implzy in FP64
-  // (per-row coefficients: k_tail_rows' rows, staged with each segment)
-  const double *fac = COMP == 1 ? a.fac_v : a.fac_u;
-  auto Pg = [&](int r) { return (double)__ldg(prod + (size_t)min(max(r, 0), ny - 1) * S); };
-  auto Vg = [&](int r) { return __ldg(vel + (size_t)min(max(r, 0), jee - 1) * S); };
-  // velocity after the pressure gradient (rhsp.F90:291-339), from global
-  // memory (boundary rows) ...
-  auto star_g = [&](int r, double o) -> double {
-    const int rp = min(r, ny - 1);
-    if (COMP == 0)
-      return last ? o
-                  : o - var1 * idxx * ((double)__ldg(pc + PV + (size_t)rp * S) - (double)__ldg(pc + (size_t)rp * S));
-    if (COMP == 1)
-      return o - var1 * c.idyy[r] *
-                     ((double)__ldg(pc + (size_t)min(r + 1, ny - 1) * S) - (double)__ldg(pc + (size_t)rp * S));
-    const double pp = (double)__ldg(pc + (size_t)rp * S + pof);
-    const double av = var1 * kz;
-    return o - (odd ? av * pp : -av * pp);
-  };
-  const int chv = which == 0 ? 3 : 1, cha = chv + 1, ic = which == 0 ? 3 : 1;
-  const W *db = cw.dcby, *vb = cw.cofvby;
-  W bot = W(0), top = W(0);
-  if (!last) {
-    bot = M4(db, chv, 1) * (W)Pg(0) + M4(db, chv, 2) * (W)Pg(1) + M4(db, chv, 3) * (W)Pg(2) + M4(db, chv, 4) * (W)Pg(3);
-    top = M4(db, cha, 1) * (W)Pg(ny - 1) + M4(db, cha, 2) * (W)Pg(ny - 2) + M4(db, cha, 3) * (W)Pg(ny - 3) +
-          M4(db, cha, 4) * (W)Pg(ny - 4);
-  }
-  const W b0 = M4(vb, ic, 1) * (W)Vg(0) + M4(vb, ic, 2) * (W)Vg(1) + M4(vb, ic, 3) * (W)Vg(2) + M4(vb, ic, 4) * (W)Vg(3);
-  const W bN = M4(vb, ic + 1, 1) * (W)Vg(jee - 1) + M4(vb, ic + 1, 2) * (W)Vg(jee - 2) +
-               M4(vb, ic + 1, 3) * (W)Vg(jee - 3) + M4(vb, ic + 1, 4) * (W)Vg(jee - 4);
-  double ub1 = 0.0, ubt = 0.0;
-  if (COMP == 1) {
-    ubt = kr == 0 ? c.vmagic[i - 1] : 0.0;
-  } else {
-    const double s2 = star_g(1, Vg(1)), s3 = star_g(2, Vg(2)), s4 = star_g(3, Vg(3));
-    const double sn = star_g(ny - 1, Vg(ny - 1)), sn1 = star_g(ny - 2, Vg(ny - 2)), sn2 = star_g(ny - 3, Vg(ny - 3));
-    ub1 = -1.0 / M4(ib, 2, 1) * (M4(ib, 2, 2) * s2 + M4(ib, 2, 3) * s3 + M4(ib, 2, 4) * s4);
-    ubt = -1.0 / M2(cc, 1, 1) * (M2(cc, 1, 2) * sn + M2(cc, 1, 3) * sn1 + M2(cc, 1, 4) * sn2);
-  }
-  // q: the row's W coefficients in shared memory (k_tail_rows' layout)
-  auto rd = [&](int r, const W *q, W gm, W g0, W gp) {
-    const W in = which == 0 ? q[1] * g0 + q[0] * gm : q[1] * gp + q[0] * g0;
-    return r == 0 ? bot : (r == jee - 1 ? top : in);
-  };
-  auto rv = [&](int r, const W *q, W um, W u0, W up) {
-    const W in = q[5] * up + q[6] * u0 + q[7] * um;
-    return r == 0 ? b0 : (r == jee - 1 ? bN : in);
-  };
-  const W *ck = reinterpret_cast<const W *>(fs.ck) + (active ? col : 0);
-  double *yq = fs.yq + (active ? col : 0);
-  const double a1raw = fac[3 * (jee + 1)], a3raw = fac[3 * (jee + 1) + 1];
-  W xd = W(0), xv = W(0);
-  double R1 = 0.0, R2 = 0.0, R3 = 0.0;
-  double res1 = 0.0, res2 = 0.0;
-  double yel = 0.0;
-  W ckd = ck[(size_t)(2 * (nseg - 1)) * ncol], ckv = ck[(size_t)(2 * (nseg - 1) + 1) * ncol];
-  const int tk = t ^ 1;  // kr+1 for even kr, kr-1 for odd kr (the chunk starts even)
-  for (int sg = nseg - 1, it = 0; sg >= 0; --sg, ++it) {
-    const int stg = it % NS;
-    const bool ok = mbar_wait_bounded(&full[stg], (it / NS) & 1, 2000000000ull);
-    if (__syncthreads_or(!ok)) {  // the stage of iteration it-1 is free from here on
-      if (t == 0) atomicExch(err, OTBL_ERR_TIMEOUT);
-      return;
-    }
-    if (t == 0 && sg >= NS - 1) issue((it + NS - 1) % NS, sg - (NS - 1));
-    const int s0 = sg * KF;
-    const unsigned char *bs = smraw + stg * B::stage;
-    const W *sp = reinterpret_cast<const W *>(bs + B::prod);
-    const double *sv = reinterpret_cast<const double *>(bs + B::vel);
-    const W *sc = reinterpret_cast<const W *>(bs + B::cx);
-    const W *sk = reinterpret_cast<const W *>(bs + B::kp);
-    const W *sh = reinterpret_cast<const W *>(bs + B::hp);
-    const W *spp = reinterpret_cast<const W *>(bs + B::p);
-    const double *rcs = reinterpret_cast<const double *>(bs + B::rc);
-    W ad = ckd, av = ckv;
-    if (sg >= 1) {  // next segment's checkpoints, ahead of use
-      ckd = ck[(size_t)(2 * (sg - 1)) * ncol];
-      ckv = ck[(size_t)(2 * (sg - 1) + 1) * ncol];
-    }
-    if (!active) continue;
-    W ydv[KF], yvv[KF];
+  if (SLOTS && blockIdx.x * L < ncm) stage(blockIdx.x);
+  for (int tile = blockIdx.x; tile * L < ncm; tile += gridDim.x) {
+    w.tile(tile, ncm);
+    const int i = w.mc / nk + 2, k = w.mc - (i - 2) * nk;
+    const bool last = i == nx;
+    const size_t PU = (size_t)(ny + 1) * nk, PV = (size_t)ny * nk;
+    const size_t pl = (size_t)(i - 1) * (COMP == 1 ? PV : PU) + k, plv = (size_t)(i - 1) * PV + k;
+    const VW *prod = reinterpret_cast<const VW *>(COMP == 0 ? a.uv : (COMP == 1 ? a.vv : a.vw)) + plv;
+    VW *hp = reinterpret_cast<VW *>(COMP == 0 ? a.rhsupa : (COMP == 1 ? a.rhsvpa : a.rhswpa)) + pl;
+    const VW *pc = reinterpret_cast<const VW *>(a.p) + plv;
+    double2 *vel = reinterpret_cast<double2 *>(COMP == 0 ? a.u : (COMP == 1 ? a.v : a.w)) + pl;
+    constexpr int PO = WH == 0 ? -1 : 0;  // product rows s + PO ..
+    VW g[K + 1];
+    double2 u[K + 2];  // velocity rows s-1 .. s+K
 #pragma unroll
-    for (int b = 0; b < KF; ++b) {
-      const int r = s0 + b;
-      const W *q = reinterpret_cast<const W *>(rcs + 16 * b + 5);
-      if (r < jee) {
-        if (!last)
-          ad = rd(r, q, sp[b * TB + t], sp[(b + 1) * TB + t], sp[(b + 2) * TB + t]) + (r > 0 ? q[2] : W(0)) * ad;
-        av = rv(r, q, (W)sv[b * TB + t], (W)sv[(b + 1) * TB + t], (W)sv[(b + 2) * TB + t]) +
-             (r > 0 ? q[8] : W(0)) * av;
-      }
-      ydv[b] = ad;
-      yvv[b] = av;
+    for (int b = 0; b <= K; ++b) {
+      const int r = s + PO + b;
+      g[b] = ld_row(prod + (ptrdiff_t)r * nk, !last && r >= 0 && r < ny);
     }
 #pragma unroll
-    for (int b = KF - 1; b >= 0; --b) {
-      const int r = s0 + b, j = r + 1;
-      if (r >= jee) continue;
-      const double *rq = rcs + 16 * b;
-      const W *q = reinterpret_cast<const W *>(rq + 5);
-      if (!last) xd = (ydv[b] - q[4] * xd) * q[3];
-      xv = (yvv[b] - q[10] * xv) * q[9];
-      // RHS assembly (rhsp.F90:164-169, 181-204, 351-418, 423-445)
-      const double d1 = last ? 0.0 : (double)xd;
-      const double u0 = sv[(b + 1) * TB + t];
-      double R = (double)sc[b * TB + t];
-      const double kzt = sgn * kz * ((!last && (COMP != 2 || r < ny)) ? (double)sk[b * TB + tk] : 0.0);
+    for (int b = 0; b < K + 2; ++b) {
+      const int r = s - 1 + b;
+      u[b] = ld_row(vel + (ptrdiff_t)r * nk, r >= 0 && r < jee);
+    }
+    VW pk = cmake<VW>(W(0), W(0));  // v: the pressure row after the chunk
+    if (COMP == 1) pk = ld_row(pc + (size_t)(s + K) * nk, s + K < ny);
+    const double kz = c.kaz[k], kv = c.kvis[k];
+    const double var1 = a.st->var1, var3 = a.st->var3, var4 = a.st->var4;
+    const double v2 = last ? 0.0 : a.st->var2;
+    const double idxx = c.S[OTBL_S_IDXX];
+    auto cvw = [](auto x) { return cmake<VW>((W)x.x, (W)x.y); };
+    // velocity after the pressure gradient (rhsp.F90:291-339)
+    auto star = [&](double2 o, double idyy, VW p0, VW p1) {
       if (COMP == 0) {
         if (!last) {
-          R = (d1 + kzt) + R;
-          if (j >= 2 && j <= ny) R = R - u0 * kv;
+          o.x = o.x - var1 * idxx * ((double)p1.x - (double)p0.x);
+          o.y = o.y - var1 * idxx * ((double)p1.y - (double)p0.y);
         }
       } else if (COMP == 1) {
-        if (!last) {
-          if (j >= 2 && j <= ny - 1) R = R - u0 * kv;
-          R = R + kzt;
-          R = R + d1;
-        }
-        if (j == 1 || j == ny) R = 0.0;
+        o.x = o.x - var1 * idyy * ((double)p1.x - (double)p0.x);
+        o.y = o.y - var1 * idyy * ((double)p1.y - (double)p0.y);
       } else {
-        if (!last) {
-          if (j >= 2 && j <= ny) R = R - u0 * kv;
-          R = R + d1;
-          if (j <= ny) R = R + kzt;
-        }
+        const double av = var1 * kz;
+        o.x = o.x + av * (double)p0.y;
+        o.y = o.y - av * (double)p0.x;
       }
-      if (COMP != 1) {  // wall and top rows of the u,w RHS (rhsp.F90:438-442)
-        if (r == jee - 1) R = 0.0;
-        if (r == 0) R = -1.0 / M4(ib, 2, 1) * (M4(ib, 2, 2) * R1 + M4(ib, 2, 3) * R2 + M4(ib, 2, 4) * R3);
-        if (r == 3) R3 = R;
-        if (r == 2) R2 = R;
-        if (r == 1) R1 = R;
-      }
-      // RK3 combination and the new RHS history (rhsp.F90:448-475); rows
-      // 1..jee-2 of the pressure box (no clamp needed there)
-      double st;
-      if (r == 0) {
-        st = ub1;
-      } else if (r == jee - 1) {
-        st = ubt;
-      } else if (COMP == 0) {
-        st = last ? u0 : u0 - var1 * idxx * ((double)spp[(B::PR + b) * TB + t] - (double)spp[b * TB + t]);
-      } else if (COMP == 1) {
-        st = u0 - var1 * rq[4] * ((double)spp[(b + 1) * TB + t] - (double)spp[b * TB + t]);
-      } else {
-        const double pp = (double)spp[b * TB + tk];
-        const double avz = var1 * kz;
-        st = u0 - (odd ? avz * pp : -avz * pp);
-      }
-      const double res = st - (var3 * R + v2 * (double)xv + var4 * (double)sh[b * TB + t]);
-      hp[(size_t)r * S] = (W)R;
-      if (r < n) {
-        double v = rq[1] * res + rq[2] * res1 + rq[3] * res2;
-        if (r == 0) v = v - a1raw * ub1;
-        if (r == n - 1) v = v - a3raw * ubt;
-        yel = v + rq[0] * yel;
-        yq[(size_t)r * ncol] = yel;
-      }
-      res2 = res1;
-      res1 = res;
+      return o;
+    };
+    // ---- right-hand sides of differzy and vistyy (table weights are 0 on the
+    // boundary rows, whose closures are added)
+    __syncthreads();  // the tables are there, the exchange buffers are free
+    VW yd[K], yv[K];
+    const int chv = WH == 0 ? 3 : 1, ic = WH == 0 ? 3 : 1;
+#pragma unroll
+    for (int b = 0; b < K; ++b) {
+      VW r = cmake<VW>(W(0), W(0));
+      fma2(r, tw[b], g[b]);
+      fma2(r, tw[K + b], g[b + 1]);
+      yd[b] = r;
+      r = cmake<VW>(W(0), W(0));
+      fma2(r, tw[5 * K + b], cvw(u[b + 2]));
+      fma2(r, tw[6 * K + b], cvw(u[b + 1]));
+      fma2(r, tw[7 * K + b], cvw(u[b]));
+      yv[b] = r;
     }
-  }
-  if (active) {
-    fs.ub[col] = ub1;
-    fs.ub[(size_t)ncol + col] = ubt;
+    if (q == 0) {
+#pragma unroll
+      for (int m = 1; m <= 4; ++m) {
+        fma2(yd[0], M4(cw.dcby, chv, m), g[m - 1 - PO]);
+        fma2(yv[0], M4(cw.cofvby, ic, m), cvw(u[m]));
+      }
+    }
+    double2 ubt = make_double2(0.0, 0.0);  // boun's top row (boun.f90:33-55)
+    if (left <= K + 1) {                   // the last chunk, or the one before a last chunk of one row
+      VW bN = cmake<VW>(W(0), W(0)), top = bN;
+      const double *cc = c.ccon;
+#pragma unroll
+      for (int m = 1; m <= 4; ++m) {
+        const double2 o = ld_row(vel + (size_t)(jee - m) * nk, true);
+        fma2(bN, M4(cw.cofvby, ic + 1, m), cvw(o));
+        fma2(top, M4(cw.dcby, chv + 1, m), ld_row(prod + (size_t)(ny - m) * nk, !last));
+        if (COMP != 1 && m > 1) {
+          const int r = jee - m;
+          const VW p0 = ld_row(pc + (size_t)r * nk, true);
+          const VW p1 = ld_row(pc + PV + (size_t)r * nk, COMP == 0 && !last);
+          const double2 v = star(o, 0.0, p0, p1);
+          ubt.x += M2(cc, 1, m) * v.x;
+          ubt.y += M2(cc, 1, m) * v.y;
+        }
+      }
+      if (COMP == 1) {
+        ubt.x = k == 0 ? c.vmagic[i - 1] : 0.0;
+      } else {
+        const double r = -1.0 / M2(cc, 1, 1);
+        ubt.x *= r;
+        ubt.y *= r;
+      }
+#pragma unroll
+      for (int b = 0; b < K; ++b) {
+        yd[b] = select2(b == left - 1, top, yd[b]);
+        yv[b] = select2(b == left - 1, bN, yv[b]);
+      }
+    }
+    // ---- both solves
+    {
+      VW *e0 = reinterpret_cast<VW *>(ex), *e1 = reinterpret_cast<VW *>(ex + NT);
+      const W *ld = tw + 2 * K, *lv = tw + 8 * K;
+      forward_local<K, 1, W>(yd, ld);
+      forward_local<K, 1, W>(yv, lv);
+      e0[t] = yd[K - 1];
+      e1[t] = yv[K - 1];
+      __syncthreads();
+      if (q > 0) {
+        forward_fix<K, 1, W>(yd, ld, chunk_carry<W>(e0 + t - L, -L, PW + q - 1, -1, q));
+        forward_fix<K, 1, W>(yv, lv, chunk_carry<W>(e1 + t - L, -L, PW + 2 * C + q - 1, -1, q));
+      }
+      e0 = reinterpret_cast<VW *>(ex + 2 * NT);
+      e1 = reinterpret_cast<VW *>(ex + 3 * NT);
+      backward_local<K, 1, W>(yd, ld + K, ld + 2 * K);
+      backward_local<K, 1, W>(yv, lv + K, lv + 2 * K);
+      e0[t] = yd[0];
+      e1[t] = yv[0];
+      __syncthreads();
+      if (q < C - 1) {
+        backward_fix<K, 1, W>(yd, ld + 2 * K, chunk_carry<W>(e0 + t + L, L, PW + C + q + 1, 1, C - 1 - q));
+        backward_fix<K, 1, W>(yv, lv + 2 * K, chunk_carry<W>(e1 + t + L, L, PW + 3 * C + q + 1, 1, C - 1 - q));
+      }
+    }
+    cp_async_wait<0>();  // the thread's own slots
+    // ---- RHS assembly (rhsp.F90:164-169, 181-204, 351-418, 423-445), RK3
+    // combination and the new RHS history (rhsp.F90:448-475)
+    double2 res[K];
+    double2 R1 = make_double2(0.0, 0.0), R2 = R1, R3 = R1, S1 = R1, S2 = R1, S3 = R1;
+#pragma unroll
+    for (int b = 0; b < K; ++b) {
+      {
+        const int r = s + b, j = r + 1;
+        VW cxv, kpv, p0, hv, p2;
+        if constexpr (SLOTS) {
+          cxv = st[b * NT], kpv = st[(K + b) * NT], p0 = st[(2 * K + b) * NT], hv = st[(3 * K + b) * NT];
+          p2 = COMP == 0 ? st[(4 * K + b) * NT] : (b < K - 1 ? st[(2 * K + (b < K - 1 ? b + 1 : b)) * NT] : pk);
+        } else {
+          const VW *kp = reinterpret_cast<const VW *>(COMP == 0 ? a.uw : (COMP == 1 ? a.vw : a.ww));
+          const VW *cx = reinterpret_cast<const VW *>(COMP == 0 ? a.cu : (COMP == 1 ? a.cv : a.cw));
+          const size_t o = (size_t)r * nk;
+          cxv = ld_row(cx + pl + o, r < jee);
+          kpv = ld_row(kp + (COMP == 0 ? pl : plv) + o, !last && r < krows);
+          p0 = ld_row(pc + o, r < ny);
+          hv = ld_row(hp + o, r < jee);
+          p2 = COMP == 0 ? ld_row(pc + PV + o, !last && r < ny) : ld_row(pc + o + nk, r + 1 < ny);
+        }
+        const double2 u0 = u[b + 1];
+        double2 R = make_double2((double)cxv.x, (double)cxv.y);
+        const double2 kzt = make_double2(-kz * (double)kpv.y, kz * (double)kpv.x);
+        if (!last) {
+          const double2 d1 = make_double2((double)yd[b].x, (double)yd[b].y);
+          if (COMP == 0) {
+            R.x = (d1.x + kzt.x) + R.x;
+            R.y = (d1.y + kzt.y) + R.y;
+            if (j >= 2 && j <= ny) {
+              R.x = R.x - u0.x * kv;
+              R.y = R.y - u0.y * kv;
+            }
+          } else if (COMP == 1) {
+            R.x = ((R.x - u0.x * kv) + kzt.x) + d1.x;
+            R.y = ((R.y - u0.y * kv) + kzt.y) + d1.y;
+          } else {
+            if (j >= 2 && j <= ny) {
+              R.x = R.x - u0.x * kv;
+              R.y = R.y - u0.y * kv;
+            }
+            R.x = (R.x + d1.x) + kzt.x;
+            R.y = (R.y + d1.y) + kzt.y;
+          }
+        }
+        if (r == jee - 1 || (COMP == 1 && r == 0)) R = make_double2(0.0, 0.0);
+        double2 sv = star(u0, COMP == 1 ? td[6 * K + b] : 0.0, p0, p2);
+        if (COMP != 1 && b >= 1 && b <= 3) {
+          (b == 1 ? R1 : (b == 2 ? R2 : R3)) = R;
+          (b == 1 ? S1 : (b == 2 ? S2 : S3)) = sv;
+        }
+        if (r == jee - 1) sv = ubt;
+        if (COMP == 1 && r == 0) sv = make_double2(0.0, 0.0);
+        const double2 xv = make_double2((double)yv[b].x, (double)yv[b].y);
+        res[b].x = sv.x - (var3 * R.x + v2 * xv.x + var4 * (double)hv.x);
+        res[b].y = sv.y - (var3 * R.y + v2 * xv.y + var4 * (double)hv.y);
+        if (w.active && r < jee && (COMP == 1 || r > 0)) hp[(size_t)r * nk] = cmake<VW>((W)R.x, (W)R.y);
+        if (COMP != 1 && b == 0 && r == 0) res[0] = make_double2((double)hv.x, (double)hv.y);  // finished below
+      }
+    }
+    const bool active = w.active;
+    if (SLOTS && (tile + gridDim.x) * L < ncm) stage(tile + gridDim.x);  // the slots are free
+    double2 ub1 = make_double2(0.0, 0.0);  // boun's wall row
+    if (COMP != 1 && q == 0) {
+      const double *ib = c.inby;
+      const double f = -1.0 / M4(ib, 2, 1);
+      ub1.x = f * (M4(ib, 2, 2) * S1.x + M4(ib, 2, 3) * S2.x + M4(ib, 2, 4) * S3.x);
+      ub1.y = f * (M4(ib, 2, 2) * S1.y + M4(ib, 2, 3) * S2.y + M4(ib, 2, 4) * S3.y);
+      const double2 R = make_double2(f * (M4(ib, 2, 2) * R1.x + M4(ib, 2, 3) * R2.x + M4(ib, 2, 4) * R3.x),
+                                     f * (M4(ib, 2, 2) * R1.y + M4(ib, 2, 3) * R2.y + M4(ib, 2, 4) * R3.y));
+      res[0].x = ub1.x - (var3 * R.x + v2 * (double)yv[0].x + var4 * res[0].x);
+      res[0].y = ub1.y - (var3 * R.y + v2 * (double)yv[0].y + var4 * res[0].y);
+      if (active) hp[0] = cmake<VW>((W)R.x, (W)R.y);
+    }
+    // ---- implzy (lip.f90:528-597): right-hand side from rows r-1..r+1 of the
+    // combination, then the solve; the boundary rows carry ub1, ubt
+    ex[t] = res[0];
+    ex[NT + t] = res[K - 1];
+    __syncthreads();
+    {
+      double2 rm = q > 0 ? ex[NT + t - L] : make_double2(0.0, 0.0);
+      const double2 rn = q < C - 1 ? ex[t + L] : make_double2(0.0, 0.0);
+#pragma unroll
+      for (int b = 0; b < K; ++b) {
+        const int r = s + b;
+        const double2 rp = b < K - 1 ? res[b < K - 1 ? b + 1 : b] : rn, r0 = res[b];
+        double2 v = make_double2(0.0, 0.0);
+        fma2(v, td[b], rm);
+        fma2(v, td[K + b], r0);
+        fma2(v, td[2 * K + b], rp);
+        if (r == 0) v = ub1;
+        if (r == 1) fma2(v, -PD[2 * C], ub1);
+        if (r == jee - 2) fma2(v, -PD[2 * C + 1], ubt);
+        if (r == jee - 1) v = ubt;
+        res[b] = v;
+        rm = r0;
+      }
+    }
+    chunk_forward<K, 1, double>(res, td + 3 * K, PD, ex + 2 * NT, q, t, L);
+    chunk_backward<K, 1, double>(res, td + 4 * K, td + 5 * K, PD + C, ex, q, C, t, L);
+    if (active) {
+#pragma unroll
+      for (int b = 0; b < K; ++b)
+        if (b < left) vel[(size_t)(s + b) * nk] = res[b];
+    }
   }
 }
 
-// Pass A of the rhsp tail fed by TMA: the same ring as k_final_tb, ascending,
-// with boxes of 128 columns x KA+2 rows of the product and the velocity
-// (KA = 8 rows per stage); the checkpoints are still written every KF rows
-// of k_final_tb's segments. The arithmetic is k_final_s1's pass A.
-template <int COMP, typename W>
-__global__ void __launch_bounds__(128) k_final_ta(DCoef c, DCoefT<W> cw, FinalStream<W> fs, int *err,
-                                                  const __grid_constant__ FinalMaps maps) {
-  constexpr int KF = FinalTune<W>::kf_tma, KA = 8, TB = 128, R = KA + 2;
-  constexpr int PB = (R * TB * (int)sizeof(W) + 127) / 128 * 128;
-  constexpr int STG = PB + R * TB * 8 + KA * 128;  // + the KA coefficient rows
-  constexpr unsigned TX = (unsigned)(R * TB * sizeof(W) + R * TB * 8 + KA * 128);
-  extern __shared__ __align__(128) unsigned char smraw[];
-  uint64_t *bar = reinterpret_cast<uint64_t *>(smraw + 2 * STG);
-  const FinalArgs<W> &a = fs.a;
-  const int nx = c.nx, ny = c.ny, nz1 = c.nz1;
-  const int ncol = (nx - 1) * nz1;
-  const int t = threadIdx.x;
-  const int i = blockIdx.y + 2, kr0 = blockIdx.x * TB, kr = kr0 + t;
-  const bool active = kr < nz1;
-  const int krc = active ? kr : 0;
-  const int col = (i - 2) * nz1 + krc;
-  const bool last = i == nx;
-  const int jee = COMP == 1 ? ny : ny + 1;
-  const int nst = (jee + KA - 1) / KA;
-  auto issue = [&](int stg, int sa) {
-    unsigned char *b = smraw + stg * STG;
-    mbar_arrive_expect_tx(&bar[stg], TX);
-    tma_load_3d(b, &maps.prod_a, kr0, sa * KA - 1, i - 1, &bar[stg]);
-    tma_load_3d(b + PB, &maps.vel_a, kr0, sa * KA - 1, i - 1, &bar[stg]);
-    tma_load_2d(b + PB + R * TB * 8, &maps.rc_a, 0, sa * KA, &bar[stg]);
-  };
-  if (t == 0) {
-    mbar_init(&bar[0], 1);
-    mbar_init(&bar[1], 1);
-    mbar_init_fence();
-  }
-  __syncthreads();
-  if (t == 0) issue(0, 0);
-  const size_t PU = (size_t)(ny + 1) * nz1, PV = (size_t)ny * nz1;
-  const size_t pl = (size_t)(i - 1) * (COMP == 1 ? PV : PU), plv = (size_t)(i - 1) * PV;
-  const size_t S = nz1;
-  const W *prod = (COMP == 0 ? a.uv : (COMP == 1 ? a.vv : a.vw)) + plv + krc;
-  const double *vel = (COMP == 0 ? a.u : (COMP == 1 ? a.v : a.w)) + pl + krc;
-  const int which = COMP == 1 ? 1 : 0;
-  // the sweeps run in W on the coefficient copy cw (FP32 on the mixed path);
-  // the per-row coefficients come staged with the boxes (k_tail_rows' rows)
-  auto Pg = [&](int r) { return (W)__ldg(prod + (size_t)min(max(r, 0), ny - 1) * S); };
-  auto Vg = [&](int r) { return (W)__ldg(vel + (size_t)min(max(r, 0), jee - 1) * S); };
-  const int chv = which == 0 ? 3 : 1, cha = chv + 1, ic = which == 0 ? 3 : 1;
-  const W *db = cw.dcby, *vb = cw.cofvby;
-  W bot = W(0), top = W(0);
-  if (!last) {
-    bot = M4(db, chv, 1) * Pg(0) + M4(db, chv, 2) * Pg(1) + M4(db, chv, 3) * Pg(2) + M4(db, chv, 4) * Pg(3);
-    top = M4(db, cha, 1) * Pg(ny - 1) + M4(db, cha, 2) * Pg(ny - 2) + M4(db, cha, 3) * Pg(ny - 3) +
-          M4(db, cha, 4) * Pg(ny - 4);
-  }
-  const W b0 = M4(vb, ic, 1) * Vg(0) + M4(vb, ic, 2) * Vg(1) + M4(vb, ic, 3) * Vg(2) + M4(vb, ic, 4) * Vg(3);
-  const W bN = M4(vb, ic + 1, 1) * Vg(jee - 1) + M4(vb, ic + 1, 2) * Vg(jee - 2) +
-               M4(vb, ic + 1, 3) * Vg(jee - 3) + M4(vb, ic + 1, 4) * Vg(jee - 4);
-  auto rd = [&](int r, const W *q, W gm, W g0, W gp) {
-    const W in = which == 0 ? q[1] * g0 + q[0] * gm : q[1] * gp + q[0] * g0;
-    return r == 0 ? bot : (r == jee - 1 ? top : in);
-  };
-  auto rv = [&](int r, const W *q, W um, W u0, W up) {
-    const W in = q[5] * up + q[6] * u0 + q[7] * um;
-    return r == 0 ? b0 : (r == jee - 1 ? bN : in);
-  };
-  W *ck = reinterpret_cast<W *>(fs.ck) + col;  // checkpoints in W, read back by k_final_tb
-  W yd = W(0), yv = W(0);
-  for (int sa = 0; sa < nst; ++sa) {
-    const int stg = sa & 1;
-    const bool ok = mbar_wait_bounded(&bar[stg], (sa >> 1) & 1, 2000000000ull);
-    if (__syncthreads_or(!ok)) {
-      if (t == 0) atomicExch(err, OTBL_ERR_TIMEOUT);
-      return;
-    }
-    if (t == 0 && sa + 1 < nst) issue(stg ^ 1, sa + 1);
-    if (!active) continue;
-    const W *sp = reinterpret_cast<const W *>(smraw + stg * STG) + t;
-    const double *sv = reinterpret_cast<const double *>(smraw + stg * STG + PB) + t;
-    const double *rcs = reinterpret_cast<const double *>(smraw + stg * STG + PB + R * TB * 8);
-    const int s0 = sa * KA;
-#pragma unroll
-    for (int b = 0; b < KA; ++b) {
-      const int r = s0 + b;
-      const W *q = reinterpret_cast<const W *>(rcs + 16 * b + 5);
-      if (r % KF == 0 && r < jee) {  // y of row r-1 at the start of segment r/KF
-        ck[(size_t)(2 * (r / KF)) * ncol] = yd;
-        ck[(size_t)(2 * (r / KF) + 1) * ncol] = yv;
-      }
-      if (r < jee) {
-        if (!last) yd = rd(r, q, sp[b * TB], sp[(b + 1) * TB], sp[(b + 2) * TB]) + (r > 0 ? q[2] : W(0)) * yd;
-        yv = rv(r, q, (W)sv[b * TB], (W)sv[(b + 1) * TB], (W)sv[(b + 2) * TB]) + (r > 0 ? q[8] : W(0)) * yv;
-      }
-    }
-  }
+template <typename W, int K>
+__global__ void __launch_bounds__(K > 7 ? 256 : 128, K > 7 ? 1 : (sizeof(W) == 8 ? 2 : 3))
+    k_tail(DCoef c, DCoefT<W> cw, TailArgs<W> a) {
+  extern __shared__ __align__(16) unsigned char smraw[];
+  const int comp = pick3(a.comp, blockIdx.y);
+  if (comp == 0)
+    tail_body<0, W, K>(c, cw, a, smraw);
+  else if (comp == 1)
+    tail_body<1, W, K>(c, cw, a, smraw);
+  else
+    tail_body<2, W, K>(c, cw, a, smraw);
 }
 
 // ---------------------------------------------------------------------------
@@ -928,160 +514,217 @@ __global__ void k_pois_lu(DCoef c, double *dinv) {
   dv[(size_t)(ny1 - 1) * nm] = 1.0 / a2p;
 }
 
-// The solve in place on phi rows 0..ny-2 of planes 2..nx, one thread per
-// column: y_r = rhs_r + l_r y_{r-1}, l_r = -ayp(1,r+1) dinv(r-1); then
-// x_r = (y_r - ayp(3,r+1) x_{r+1}) dinv(r). The singular (i = 2, k = 0)
-// system has its last row zeroed first (pois.f90:111-114). The launch takes
-// the columns kr0 <= kr < kr0 + nkr of every plane, in T (FP64, or FP32 for
-// the higher spanwise modes of the mixed path, with FP32 coefficients and
-// pivots); phi and the checkpoints hold T.
-template <typename T>
-__global__ void __launch_bounds__(128) k_pois_solve(DCoefT<T> c, T *phi, const T *__restrict__ dinv, T *ckbuf,
-                                                    int kr0, int nkr) {
-  const int ny = c.ny, ny1 = ny - 1, nz1 = c.nz1, nm = c.nz2 + 1;
-  const int ncol = (c.nx - 1) * nkr;
-  const int col = blockIdx.x * blockDim.x + threadIdx.x;
-  if (col >= ncol) return;
-  const int i = col / nkr + 2, kr = kr0 + (col - (i - 2) * nkr), k = kr >> 1;
-  const size_t S = nz1;
-  T *x = phi + (size_t)(i - 1) * ny * nz1 + kr;
-  const T *dv = dinv + (size_t)(i - 1) * ny * nm + k;
-  T *ck = ckbuf + col;
-  const T *ayp = c.ayp;
+// The solve in place on phi rows 0..ny-2 of planes 2..nx: y_r = rhs_r + l_r
+// y_{r-1}, l_r = -ayp(1,r+1) dinv(r-1); then x_r = (y_r - ayp(3,r+1)
+// x_{r+1}) dinv(r). The singular (i = 2, k = 0) system has its last row
+// zeroed first (pois.f90:111-114). The launch takes the modes k0 <= k < k0 +
+// nkm of every plane, in T (FP64, or FP32 for the higher spanwise modes of
+// the mixed path, with FP32 coefficients and pivots); phi holds T. The chunk
+// products differ per mode and are exchanged with the values; the smooth
+// modes' products do not decay and take every chunk.
+template <typename T, int K>
+__global__ void __launch_bounds__(256, 2) k_pois_solve(DCoefT<T> c, T *phi, const T *__restrict__ dinv, int k0,
+                                                       int nkm, int C, int L) {
+  using V = V2<T>;
+  extern __shared__ __align__(16) unsigned char smraw[];
+  const int ny = c.ny, ny1 = ny - 1, nk = c.nz1 >> 1;
+  YPlace w(L, C, K);
+  w.tile(blockIdx.x, (c.nx - 1) * nkm);
+  const int i = w.mc / nkm + 2, k = k0 + w.mc - (i - 2) * nkm, s = w.s, t = w.t, q = w.q;
+  V *x = reinterpret_cast<V *>(phi) + ((size_t)(i - 1) * ny + s) * nk + k;
+  const T *dv = dinv + ((size_t)(i - 1) * ny + s) * nk + k;
+  const T *ayp = c.ayp + 3 * s;
   const bool sing = i == 2 && k == 0;
-  auto X = [&](int r) { return (sing && r == ny1 - 1) ? (T)0 : x[(size_t)min(r, ny1 - 1) * S]; };
-  auto D = [&](int r) { return __ldg(dv + (size_t)min(max(r, 0), ny1 - 1) * nm); };
-  const int nseg = (ny1 + KY - 1) / KY;
-  T y = 0;
-  for (int sg = 0; sg < nseg; ++sg) {
-    const int s0 = sg * KY;
-    ck[(size_t)sg * ncol] = y;
-    T bv[KY], dp[KY + 1];
+  V y[K];
+  T l[K], d[K];
+  T dp = q > 0 ? __ldg(dv - nk) : T(0);
 #pragma unroll
-    for (int b = 0; b < KY; ++b) bv[b] = X(s0 + b);
-#pragma unroll
-    for (int b = 0; b <= KY; ++b) dp[b] = D(s0 + b - 1);
-#pragma unroll
-    for (int b = 0; b < KY; ++b) {
-      const int r = s0 + b;
-      if (r < ny1) y = bv[b] + (r > 0 ? -A3(ayp, 1, r + 1) * dp[b] : (T)0) * y;
-    }
+  for (int b = 0; b < K; ++b) {
+    const int r = s + b;
+    y[b] = ld_row(x + (size_t)b * nk, r < ny1 && !(sing && r == ny1 - 1));
+    d[b] = r < ny1 ? __ldg(dv + (size_t)b * nk) : T(0);
   }
-  T xn = 0;
-  for (int sg = nseg - 1; sg >= 0; --sg) {
-    const int s0 = sg * KY;
-    T bv[KY], dp[KY + 1], yv[KY];
+  V *e0 = reinterpret_cast<V *>(smraw), *e1 = e0 + w.NT;
+  T *p0 = reinterpret_cast<T *>(e1 + w.NT), *p1 = p0 + w.NT;
+  T pr = T(1);
 #pragma unroll
-    for (int b = 0; b < KY; ++b) bv[b] = X(s0 + b);
-#pragma unroll
-    for (int b = 0; b <= KY; ++b) dp[b] = D(s0 + b - 1);
-    T yy = ck[(size_t)sg * ncol];
-#pragma unroll
-    for (int b = 0; b < KY; ++b) {
-      const int r = s0 + b;
-      if (r < ny1) yy = bv[b] + (r > 0 ? -A3(ayp, 1, r + 1) * dp[b] : (T)0) * yy;
-      yv[b] = yy;
-    }
-#pragma unroll
-    for (int b = KY - 1; b >= 0; --b) {
-      const int r = s0 + b;
-      if (r < ny1) {
-        xn = (yv[b] - (r < ny1 - 1 ? A3(ayp, 3, r + 1) : (T)0) * xn) * dp[b + 1];
-        x[(size_t)r * S] = xn;
-      }
-    }
+  for (int b = 0; b < K; ++b) {
+    l[b] = s + b < ny1 ? -__ldg(ayp + 3 * b) * dp : T(0);
+    pr *= l[b];
+    dp = d[b];
   }
+  forward_local<K, 1, T>(y, l);
+  e0[t] = y[K - 1];
+  p0[t] = pr;
+  __syncthreads();
+  if (q > 0) forward_fix<K, 1, T>(y, l, chunk_carry<T>(e0 + t - w.L, -w.L, p0 + t - w.L, -w.L, q));
+  pr = T(1);
+#pragma unroll
+  for (int b = 0; b < K; ++b) {  // l holds e from here on
+    l[b] = s + b < ny1 - 1 ? -__ldg(ayp + 3 * b + 2) * d[b] : T(0);
+    pr *= l[b];
+  }
+  backward_local<K, 1, T>(y, d, l);
+  e1[t] = y[0];
+  p1[t] = pr;
+  __syncthreads();
+  if (q < C - 1) backward_fix<K, 1, T>(y, l, chunk_carry<T>(e1 + t + w.L, w.L, p1 + t + w.L, w.L, C - 1 - q));
+  if (!w.active) return;
+#pragma unroll
+  for (int b = 0; b < K; ++b)
+    if (s + b < ny1) x[(size_t)b * nk] = y[b];
 }
 
 // ---------------------------------------------------------------------------
-// launch wrappers
+// tables and launch wrappers
 // ---------------------------------------------------------------------------
-// Checkpoints of interpyy at the tail of each line scratch, so that
-// interpyy can run beside interpxx (whose checkpoints start at the head);
-// nullptr when the two would overlap.
-double *interpy_ck_tail(otbl_ctx *c, double *s) {
-  const int nx = c->cfg.nx, ny = c->cfg.ny, nz = c->cfg.nz, nz1 = c->dc.nz1;
-  const size_t lu = otbl_field_len(nx, ny, nz, 1);  // doubles in s2, s3 (s1 may be larger)
-  const size_t ncol = (size_t)nx * nz1;
-  // the shorter of the register-streamed and the TMA-fed segments
-  const int ky = KY < YTune<double>::kt ? KY : YTune<double>::kt;
-  const size_t y_need = (size_t)((ny + ky - 1) / ky) * ncol;  // doubles (floats need less)
-  // interpxx: at most one checkpoint per 4 planes per line (4 is its shortest segment)
-  const size_t x_need = (size_t)((nx + 3) / 4) * (size_t)(ny + 1) * nz1;
-  if (x_need + y_need + 64 > lu) return nullptr;
-  return s + ((lu - y_need) & ~(size_t)31);
+// Work::ytab in T: interpyy (u-type, v-type), then differzy and vistyy
+// (u-type, v-type); Work::tdtab in FP64: implzy (u-type, v-type), whose l, d,
+// e and products k_dt writes for the substep's dt
+struct YSizes {
+  int K, C[2], Ci;            // rows per chunk; chunks of the tail (u-, v-type) and of interpyy
+  size_t in, tw[2], td[2];    // elements of each table
+  int QS;                     // row stride of interpyy's
+};
+static YSizes y_sizes(int ny) {
+  YSizes z;
+  z.K = y_chunk(ny);
+  z.Ci = (ny + z.K - 1) / z.K;
+  z.QS = z.K == 7 ? 64 : 256;
+  z.in = (size_t)(kYInterp * z.K + 2) * z.QS;
+  for (int wh = 0; wh < 2; ++wh) {
+    z.C[wh] = ((wh ? ny : ny + 1) + z.K - 1) / z.K;
+    z.tw[wh] = ytab_elems(z.K, z.C[wh], kTailW, 4);
+    z.td[wh] = ytab_elems(z.K, z.C[wh], kTailD, 2);
+  }
+  return z;
+}
+size_t ytab_bytes(int ny, bool mixed) {
+  const YSizes z = y_sizes(ny);
+  return (2 * z.in + z.tw[0] + z.tw[1]) * (mixed ? sizeof(float) : sizeof(double));
+}
+size_t tdtab_doubles(int ny) {
+  const YSizes z = y_sizes(ny);
+  return z.td[0] + z.td[1];
+}
+
+ImplzyTab implzy_tab(otbl_ctx *c, int which) {
+  const YSizes z = y_sizes(c->cfg.ny);
+  double *t = c->w.tdtab + (which ? z.td[0] : 0);
+  return {t + 3 * z.K, t + (size_t)z.C[which] * kTailD * z.K, z.K, kTailD * z.K, z.C[which]};
+}
+
+template <typename T>
+static cudaError_t y_tables(otbl_ctx *c) {
+  const int ny = c->cfg.ny;
+  const YSizes z = y_sizes(ny);
+  const int K = z.K;
+  otbl_coef_offsets o;
+  otbl_coef_layout(c->cfg.nx, ny, c->cfg.nz, &o);
+  std::vector<T> cf(c->coef_host.begin(), c->coef_host.end());
+  auto A = [&](int id) { return cf.data() + o.off[id]; };
+  std::vector<T> all(2 * z.in + z.tw[0] + z.tw[1], T(0));
+  T *tab = all.data();
+  for (int wh = 0; wh < 2; ++wh, tab += z.in) {
+    const T *e = A(wh ? OTBL_C_COFIVY : OTBL_C_COFIUY);
+    auto put = [&](int i, int r, T v) { tab[(size_t)(i * K + r % K) * z.QS + r / K] = v; };
+    for (int r = 1; r < ny - 1; ++r) {
+      put(0, r, e[2 * r]);
+      put(1, r, e[2 * r + 1]);
+    }
+    T *P = tab + (size_t)kYInterp * K * z.QS;
+    chunk_factors<T>([&](int i, int r, T v) { put(2 + i, r, v); }, K, ny, A(wh ? OTBL_C_INYV : OTBL_C_INYU), 0, P,
+                     P + z.QS);
+  }
+  const int S = kTailW * K;
+  auto put = [&](int i, int r, T v) { tab[(size_t)(r / K) * S + i * K + r % K] = v; };
+  auto lde = [&](int at) { return [&put, at](int i, int r, T v) { put(at + i, r, v); }; };
+  for (int wh = 0; wh < 2; tab += z.tw[wh], ++wh) {
+    const int jee = wh ? ny : ny + 1, C = z.C[wh];
+    const T *e = A(wh ? OTBL_C_COFCYV : OTBL_C_COFCYU), *ev = A(wh ? OTBL_C_COFVYV : OTBL_C_COFVYU);
+    for (int r = 1; r < jee - 1; ++r) {
+      put(0, r, e[2 * r]);
+      put(1, r, e[2 * r + 1]);
+      for (int k = 0; k < 3; ++k) put(5 + k, r, ev[3 * r + k]);
+    }
+    T *P = tab + (size_t)C * S;
+    chunk_factors<T>(lde(2), K, jee, A(wh ? OTBL_C_DCYV : OTBL_C_DCYU), 0, P, P + C);
+    chunk_factors<T>(lde(8), K, jee, A(wh ? OTBL_C_VIYV : OTBL_C_VIYU), 0, P + 2 * C, P + 3 * C);
+  }
+  std::vector<double> dt(z.td[0] + z.td[1], 0.0);
+  for (int wh = 0; wh < 2; ++wh) {
+    double *td = dt.data() + (wh ? z.td[0] : 0);
+    const int jee = wh ? ny : ny + 1;
+    const double *vyi = c->coef_host.data() + o.off[wh ? OTBL_C_VYVI : OTBL_C_VYUI];
+    const double *idyy = c->coef_host.data() + o.off[OTBL_C_IDYY];
+    for (int r = 0; r < jee; ++r) {
+      double *row = td + (size_t)(r / K) * kTailD * K + r % K;
+      if (r > 0 && r < jee - 1)
+        for (int k = 0; k < 3; ++k) row[k * K] = vyi[3 * r + k];
+      if (wh && r < ny) row[6 * K] = idyy[r];
+    }
+  }
+  cudaError_t e = cudaMemcpyAsync(c->w.ytab, all.data(), all.size() * sizeof(T), cudaMemcpyHostToDevice, c->stream);
+  if (e == cudaSuccess)
+    e = cudaMemcpyAsync(c->w.tdtab, dt.data(), dt.size() * sizeof(double), cudaMemcpyHostToDevice, c->stream);
+  return e == cudaSuccess ? cudaStreamSynchronize(c->stream) : e;
+}
+
+cudaError_t prepare_ylines(otbl_ctx *c) { return c->mixed ? y_tables<float>(c) : y_tables<double>(c); }
+
+// tiles of a persistent launch: what `per` CTAs per SM take at once, shared by
+// ncomp fields, unless there are fewer
+static int y_grid(int ntile, int per, int ncomp) {
+  return std::min(ntile, std::max(1, (per * sm_count() + ncomp - 1) / ncomp));
+}
+
+template <typename T>
+static void interpy_t(otbl_ctx *c, const DCoefT<T> &dc, InterpyArgs &a) {
+  const YSizes z = y_sizes(c->cfg.ny);
+  for (int wh = 0; wh < 2; ++wh) a.tab[wh] = static_cast<const T *>(c->w.ytab) + wh * z.in;
+  a.C = z.Ci;
+  // as wide as the threads allow, or narrower when the autotuner found that
+  // faster (tune_bs 128, 64, 32)
+  a.L = std::max(1, y_lanes(a.C, 256) * c->tune_bs[2] / 128);
+  const int NT = y_threads(a.C, a.L), ncm = c->cfg.nx * (c->dc.nz1 / 2);
+  const dim3 gr((ncm + a.L - 1) / a.L, 3);
+  const size_t sm = (size_t)2 * NT * sizeof(V2<T>);
+  if (z.K == 7)
+    k_interpy<T, 7, 64><<<gr, NT, sm, c->stream>>>(dc, a);
+  else
+    k_interpy<T, 15, 256><<<gr, NT, sm, c->stream>>>(dc, a);
 }
 
 cudaError_t launch_interpy(otbl_ctx *c) {
-  InterpyArgs a;
-  const double *ins[3] = {c->f[OTBL_F_U], c->f[OTBL_F_W], c->f[OTBL_F_V]};
-  void *outs[3] = {c->w.uy, c->w.wy, c->w.vy};
-  double *tail[3] = {interpy_ck_tail(c, c->w.s1), interpy_ck_tail(c, c->w.s2), interpy_ck_tail(c, c->w.s3)};
-  double *cks[3] = {tail[0] ? tail[0] : c->w.s1, tail[1] ? tail[1] : c->w.s2, tail[2] ? tail[2] : c->w.s3};
-  const int which[3] = {0, 0, 1};
-  for (int f = 0; f < 3; ++f) {
-    a.in[f] = ins[f];
-    a.out[f] = outs[f];
-    a.ck[f] = cks[f];
-    a.which[f] = which[f];
-  }
-  const int ncol = c->cfg.nx * c->dc.nz1;
   prof_begin(c, PK_INTERPY);
   if (ydense_ready(c)) {
     const cudaError_t e = launch_interpy_dense(c);
     prof_end(c);
     return e;
   }
-  const int bs = c->tune_bs[2];
-  if (c->ymaps_ok) {
-    const dim3 gt((c->dc.nz1 + 127) / 128, c->cfg.nx, 3);
-    if (c->mixed) {
-      const int sm = 2 * ((YTune<float>::kt + 2) * 128 * 8 + YTune<float>::kt * 8 * 4) + 128;
-      cudaFuncSetAttribute(k_interpy_t<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm);
-      k_interpy_t<float><<<gt, 128, sm, c->stream>>>(c->dcf, a, &c->st->err, c->ymi);
-    } else {
-      const int sm = 2 * ((YTune<double>::kt + 2) * 128 * 8 + YTune<double>::kt * 8 * 8) + 128;
-      cudaFuncSetAttribute(k_interpy_t<double>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm);
-      k_interpy_t<double><<<gt, 128, sm, c->stream>>>(c->dc, a, &c->st->err, c->ymi);
-    }
-  } else if (c->mixed)
-    k_interpy<float><<<dim3((ncol + bs - 1) / bs, 3), bs, 0, c->stream>>>(c->dcf, a);
+  if (stream_interpy(c)) {
+    const cudaError_t e = launch_interpy_stream(c);
+    prof_end(c);
+    c->launches += 1;
+    return e;
+  }
+  InterpyArgs a;
+  const double *ins[3] = {c->f[OTBL_F_U], c->f[OTBL_F_W], c->f[OTBL_F_V]};
+  void *outs[3] = {c->w.uy, c->w.wy, c->w.vy};
+  for (int f = 0; f < 3; ++f) {
+    a.in[f] = ins[f];
+    a.out[f] = outs[f];
+    a.which[f] = f == 2;
+  }
+  if (c->mixed)
+    interpy_t<float>(c, c->dcf, a);
   else
-    k_interpy<double><<<dim3((ncol + bs - 1) / bs, 3), bs, 0, c->stream>>>(c->dc, a);
+    interpy_t<double>(c, c->dc, a);
   prof_end(c);
   c->launches += 1;
   return cudaGetLastError();
 }
 
-// One row of 8 T per y row r of each table (which 0: u-type input, u and w;
-// 1: v-type input, v): interpyy's right-hand-side weights econ[2r],
-// econ[2r+1] and LU coefficients iny[3r..3r+2]; the rest 0. k_interpy_t's
-// ring stages a segment's rows with its field box.
-template <typename T>
-__global__ void __launch_bounds__(128) k_y_rows(DCoefT<T> c, T *tab) {
-  const int ny = c.ny;
-  const int e = blockIdx.x * blockDim.x + threadIdx.x;
-  if (e >= 2 * ny) return;
-  const int which = e / ny, r = e - which * ny;
-  const T *iny = which == 0 ? c.inyu : c.inyv, *econ = which == 0 ? c.cofiuy : c.cofivy;
-  T *q = tab + (size_t)e * 8;
-  q[0] = econ[2 * r];
-  q[1] = econ[2 * r + 1];
-  for (int k = 0; k < 3; ++k) q[2 + k] = iny[3 * r + k];
-  for (int k = 5; k < 8; ++k) q[k] = T(0);
-}
-
-cudaError_t launch_y_rows(otbl_ctx *c) {
-  const int n = 2 * c->cfg.ny;
-  if (c->mixed)
-    k_y_rows<float><<<(n + 127) / 128, 128, 0, c->stream>>>(c->dcf, static_cast<float *>(c->w.yrowc));
-  else
-    k_y_rows<double><<<(n + 127) / 128, 128, 0, c->stream>>>(c->dc, static_cast<double *>(c->w.yrowc));
-  c->launches += 1;
-  return cudaGetLastError();
-}
-
-// ---- TMA descriptors (host) ----
 // cuTensorMapEncodeTiled from the driver, looked up once (thread-safe
 // initialisation of a function-local static); nullptr if unavailable
 void *tensor_map_encoder() {
@@ -1097,155 +740,10 @@ void *tensor_map_encoder() {
   return fn;
 }
 
-// a field [planes][rows][nz1] of element size esz, boxes of 128 x brows x bplanes
-static bool encode_field(CUtensorMap *m, const void *base, size_t esz, int planes, int rows, int nz1, int brows,
-                         int bplanes) {
-  auto fn = reinterpret_cast<PFN_cuTensorMapEncodeTiled_v12000>(tensor_map_encoder());
-  if (!fn || (nz1 * esz) % 16 != 0 || ((uintptr_t)base) % 16 != 0) return false;
-  const cuuint64_t dims[3] = {(cuuint64_t)nz1, (cuuint64_t)rows, (cuuint64_t)planes};
-  const cuuint64_t strides[2] = {(cuuint64_t)nz1 * esz, (cuuint64_t)rows * nz1 * esz};
-  const cuuint32_t box[3] = {128, (cuuint32_t)brows, (cuuint32_t)bplanes};
-  const cuuint32_t es[3] = {1, 1, 1};
-  const CUtensorMapDataType dt = esz == 8 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT64 : CU_TENSOR_MAP_DATA_TYPE_FLOAT32;
-  return fn(m, dt, 3, const_cast<void *>(base), dims, strides, box, es, CU_TENSOR_MAP_INTERLEAVE_NONE,
-            CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
-            CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
-}
-
-static bool encode_rows(CUtensorMap *m, const double *base, int rows, int brows);
-
-// 2D map of a coefficient table [rows][width elements of esz bytes], boxes
-// of brows full rows
-static bool encode_table(CUtensorMap *m, const void *base, size_t esz, int width, int rows, int brows) {
-  auto fn = reinterpret_cast<PFN_cuTensorMapEncodeTiled_v12000>(tensor_map_encoder());
-  if (!fn || ((uintptr_t)base) % 16 != 0 || (width * esz) % 16 != 0) return false;
-  const cuuint64_t dims[2] = {(cuuint64_t)width, (cuuint64_t)rows};
-  const cuuint64_t strides[1] = {width * esz};
-  const cuuint32_t box[2] = {(cuuint32_t)width, (cuuint32_t)brows};
-  const cuuint32_t es[2] = {1, 1};
-  const CUtensorMapDataType dt = esz == 8 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT64 : CU_TENSOR_MAP_DATA_TYPE_FLOAT32;
-  return fn(m, dt, 2, const_cast<void *>(base), dims, strides, box, es, CU_TENSOR_MAP_INTERLEAVE_NONE,
-            CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
-            CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
-}
-
 template <typename W>
-static bool build_maps_t(otbl_ctx *c) {
-  constexpr int KF = FinalTune<W>::kf_tma;
-  const int nx = c->cfg.nx, ny = c->cfg.ny, nz1 = c->dc.nz1;
-  const size_t ew = sizeof(W);
-  bool ok = nz1 >= 2;
-  for (int comp = 0; comp < 3 && ok; ++comp) {
-    FinalMaps &m = c->fmaps[comp];
-    const int jee = comp == 1 ? ny : ny + 1;
-    const void *prod = comp == 0 ? c->w.uv : (comp == 1 ? c->w.vv : c->w.vw);
-    const void *kp = comp == 0 ? c->w.uw : (comp == 1 ? c->w.vw : c->w.ww);
-    const int kprows = comp == 0 ? ny + 1 : ny;
-    const double *vel = c->f[comp == 0 ? OTBL_F_U : (comp == 1 ? OTBL_F_V : OTBL_F_W)];
-    const void *cx = comp == 0 ? c->w.cu : (comp == 1 ? c->w.cv : c->w.cw);
-    const void *hp = c->f[comp == 0 ? OTBL_F_RHSUPA : (comp == 1 ? OTBL_F_RHSVPA : OTBL_F_RHSWPA)];
-    ok = ok && encode_field(&m.prod, prod, ew, nx, ny, nz1, KF + 2, 1);
-    ok = ok && encode_field(&m.prod_a, prod, ew, nx, ny, nz1, 8 + 2, 1);
-    ok = ok && encode_field(&m.vel_a, vel, 8, nx, jee, nz1, 8 + 2, 1);
-    ok = ok && encode_field(&m.kp, kp, ew, nx, kprows, nz1, KF, 1);
-    ok = ok && encode_field(&m.vel, vel, 8, nx, jee, nz1, KF + 2, 1);
-    ok = ok && encode_field(&m.cx, cx, ew, nx, jee, nz1, KF, 1);
-    ok = ok && encode_field(&m.hp, hp, ew, nx, jee, nz1, KF, 1);
-    ok = ok && encode_field(&m.p, c->f[OTBL_F_P], ew, nx, ny, nz1, comp == 1 ? KF + 1 : KF, comp == 0 ? 2 : 1);
-    ok = ok && encode_rows(&m.rc, c->w.rowc + (comp == 1 ? (size_t)16 * (ny + 2) : 0), ny + 2, KF);
-    ok = ok && encode_rows(&m.rc_a, c->w.rowc + (comp == 1 ? (size_t)16 * (ny + 2) : 0), ny + 2, 8);
-  }
-  return ok;
-}
-
-bool build_y_maps(otbl_ctx *c) {
-  const int K = c->mixed ? YTune<float>::kt : YTune<double>::kt;
-  const int nx = c->cfg.nx, ny = c->cfg.ny, nz1 = c->dc.nz1;
-  const double *in[3] = {c->f[OTBL_F_U], c->f[OTBL_F_W], c->f[OTBL_F_V]};
-  const int rows[3] = {ny + 1, ny + 1, ny};
-  bool ok = true;
-  const size_t ew = c->mixed ? sizeof(float) : sizeof(double);
-  const int which[3] = {0, 0, 1};
-  for (int f = 0; f < 3 && ok; ++f) {
-    ok = encode_field(&c->ymi.g[f], in[f], 8, nx, rows[f], nz1, K + 2, 1);
-    const char *tab = static_cast<const char *>(c->w.yrowc) + (size_t)which[f] * ny * 8 * ew;
-    ok = ok && encode_table(&c->ymi.r[f], tab, ew, 8, ny, K);
-  }
-  c->ymaps_ok = ok;
-  return ok;
-}
-
-// One 128-byte row per y row r and tail kind (table 0: the u and w tails,
-// u-type coefficients; table 1: the v tail): the FP64 values fac[3(r+2)+2]
-// (the implzy factor of the descending elimination), vyi[3(r+1)+0..2] and
-// idyy[r], then in W ecd[2r+0..1], dcy[3r+0..2], ecv[3r+0..2],
-// viy[3r+0..2] (differzy's and vistyy's right-hand-side and LU
-// coefficients). k_final_tb's ring stages a segment's rows with its field
-// boxes, so its sweeps read them from shared memory as broadcasts. Entries
-// that a row does not use are 0.
-template <typename W>
-__global__ void __launch_bounds__(128) k_tail_rows(DCoef c, DCoefT<W> cw, const double *fac_u, const double *fac_v,
-                                                   double *rowc) {
-  const int ny = c.ny, R = ny + 2;
-  const int e = blockIdx.x * blockDim.x + threadIdx.x;
-  if (e >= 2 * R) return;
-  const int which = e / R, r = e - which * R;
-  const int jee = which == 1 ? ny : ny + 1, n = jee - 2;
-  double *row = rowc + (size_t)e * 16;
-  const double *fac = which == 1 ? fac_v : fac_u;
-  const double *vyi = which == 0 ? c.vyui : c.vyvi;
-  row[0] = r < n ? fac[3 * (r + 2) + 2] : 0.0;
-  for (int q = 0; q < 3; ++q) row[1 + q] = r < n ? vyi[3 * (r + 1) + q] : 0.0;
-  row[4] = (which == 1 && r < ny) ? c.idyy[r] : 0.0;
-  W *q = reinterpret_cast<W *>(row + 5);
-  constexpr int NW = (int)((128 - 5 * sizeof(double)) / sizeof(W));
-  for (int k = 0; k < NW; ++k) q[k] = W(0);
-  if (r < jee) {
-    const W *dcy = which == 0 ? cw.dcyu : cw.dcyv, *ecd = which == 0 ? cw.cofcyu : cw.cofcyv;
-    const W *viy = which == 0 ? cw.viyu : cw.viyv, *ecv = which == 0 ? cw.cofvyu : cw.cofvyv;
-    q[0] = ecd[2 * r];
-    q[1] = ecd[2 * r + 1];
-    for (int k = 0; k < 3; ++k) {
-      q[2 + k] = dcy[3 * r + k];
-      q[5 + k] = ecv[3 * r + k];
-      q[8 + k] = viy[3 * r + k];
-    }
-  }
-}
-
-cudaError_t launch_tail_rows(otbl_ctx *c) {
-  if (!c->fmaps_ok) return cudaSuccess;
-  const int n = 2 * (c->cfg.ny + 2);
-  if (c->mixed)
-    k_tail_rows<float><<<(n + 127) / 128, 128, 0, c->stream>>>(c->dc, c->dcf, c->w.fac_u, c->w.fac_v, c->w.rowc);
-  else
-    k_tail_rows<double><<<(n + 127) / 128, 128, 0, c->stream>>>(c->dc, c->dc, c->w.fac_u, c->w.fac_v, c->w.rowc);
-  c->launches += 1;
-  return cudaGetLastError();
-}
-
-// 2D map of one table of Work::rowc: [ny+2 rows][16 doubles], boxes of KF rows
-static bool encode_rows(CUtensorMap *m, const double *base, int rows, int brows) {
-  auto fn = reinterpret_cast<PFN_cuTensorMapEncodeTiled_v12000>(tensor_map_encoder());
-  if (!fn || ((uintptr_t)base) % 16 != 0) return false;
-  const cuuint64_t dims[2] = {16, (cuuint64_t)rows};
-  const cuuint64_t strides[1] = {16 * sizeof(double)};
-  const cuuint32_t box[2] = {16, (cuuint32_t)brows};
-  const cuuint32_t es[2] = {1, 1};
-  return fn(m, CU_TENSOR_MAP_DATA_TYPE_FLOAT64, 2, const_cast<double *>(base), dims, strides, box, es,
-            CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
-            CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
-}
-
-bool build_final_maps(otbl_ctx *c) {
-  c->fmaps_ok = c->mixed ? build_maps_t<float>(c) : build_maps_t<double>(c);
-  return c->fmaps_ok;
-}
-
-template <typename W>
-static int final_t(otbl_ctx *c, unsigned comps, cudaEvent_t before_vel, bool second_scratch) {
-  FinalStream<W> fs;
-  FinalArgs<W> &a = fs.a;
+static void tail_t(otbl_ctx *c, const DCoefT<W> &cw, unsigned comps) {
+  const YSizes z = y_sizes(c->cfg.ny);
+  TailArgs<W> a;
   a.u = c->f[OTBL_F_U];
   a.v = c->f[OTBL_F_V];
   a.w = c->f[OTBL_F_W];
@@ -1261,61 +759,45 @@ static int final_t(otbl_ctx *c, unsigned comps, cudaEvent_t before_vel, bool sec
   a.vw = static_cast<const W *>(c->w.vw);
   a.vv = static_cast<const W *>(c->w.vv);
   a.ww = static_cast<const W *>(c->w.ww);
-  a.fac_u = c->w.fac_u;
-  a.fac_v = c->w.fac_v;
   a.st = c->st;
-  const int ncol = (c->cfg.nx - 1) * c->dc.nz1;
-  fs.ck = second_scratch ? c->w.t1 : c->w.s1;
-  fs.yq = second_scratch ? c->w.t2 : c->w.s2;
-  fs.ub = second_scratch ? c->w.t3 : c->w.s3;
-  const dim3 g((ncol + 127) / 128);
-  double *U = c->f[OTBL_F_U], *V = c->f[OTBL_F_V], *Wv = c->f[OTBL_F_W];
-  const bool tma = c->fmaps_ok;
-  DCoefT<W> cw;  // the sweeps' coefficients in W
-  if constexpr (std::is_same<W, float>::value)
-    cw = c->dcf;
-  else
-    cw = c->dc;
-  const dim3 gt((c->dc.nz1 + 127) / 128, c->cfg.nx - 1);
-  auto comp = [&](auto C) {
-    constexpr int K = decltype(C)::value;
-    const int smem_t = FinalBox<W, K>::smem;
-    if (tma) {
-      // pass A (register-streamed or TMA-fed), then the TMA-fed pass B
-      if constexpr (FinalTune<W>::tma_a) {
-        constexpr int sma = 2 * ((10 * 128 * (int)sizeof(W) + 127) / 128 * 128 + 10 * 128 * 8 + 8 * 128) + 128;
-        cudaFuncSetAttribute(k_final_ta<K, W>, cudaFuncAttributeMaxDynamicSharedMemorySize, sma);
-        k_final_ta<K, W><<<gt, 128, sma, c->stream>>>(c->dc, cw, fs, &c->st->err, c->fmaps[K]);
-      } else {
-        k_final_s1<K, W, 1, FinalTune<W>::kf_tma><<<g, 128, 0, c->stream>>>(c->dc, fs);
-      }
-      cudaFuncSetAttribute(k_final_tb<K, W>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_t);
-      k_final_tb<K, W><<<gt, 128, smem_t, c->stream>>>(c->dc, cw, fs, &c->st->err, c->fmaps[K]);
-    } else if constexpr (FinalTune<W>::split) {
-      k_final_s1<K, W, 1><<<g, 128, 0, c->stream>>>(c->dc, fs);
-      k_final_s1<K, W, 2><<<g, 128, 0, c->stream>>>(c->dc, fs);
-    } else {
-      k_final_s1<K, W, 3><<<g, 128, 0, c->stream>>>(c->dc, fs);
-    }
-    if (before_vel) {  // the first velocity write waits for this event
-      cudaStreamWaitEvent(c->stream, before_vel, 0);
-      before_vel = nullptr;
-    }
-    k_final_s2<K><<<g, 128, 0, c->stream>>>(c->dc, U, V, Wv, c->w.fac_u, c->w.fac_v, fs.yq, fs.ub);
+  const bool gt = y_table_global(z.K);
+  int NT = 0, lmin = 32, n = 0;
+  size_t tabs = 0;
+  for (int wh = 0; wh < 2; ++wh) {
+    a.tw[wh] = static_cast<const W *>(c->w.ytab) + 2 * z.in + (wh ? z.tw[0] : 0);
+    a.td[wh] = c->w.tdtab + (wh ? z.td[0] : 0);
+    a.C[wh] = z.C[wh];
+    a.nw[wh] = (int)z.tw[wh];
+    a.nd[wh] = (int)z.td[wh];
+    a.L[wh] = y_lanes(z.C[wh], gt ? 256 : 128);
+    lmin = std::min(lmin, a.L[wh]);
+    NT = std::max(NT, y_threads(z.C[wh], a.L[wh]));
+    if (!gt) tabs = std::max(tabs, z.td[wh] * sizeof(double) + z.tw[wh] * sizeof(W));
+  }
+  for (int k = 0; k < 3; ++k) a.comp[k] = 0;
+  for (int k = 0; k < 3; ++k)
+    if (comps & (1u << k)) a.comp[n++] = k;
+  const int ncm = (c->cfg.nx - 1) * (c->dc.nz1 / 2), ntile = (ncm + lmin - 1) / lmin;
+  const size_t sm = (size_t)4 * NT * 16 + (gt ? 0 : (size_t)5 * z.K * NT * sizeof(V2<W>)) + tabs;
+  const int per = std::max(1, std::min((int)(233472 / (sm + 1024)), gt ? 1 : (sizeof(W) == 8 ? 256 : 384) / NT));
+  auto go = [&](auto kern) {
+    if (sm > 48 * 1024) cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+    kern<<<dim3(y_grid(ntile, per, n), n), NT, sm, c->stream>>>(c->dc, cw, a);
   };
-  int n = 0;
-  if (comps & 1) comp(std::integral_constant<int, 0>{}), ++n;
-  if (comps & 2) comp(std::integral_constant<int, 1>{}), ++n;
-  if (comps & 4) comp(std::integral_constant<int, 2>{}), ++n;
-  return n * ((tma || FinalTune<W>::split) ? 3 : 2);
+  if (z.K == 7)
+    go(k_tail<W, 7>);
+  else
+    go(k_tail<W, 15>);
 }
 
-cudaError_t launch_final(otbl_ctx *c, unsigned comps, cudaEvent_t before_vel, bool second_scratch) {
+cudaError_t launch_final(otbl_ctx *c, unsigned comps) {
   prof_begin(c, PK_FINAL);
-  const int nl = c->mixed ? final_t<float>(c, comps, before_vel, second_scratch)
-                          : final_t<double>(c, comps, before_vel, second_scratch);
+  if (c->mixed)
+    tail_t<float>(c, c->dcf, comps);
+  else
+    tail_t<double>(c, c->dc, comps);
   prof_end(c);
-  c->launches += nl;
+  c->launches += 1;
   return cudaGetLastError();
 }
 
@@ -1331,20 +813,25 @@ cudaError_t launch_pois_lu(otbl_ctx *c) {
   return cudaGetLastError();
 }
 
-// columns kr0 <= kr < kr0 + nkr of every plane; phi holds T
+// modes k0 <= k < k0 + nkm of every plane; phi holds T
 template <typename T>
-static void pois_solve_t(otbl_ctx *c, const DCoefT<T> &dc, T *phi, const T *dinv, int kr0, int nkr) {
-  const int ncol = (c->cfg.nx - 1) * nkr;
-  k_pois_solve<T><<<(ncol + 127) / 128, 128, 0, c->stream>>>(dc, phi, dinv, reinterpret_cast<T *>(c->w.s1), kr0,
-                                                            nkr);
+static void pois_solve_t(otbl_ctx *c, const DCoefT<T> &dc, T *phi, const T *dinv, int k0, int nkm) {
+  const int K = c->cfg.ny - 1 <= 7 * 64 ? 7 : 15;
+  const int C = (c->cfg.ny - 1 + K - 1) / K, L = std::max(1, std::min(32, 224 / C)), NT = y_threads(C, L);
+  const int ncm = (c->cfg.nx - 1) * nkm, nb = (ncm + L - 1) / L;
+  const size_t sm = (size_t)2 * NT * (sizeof(V2<T>) + sizeof(T));
+  if (K == 7)
+    k_pois_solve<T, 7><<<nb, NT, sm, c->stream>>>(dc, phi, dinv, k0, nkm, C, L);
+  else
+    k_pois_solve<T, 15><<<nb, NT, sm, c->stream>>>(dc, phi, dinv, k0, nkm, C, L);
   c->launches += 1;
 }
 
 cudaError_t launch_pois_solve(otbl_ctx *c, double *phi64, float *phi32, int kr_split) {
-  const int nz1 = c->dc.nz1;
+  const int nk = c->dc.nz1 / 2, ks = kr_split / 2;
   prof_begin(c, PK_POIS_SOLVE);
-  if (kr_split > 0) pois_solve_t<double>(c, c->dc, phi64, c->w.pois_dinv, 0, kr_split);
-  if (kr_split < nz1) pois_solve_t<float>(c, c->dcf, phi32, c->w.pois_dinvf, kr_split, nz1 - kr_split);
+  if (ks > 0) pois_solve_t<double>(c, c->dc, phi64, c->w.pois_dinv, 0, ks);
+  if (ks < nk) pois_solve_t<float>(c, c->dcf, phi32, c->w.pois_dinvf, ks, nk - ks);
   prof_end(c);
   return cudaGetLastError();
 }

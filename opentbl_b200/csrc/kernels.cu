@@ -442,51 +442,42 @@ __global__ void __launch_bounds__(128, std::is_same<T, double>::value ? OTBL_PR_
 // ---------------------------------------------------------------------------
 // dt (rhsp.F90:214-267), RK3 factors, implzy LU (lip.f90:545-568)
 // ---------------------------------------------------------------------------
-// Factors of (A + var1*B) for implzy (lip.f90:545-568, rows j = 2..jee-1),
-// eliminated from the top row down (a UL factorisation; the reference's LU
-// eliminates from the bottom, and both solve the same diagonally dominant
-// system to rounding), so that the rhsp tail, which forms the right-hand
-// side from the top row down, eliminates as it goes. With A_j, B_j, C_j the
-// sub-, main and super-diagonal of row j:
-//   B'_{jee-1} = B_{jee-1},  m_j = C_j / B'_{j+1},  B'_j = B_j - m_j A_{j+1}
-//   fac[3j] = A_j (0 for j = 2), fac[3j+1] = 1/B'_j, fac[3j+2] = -m_j (0 for
-//   j = jee-1); descending y_j = r_j + fac[3j+2] y_{j+1}, ascending
-//   x_j = (y_j - fac[3j] x_{j-1}) fac[3j+1].
-// The two boundary couplings that implzy moves to the right-hand side:
-// fac[3*(jee+1)] = A_2, fac[3*(jee+1)+1] = C_{jee-1}.
-__device__ void implzy_factor(const DCoef &c, double *fac, int which, double var1) {
-  const int ny = c.ny, jee = which == 0 ? ny + 1 : ny;
-  const double *icon = which == 0 ? c.vyui : c.vyvi;
-  const double *econ = which == 0 ? c.cofvyu : c.cofvyv;
-  auto Aj = [&](int j) { return A3(icon, 1, j) + var1 * A3(econ, 3, j); };
-  auto Bj = [&](int j) { return A3(icon, 2, j) + var1 * A3(econ, 2, j); };
-  auto Cj = [&](int j) { return A3(icon, 3, j) + var1 * A3(econ, 1, j); };
-  fac[3 * (jee + 1)] = Aj(2);
-  fac[3 * (jee + 1) + 1] = Cj(jee - 1);
-  double bp = Bj(jee - 1);
-  fac[3 * (jee - 1) + 2] = 0.0;
-  for (int j = jee - 1;; --j) {
-    const double ib = 1.0 / bp;
-    fac[3 * j + 1] = ib;
-    fac[3 * j] = j == 2 ? 0.0 : Aj(j);
-    if (j == 2) break;
-    const double m = Cj(j - 1) * ib;  // m_{j-1} = C_{j-1} / B'_j
-    fac[3 * (j - 1) + 2] = -m;
-    bp = Bj(j - 1) - m * Aj(j);
-  }
+// Factors of (A + var1*B) for implzy (lip.f90:545-568): with A_r, B_r, C_r the
+// sub-, main and super-diagonal of row r (0-based, the unknowns r = 1..jee-2),
+// pivot_r = B_r - A_r C_{r-1} / pivot_{r-1}, l_r = -A_r / pivot_{r-1}, d_r =
+// 1 / pivot_r, e_r = -C_r d_r; the boundary rows pass their value through (l =
+// e = 0, d = 1). The pivots are the ratios of the continuants t_r = B_r
+// t_{r-1} - A_r C_{r-1} t_{r-2}, which leaves no division on the serial
+// chain (one multiply-add a row instead of a division and two; computed
+// ratios satisfy the pivot recurrence to one rounding, so it loses nothing).
+// The reference's two boundary couplings: P[2 C] = A_1, P[2 C + 1] =
+// C_{jee-2}.
+struct ImplzyRow {
+  double A, B, C;
+};
+__device__ __forceinline__ ImplzyRow implzy_row(const DCoef &c, int which, int r, double var1) {
+  const double *icon = (which == 0 ? c.vyui : c.vyvi) + 3 * r, *econ = (which == 0 ? c.cofvyu : c.cofvyv) + 3 * r;
+  return {icon[0] + var1 * econ[2], icon[1] + var1 * econ[1], icon[2] + var1 * econ[0]};
 }
 
-// One CTA of 64 threads: the CFL reduction over the rows, then dt, the RK3
-// factors and the two implzy factorisations (one warp each).
-__global__ void __launch_bounds__(64) k_dt(DCoef c, DState *st, const unsigned long long *vm_bits, double *fac_u,
-                                           double *fac_v, int m, int setstep, int dt_mode, double dt_fixed) {
-  __shared__ double s_dt3[2], s_vmax[2];
-  const int t = threadIdx.x, lane = t & 31, wid = t >> 5;
+// One CTA: the CFL reduction over the rows, then dt, the RK3 factors and the
+// two implzy factorisations. Shared memory: 8 (ny+1) doubles, 12 with fac_u.
+// fac_u, fac_v (null when the tail is not streamed): the factors of the
+// elimination from the top row down, in 1-based rows j = 2..jee-1: B'_j = B_j -
+// C_j A_{j+1} / B'_{j+1}; fac[3j] = A_j (0 for j = 2), fac[3j+1] = 1/B'_j,
+// fac[3j+2] = -C_j / B'_{j+1} (0 for j = jee-1); descending y_j = r_j +
+// fac[3j+2] y_{j+1}, ascending x_j = (y_j - fac[3j] x_{j-1}) fac[3j+1];
+// fac[3(jee+1)] = A_2, fac[3(jee+1)+1] = C_{jee-1}.
+__global__ void __launch_bounds__(256) k_dt(DCoef c, DState *st, const unsigned long long *vm_bits, ImplzyTab tu,
+                                            ImplzyTab tv, double *fac_u, double *fac_v, int m, int setstep, int dt_mode, double dt_fixed) {
+  extern __shared__ double dsm[];
+  __shared__ double s_dt3[8], s_vmax[8], s_rkk;
+  const int t = threadIdx.x, lane = t & 31, wid = t >> 5, N1 = c.ny + 1;
   const double *S = c.S;
   const double poco = 1e-7;
   if (setstep) {
     double dt3 = DBL_MAX, vmax = 0.0;
-    for (int j = t + 1; j <= c.ny; j += 64) {
+    for (int j = t + 1; j <= c.ny; j += 256) {
       const double vm = __longlong_as_double((long long)vm_bits[j]);
       dt3 = fmin(dt3, c.dymin[j - 1] / fmax(poco, vm));
       vmax = nmax(vmax, vm);
@@ -508,8 +499,11 @@ __global__ void __launch_bounds__(64) k_dt(DCoef c, DState *st, const unsigned l
       const double wm = __longlong_as_double((long long)st->wmax_bits);
       const double dt1 = S[OTBL_S_DXMIN] / fmax(poco, um);
       const double dt2 = S[OTBL_S_DXMIN] / fmax(poco, wm);
-      const double dt3 = fmin(s_dt3[0], s_dt3[1]);
-      const double vmax = nmax(s_vmax[0], s_vmax[1]);
+      double dt3 = s_dt3[0], vmax = s_vmax[0];
+      for (int q = 1; q < 8; ++q) {
+        dt3 = fmin(dt3, s_dt3[q]);
+        vmax = nmax(vmax, s_vmax[q]);
+      }
       const double dtloc = fmin(fmin(dt1, dt2), fmin(dt3, S[OTBL_S_DTRET]));
       st->umax = um;
       st->wmax = wm;
@@ -529,16 +523,88 @@ __global__ void __launch_bounds__(64) k_dt(DCoef c, DState *st, const unsigned l
     st->var2 = dt * S[OTBL_S_REX] * S[OTBL_S_RKCV + q];
     st->var3 = dt * S[OTBL_S_RKC + q];
     st->var4 = dt * S[OTBL_S_RKD + q];
-    st->rkk = S[OTBL_S_REX] * dt * S[OTBL_S_RKDV + q];
+    s_rkk = S[OTBL_S_REX] * dt * S[OTBL_S_RKDV + q];
+    st->rkk = s_rkk;
     st->varstep = 5e-1 / dt / S[OTBL_S_RKDV + q];
   }
   __syncthreads();
-  if (lane == 0) {
-    const double rkk = *(volatile double *)&st->rkk;
-    if (wid == 0)
-      implzy_factor(c, fac_u, 0, rkk);
-    else
-      implzy_factor(c, fac_v, 1, rkk);
+  const double rkk = s_rkk;
+  double *bs = dsm, *ac = bs + 2 * N1, *num = ac + 2 * N1, *den = num + 2 * N1;
+  for (int e = t; e < 2 * N1; e += 256) {
+    const int which = e / N1, r = e - which * N1, jee = which == 0 ? N1 : N1 - 1;
+    if (r < 1 || r > jee - 2) continue;
+    const ImplzyRow w = implzy_row(c, which, r, rkk);
+    bs[e] = w.B;
+    ac[e] = r > 1 ? w.A * implzy_row(c, which, r - 1, rkk).C : 0.0;
+  }
+  __syncthreads();
+  double *top = den + 2 * N1;  // 1 / B' of the top-down elimination
+  if (lane == 0 && wid < (fac_u ? 4 : 2)) {
+    const int which = wid & 1, o = which * N1, n = (which == 0 ? N1 : N1 - 1) - 2;
+    double t1 = 1.0, t2 = 0.0;  // the continuants of the two rows before
+    for (int i = 1; i <= n; ++i) {
+      const int r = wid < 2 ? i : n + 1 - i;
+      const double t0 = bs[o + r] * t1 - (wid < 2 ? ac[o + r] : (i > 1 ? ac[o + r + 1] : 0.0)) * t2;
+      if (wid < 2) {
+        num[o + r] = t0;
+        den[o + r] = t1;
+      } else {
+        top[o + r] = t1;
+        top[2 * N1 + o + r] = t0;
+      }
+      t2 = t1;
+      t1 = t0;
+      if (fabs(t1) > 0x1p300) {
+        t1 *= 0x1p-300;
+        t2 *= 0x1p-300;
+      } else if (fabs(t1) < 0x1p-300) {
+        t1 *= 0x1p300;
+        t2 *= 0x1p300;
+      }
+    }
+  }
+  __syncthreads();
+  for (int e = t; e < 2 * N1; e += 256) {
+    const int which = e / N1, r = e - which * N1, jee = which == 0 ? N1 : N1 - 1;
+    if (r >= jee) continue;
+    const ImplzyTab &tb = which == 0 ? tu : tv;
+    double l = 0.0, d = 1.0, u = 0.0;
+    if (r >= 1 && r <= jee - 2) {
+      const ImplzyRow w = implzy_row(c, which, r, rkk);
+      d = den[e] / num[e];
+      if (r > 1) l = -w.A * (den[e - 1] / num[e - 1]);
+      if (r < jee - 2) u = -w.C * d;
+      if (fac_u) {
+        double *fac = which == 0 ? fac_u : fac_v;
+        const double *tp = top + e;
+        fac[3 * (r + 1)] = r == 1 ? 0.0 : w.A;
+        fac[3 * (r + 1) + 1] = tp[0] / tp[2 * N1];
+        fac[3 * (r + 1) + 2] = r == jee - 2 ? 0.0 : -w.C * (tp[1] / tp[2 * N1 + 1]);
+        if (r == 1) fac[3 * (jee + 1)] = w.A;
+        if (r == jee - 2) fac[3 * (jee + 1) + 1] = w.C;
+      }
+      if (r == 1) tb.P[2 * tb.C] = w.A;
+      if (r == jee - 2) tb.P[2 * tb.C + 1] = w.C;
+    }
+    bs[e] = l;  // free since the chain
+    ac[e] = u;
+    double *row = tb.lde + (size_t)(r / tb.K) * tb.S + r % tb.K;
+    row[0] = l;
+    row[tb.K] = d;
+    row[2 * tb.K] = u;
+  }
+  __syncthreads();
+  for (int e = t; e < 2 * N1; e += 256) {  // chunk products
+    const int which = e / N1, q = e - which * N1, jee = which == 0 ? N1 : N1 - 1;
+    const ImplzyTab &tb = which == 0 ? tu : tv;
+    if (q * tb.K >= jee) continue;
+    double p = 1.0, x = 1.0;
+    for (int r = q * tb.K; r < min((q + 1) * tb.K, jee); ++r) {
+      p *= bs[which * N1 + r];
+      x *= ac[which * N1 + r];
+    }
+    tb.P[q] = p;
+    tb.P[tb.C + q] = x;
   }
 }
 
@@ -872,13 +938,18 @@ __global__ void __launch_bounds__(128) k_genflu_cols(DCoef c, GenArgs a) {
   out[(size_t)r * nz1] = v;
 }
 
-cudaError_t genflu_launch(otbl_ctx *c, const GenArgs &a) {
+cudaError_t genflu_tab_launch(otbl_ctx *c, const GenArgs &a) {
   const size_t smem = genflu_smem_bytes(c->cfg.ny);
   if (smem > 48 * 1024) cudaFuncSetAttribute(k_genflu_tab, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   k_genflu_tab<<<1, 256, smem, c->stream>>>(c->dc, a);
+  c->launches += 1;
+  return cudaGetLastError();
+}
+
+cudaError_t genflu_cols_launch(otbl_ctx *c, const GenArgs &a) {
   dim3 g((c->dc.nz1 + 127) / 128, 3, c->cfg.ny + 1);
   k_genflu_cols<<<g, 128, 0, c->stream>>>(c->dc, a);
-  c->launches += 2;
+  c->launches += 1;
   return cudaGetLastError();
 }
 
@@ -1646,16 +1717,20 @@ cudaError_t launch_products(otbl_ctx *c, int setstep, int part) {
 
 cudaError_t launch_dt(otbl_ctx *c, int m, int setstep) {
   prof_begin(c, PK_DT);
-  k_dt<<<1, 64, 0, c->stream>>>(c->dc, c->st, c->w.vm_bits, c->w.fac_u, c->w.fac_v, m, setstep,
-                                c->cfg.dt_mode, c->cfg.dt_fixed);
+  const bool st = stream_tail(c);
+  const size_t smem = (size_t)(st ? 12 : 8) * (c->cfg.ny + 1) * sizeof(double);
+  if (smem > 40 * 1024) cudaFuncSetAttribute(k_dt, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  k_dt<<<1, 256, smem, c->stream>>>(c->dc, c->st, c->w.vm_bits, implzy_tab(c, 0), implzy_tab(c, 1),
+                                    st ? c->w.fac_u : nullptr, st ? c->w.fac_v : nullptr, m, setstep,
+                                    c->cfg.dt_mode, c->cfg.dt_fixed);
   c->launches += 1;
   cudaError_t e = cudaGetLastError();
-  if (e == cudaSuccess) e = launch_tail_rows(c);
+  if (e == cudaSuccess && st) e = launch_tail_rows(c);
   prof_end(c);
   return e;
 }
 
-cudaError_t launch_genflu(otbl_ctx *c, int tail) {
+static GenArgs genflu_args(otbl_ctx *c, int tail) {
   GenArgs a;
   a.u = c->f[OTBL_F_U];
   a.v = c->f[OTBL_F_V];
@@ -1681,8 +1756,19 @@ cudaError_t launch_genflu(otbl_ctx *c, int tail) {
   a.err = &st->err;
   a.err_code = OTBL_DEVERR_GENFLU_GRID;
   a.tail = tail;
+  return a;
+}
+
+cudaError_t launch_genflu_tab(otbl_ctx *c, int tail) {
   prof_begin(c, PK_GENFLU);
-  const cudaError_t e = genflu_launch(c, a);
+  const cudaError_t e = genflu_tab_launch(c, genflu_args(c, tail));
+  prof_end(c);
+  return e;
+}
+
+cudaError_t launch_genflu_cols(otbl_ctx *c, int tail) {
+  prof_begin(c, PK_GENFLU);
+  const cudaError_t e = genflu_cols_launch(c, genflu_args(c, tail));
   prof_end(c);
   return e;
 }
@@ -1749,7 +1835,8 @@ cudaError_t launch_genflu_noalloc(otbl_ctx *c, double *wk, double *u, double *v,
   a.err = err;
   a.err_code = OTBL_ERR_NAN;
   a.tail = 0;
-  return genflu_launch(c, a);
+  const cudaError_t e = genflu_tab_launch(c, a);
+  return e == cudaSuccess ? genflu_cols_launch(c, a) : e;
 }
 
 cudaError_t launch_outflow(otbl_ctx *c) {
@@ -1793,7 +1880,7 @@ bool build_pois_maps(otbl_ctx *c) {
 
 // SMs of the current device (the persistent x-DCT grids; any grid size is
 // correct, the count only spreads the tiles), cached per device ordinal
-static int sm_count() {
+int sm_count() {
   constexpr int kDevs = 64;
   static int nsm[kDevs] = {0};  // the same value if two host threads race
   int dev = 0;

@@ -243,12 +243,10 @@ extern "C" int otbl_ctx_create(const otbl_config *cfg, const double *coef, int d
       *b = q;
     }
   }
-  // s1 holds the line kernels' checkpoints; the rhsp tail's, at segments of
-  // 2 rows, take 2*ceil((ny+1)/2) <= ny+2 rows of (nx-1)*nz1 columns
-  TRY(dalloc(c, &w.s1, std::max(lu, (size_t)(ny + 2) * (nx - 1) * nz1)));
+  TRY(dalloc(c, &w.s1, lu));
   TRY(dalloc(c, &w.s2, lu));
   TRY(dalloc(c, &w.s3, lu));
-  TRY(dalloc(c, &w.t1, std::max(lu, (size_t)(ny + 2) * (nx - 1) * nz1)));
+  TRY(dalloc(c, &w.t1, lu));
   TRY(dalloc(c, &w.t2, lu));
   TRY(dalloc(c, &w.t3, lu));
   const int M = nz / 2, n = nx - 1;
@@ -265,24 +263,26 @@ extern "C" int otbl_ctx_create(const otbl_config *cfg, const double *coef, int d
     TRY(dalloc(c, &w.twx2f, 2 * (size_t)n));
   }
   TRY(dalloc(c, &w.vm_bits, (size_t)ny + 1));
-  TRY(dalloc(c, &w.fac_u, 3 * (size_t)(ny + 4)));
-  TRY(dalloc(c, &w.fac_v, 3 * (size_t)(ny + 4)));
-  TRY(dalloc(c, &w.rowc, 2 * 16 * (size_t)(ny + 2)));
   {
-    double *q = nullptr;
-    TRY(dalloc(c, &q, 4 * 16 * (size_t)nx));
-    w.xrowc = q;
-    TRY(dalloc(c, &q, 2 * 8 * (size_t)ny));
-    w.yrowc = q;
+    char *xt = nullptr;
+    TRY(dalloc(c, &xt, xline_table_bytes(nx, c->mixed)));
+    w.xtab = xt;
+    TRY(dalloc(c, &xt, 64 * (size_t)nx * (c->mixed ? sizeof(float) : sizeof(double))));
+    w.xrowc = xt;
+    TRY(dalloc(c, &xt, ytab_bytes(ny, c->mixed)));
+    w.ytab = xt;
+    TRY(dalloc(c, &w.tdtab, tdtab_doubles(ny)));
+    TRY(dalloc(c, &w.yrowc, 16 * (size_t)ny));
+    TRY(dalloc(c, &w.rowc, 32 * (size_t)(ny + 2)));
+    TRY(dalloc(c, &w.fac_u, 3 * (size_t)(ny + 4)));
+    TRY(dalloc(c, &w.fac_v, 3 * (size_t)(ny + 4)));
   }
   TRY(dalloc(c, &w.gf, genflu_tab_doubles(ny)));
   TRY(dalloc(c, &w.pois_dinv, (size_t)nx * ny * (nz1 / 2)));
   if (c->mixed) TRY(dalloc(c, &w.pois_dinvf, (size_t)nx * ny * (nz1 / 2)));
 #undef TRY
   if (!getenv("OTBL_NO_TMA")) {
-    build_final_maps(c);
-    build_x_maps(c);
-    build_y_maps(c);
+    build_stream_maps(c);
     build_pois_maps(c);
   }
   c->ydense = (cfg->options & OTBL_OPT_YDENSE) != 0;
@@ -292,7 +292,7 @@ extern "C" int otbl_ctx_create(const otbl_config *cfg, const double *coef, int d
   }
   if (c->ydense && !getenv("OTBL_NO_TMA")) build_ydense_maps(c);
   if (check(c, launch_twiddles(c), "twiddles") != OTBL_OK || check(c, launch_pois_lu(c), "pois_lu") != OTBL_OK ||
-      check(c, launch_x_rows(c), "x rows") != OTBL_OK || check(c, launch_y_rows(c), "y rows") != OTBL_OK ||
+      check(c, prepare_xlines(c), "x-line tables") != OTBL_OK || check(c, prepare_ylines(c), "y-line tables") != OTBL_OK || check(c, prepare_stream(c), "ring rows") != OTBL_OK ||
       check(c, cudaStreamSynchronize(c->stream), "init")) {
     *out = c;
     return OTBL_ERR_CUDA;
@@ -312,12 +312,14 @@ extern "C" size_t otbl_ctx_bytes(const otbl_config *cfg) {
   b += (2 * lu + lv) * sizeof(double) + (2 * lu + 2 * lv) * (mixed ? sizeof(float) : sizeof(double));  // state
   b += 3 * (size_t)(ny + 1) * sizeof(double) + sizeof(DState);   // u0, v0, um, scalars
   b += 15 * lu * (mixed ? sizeof(float) : sizeof(double));       // intermediates
-  b += 2 * (std::max(lu, (size_t)(ny + 2) * (nx - 1) * nz1) + 2 * lu) * sizeof(double);  // s1..s3, t1..t3
+  b += 6 * lu * sizeof(double);  // s1..s3, t1..t3
   b += (4 * (size_t)M + 4 * (size_t)n) * sizeof(double) + (mixed ? (4 * (size_t)M + 4 * (size_t)n) * sizeof(float) : 0);
-  b += (size_t)(ny + 1) * 8 + 6 * (size_t)(ny + 4) * sizeof(double) + genflu_tab_doubles(ny) * sizeof(double);
+  b += (size_t)(ny + 1) * 8 + genflu_tab_doubles(ny) * sizeof(double);
   b += (size_t)nx * ny * (nz1 / 2) * (sizeof(double) + (mixed ? sizeof(float) : 0));  // Poisson pivots
   if (cfg->options & OTBL_OPT_YDENSE) b += ydense_bytes(ny);     // dense interpyy operators
-  b += (2 * 16 * (size_t)(ny + 2) + 4 * 16 * (size_t)nx + 2 * 8 * (size_t)ny) * sizeof(double);  // coefficient rows
+  b += xline_table_bytes(nx, mixed) + ytab_bytes(ny, mixed) + tdtab_doubles(ny) * sizeof(double);  // coefficient tables
+  b += 64 * (size_t)nx * (mixed ? sizeof(float) : sizeof(double));                 // streamed kernels' rows, factors
+  b += (16 * (size_t)ny + 32 * (size_t)(ny + 2) + 6 * (size_t)(ny + 4)) * sizeof(double);
   return b;
 }
 
@@ -348,8 +350,9 @@ extern "C" int otbl_ctx_rebind(otbl_ctx *c, const otbl_config *cfg, const double
   }
   if (check(c, launch_pois_lu(c), "pois_lu") != OTBL_OK) return OTBL_ERR_CUDA;
   if (c->ydense && check(c, ydense_prepare(c), "dense interpyy operator") != OTBL_OK) return OTBL_ERR_CUDA;
-  if (check(c, launch_x_rows(c), "x rows") != OTBL_OK) return OTBL_ERR_CUDA;
-  if (check(c, launch_y_rows(c), "y rows") != OTBL_OK) return OTBL_ERR_CUDA;
+  if (check(c, prepare_xlines(c), "x-line tables") != OTBL_OK) return OTBL_ERR_CUDA;
+  if (check(c, prepare_ylines(c), "y-line tables") != OTBL_OK) return OTBL_ERR_CUDA;
+  if (check(c, prepare_stream(c), "ring rows") != OTBL_OK) return OTBL_ERR_CUDA;
   OTBL_CUDA_TRY(c, cudaStreamSynchronize(c->stream));
   return OTBL_OK;
 }
@@ -535,32 +538,27 @@ static int rhsp_issue(otbl_ctx *c, int m, int setstep) {
   cudaError_t e = cudaSuccess;
   // Streams (all forks and joins by events, so a graph capture records them):
   //   main:    interpxx, products 0 (uu, uw), [interpyy] products 2 (uv),
-  //            difvisxx, [k_dt] u tail ([genflu] before its velocity write),
-  //            [products 1] v tail, [w tail]
-  //   side:    interpyy, [products 0, 2] k_dt, [difvisxx] genflu,
-  //            [products 1] w tail on its own line scratch
+  //            difvisxx, [genflu] u tail, [products 1] v and w tails
+  //   side:    interpyy, [products 2] k_dt, genflu's tables, [difvisxx]
+  //            genflu's plane 1
   //   side_lo: [products 2] products 1 (vw, vv, ww)
-  // interpyy and interpxx only read the state (their checkpoints take the
-  // head and the tail of the line scratch); each products part reads and
-  // writes fields no kernel beside it touches; difvisxx reads parts 0 and
-  // 2; k_dt needs the CFL maxima of parts 0 and 2; genflu needs dt, writes
-  // plane 1 of u, v, w after difvisxx has read it and reads plane xout
-  // before a tail rewrites it.
-  const bool ypar = interpy_ck_tail(c, c->w.s2) != nullptr;
-  if (ypar) {
-    OTBL_CUDA_TRY(c, cudaEventRecord(c->ev[0], main_s));
-    OTBL_CUDA_TRY(c, cudaStreamWaitEvent(side, c->ev[0], 0));
-    c->stream = side;
-    e = launch_interpy(c);
-    if (e == cudaSuccess) e = cudaEventRecord(c->ev[1], side);
-    c->stream = main_s;
-    if (check(c, e, "launch_interpy") != OTBL_OK) return OTBL_ERR_CUDA;
-    LAUNCH(c, launch_interpx(c));
-  } else {
-    LAUNCH(c, launch_interpx(c));
-    LAUNCH(c, launch_interpy(c));
-    OTBL_CUDA_TRY(c, cudaEventRecord(c->ev[1], main_s));
-  }
+  // With the streamed tail (the largest boxes): main: [k_dt] u tail ([genflu]
+  // before its velocity write), [products 1] v tail, [w tail]; side: [products
+  // 1] w tail on line scratch of its own.
+  // interpyy and interpxx only read the state; each products part reads and
+  // writes fields no kernel beside it touches; difvisxx reads parts 0 and 2;
+  // k_dt needs the CFL maxima of parts 0 and 2; genflu needs dt, writes plane
+  // 1 of u, v, w after difvisxx has read it and reads plane xout before the
+  // tails rewrite it.
+  const bool st = stream_tail(c);
+  OTBL_CUDA_TRY(c, cudaEventRecord(c->ev[0], main_s));
+  OTBL_CUDA_TRY(c, cudaStreamWaitEvent(side, c->ev[0], 0));
+  c->stream = side;
+  e = launch_interpy(c);
+  if (e == cudaSuccess) e = cudaEventRecord(c->ev[1], side);
+  c->stream = main_s;
+  if (check(c, e, "launch_interpy") != OTBL_OK) return OTBL_ERR_CUDA;
+  LAUNCH(c, launch_interpx(c));
   LAUNCH(c, launch_products(c, setstep, 0));
   OTBL_CUDA_TRY(c, cudaStreamWaitEvent(main_s, c->ev[1], 0));
   LAUNCH(c, launch_products(c, setstep, 2));
@@ -576,28 +574,36 @@ static int rhsp_issue(otbl_ctx *c, int m, int setstep) {
   OTBL_CUDA_TRY(c, cudaStreamWaitEvent(side, c->ev[0], 0));
   c->stream = side;
   e = launch_dt(c, m, setstep);
-  if (e == cudaSuccess) e = cudaEventRecord(c->ev[1], side);
+  if (e == cudaSuccess && st) e = cudaEventRecord(c->ev[1], side);
+  if (e == cudaSuccess) e = launch_genflu_tab(c, 1);
   c->stream = main_s;
   if (check(c, e, "k_dt") != OTBL_OK) return OTBL_ERR_CUDA;
   LAUNCH(c, launch_difvisx(c));
   OTBL_CUDA_TRY(c, cudaEventRecord(c->ev[2], main_s));
   OTBL_CUDA_TRY(c, cudaStreamWaitEvent(side, c->ev[2], 0));
   c->stream = side;
-  e = launch_genflu(c, 1);
+  e = launch_genflu_cols(c, 1);
   if (e == cudaSuccess) e = cudaEventRecord(c->ev[3], side);
   c->stream = main_s;
   if (check(c, e, "launch_genflu") != OTBL_OK) return OTBL_ERR_CUDA;
-  OTBL_CUDA_TRY(c, cudaStreamWaitEvent(main_s, c->ev[1], 0));
-  LAUNCH(c, launch_final(c, 1, c->ev[3]));
-  OTBL_CUDA_TRY(c, cudaStreamWaitEvent(side, c->ev[4], 0));
-  c->stream = side;
-  e = launch_final(c, 4, nullptr, true);
-  if (e == cudaSuccess) e = cudaEventRecord(c->ev[5], side);
-  c->stream = main_s;
-  if (check(c, e, "w tail") != OTBL_OK) return OTBL_ERR_CUDA;
+  if (st) {
+    OTBL_CUDA_TRY(c, cudaStreamWaitEvent(main_s, c->ev[1], 0));
+    LAUNCH(c, launch_final_stream(c, 1, c->ev[3]));
+    OTBL_CUDA_TRY(c, cudaStreamWaitEvent(side, c->ev[4], 0));
+    c->stream = side;
+    e = launch_final_stream(c, 4, nullptr, true);
+    if (e == cudaSuccess) e = cudaEventRecord(c->ev[5], side);
+    c->stream = main_s;
+    if (check(c, e, "w tail") != OTBL_OK) return OTBL_ERR_CUDA;
+    OTBL_CUDA_TRY(c, cudaStreamWaitEvent(main_s, c->ev[4], 0));
+    LAUNCH(c, launch_final_stream(c, 2));
+    OTBL_CUDA_TRY(c, cudaStreamWaitEvent(main_s, c->ev[5], 0));
+    return OTBL_OK;
+  }
+  OTBL_CUDA_TRY(c, cudaStreamWaitEvent(main_s, c->ev[3], 0));
+  LAUNCH(c, launch_final(c, 1));
   OTBL_CUDA_TRY(c, cudaStreamWaitEvent(main_s, c->ev[4], 0));
-  LAUNCH(c, launch_final(c, 2));
-  OTBL_CUDA_TRY(c, cudaStreamWaitEvent(main_s, c->ev[5], 0));
+  LAUNCH(c, launch_final(c, 2 | 4));
   return OTBL_OK;
 }
 
@@ -666,9 +672,7 @@ static int bind_fields(otbl_ctx *c, double *const *ptr, const bool *use) {
   for (int id = 0; id < OTBL_F_COUNT; ++id)
     if (use[id]) c->f[id] = ptr[id] ? ptr[id] : c->f_own[id];
   if (!getenv("OTBL_NO_TMA")) {
-    build_final_maps(c);
-    build_x_maps(c);
-    build_y_maps(c);
+    build_stream_maps(c);
     build_ydense_maps(c);
     build_pois_maps(c);
   }
@@ -820,7 +824,8 @@ extern "C" int otbl_boun(otbl_ctx *c) {
 extern "C" int otbl_genflu(otbl_ctx *c) {
   if (!c) return OTBL_ERR_ARG;
   cudaSetDevice(c->device);
-  LAUNCH(c, launch_genflu(c, 0));
+  LAUNCH(c, launch_genflu_tab(c, 0));
+  LAUNCH(c, launch_genflu_cols(c, 0));
   return OTBL_OK;
 }
 

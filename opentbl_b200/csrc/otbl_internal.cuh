@@ -56,40 +56,47 @@ struct Work {
   void *uy, *wy, *vy;          // interpyy outputs (ny rows each)
   void *uu, *uw, *uv, *vw, *vv, *ww;  // products (uu, uw u-type; others ny rows)
   void *cu, *cv, *cw;          // difvisxx outputs
-  double *s1, *s2, *s3;        // line-solve scratch and pois' phi (u-type size)
-  double *t1, *t2, *t3;        // the w tail's scratch (beside the v tail), as s1..s3
+  double *s1, *s2, *s3;        // pois' phi (s2, s3), streamed lines' and statistics' scratch (u-type size)
+  double *t1, *t2, *t3;        // the streamed w tail's and the statistics' scratch, as s1..s3
   double *twz, *twz2;          // z-FFT twiddles exp(-2 pi i t/M), exp(-2 pi i t/nz)
   float *twzf, *twz2f;         // the same rounded to FP32 (mixed path)
   double *twx;                 // x-DCT twiddles for the length nx-1 FFT
   double *twx2;                // exp(-i pi k/(2n)), k = 0..n-1
   float *twxf, *twx2f;         // the same rounded to FP32 (mixed path)
   unsigned long long *vm_bits; // vm(j) maxima, j = 1..ny
-  double *fac_u, *fac_v;       // implzy LU factors for the current dt (3*(ny+1))
-  double *rowc;                // k_final_tb's per-row coefficients, [2][ny+2][16]
-  void *xrowc;                 // k_xline_t's per-plane coefficients, [2][2][nx][16] (T)
-  void *yrowc;                 // k_interpy_t's per-row coefficients, [2][ny][8] (T)
+  void *xtab;                  // k_xline's coefficient tables (T): interpxx u, v, difvisxx u, v
+  // streamed kernels of the largest boxes (k_stream.cu): per-plane and per-row
+  // coefficients of their rings, implzy's top-down factors
+  void *xrowc;                 // [2][2][nx][16] (T)
+  double *yrowc, *rowc;        // [2][ny][8], [2][ny+2][16]
+  double *fac_u, *fac_v;
+  void *ytab;                  // k_interpy's and k_tail's coefficient tables (T)
+  double *tdtab;               // implzy's tables (k_tail), its factors for the current dt
   double *gf;                  // genflu tables (genflu_tab_doubles)
   double *pois_dinv;           // pivots of the (x-mode, kz) y-systems, [i][j][k]
   float *pois_dinvf;           // the same rounded to FP32 (mixed path, modes >= kPoisLow)
 };
 
-// TMA descriptors (opaque 128-byte CUtensorMap objects) of the fields the
-// rhsp tail's descending pass reads, for one velocity component (k_final_tb)
-struct FinalMaps {
-  CUtensorMap prod, kp, vel, cx, hp, p;
-  CUtensorMap prod_a, vel_a;  // pass A: boxes of 8 + 2 rows
-  CUtensorMap rc, rc_a;       // per-row coefficients (Work::rowc), KF / 8 rows
+// where k_dt writes implzy's factors of one velocity type: l, d, e (row r at
+// lde[(r / K) S + i K + r mod K], i = 0, 1, 2), the products P, Q of the C
+// chunks and the two boundary couplings
+struct ImplzyTab {
+  double *lde, *P;
+  int K, S, C;
 };
 
-// TMA descriptors of interpyy's inputs (u, w, v), boxes of 128 kr x rows,
-// and the per-row coefficient rows of each field's operator (Work::yrowc)
+// TMA descriptors of the streamed kernels (k_stream.cu): the tail's fields of
+// one velocity component (pass A: boxes of 8 + 2 rows), interpyy's inputs (u,
+// w, v), the x-lines' inputs per field (u, v, w; 2D tensors [plane][line]), and
+// the coefficient rows of each
+struct FinalMaps {
+  CUtensorMap prod, kp, vel, cx, hp, p;
+  CUtensorMap prod_a, vel_a;
+  CUtensorMap rc, rc_a;
+};
 struct YMaps {
   CUtensorMap g[3], r[3];
 };
-
-// TMA descriptors of the x-line kernels' inputs, per field (u, v, w): 2D
-// tensors [plane][line] with boxes of 32 lines, and the per-plane
-// coefficient rows of the field's operator (Work::xrowc)
 struct XMaps {
   CUtensorMap g[3], u[3], r[3];
 };
@@ -124,8 +131,8 @@ struct otbl_ctx {
   otbl::DCoef dc;
   otbl::DCoefT<float> dcf;  // FP32 coefficients (mixed path)
   // threads per CTA of the line kernels that otbl_autotune times:
-  // [0] k_interpx, [1] k_difvisx, [2] k_interpy (one thread per line, so the
-  // choice changes the schedule, never the arithmetic)
+  // [0] interpxx, [1] difvisxx (half the CTA's threads), [2] k_interpy; the
+  // choice changes the schedule, never the arithmetic
   int tune_bs[3] = {128, 128, 128};
   int pois_klo = 0;  // mixed path: spanwise modes k < pois_klo solve in FP64 (kPoisCond)
   // interpyy of the mixed path as a dense operator on the tensor cores
@@ -143,13 +150,10 @@ struct otbl_ctx {
   // allocated by the first otbl_statsp, and the number of samples in them
   double *stats = nullptr;
   int stats_samples = 0;
-  // TMA descriptors of the rhsp tail's inputs, per velocity component
-  otbl::FinalMaps fmaps[3];
-  bool fmaps_ok = false;
-  otbl::XMaps xmi, xmd;  // k_interpx_t (state), k_difvisx_t (products, state)
-  bool xmaps_ok = false;
-  otbl::YMaps ymi;       // k_interpy_t
-  bool ymaps_ok = false;
+  otbl::FinalMaps fmaps[3];  // k_stream.cu
+  otbl::XMaps xmi, xmd;
+  otbl::YMaps ymi;
+  bool fmaps_ok = false, xmaps_ok = false, ymaps_ok = false;
   otbl::PoisMaps pmaps;  // k_pois_fwd_t / k_pois_bwd_t
   bool pmaps_vel = false, pmaps_phi64 = false, pmaps_phi32 = false;
   int mixed;                // cfg.precision == OTBL_PREC_MIXED
@@ -219,41 +223,48 @@ namespace otbl {
 // kernel launch wrappers (kernels.cu); each returns cudaGetLastError()
 cudaError_t launch_interpx(otbl_ctx *c);
 cudaError_t launch_interpy(otbl_ctx *c);
-// interpyy's checkpoint region in a line scratch when it can run beside
-// interpxx, else nullptr
-double *interpy_ck_tail(otbl_ctx *c, double *s);
 // part 0: uu, uw and the u, w CFL maxima; part 2: uv and the v maxima;
 // part 1: vw, vv, ww
 cudaError_t launch_products(otbl_ctx *c, int setstep, int part);
 cudaError_t launch_difvisx(otbl_ctx *c);
 cudaError_t launch_dt(otbl_ctx *c, int m, int setstep);
-cudaError_t launch_genflu(otbl_ctx *c, int tail);
+// genflu's two kernels: the tables (needs dt, reads plane xout) and the new
+// plane 1
+cudaError_t launch_genflu_tab(otbl_ctx *c, int tail);
+cudaError_t launch_genflu_cols(otbl_ctx *c, int tail);
 // the rhsp tail of the velocity components in the bit mask comps (1 u, 2 v,
-// 4 w), in that order, on line scratch s1..s3 (second_scratch: t1..t3); the
-// first kernel that writes a velocity component waits for before_vel when
-// it is not null
-cudaError_t launch_final(otbl_ctx *c, unsigned comps, cudaEvent_t before_vel = nullptr,
-                         bool second_scratch = false);
+// 4 w), one launch
+cudaError_t launch_final(otbl_ctx *c, unsigned comps);
+// the streamed forms for the largest boxes (k_stream.cu) and where they are
+// the faster ones; the streamed tail works on line scratch s1..s3
+// (second_scratch: t1..t3), needs launch_tail_rows after k_dt, and its first
+// velocity write waits for before_vel when it is not null
+bool stream_xlines(const otbl_ctx *c, bool dv);
+bool stream_interpy(const otbl_ctx *c);
+bool stream_tail(const otbl_ctx *c);
+cudaError_t launch_xlines_stream(otbl_ctx *c, bool dv);
+cudaError_t launch_interpy_stream(otbl_ctx *c);
+cudaError_t launch_tail_rows(otbl_ctx *c);
+cudaError_t launch_final_stream(otbl_ctx *c, unsigned comps, cudaEvent_t before_vel = nullptr,
+                                bool second_scratch = false);
+void build_stream_maps(otbl_ctx *c);
+cudaError_t prepare_stream(otbl_ctx *c);
 cudaError_t launch_outflow(otbl_ctx *c);
 cudaError_t launch_pois(otbl_ctx *c, int m);
 cudaError_t launch_reset_max(otbl_ctx *c);
 cudaError_t launch_boun_all(otbl_ctx *c);
 cudaError_t launch_tiempo(otbl_ctx *c);
 cudaError_t launch_energies(otbl_ctx *c);
-// builds c->fmaps (false if TMA cannot address the fields, e.g. an FP32 row
-// pitch that is not a multiple of 16 bytes)
-bool build_final_maps(otbl_ctx *c);
-// fills Work::rowc from the coefficients and this substep's implzy factors
-// (after k_dt, on the same stream); a no-op without the TMA-fed tail
-cudaError_t launch_tail_rows(otbl_ctx *c);
+int sm_count();  // SMs of the current device
 // the driver's cuTensorMapEncodeTiled (as void *), nullptr if unavailable
 void *tensor_map_encoder();
-bool build_x_maps(otbl_ctx *c);
-// fill Work::xrowc and Work::yrowc from the coefficients (at creation and on
-// new coefficients)
-cudaError_t launch_x_rows(otbl_ctx *c);
-cudaError_t launch_y_rows(otbl_ctx *c);
-bool build_y_maps(otbl_ctx *c);
+// fill the coefficient tables (at creation and on new coefficients)
+cudaError_t prepare_xlines(otbl_ctx *c);
+cudaError_t prepare_ylines(otbl_ctx *c);
+size_t xline_table_bytes(int nx, bool mixed);
+size_t ytab_bytes(int ny, bool mixed);
+size_t tdtab_doubles(int ny);
+ImplzyTab implzy_tab(otbl_ctx *c, int which);
 cudaError_t launch_twiddles(otbl_ctx *c);
 cudaError_t launch_pois_lu(otbl_ctx *c);
 // columns kr < kr_split solve in FP64 on phi64, the others in FP32 on phi32
