@@ -137,6 +137,37 @@ __device__ __forceinline__ void dft5(V *v) {
   v[3] = csub(r2, i2);
 }
 
+// 16 = 4 x 4: DFT4 over r, r + 4, r + 8, r + 12, twiddles W16^(r q), DFT4 over
+// r; output q + 4 p comes from v[4 q + p]
+template <int SIGN, typename V>
+__device__ __forceinline__ void dft16(V *v) {
+  using S = decltype(V{}.x);
+  const S c1 = S(0.92387953251128675613), s1 = S(0.38268343236508977173);  // cos, sin of pi/8
+  const S c2 = S(0.70710678118654752440);
+#pragma unroll
+  for (int r = 0; r < 4; ++r) dft4<SIGN>(v[r], v[r + 4], v[r + 8], v[r + 12]);
+  const V w1 = cmake<V>(c1, SIGN * s1), w2 = cmake<V>(c2, SIGN * c2), w3 = cmake<V>(s1, SIGN * c1);
+  v[5] = cmul(v[5], w1);
+  v[6] = cmul(v[6], w2);
+  v[7] = cmul(v[7], w3);
+  v[9] = cmul(v[9], w2);
+  v[10] = cmul_i(v[10], SIGN);
+  v[11] = cmul(v[11], cmake<V>(-c2, SIGN * c2));
+  v[13] = cmul(v[13], w3);
+  v[14] = cmul(v[14], cmake<V>(-c2, SIGN * c2));
+  v[15] = cmul(v[15], cmake<V>(-c1, -SIGN * s1));
+#pragma unroll
+  for (int q = 0; q < 4; ++q) dft4<SIGN>(v[4 * q], v[4 * q + 1], v[4 * q + 2], v[4 * q + 3]);
+#pragma unroll
+  for (int q = 0; q < 4; ++q)
+#pragma unroll
+    for (int p = q + 1; p < 4; ++p) {
+      const V x = v[4 * q + p];
+      v[4 * q + p] = v[4 * p + q];
+      v[4 * p + q] = x;
+    }
+}
+
 // In-register DFT of size R; SIGN = -1 forward (e^{-}), +1 backward (e^{+}).
 template <int R, int SIGN, typename V>
 __device__ __forceinline__ void dft_small(V *v) {
@@ -150,8 +181,10 @@ __device__ __forceinline__ void dft_small(V *v) {
     dft4<SIGN>(v[0], v[1], v[2], v[3]);
   } else if constexpr (R == 5) {
     dft5<SIGN>(v);
+  } else if constexpr (R == 16) {
+    dft16<SIGN>(v);
   } else {
-    static_assert(R == 8, "radix 2, 3, 4, 5 or 8");
+    static_assert(R == 8, "radix 2, 3, 4, 5, 8 or 16");
     dft8<SIGN>(v);
   }
 }

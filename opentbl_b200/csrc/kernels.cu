@@ -148,201 +148,6 @@ __global__ void __launch_bounds__(128) k_products(DCoef c, ZTabT<T> z, ProdArgs<
   }
 }
 
-// ---------------------------------------------------------------------------
-// k_products for M = nz/2 = 32..256 (nz = 64..512): the transforms and
-// products of k_products with each line kept in registers between the
-// inverse transform's last Stockham pass and the forward transform's first
-// one. Register layout L: lane t holds complex element n = t + 32 m in v[m],
-// m < E = M/32. Passes: radix E (Ns = 1; its butterflies' inputs j + 32 r are
-// one lane's registers; a copy for E = 1), radix 8 (Ns = E), radix 4 (Ns =
-// 8 E = M/4); the first reads L, the last writes L (for M < 128 through the
-// buffer, its outputs not being in layout L), the two in between go through
-// a per-warp shared buffer. M = 256: radices 8, 8, 4, warp_fft's order;
-// M = 128: 4, 8, 4, M = 64: 2, 8, 4, M = 32: 8, 4 (warp_fft's order would
-// need eight register inputs per butterfly). The buffer's element i is
-// stored at i + i/8 for 16-byte (FP64) elements and at i ^ ((i/8) mod 16)
-// for 8-byte (FP32) ones, which at M = 256 makes every exchange of the three
-// passes conflict-free for its element size (a bank model of the access
-// patterns: the FP32 buffer at i + i/8 needed 160 wavefronts per transform
-// where 96 is the minimum, and ncu showed 15 M of its 42 M shared wavefronts
-// as conflicts at 257x193x512; 0.4 M with the swizzle). The real-to-complex post-step takes the mirrored element
-// Z[M-k] from the lane that holds it by warp shuffles instead of a round
-// trip through the buffer. For M = 256 the arithmetic is warp_fft's,
-// operation for operation.
-// ---------------------------------------------------------------------------
-template <int M>
-struct ZPlan {
-  static_assert(M == 256 || M == 128 || M == 64 || M == 32, "register transforms for M = 32..256");
-  static constexpr int E = M / 32;
-  static constexpr int R3 = 4;  // M = E x 8 x 4
-};
-template <typename V>
-__device__ __forceinline__ int zpad(int i) {
-  if constexpr (sizeof(V) == 16)
-    return i + (i >> 3);
-  else
-    return i ^ ((i >> 3) & 15);
-}
-template <typename V>
-__device__ __forceinline__ V shfl_cx(V v, int src) {
-  V r;
-  r.x = __shfl_sync(0xffffffffu, v.x, src);
-  r.y = __shfl_sync(0xffffffffu, v.y, src);
-  return r;
-}
-
-// inverse (SIGN = +1) or forward (SIGN = -1) FFT of a line in layout L
-template <int M, int SIGN, typename V>
-__device__ __forceinline__ void zfft_regs(V (&L)[M / 32], V *buf, const V *__restrict__ tw, int t) {
-  constexpr int E = M / 32, R3 = ZPlan<M>::R3;
-  // pass A: radix E, Ns = 1, input from registers (inputs t + 32 r; a copy
-  // for E = 1)
-  {
-    V v[E];
-#pragma unroll
-    for (int r = 0; r < E; ++r) v[r] = L[r];
-    if constexpr (E > 1) dft_small<E, SIGN>(v);
-#pragma unroll
-    for (int r = 0; r < E; ++r) buf[zpad<V>(t * E + r)] = v[r];
-  }
-  __syncwarp();
-  // pass B: radix 8, Ns = E (M / 8 butterflies: IB per lane, or the first
-  // M / 8 lanes)
-  {
-    constexpr int NB = M / 8, IB = (NB + 31) / 32;
-    V v[IB][8];
-#pragma unroll
-    for (int it = 0; it < IB; ++it) {
-      const int j = t + 32 * it;
-      if (j < NB) {
-#pragma unroll
-        for (int r = 0; r < 8; ++r) v[it][r] = buf[zpad<V>(j + r * NB)];
-      }
-    }
-    __syncwarp();
-#pragma unroll
-    for (int it = 0; it < IB; ++it) {
-      const int j = t + 32 * it, k = j % E;
-      if (j < NB) {
-        if constexpr (E > 1) {  // Ns = 1 has no twiddles
-#pragma unroll
-          for (int r = 1; r < 8; ++r) {
-            V w = __ldg(&tw[r * k * (M / (8 * E))]);
-            if (SIGN > 0) w.y = -w.y;
-            v[it][r] = cmul(v[it][r], w);
-          }
-        }
-        dft_small<8, SIGN>(v[it]);
-        const int base = (j / E) * (8 * E) + k;
-#pragma unroll
-        for (int r = 0; r < 8; ++r) buf[zpad<V>(base + r * E)] = v[it][r];
-      }
-    }
-  }
-  __syncwarp();
-  // pass C: radix R3, Ns = M / R3, output to registers (for M < 128, whose
-  // outputs j + r M/R3 are not in layout L, through the buffer)
-  {
-    constexpr int NC = M / R3, IC = (NC + 31) / 32;
-    V v[IC][R3];
-#pragma unroll
-    for (int it = 0; it < IC; ++it) {
-      const int j = t + 32 * it;
-      if (j < NC) {
-#pragma unroll
-        for (int r = 0; r < R3; ++r) v[it][r] = buf[zpad<V>(j + r * NC)];
-      }
-    }
-    __syncwarp();
-#pragma unroll
-    for (int it = 0; it < IC; ++it) {
-      const int j = t + 32 * it;  // k = j mod (M / R3) = j, twiddle stride M/(Ns R3) = 1
-      if (j < NC) {
-#pragma unroll
-        for (int r = 1; r < R3; ++r) {
-          V w = __ldg(&tw[r * j]);
-          if (SIGN > 0) w.y = -w.y;
-          v[it][r] = cmul(v[it][r], w);
-        }
-        dft_small<R3, SIGN>(v[it]);
-#pragma unroll
-        for (int r = 0; r < R3; ++r) {
-          if constexpr (NC >= 32)
-            L[it + r * IC] = v[it][r];
-          else
-            buf[zpad<V>(j + r * NC)] = v[it][r];
-        }
-      }
-    }
-    if constexpr (NC < 32) {
-      __syncwarp();
-#pragma unroll
-      for (int m = 0; m < E; ++m) L[m] = buf[zpad<V>(t + 32 * m)];
-      __syncwarp();
-    }
-  }
-}
-
-// c2r of fou (modes 0..nz2, global) into layout L (physical values packed
-// as complex), the line_c2r pre-step followed by the inverse FFT
-template <int M, typename T, typename TI>
-__device__ __forceinline__ void zc2r_regs(const ZTabT<T> &z, const TI *__restrict__ fou, V2<T> (&L)[M / 32],
-                                          V2<T> *buf, int t) {
-  using V = V2<T>;
-  constexpr int E = M / 32;
-  const int nz2 = z.nz2;
-  V a[E], b[E];
-#pragma unroll
-  for (int m = 0; m < E; ++m) {  // modes above nz2 are not read (they are 0)
-    const int k = t + 32 * m, km = M - k;
-    a[m] = k <= nz2 ? ldcx<T>(fou, k) : cmake<V>(T(0), T(0));
-    b[m] = km <= nz2 ? ldcx<T>(fou, km) : cmake<V>(T(0), T(0));
-  }
-#pragma unroll
-  for (int m = 0; m < E; ++m) {
-    const int k = t + 32 * m, km = M - k;
-    V aa = k <= nz2 ? a[m] : cmake<V>(T(0), T(0));
-    if (k == 0) aa.y = T(0);  // c2r ignores Im X[0]
-    V bb = km <= nz2 ? b[m] : cmake<V>(T(0), T(0));
-    bb.y = -bb.y;
-    const V s = cadd(aa, bb), d = csub(aa, bb);
-    const V tt = cmul(cconj(__ldg(z.tw2 + k)), d);  // W^{-k} d
-    L[m] = cmake<V>(s.x - tt.y, s.y + tt.x);       // s + i t
-  }
-  zfft_regs<M, 1>(L, buf, z.tw, t);
-}
-
-// r2c of layout L (physical values packed as complex) into fou (modes
-// 0..nz2) x 1/nz: forward FFT, then the line_r2c post-step
-template <int M, typename T, typename TO>
-__device__ __forceinline__ void zr2c_regs(const ZTabT<T> &z, V2<T> (&L)[M / 32], TO *__restrict__ fou, V2<T> *buf,
-                                          int t) {
-  using V = V2<T>;
-  constexpr int E = M / 32;
-  zfft_regs<M, -1>(L, buf, z.tw, t);
-  const int nz2 = z.nz2;
-  const T dnf = T(1) / (T)z.nz;
-#pragma unroll
-  for (int m = 0; m < E; ++m) {
-    // Z[(M - k) mod M], k = t + 32 m: element (32 - t) + 32 (E - 1 - m), held
-    // by lane 32 - t in L[E - 1 - m] for t >= 1; element 32 ((E - m) mod E),
-    // this lane's own L[(E - m) mod E], for t = 0
-    const V other = shfl_cx(L[E - 1 - m], (32 - t) & 31);
-    const V zm = t == 0 ? L[(E - m) % E] : other;
-    const int k = t + 32 * m;
-    if (k <= nz2) {
-      const V zk = L[m];
-      const V zc = cconj(zm);
-      const V e = cmake<V>(T(0.5) * (zk.x + zc.x), T(0.5) * (zk.y + zc.y));
-      const V d = csub(zk, zc);
-      const V o = cmake<V>(T(0.5) * d.y, T(-0.5) * d.x);  // -i d / 2
-      const V xk = cadd(e, cmul(__ldg(z.tw2 + k), o));
-      stcx(fou, k, cmake<V>(dnf * xk.x, dnf * xk.y));
-    }
-  }
-  __syncwarp();
-}
-
 template <int E, typename V>
 __device__ __forceinline__ void regs_mul(V (&a)[E], const V (&b)[E]) {
 #pragma unroll
@@ -361,81 +166,87 @@ __device__ __forceinline__ double regs_absmax(const V (&a)[E]) {
   return mx;
 }
 
-// CTAs per SM bound: FP64 unbounded (252 registers, 4.49 ms per substep at
-// 1025x193x512; 5.02 at >= 3 CTAs with spills), FP32 >= 4 CTAs (126-128
-// registers, 36 bytes of spills in part 0; 2.29-2.30 ms per substep against
-// 2.34-2.43 at >= 3 CTAs and 162-168 registers, after the exchange buffer's
-// swizzle; 3.16 unbounded before it). M < 256: FP32 >= 5 CTAs (M = 128: 96
-// registers, 0.69 against 0.72 ms per substep at 513x193x256 at 111); FP64
-// unbounded (M = 128: 152-168 registers, three CTAs; four at 128 registers
-// took 1.10-1.11 against 1.08-1.10 ms). A variant with two warps per line (4
-// elements per thread, radix-4 passes, named barriers) measured slower in
-// both precisions (4.92 and 3.61 ms) and was dropped.
+// k_products for M = nz/2 = 16..256 (nz = 32..512), each line kept in the
+// registers of ZGroup<M>::G lanes between the inverse transform's last pass and
+// the forward transform's first one. The lines of a part are counted through
+// planes and rows, so only the last warp has idle lanes. us per substep, one
+// warp per line with 2 to 8 elements a lane (three passes; nz = 32 the
+// shared-memory kernel) -> this: 33x41x32 55 -> 26, 257x97x128 229 -> 109,
+// 513x129x256 719 -> 538, 1025x193x512 4170 -> 3160; FP32 257x97x128 172 -> 84,
+// 513x129x256 472 -> 358, 1025x193x512 2110 -> 2056 (at three CTAs per SM
+// instead of four 2167).
 #ifndef OTBL_PR_MB_D
-#define OTBL_PR_MB_D 1
+#define OTBL_PR_MB_D 2
 #endif
 #ifndef OTBL_PR_MB_F
 #define OTBL_PR_MB_F 4
 #endif
+template <int M, typename T>
+constexpr int prod_min_ctas() {
+  return M >= 128 ? (sizeof(T) == 8 ? OTBL_PR_MB_D : OTBL_PR_MB_F) : (sizeof(T) == 8 ? 3 : 5);
+}
 template <int M, typename T, int PART>
-__global__ void __launch_bounds__(128, std::is_same<T, double>::value ? OTBL_PR_MB_D : (M < 256 ? 5 : OTBL_PR_MB_F))
-    k_products_r(DCoef c, ZTabT<T> z, ProdArgs<T> a) {
+__global__ void __launch_bounds__(128, prod_min_ctas<M, T>()) k_products_r(DCoef c, ZTabT<T> z, ProdArgs<T> a,
+                                                                         int nlines) {
   using V = V2<T>;
+  using Z = ZGroup<M>;
   extern __shared__ __align__(16) unsigned char smraw[];
-  V *sm = reinterpret_cast<V *>(smraw);
-  constexpr int E = M / 32;
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  const int j = blockIdx.x * 4 + wid + 1;
-  const int i = blockIdx.y + ProdPart<PART>::i0;
-  const int ny = c.ny, nz1 = c.nz1;
-  if (j > ny + ProdPart<PART>::extra) return;
-  V *buf = sm + (size_t)wid * (M + M / 8);
-  const size_t offu = ((size_t)(i - 1) * (ny + 1) + (j - 1)) * nz1;
-  const size_t offv = ((size_t)(i - 1) * ny + (j - 1)) * nz1;
+  constexpr int E = Z::E, G = Z::G;
+  const int grp = threadIdx.x / G, t = threadIdx.x & (G - 1);
+  const int line = blockIdx.x * (128 / G) + grp;
+  const bool on = line < nlines;
+  const int ny = c.ny, nz1 = c.nz1, rows = ny + ProdPart<PART>::extra;
+  const int ln = min(line, nlines - 1), i0 = ln / rows, j0 = ln - i0 * rows;
+  const int i = i0 + ProdPart<PART>::i0;
+  V *buf = reinterpret_cast<V *>(smraw) + grp * Z::BUF;
+  const size_t offu = ((size_t)(i - 1) * (ny + 1) + j0) * nz1;
+  const size_t offv = ((size_t)(i - 1) * ny + j0) * nz1;
   V A[E], B[E];
   if (PART == 1) {  // planes 2..nx-1, rows 1..ny
-    zc2r_regs<M>(z, a.v + offv, A, buf, lane);  // vw = v wy
-    zc2r_regs<M>(z, a.wy + offv, B, buf, lane);
+    zc2r_group<M>(z, a.v + offv, A, buf, t);  // vw = v wy
+    zc2r_group<M>(z, a.wy + offv, B, buf, t);
     regs_mul<E>(A, B);
-    zr2c_regs<M>(z, A, a.vw + offv, buf, lane);
-    zc2r_regs<M>(z, a.vy + offv, A, buf, lane);  // vv = vy^2
+    zr2c_group<M>(z, A, a.vw + offv, buf, t, on);
+    zc2r_group<M>(z, a.vy + offv, A, buf, t);  // vv = vy^2
     regs_sq<E>(A);
-    zr2c_regs<M>(z, A, a.vv + offv, buf, lane);
-    zc2r_regs<M>(z, a.w + offu, A, buf, lane);  // ww = w^2
+    zr2c_group<M>(z, A, a.vv + offv, buf, t, on);
+    zc2r_group<M>(z, a.w + offu, A, buf, t);  // ww = w^2
     regs_sq<E>(A);
-    zr2c_regs<M>(z, A, a.ww + offv, buf, lane);
+    zr2c_group<M>(z, A, a.ww + offv, buf, t, on);
     return;
   }
+  auto group_max = [&](double m) {
+#pragma unroll
+    for (int o = G / 2; o > 0; o >>= 1) m = nmax(m, __shfl_xor_sync(0xffffffffu, m, o));
+    return (unsigned long long)__double_as_longlong(m);
+  };
+  // an atomic only where it would change the maximum seen so far
+  auto raise = [&](unsigned long long *p, unsigned long long v) {
+    if (t == 0 && on && v > *(volatile unsigned long long *)p) atomicMax(p, v);
+  };
   if (PART == 2) {  // all planes, rows 1..ny
     double mv = 0.0;
-    zc2r_regs<M>(z, a.vx + offv, A, buf, lane);  // uv = vx uy
+    zc2r_group<M>(z, a.vx + offv, A, buf, t);  // uv = vx uy
     if (a.setstep) mv = regs_absmax<E>(A);
-    zc2r_regs<M>(z, a.uy + offv, B, buf, lane);
+    zc2r_group<M>(z, a.uy + offv, B, buf, t);
     regs_mul<E>(A, B);
-    zr2c_regs<M>(z, A, a.uv + offv, buf, lane);
-    if (a.setstep) {
-      mv = warp_nmax(mv);
-      if (lane == 0) atomicMax(&a.vm_bits[j], (unsigned long long)__double_as_longlong(mv));
-    }
+    zr2c_group<M>(z, A, a.uv + offv, buf, t, on);
+    if (a.setstep) raise(&a.vm_bits[j0 + 1], group_max(mv));
     return;
   }
   double mu = 0.0, mw = 0.0;
-  zc2r_regs<M>(z, a.ux + offu, A, buf, lane);  // uu = ux^2
+  zc2r_group<M>(z, a.ux + offu, A, buf, t);  // uu = ux^2
   regs_sq<E>(A);
-  zr2c_regs<M>(z, A, a.uu + offu, buf, lane);
-  zc2r_regs<M>(z, a.u + offu, B, buf, lane);  // uw = wx u
+  zr2c_group<M>(z, A, a.uu + offu, buf, t, on);
+  zc2r_group<M>(z, a.u + offu, B, buf, t);  // uw = wx u
   if (a.setstep) mu = regs_absmax<E>(B);
-  zc2r_regs<M>(z, a.wx + offu, A, buf, lane);
+  zc2r_group<M>(z, a.wx + offu, A, buf, t);
   if (a.setstep) mw = regs_absmax<E>(A);
   regs_mul<E>(A, B);
-  zr2c_regs<M>(z, A, a.uw + offu, buf, lane);
+  zr2c_group<M>(z, A, a.uw + offu, buf, t, on);
   if (a.setstep) {
-    mu = warp_nmax(mu);
-    mw = warp_nmax(mw);
-    if (lane == 0) {
-      atomicMax(&a.st->umax_bits, (unsigned long long)__double_as_longlong(mu));
-      atomicMax(&a.st->wmax_bits, (unsigned long long)__double_as_longlong(mw));
-    }
+    raise(&a.st->umax_bits, group_max(mu));
+    raise(&a.st->wmax_bits, group_max(mw));
   }
 }
 
@@ -1666,26 +1477,26 @@ static cudaError_t products_t(otbl_ctx *c, int setstep, int part, const ZTabT<T>
   // part 0: all planes, rows 1..ny+1; part 2: all planes, rows 1..ny;
   // part 1: planes 2..nx-1, rows 1..ny
   const dim3 g((c->cfg.ny + (part == 0 ? 1 : 0) + 3) / 4, c->cfg.nx - (part == 1 ? 2 : 0));
-  // the register-pipelined transforms for M = 32..256; other M (and
+  // the register-pipelined transforms for M = 16..256; other M (and
   // OTBL_PRODUCTS_SMEM=1) the shared-memory kernel
-  if ((M == 32 || M == 64 || M == 128 || M == 256) && !getenv("OTBL_PRODUCTS_SMEM")) {
-    const size_t smem = (size_t)4 * (M + M / 8) * sizeof(V2<T>);
-    auto go = [&](auto k0, auto k1, auto k2) {
-      if (part == 0)
-        k0<<<g, 128, smem, c->stream>>>(c->dc, z, a);
-      else if (part == 1)
-        k1<<<g, 128, smem, c->stream>>>(c->dc, z, a);
-      else
-        k2<<<g, 128, smem, c->stream>>>(c->dc, z, a);
+  if (M >= 16 && M <= 256 && !getenv("OTBL_PRODUCTS_SMEM")) {
+    const int nlines = (c->cfg.ny + (part == 0 ? 1 : 0)) * (c->cfg.nx - (part == 1 ? 2 : 0));
+    auto go = [&](auto m) {
+      constexpr int MM = decltype(m)::value, per = 128 / ZGroup<MM>::G;
+      const size_t smem = (size_t)per * ZGroup<MM>::BUF * sizeof(V2<T>);
+      auto k = part == 0 ? k_products_r<MM, T, 0> : (part == 1 ? k_products_r<MM, T, 1> : k_products_r<MM, T, 2>);
+      k<<<(nlines + per - 1) / per, 128, smem, c->stream>>>(c->dc, z, a, nlines);
     };
     if (M == 256)
-      go(k_products_r<256, T, 0>, k_products_r<256, T, 1>, k_products_r<256, T, 2>);
+      go(std::integral_constant<int, 256>{});
     else if (M == 128)
-      go(k_products_r<128, T, 0>, k_products_r<128, T, 1>, k_products_r<128, T, 2>);
+      go(std::integral_constant<int, 128>{});
     else if (M == 64)
-      go(k_products_r<64, T, 0>, k_products_r<64, T, 1>, k_products_r<64, T, 2>);
+      go(std::integral_constant<int, 64>{});
+    else if (M == 32)
+      go(std::integral_constant<int, 32>{});
     else
-      go(k_products_r<32, T, 0>, k_products_r<32, T, 1>, k_products_r<32, T, 2>);
+      go(std::integral_constant<int, 16>{});
   } else {
     const size_t smem = (size_t)4 * 3 * M * sizeof(V2<T>);
     auto k = part == 0 ? k_products<T, 0> : (part == 1 ? k_products<T, 1> : k_products<T, 2>);
