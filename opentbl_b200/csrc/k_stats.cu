@@ -2,12 +2,12 @@
 // does when dostat is set (rhsp.F90:70-92). Not on the substep path: the
 // reference computes them every avcrt steps (bl_1.F90:92).
 //
-//   k_stats_x    one thread per x-line (j, kr), coalesced across kr:
+//   k_stats_x    tiles of neighbouring x-lines in shared memory:
 //                u_x = interpx_new(u) shifted by one plane (rhsp.F90:71-79),
 //                dudx = diffx(u_x), dwdx = diffx(w), dvdx = diffx(v)
 //                (lip.f90:703-765, fd_ix and fd_dx), into the line scratch
 //                s1, s2, s3, t1
-//   k_stats_y    one thread per y-column (i, kr) of a group of planes:
+//   k_stats_y    tiles of neighbouring y-columns of a group of planes:
 //                buf1..buf5 = interpy_new of u_x, w, dwdx, dudx (fd_iy) and
 //                p (fd_iyp) onto the wall positions, buf6..buf8 = diffy of
 //                buf1, buf2, v (fd_dvdy) (stotf.F90:101-110,
@@ -19,12 +19,13 @@
 //                transforms (stotf.F90:264-285), added to the accumulators
 //
 // The groups of planes are sized so that the eight buffers fit in t2 and
-// t3. Every compact solve is the reference's serial recurrence in its order;
-// the sums over k and over the physical points are reduced in a different
+// t3. Every compact solve is the reference's recurrence in chunks of K rows
+// per thread (lines.cuh); the sums over k and over the physical points are reduced in a different
 // order than the reference's serial loops (rounding-level differences).
 #include <algorithm>
 
 #include "devcommon.cuh"
+#include "lines.cuh"
 #include "otbl_internal.cuh"
 #include "zline.cuh"
 
@@ -36,144 +37,96 @@ namespace {
 
 __device__ __forceinline__ double rd(double x, int xr) { return xr ? (double)(float)x : x; }
 
-// interpx_new (lip.f90:736-765) of a line of nx values at stride st, the
-// input rounded to REAL4 when xr (the chp2x transpose), the result written
-// shifted by one plane as rhsp.F90:75-79 does: out(i+1) = interp(i), out(1)
-// = interp(1). The backward sweep writes x_j into row j+1, whose forward
-// value it has already consumed.
-__device__ void interpx_shift(const double *c, int nx, const double *in, double *out, size_t st, int xr) {
-  auto I = [&](int i) { return rd(in[(size_t)(i - 1) * st], xr); };
-  auto O = [&](int i) -> double & { return out[(size_t)(i - 1) * st]; };
-  double s = 0.0;
-  for (int m = 1; m <= 4; ++m) s += C8(c, m, 1) * I(m);
-  O(1) = s;
-  for (int i = 2; i <= nx - 2; ++i) {
-    s = 0.0;
-    for (int m = 1; m <= 4; ++m) s += C8(c, m, 3) * I(i - 2 + m);
-    O(i) = s;
+// The window and weights of a compact operator's right-hand side: row r (of n)
+// takes cnt weights of row wr of the table times the input rows o..o+cnt-1;
+// its recurrence starts at row `first` (rows before it are the right-hand side
+// itself).
+struct Win {
+  int o, cnt, wr;
+};
+// interpx_new (lip.f90:736-765)
+struct OpIntX {
+  static constexpr int first = 0;
+  __device__ static Win win(int r, int n) {
+    if (r == 0) return {0, 4, 0};
+    return r <= n - 3 ? Win{r - 1, 4, 2} : Win{n - 4, 4, r};
   }
-  s = 0.0;
-  for (int m = 1; m <= 4; ++m) s += C8(c, m, nx - 1) * I(nx - 4 + m);
-  O(nx - 1) = s;
-  s = 0.0;
-  for (int m = 1; m <= 4; ++m) s += C8(c, m, nx) * I(nx - 4 + m);
-  O(nx) = s;
-  double prev = O(1);
-  for (int j = 2; j <= nx; ++j) {
-    prev = O(j) - C8(c, 6, j) * prev;
-    O(j) = prev;
+};
+// diffx_inplace (lip.f90:703-731)
+struct OpDifX {
+  static constexpr int first = 0;
+  __device__ static Win win(int r, int n) {
+    if (r < 2) return {0, 5, r};
+    return r <= n - 3 ? Win{r - 2, 5, 2} : Win{n - 5, 5, r};
   }
-  double xn = prev * C8(c, 7, nx);  // interp(nx): dropped by the shift
-  for (int j = nx - 1; j >= 1; --j) {
-    xn = (O(j) - C8(c, 8, j) * xn) * C8(c, 7, j);
-    O(j + 1) = xn;
+};
+// interpy_new (lip.f90:767-809): TIPO 0 from ny+1 rows, zero at the wall, TIPO
+// 1 from ny rows
+template <int TIPO>
+struct OpIntY {
+  static constexpr int first = 1;
+  __device__ static Win win(int r, int n) {
+    if (r == 0) return {1, TIPO == 0 ? 0 : 4, 0};
+    if (r == 1) return {1, 5, 1};
+    return r <= n - 3 ? Win{r - 1, 4, r} : Win{n - 3, TIPO == 1 ? 3 : 4, r};
   }
-  O(1) = xn;
-}
+};
+// diffy_inplace (lip.f90:666-699)
+struct OpDifY {
+  static constexpr int first = 0;
+  __device__ static Win win(int r, int n) {
+    if (r < 2) return {0, 4, r};
+    return r <= n - 3 ? Win{r - 2, 5, r} : Win{n - 4, 4, r};
+  }
+};
 
-// diffx_inplace (lip.f90:703-731) of a line at stride st
-__device__ void diffx_line(const double *c, int nx, const double *in, double *out, size_t st, int xr) {
-  auto I = [&](int i) { return rd(in[(size_t)(i - 1) * st], xr); };
-  auto O = [&](int i) -> double & { return out[(size_t)(i - 1) * st]; };
-  double s = 0.0;
-  for (int m = 1; m <= 5; ++m) s += C8(c, m, 1) * I(m);
-  O(1) = s;
-  s = 0.0;
-  for (int m = 1; m <= 5; ++m) s += C8(c, m, 2) * I(m);
-  O(2) = s;
-  for (int i = 3; i <= nx - 2; ++i) {
-    s = 0.0;
-    for (int m = 1; m <= 5; ++m) s += C8(c, m, 3) * I(i - 3 + m);
-    O(i) = s;
+// One operator (table c8, 8 values per row: five weights, then l, 1/pivot,
+// upper) on the lines of a tile in shared memory ([rows][L] pairs), chunk q of
+// K rows of lane `lane` to y. Uses ex (2 x blockDim values) and px (2 x
+// blockDim products). On return every thread has read the tile.
+template <typename OP, int K>
+__device__ __forceinline__ void stats_solve(const double *__restrict__ c8, const double2 *tile, int n, int C, int L,
+                                            int q, int lane, int xr, double2 (&y)[K], double2 *ex, double *px) {
+  const int t = threadIdx.x, NT = blockDim.x, s = q * K;
+  double l[K], d[K], e[K], pl = 1.0, pe = 1.0;
+#pragma unroll
+  for (int b = 0; b < K; ++b) {
+    const int r = s + b;
+    y[b] = make_double2(0.0, 0.0);
+    l[b] = d[b] = e[b] = 0.0;
+    if (r < n) {
+      const Win w = OP::win(r, n);
+      const double *cw = c8 + (size_t)w.wr * 8, *cr = c8 + (size_t)r * 8;
+#pragma unroll
+      for (int m = 0; m < 5; ++m) {
+        if (m < w.cnt) {
+          const double2 v = tile[(w.o + m) * L + lane];
+          fma2(y[b], __ldg(cw + m), make_double2(rd(v.x, xr), rd(v.y, xr)));
+        }
+      }
+      if (r < OP::first) {
+        d[b] = 1.0;
+      } else {
+        d[b] = __ldg(cr + 6);
+        if (r > OP::first) l[b] = -__ldg(cr + 5);
+        if (r < n - 1) e[b] = -__ldg(cr + 7) * d[b];
+      }
+    }
+    pl *= l[b];
   }
-  s = 0.0;
-  for (int m = 1; m <= 5; ++m) s += C8(c, m, nx - 1) * I(nx - 5 + m);
-  O(nx - 1) = s;
-  s = 0.0;
-  for (int m = 1; m <= 5; ++m) s += C8(c, m, nx) * I(nx - 5 + m);
-  O(nx) = s;
-  double prev = O(1);
-  for (int j = 2; j <= nx; ++j) {
-    prev = O(j) - C8(c, 6, j) * prev;
-    O(j) = prev;
-  }
-  double xn = prev * C8(c, 7, nx);
-  O(nx) = xn;
-  for (int j = nx - 1; j >= 1; --j) {
-    xn = (O(j) - C8(c, 8, j) * xn) * C8(c, 7, j);
-    O(j) = xn;
-  }
-}
-
-// interpy_new (lip.f90:767-809) of a column at stride st: ny+1-tipo input
-// rows of element type TI, ny output rows
-template <typename TI>
-__device__ void interpy_col(const double *c, int ny, const TI *in, double *out, size_t st, int tipo) {
-  auto I = [&](int j) { return (double)in[(size_t)(j - 1) * st]; };
-  auto O = [&](int j) -> double & { return out[(size_t)(j - 1) * st]; };
-  const int ch = tipo == 1 ? 0 : 1;
-  double s = 0.0;
-  for (int m = 1; m <= 4; ++m) s += C8(c, m, 1) * I(m + 1);
-  O(1) = tipo == 0 ? 0.0 : s;  // u and w vanish at the wall
-  s = 0.0;
-  for (int m = 1; m <= 5; ++m) s += C8(c, m, 2) * I(m + 1);
-  O(2) = s;
-  for (int j = 3; j <= ny - 2; ++j) {
-    s = 0.0;
-    for (int m = 1; m <= 4; ++m) s += C8(c, m, j) * I(j - 2 + m);
-    O(j) = s;
-  }
-  s = 0.0;
-  for (int m = 1; m <= 3 + ch; ++m) s += C8(c, m, ny - 1) * I(ny - 3 + m);
-  O(ny - 1) = s;
-  s = 0.0;
-  for (int m = 1; m <= 3 + ch; ++m) s += C8(c, m, ny) * I(ny - 3 + m);
-  O(ny) = s;
-  double prev = O(2);
-  for (int j = 3; j <= ny; ++j) {
-    prev = O(j) - C8(c, 6, j) * prev;
-    O(j) = prev;
-  }
-  double xn = prev * C8(c, 7, ny);
-  O(ny) = xn;
-  for (int j = ny - 1; j >= 2; --j) {
-    xn = (O(j) - C8(c, 8, j) * xn) * C8(c, 7, j);
-    O(j) = xn;
-  }
-}
-
-// diffy_inplace (lip.f90:666-699) of a column of ny rows at stride st
-__device__ void diffy_col(const double *c, int ny, const double *in, double *out, size_t st) {
-  auto I = [&](int j) { return in[(size_t)(j - 1) * st]; };
-  auto O = [&](int j) -> double & { return out[(size_t)(j - 1) * st]; };
-  double s = 0.0;
-  for (int m = 1; m <= 4; ++m) s += C8(c, m, 1) * I(m);
-  O(1) = s;
-  s = 0.0;
-  for (int m = 1; m <= 4; ++m) s += C8(c, m, 2) * I(m);
-  O(2) = s;
-  for (int j = 3; j <= ny - 2; ++j) {
-    s = 0.0;
-    for (int m = 1; m <= 5; ++m) s += C8(c, m, j) * I(j - 3 + m);
-    O(j) = s;
-  }
-  s = 0.0;
-  for (int m = 1; m <= 4; ++m) s += C8(c, m, ny - 1) * I(ny - 4 + m);
-  O(ny - 1) = s;
-  s = 0.0;
-  for (int m = 1; m <= 4; ++m) s += C8(c, m, ny) * I(ny - 4 + m);
-  O(ny) = s;
-  double prev = O(1);
-  for (int j = 2; j <= ny; ++j) {
-    prev = O(j) - C8(c, 6, j) * prev;
-    O(j) = prev;
-  }
-  double xn = prev * C8(c, 7, ny);
-  O(ny) = xn;
-  for (int j = ny - 1; j >= 1; --j) {
-    xn = (O(j) - C8(c, 8, j) * xn) * C8(c, 7, j);
-    O(j) = xn;
-  }
+#pragma unroll
+  for (int b = 0; b < K; ++b) pe *= e[b];
+  forward_local<K, 1, double>(y, l);
+  ex[t] = y[K - 1];
+  px[t] = pl;
+  px[NT + t] = pe;
+  __syncthreads();
+  if (q > 0) forward_fix<K, 1, double>(y, l, chunk_carry<double>(ex + t - L, -L, px + t - L, -L, q));
+  backward_local<K, 1, double>(y, d, e);
+  ex[NT + t] = y[0];
+  __syncthreads();
+  if (q < C - 1)
+    backward_fix<K, 1, double>(y, e, chunk_carry<double>(ex + NT + t + L, L, px + NT + t + L, L, C - 1 - q));
 }
 
 struct StatsOps {
@@ -186,47 +139,115 @@ struct StatsBufs {
   double *b[8];
 };
 
-__global__ void __launch_bounds__(128) k_stats_x(DCoef c, StatsOps op, const double *__restrict__ u,
+// blockIdx.y: 0 u (u_x, dudx), 1 w (dwdx), 2 v (dvdx); a CTA takes L pairs of
+// neighbouring lines
+template <int K>
+__global__ void __launch_bounds__(256) k_stats_x(DCoef c, StatsOps op, const double *__restrict__ u,
                                                  const double *__restrict__ v, const double *__restrict__ w,
-                                                 double *ux, double *dudx, double *dwdx, double *dvdx) {
-  const int nx = c.nx, ny = c.ny, nz1 = c.nz1, xr = c.xround;
-  const size_t PU = (size_t)(ny + 1) * nz1, PV = (size_t)ny * nz1;
-  const size_t line = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (line >= PU) return;
-  interpx_shift(op.fix, nx, u + line, ux + line, PU, xr);
-  diffx_line(op.fdx, nx, ux + line, dudx + line, PU, 0);  // of the unrounded u_x
-  diffx_line(op.fdx, nx, w + line, dwdx + line, PU, xr);
-  if (line < PV) diffx_line(op.fdx, nx, v + line, dvdx + line, PV, xr);
-  if (xr) {  // the chx2p transposes back to planes round to REAL4
-    for (int i = 0; i < nx; ++i) {
-      ux[(size_t)i * PU + line] = rd(ux[(size_t)i * PU + line], 1);
-      dudx[(size_t)i * PU + line] = rd(dudx[(size_t)i * PU + line], 1);
-      dwdx[(size_t)i * PU + line] = rd(dwdx[(size_t)i * PU + line], 1);
-      if (line < PV) dvdx[(size_t)i * PV + line] = rd(dvdx[(size_t)i * PV + line], 1);
-    }
+                                                 double *ux, double *dudx, double *dwdx, double *dvdx, int C, int L) {
+  extern __shared__ __align__(16) unsigned char stsm[];
+  const int nx = c.nx, ny = c.ny, xr = c.xround, f = blockIdx.y, t = threadIdx.x, NT = blockDim.x;
+  const int npp = (c.nz1 >> 1) * (f == 2 ? ny : ny + 1), p0 = blockIdx.x * L;
+  if (p0 >= npp) return;  // the whole CTA
+  const int q = min(t / L, C - 1), lane = t % L, s = q * K;
+  const bool on = t < C * L && p0 + lane < npp;
+  double2 *tile = reinterpret_cast<double2 *>(stsm), *ex = tile + (size_t)nx * L;
+  double *px = reinterpret_cast<double *>(ex + 2 * NT);
+  const double2 *in = reinterpret_cast<const double2 *>(f == 0 ? u : (f == 1 ? w : v));
+  for (int e = t; e < nx * L; e += NT) {
+    const int r = e / L, m = p0 + (e - r * L);
+    cp_async_v(tile + e, in + (size_t)r * npp + min(m, npp - 1), m < npp);
   }
+  cp_async_commit();
+  cp_async_wait<0>();
+  __syncthreads();
+  double2 y[K];
+  double *out = f == 0 ? dudx : (f == 1 ? dwdx : dvdx);
+  if (f == 0) {
+    stats_solve<OpIntX, K>(op.fix, tile, nx, C, L, q, lane, xr, y, ex, px);
+    // shifted by one plane: out(i+1) = interp(i), out(1) = interp(1)
+    if (t < C * L) {
+#pragma unroll
+      for (int b = 0; b < K; ++b) {
+        const int r = s + b;
+        if (r < nx - 1) tile[(r + 1) * L + lane] = y[b];
+        if (r == 0) tile[lane] = y[b];
+      }
+    }
+    __syncthreads();
+    double2 *o = reinterpret_cast<double2 *>(ux);
+    for (int e = t; e < nx * L; e += NT) {  // the chx2p transposes back to planes round to REAL4
+      const int r = e / L, m = p0 + (e - r * L);
+      const double2 x = tile[e];
+      if (m < npp) o[(size_t)r * npp + m] = make_double2(rd(x.x, xr), rd(x.y, xr));
+    }
+    stats_solve<OpDifX, K>(op.fdx, tile, nx, C, L, q, lane, 0, y, ex, px);  // of the unrounded u_x
+  } else {
+    stats_solve<OpDifX, K>(op.fdx, tile, nx, C, L, q, lane, xr, y, ex, px);
+  }
+  if (!on) return;
+  double2 *o = reinterpret_cast<double2 *>(out) + (size_t)s * npp + p0 + lane;
+#pragma unroll
+  for (int b = 0; b < K; ++b)
+    if (s + b < nx) o[(size_t)b * npp] = make_double2(rd(y[b].x, xr), rd(y[b].y, xr));
 }
 
-template <typename TP>
-__global__ void __launch_bounds__(128) k_stats_y(DCoef c, StatsOps op, const double *__restrict__ ux,
+// blockIdx.y: 0 u_x (buf1, buf6), 1 w (buf2, buf7), 2 dwdx (buf3), 3 dudx
+// (buf4), 4 p (buf5), 5 v (buf8); a CTA takes L neighbouring modes of the G
+// planes from i0 on
+template <typename TP, int K>
+__global__ void __launch_bounds__(256) k_stats_y(DCoef c, StatsOps op, const double *__restrict__ ux,
                                                  const double *__restrict__ w, const double *__restrict__ dwdx,
                                                  const double *__restrict__ dudx, const TP *__restrict__ p,
-                                                 const double *__restrict__ v, StatsBufs bf, int i0, int G) {
-  const int ny = c.ny, nz1 = c.nz1;
-  const int col = blockIdx.x * blockDim.x + threadIdx.x;
-  if (col >= G * nz1) return;
-  const int il = col / nz1, kr = col - il * nz1, i = i0 + il;
-  const size_t PU = (size_t)(ny + 1) * nz1, PV = (size_t)ny * nz1;
-  const size_t cu = (size_t)(i - 1) * PU + kr, cv = (size_t)(i - 1) * PV + kr;
-  const size_t cb = (size_t)il * PV + kr;
-  interpy_col(op.fiy, ny, ux + cu, bf.b[0] + cb, nz1, 0);
-  interpy_col(op.fiy, ny, w + cu, bf.b[1] + cb, nz1, 0);
-  interpy_col(op.fiy, ny, dwdx + cu, bf.b[2] + cb, nz1, 0);
-  interpy_col(op.fiy, ny, dudx + cu, bf.b[3] + cb, nz1, 0);
-  interpy_col(op.fiyp, ny, p + cv, bf.b[4] + cb, nz1, 1);
-  diffy_col(op.fdvdy, ny, bf.b[0] + cb, bf.b[5] + cb, nz1);
-  diffy_col(op.fdvdy, ny, bf.b[1] + cb, bf.b[6] + cb, nz1);
-  diffy_col(op.fdvdy, ny, v + cv, bf.b[7] + cb, nz1);
+                                                 const double *__restrict__ v, StatsBufs bf, int i0, int G, int C,
+                                                 int L) {
+  extern __shared__ __align__(16) unsigned char stsm[];
+  const int ny = c.ny, nk = c.nz1 >> 1, f = blockIdx.y, t = threadIdx.x, NT = blockDim.x;
+  const int rows = f < 4 ? ny + 1 : ny, ncm = G * nk, m0 = blockIdx.x * L;
+  const int q = min(t / L, C - 1), lane = t % L, s = q * K;
+  double2 *tile = reinterpret_cast<double2 *>(stsm), *ex = tile + (size_t)(ny + 1) * L;
+  double *px = reinterpret_cast<double *>(ex + 2 * NT);
+  const double *in = f == 0 ? ux : (f == 1 ? w : (f == 2 ? dwdx : (f == 3 ? dudx : v)));
+  for (int e = t; e < rows * L; e += NT) {
+    const int r = e / L, m = min(m0 + (e - r * L), ncm - 1), il = m / nk, k = m - il * nk;
+    const size_t at = ((size_t)(i0 - 1 + il) * rows + r) * nk + k;
+    if (f == 4) {
+      const V2<TP> x = __ldg(reinterpret_cast<const V2<TP> *>(p) + at);
+      tile[e] = make_double2((double)x.x, (double)x.y);
+    } else {
+      tile[e] = __ldg(reinterpret_cast<const double2 *>(in) + at);
+    }
+  }
+  __syncthreads();
+  const int m = min(m0 + lane, ncm - 1), il = m / nk, k = m - il * nk;
+  const bool on = t < C * L && m0 + lane < ncm;
+  double2 y[K];
+  auto store = [&](double *base) {
+    double2 *o = reinterpret_cast<double2 *>(base) + ((size_t)il * ny + s) * nk + k;
+#pragma unroll
+    for (int b = 0; b < K; ++b)
+      if (on && s + b < ny) o[(size_t)b * nk] = y[b];
+  };
+  if (f < 4) {
+    stats_solve<OpIntY<0>, K>(op.fiy, tile, ny, C, L, q, lane, 0, y, ex, px);
+    store(f == 0 ? bf.b[0] : (f == 1 ? bf.b[1] : (f == 2 ? bf.b[2] : bf.b[3])));
+    if (f < 2) {
+      if (t < C * L) {
+#pragma unroll
+        for (int b = 0; b < K; ++b)
+          if (s + b < ny) tile[(s + b) * L + lane] = y[b];
+      }
+      __syncthreads();
+      stats_solve<OpDifY, K>(op.fdvdy, tile, ny, C, L, q, lane, 0, y, ex, px);
+      store(f == 0 ? bf.b[5] : bf.b[6]);
+    }
+  } else if (f == 4) {
+    stats_solve<OpIntY<1>, K>(op.fiyp, tile, ny, C, L, q, lane, 0, y, ex, px);
+    store(bf.b[4]);
+  } else {
+    stats_solve<OpDifY, K>(op.fdvdy, tile, ny, C, L, q, lane, 0, y, ex, px);
+    store(bf.b[7]);
+  }
 }
 
 __device__ __forceinline__ double warp_sum(double x) {
@@ -372,9 +393,27 @@ cudaError_t launch_statsp(otbl_ctx *c) {
   op.fiyp = c->coef_dev + o.off[OTBL_C_FD_IYP];
   const size_t PU = (size_t)(ny + 1) * nz1, PV = (size_t)ny * nz1;
   double *ux = c->w.s1, *dudx = c->w.s2, *dwdx = c->w.s3, *dvdx = c->w.t1;
-  k_stats_x<<<(unsigned)((PU + 127) / 128), 128, 0, s>>>(c->dc, op, c->f[OTBL_F_U], c->f[OTBL_F_V],
-                                                          c->f[OTBL_F_W], ux, dudx, dwdx, dvdx);
-  c->launches += 1;
+  // a chunk of 9 (longer lines: 33) rows per thread, as many lanes as 256
+  // threads and 96 KB of tile hold
+  auto shape = [](int n, int &K, int &C, int &L, int &NT, size_t &smem) {
+    K = n <= 9 * 128 ? 9 : 33;
+    C = (n + K - 1) / K;
+    L = std::max(1, std::min(std::min(256 / C, 16), 6144 / (n + 1)));
+    NT = (C * L + 31) / 32 * 32;
+    smem = (size_t)(n + 1) * L * 16 + (size_t)NT * (32 + 16);
+    return K == 9;
+  };
+  int K, C, L, NT;
+  size_t sm;
+  auto go = [&](auto kern, dim3 g, auto... args) {
+    if (sm > 48 * 1024) cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+    kern<<<g, NT, sm, s>>>(c->dc, op, args..., C, L);
+    c->launches += 1;
+  };
+  const bool sx = shape(nx, K, C, L, NT, sm);
+  const dim3 gx((unsigned)((PU / 2 + L - 1) / L), 3);
+  go(sx ? k_stats_x<9> : k_stats_x<33>, gx, (const double *)c->f[OTBL_F_U], (const double *)c->f[OTBL_F_V],
+     (const double *)c->f[OTBL_F_W], ux, dudx, dwdx, dvdx);
   // groups of G planes: four buffers of G planes in each of t2 and t3
   const size_t lu = otbl_field_len(nx, ny, nz, 1);
   const int G = (int)std::max<size_t>(1, std::min<size_t>(nx, lu / (4 * PV)));
@@ -390,16 +429,17 @@ cudaError_t launch_statsp(otbl_ctx *c) {
     const int g = std::min(G, nx - i0 + 1);
     StatsBufs bf;
     for (int b = 0; b < 8; ++b) bf.b[b] = (b < 4 ? c->w.t2 : c->w.t3) + (size_t)(b % 4) * G * PV;
-    const int ncol = g * nz1;
+    const bool sy = shape(ny, K, C, L, NT, sm);
+    const dim3 gy((g * (nz1 / 2) + L - 1) / L, 6);
+    const double *cx = ux, *cw = c->f[OTBL_F_W], *cdw = dwdx, *cdu = dudx, *cv = c->f[OTBL_F_V];
     if (c->f32[OTBL_F_P])
-      k_stats_y<float><<<(ncol + 127) / 128, 128, 0, s>>>(c->dc, op, ux, c->f[OTBL_F_W], dwdx, dudx,
-                                                         reinterpret_cast<const float *>(c->f[OTBL_F_P]),
-                                                         c->f[OTBL_F_V], bf, i0, g);
+      go(sy ? k_stats_y<float, 9> : k_stats_y<float, 33>, gy, cx, cw, cdw, cdu,
+         reinterpret_cast<const float *>(c->f[OTBL_F_P]), cv, bf, i0, g);
     else
-      k_stats_y<double><<<(ncol + 127) / 128, 128, 0, s>>>(c->dc, op, ux, c->f[OTBL_F_W], dwdx, dudx,
-                                                          c->f[OTBL_F_P], c->f[OTBL_F_V], bf, i0, g);
+      go(sy ? k_stats_y<double, 9> : k_stats_y<double, 33>, gy, cx, cw, cdw, cdu, (const double *)c->f[OTBL_F_P], cv,
+         bf, i0, g);
     k_stats_acc<<<(g * ny + 3) / 4, 128, smem, s>>>(c->dc, z, bf, c->f[OTBL_F_V], dvdx, c->stats, i0, g);
-    c->launches += 2;
+    c->launches += 1;
   }
   c->stats_samples += 1;
   return cudaGetLastError();
