@@ -186,14 +186,13 @@ constexpr int prod_min_ctas() {
   return M >= 128 ? (sizeof(T) == 8 ? OTBL_PR_MB_D : OTBL_PR_MB_F) : (sizeof(T) == 8 ? 3 : 5);
 }
 template <int M, typename T, int PART>
-__global__ void __launch_bounds__(128, prod_min_ctas<M, T>()) k_products_r(DCoef c, ZTabT<T> z, ProdArgs<T> a,
-                                                                         int nlines) {
+__device__ __forceinline__ void products_body(const DCoef &c, const ZTabT<T> &z, const ProdArgs<T> &a, int block,
+                                              int nlines, unsigned char *smraw) {
   using V = V2<T>;
   using Z = ZGroup<M>;
-  extern __shared__ __align__(16) unsigned char smraw[];
   constexpr int E = Z::E, G = Z::G;
   const int grp = threadIdx.x / G, t = threadIdx.x & (G - 1);
-  const int line = blockIdx.x * (128 / G) + grp;
+  const int line = block * (128 / G) + grp;
   const bool on = line < nlines;
   const int ny = c.ny, nz1 = c.nz1, rows = ny + ProdPart<PART>::extra;
   const int ln = min(line, nlines - 1), i0 = ln / rows, j0 = ln - i0 * rows;
@@ -250,6 +249,31 @@ __global__ void __launch_bounds__(128, prod_min_ctas<M, T>()) k_products_r(DCoef
   }
 }
 
+// lines of each part
+template <int PART>
+__host__ __device__ constexpr int prod_lines(int nx, int ny) {
+  return (ny + ProdPart<PART>::extra) * (nx - (PART == 1 ? 2 : 0));
+}
+template <int M, typename T, int PART>
+__global__ void __launch_bounds__(128, prod_min_ctas<M, T>()) k_products_r(DCoef c, ZTabT<T> z, ProdArgs<T> a) {
+  extern __shared__ __align__(16) unsigned char smraw[];
+  products_body<M, T, PART>(c, z, a, blockIdx.x, prod_lines<PART>(c.nx, c.ny), smraw);
+}
+// the three parts in one launch, for boxes whose single parts leave SMs idle
+template <int M, typename T>
+__global__ void __launch_bounds__(128, prod_min_ctas<M, T>()) k_products_all(DCoef c, ZTabT<T> z, ProdArgs<T> a) {
+  extern __shared__ __align__(16) unsigned char smraw[];
+  constexpr int per = 128 / ZGroup<M>::G;
+  const int n0 = prod_lines<0>(c.nx, c.ny), n2 = prod_lines<2>(c.nx, c.ny), n1 = prod_lines<1>(c.nx, c.ny);
+  const int b1 = (n1 + per - 1) / per, b0 = (n0 + per - 1) / per, b = blockIdx.x;
+  if (b < b1)
+    products_body<M, T, 1>(c, z, a, b, n1, smraw);
+  else if (b < b1 + b0)
+    products_body<M, T, 0>(c, z, a, b - b1, n0, smraw);
+  else
+    products_body<M, T, 2>(c, z, a, b - b1 - b0, n2, smraw);
+}
+
 // ---------------------------------------------------------------------------
 // dt (rhsp.F90:214-267), RK3 factors, implzy LU (lip.f90:545-568)
 // ---------------------------------------------------------------------------
@@ -279,7 +303,7 @@ __device__ __forceinline__ ImplzyRow implzy_row(const DCoef &c, int which, int r
 // fac[3j+2] = -C_j / B'_{j+1} (0 for j = jee-1); descending y_j = r_j +
 // fac[3j+2] y_{j+1}, ascending x_j = (y_j - fac[3j] x_{j-1}) fac[3j+1];
 // fac[3(jee+1)] = A_2, fac[3(jee+1)+1] = C_{jee-1}.
-__global__ void __launch_bounds__(256) k_dt(DCoef c, DState *st, const unsigned long long *vm_bits, ImplzyTab tu,
+__global__ void __launch_bounds__(256) k_dt(DCoef c, DState *st, unsigned long long *vm_bits, ImplzyTab tu,
                                             ImplzyTab tv, double *fac_u, double *fac_v, int m, int setstep, int dt_mode, double dt_fixed) {
   extern __shared__ double dsm[];
   __shared__ double s_dt3[8], s_vmax[8], s_rkk;
@@ -292,6 +316,7 @@ __global__ void __launch_bounds__(256) k_dt(DCoef c, DState *st, const unsigned 
       const double vm = __longlong_as_double((long long)vm_bits[j]);
       dt3 = fmin(dt3, c.dymin[j - 1] / fmax(poco, vm));
       vmax = nmax(vmax, vm);
+      vm_bits[j] = 0ull;
     }
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) {
@@ -327,6 +352,7 @@ __global__ void __launch_bounds__(256) k_dt(DCoef c, DState *st, const unsigned 
         st->dt_frozen = 1;
       }
     }
+    if (setstep) st->umax_bits = st->wmax_bits = 0ull;  // consumed: the next reduction starts from 0
     const double dt = st->dt;
     if (!(dt > 0.0) || !isfinite(dt)) atomicCAS(&st->err, 0, OTBL_ERR_NAN);
     const int q = m - 1;
@@ -353,18 +379,28 @@ __global__ void __launch_bounds__(256) k_dt(DCoef c, DState *st, const unsigned 
   if (lane == 0 && wid < (fac_u ? 4 : 2)) {
     const int which = wid & 1, o = which * N1, n = (which == 0 ? N1 : N1 - 1) - 2;
     double t1 = 1.0, t2 = 0.0;  // the continuants of the two rows before
-    for (int i = 1; i <= n; ++i) {
-      const int r = wid < 2 ? i : n + 1 - i;
-      const double t0 = bs[o + r] * t1 - (wid < 2 ? ac[o + r] : (i > 1 ? ac[o + r + 1] : 0.0)) * t2;
-      if (wid < 2) {
-        num[o + r] = t0;
-        den[o + r] = t1;
-      } else {
-        top[o + r] = t1;
-        top[2 * N1 + o + r] = t0;
+    const bool up = wid < 2;
+    double *pd = (up ? den : top) + o, *pn = (up ? num : top + 2 * N1) + o;
+    // four rows between the range checks (a row's factor stays far below 2^75)
+    for (int i0 = 1; i0 <= n; i0 += 4) {
+      double b[4], a[4];
+#pragma unroll
+      for (int x = 0; x < 4; ++x) {
+        const int i = min(i0 + x, n), r = up ? i : n + 1 - i;
+        b[x] = bs[o + r];
+        a[x] = up ? ac[o + r] : (i > 1 ? ac[o + r + 1] : 0.0);
       }
-      t2 = t1;
-      t1 = t0;
+#pragma unroll
+      for (int x = 0; x < 4; ++x) {
+        const int i = i0 + x, r = up ? i : n + 1 - i;
+        if (i <= n) {
+          const double t0 = b[x] * t1 - a[x] * t2;
+          pn[r] = t0;
+          pd[r] = t1;
+          t2 = t1;
+          t1 = t0;
+        }
+      }
       if (fabs(t1) > 0x1p300) {
         t1 *= 0x1p-300;
         t2 *= 0x1p-300;
@@ -417,15 +453,6 @@ __global__ void __launch_bounds__(256) k_dt(DCoef c, DState *st, const unsigned 
     tb.P[q] = p;
     tb.P[tb.C + q] = x;
   }
-}
-
-__global__ void k_reset_max(DState *st, unsigned long long *vm_bits, int ny) {
-  const int t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (t == 0) {
-    st->umax_bits = 0ull;
-    st->wmax_bits = 0ull;
-  }
-  if (t <= ny) vm_bits[t] = 0ull;
 }
 
 // energies + ministats (rhsp.F90:493-509, stotf.F90:395-440) when one
@@ -524,13 +551,14 @@ __global__ void __launch_bounds__(256) k_genflu_tab(DCoef c, GenArgs a) {
   int *kf = reinterpret_cast<int *>(um + ny + 2);  // [2][ny+1] fresh bisection, -1 = outside
   int *kh = kf + 2 * N1;                            // [2][ny+1] its khh
   __shared__ double s_timec, s_g1, s_g2, s_www1[2];
-  __shared__ int s_jfirst;
+  __shared__ int s_jfirst, s_nt[2];
   const double re = c.S[OTBL_S_RE], din = c.S[OTBL_S_DIN], rthin = c.S[OTBL_S_RTHIN];
   const double dt = *a.dt;
   if (t == 0) {
     const double tloc = *a.tiempo - *a.timeinit;
     s_timec = tloc < 20 ? 20.0 : (tloc < 100 ? 100.0 : tloc);
     s_jfirst = ny - 1;
+    s_nt[0] = s_nt[1] = 0;
   }
   __syncthreads();
   const double timec = s_timec;
@@ -551,14 +579,17 @@ __global__ void __launch_bounds__(256) k_genflu_tab(DCoef c, GenArgs a) {
   for (int j = t + 1; j <= ny - 2; j += T)
     if (um[j] >= u99) atomicMin(&s_jfirst, j);
   __syncthreads();
-  if (t == 0) {
+  if (t < 32) {
     const int jf = s_jfirst;
     const int jtop = jf == 1 ? 0 : jf;
+    double s = 0.0;  // the momentum integral, summed across the warp
+    for (int q = t; q < jtop + 2; q += 32) s += (uinf - um[2 + q]) * um[2 + q] * dy[1 + q];
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+    if (t == 0) {
     *a.timec = timec;
     *a.utauout = sqrt(fabs((um[2] - um[1]) / (y[2] - y[1]) / re));
     *a.dout = y[jtop];
-    double s = 0.0;
-    for (int q = 0; q < jtop + 2; ++q) s += (uinf - um[2 + q]) * um[2 + q] * dy[1 + q];
     const double rthout = s * re / uinf;
     *a.rthout = rthout;
     const double gamma2 = rthin / rthout;
@@ -568,6 +599,7 @@ __global__ void __launch_bounds__(256) k_genflu_tab(DCoef c, GenArgs a) {
     s_g1 = gamma1;
     s_g2 = gamma2;
     a.tab[3 * N1] = 1.0 / gamma1;  // ggg
+    }
   }
   // rescaled grids: kk = 0 (u rows, cell centres) and kk = 1 (v rows)
   for (int e = t; e < 2 * N1; e += T) {
@@ -576,7 +608,7 @@ __global__ void __launch_bounds__(256) k_genflu_tab(DCoef c, GenArgs a) {
   }
   __syncthreads();
   // dobleu (genflu.F90:250-298): the tanh weights element-wise, the running
-  // integral sequentially
+  // integral as a scan of one warp per grid
   {
     const double ag = 4.0, bg = 0.2;
     const double bg2 = 1.0 - 2.0 * bg, tag = 1.0 / tanh(ag);
@@ -589,17 +621,31 @@ __global__ void __launch_bounds__(256) k_genflu_tab(DCoef c, GenArgs a) {
     }
   }
   __syncthreads();
-  if (t == 0 || t == 32) {
-    const int kk = t / 32;
+  if (t < 64) {
+    const int kk = t / 32, lane = t & 31;
     const double *eta = ysca + kk * N1, *yy = yyy + kk * N1;
     double *ww = www + kk * N1;
-    double www1 = (double)0.7895f;
-    ww[1] = 0.0;
-    for (int i = 2; i <= ny; ++i) {
-      ww[i] = ww[i - 1] + yy[i] * (eta[i] - eta[i - 1]);
-      if (eta[i] >= 1.0 && eta[i - 1] < 1.0) www1 = ww[i - 1] + (1.0 - eta[i - 1]) * yy[i];
+    if (lane == 0) {
+      s_www1[kk] = (double)0.7895f;
+      ww[1] = 0.0;
     }
-    s_www1[kk] = www1;
+    __syncwarp();
+    double before = 0.0;
+    for (int i0 = 2; i0 <= ny; i0 += 32) {
+      const int i = i0 + lane;
+      double s = i <= ny ? yy[i] * (eta[i] - eta[i - 1]) : 0.0;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const double x = __shfl_up_sync(0xffffffffu, s, o);
+        if (lane >= o) s += x;
+      }
+      if (i <= ny) {
+        ww[i] = before + s;
+        if (eta[i] >= 1.0 && eta[i - 1] < 1.0)
+          s_www1[kk] = before + s - yy[i] * (eta[i] - eta[i - 1]) + (1.0 - eta[i - 1]) * yy[i];
+      }
+      before += __shfl_sync(0xffffffffu, s, 31);
+    }
   }
   __syncthreads();
   const double gamma1 = s_g1, gamma2 = s_g2;
@@ -633,8 +679,18 @@ __global__ void __launch_bounds__(256) k_genflu_tab(DCoef c, GenArgs a) {
   __syncthreads();
   // the reference carries kll from one row to the next; a bisection started
   // at the carried kll = lo ends where the fresh one does unless the target
-  // lies at or below ys[lo], where it stays at lo (redone sequentially)
-  if (t == 0 || t == 32) {
+  // lies at or below ys[lo], where it stays at lo (then redone sequentially;
+  // it takes a rescaled grid that is not increasing)
+  int redo = 0;
+  for (int e = t; e < 2 * N1; e += T) {
+    const int kk = e / N1, i = e - kk * N1;
+    if (i < 1 || kf[e] < 0) continue;
+    atomicMax(&s_nt[kk], i);
+    if (i > 1 && (kf[e - 1] < 0 || !(ysca[kk * N1 + kf[e - 1]] < www[e]))) redo = 1;
+  }
+  redo = __syncthreads_or(redo);
+  if (!redo && t < 2) ntop[t] = s_nt[t];
+  if (redo && (t == 0 || t == 32)) {
     const int kk = t / 32;
     const double *ys = ysca + kk * N1, *wl = www + kk * N1;
     int *kfk = kf + kk * N1, *khk = kh + kk * N1;
@@ -786,22 +842,9 @@ __global__ void k_boun(DCoef c, double *u, double *v, double *w) {
 // ---------------------------------------------------------------------------
 // outflow_correction, boun.f90:63-93: one CTA, fixed-order reductions.
 // ---------------------------------------------------------------------------
-__device__ double block_sum(double v, double *red) {
-  const int t = threadIdx.x;
-  red[t] = v;
-  __syncthreads();
-  for (int s = blockDim.x / 2; s > 0; s >>= 1) {
-    if (t < s) red[t] = red[t] + red[t + s];
-    __syncthreads();
-  }
-  const double r = red[0];
-  __syncthreads();
-  return r;
-}
-
 template <typename TR>
 __global__ void __launch_bounds__(256) k_outflow(DCoef c, double *u, const double *v, TR *rhsupa) {
-  __shared__ double red[256];
+  __shared__ double red[3][8];
   const int t = threadIdx.x, nx = c.nx, ny = c.ny, nz1 = c.nz1;
   const size_t PU = (size_t)(ny + 1) * nz1, PV = (size_t)ny * nz1;
   double a = 0.0, b = 0.0, d = 0.0;
@@ -810,16 +853,35 @@ __global__ void __launch_bounds__(256) k_outflow(DCoef c, double *u, const doubl
     b += u[(size_t)(j - 1) * nz1] * c.dy[j - 1];
     d += u[(size_t)(nx - 1) * PU + (size_t)(j - 1) * nz1] * c.dy[j - 1];
   }
-  const double sv = block_sum(a, red), s1 = block_sum(b, red), s2 = block_sum(d, red);
-  double sumax = sv * c.S[OTBL_S_DX1];
+  const double ly = c.y[ny] - c.y[1], dx1 = c.S[OTBL_S_DX1], idx = c.S[OTBL_S_IDX];
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    a += __shfl_xor_sync(0xffffffffu, a, o);
+    b += __shfl_xor_sync(0xffffffffu, b, o);
+    d += __shfl_xor_sync(0xffffffffu, d, o);
+  }
+  if ((t & 31) == 0) {
+    red[0][t >> 5] = a;
+    red[1][t >> 5] = b;
+    red[2][t >> 5] = d;
+  }
+  __syncthreads();
+  double sv = 0.0, s1 = 0.0, s2 = 0.0;
+#pragma unroll
+  for (int w = 0; w < 8; ++w) {
+    sv += red[0][w];
+    s1 += red[1][w];
+    s2 += red[2][w];
+  }
+  double sumax = sv * dx1;
   sumax = sumax - s1;
   sumax = sumax + s2;
-  const double alpha = -sumax / (c.y[ny] - c.y[1]);
+  const double alpha = -sumax / ly;
   for (int j = 2 + t; j <= ny; j += 256) {
     double *q = u + (size_t)(nx - 1) * PU + (size_t)(j - 1) * nz1;
     q[0] = q[0] + alpha;
     TR *h = rhsupa + (size_t)(nx - 1) * PU + (size_t)(j - 1) * nz1;
-    h[0] = (TR)((double)h[0] + alpha * c.S[OTBL_S_IDX]);
+    h[0] = (TR)((double)h[0] + alpha * idx);
   }
 }
 
@@ -1475,10 +1537,11 @@ cudaError_t launch_twiddles(otbl_ctx *c) {
   return cudaGetLastError();
 }
 
-cudaError_t launch_reset_max(otbl_ctx *c) {
-  k_reset_max<<<(c->cfg.ny + 1 + 255) / 256, 256, 0, c->stream>>>(c->st, c->w.vm_bits, c->cfg.ny);
-  c->launches += 1;
-  return cudaGetLastError();
+static bool products_in_registers(int M) { return M >= 16 && M <= 256 && !getenv("OTBL_PRODUCTS_SMEM"); }
+// one launch for the three parts: below 12 thousand rows a part takes one wave
+// of CTAs or less (129x65x64: 22 us in three launches)
+bool products_merged(const otbl_ctx *c) {
+  return c->cfg.nx > 2 && c->cfg.nx * c->cfg.ny < 12000 && products_in_registers(c->cfg.nz / 2);
 }
 
 template <typename T>
@@ -1508,13 +1571,19 @@ static cudaError_t products_t(otbl_ctx *c, int setstep, int part, const ZTabT<T>
   const dim3 g((c->cfg.ny + (part == 0 ? 1 : 0) + 3) / 4, c->cfg.nx - (part == 1 ? 2 : 0));
   // the register-pipelined transforms for M = 16..256; other M (and
   // OTBL_PRODUCTS_SMEM=1) the shared-memory kernel
-  if (M >= 16 && M <= 256 && !getenv("OTBL_PRODUCTS_SMEM")) {
-    const int nlines = (c->cfg.ny + (part == 0 ? 1 : 0)) * (c->cfg.nx - (part == 1 ? 2 : 0));
+  if (products_in_registers(M)) {
+    const int nx = c->cfg.nx, ny = c->cfg.ny;
+    const int n[3] = {prod_lines<0>(nx, ny), prod_lines<1>(nx, ny), prod_lines<2>(nx, ny)};
     auto go = [&](auto m) {
       constexpr int MM = decltype(m)::value, per = 128 / ZGroup<MM>::G;
       const size_t smem = (size_t)per * ZGroup<MM>::BUF * sizeof(V2<T>);
+      auto nb = [&](int p) { return (n[p] + per - 1) / per; };
+      if (part == 3) {
+        k_products_all<MM, T><<<nb(0) + nb(1) + nb(2), 128, smem, c->stream>>>(c->dc, z, a);
+        return;
+      }
       auto k = part == 0 ? k_products_r<MM, T, 0> : (part == 1 ? k_products_r<MM, T, 1> : k_products_r<MM, T, 2>);
-      k<<<(nlines + per - 1) / per, 128, smem, c->stream>>>(c->dc, z, a, nlines);
+      k<<<nb(part), 128, smem, c->stream>>>(c->dc, z, a);
     };
     if (M == 256)
       go(std::integral_constant<int, 256>{});

@@ -529,8 +529,6 @@ extern "C" int otbl_rhsp(otbl_ctx *c, int m, int setstep) {
 }
 
 static int rhsp_issue(otbl_ctx *c, int m, int setstep) {
-  if (m == 1) LAUNCH(c, launch_energies(c));
-  if (setstep) LAUNCH(c, launch_reset_max(c));
   cudaStream_t main_s = c->stream;
   // with per-kernel timing on, everything runs on the context stream, so
   // that each event pair brackets its own kernels only
@@ -539,13 +537,14 @@ static int rhsp_issue(otbl_ctx *c, int m, int setstep) {
   // Streams (all forks and joins by events, so a graph capture records them):
   //   main:    interpxx, products 0 (uu, uw), [interpyy] products 2 (uv),
   //            difvisxx, [genflu] u tail, [products 1] v and w tails
-  //   side:    interpyy, [products 2] k_dt, genflu's tables, [difvisxx]
+  //   side:    interpyy, (m = 1) the energies, [products 2] k_dt, genflu's tables, [difvisxx]
   //            genflu's plane 1
   //   side_lo: [products 2] products 1 (vw, vv, ww)
-  // With the streamed tail (the largest boxes): main: [k_dt] u tail ([genflu]
+  // Small boxes (products_merged): all products and all tails in one launch
+  // each on main. With the streamed tail (the largest boxes): main: [k_dt] u tail ([genflu]
   // before its velocity write), [products 1] v tail, [w tail]; side: [products
   // 1] w tail on line scratch of its own.
-  // interpyy and interpxx only read the state; each products part reads and
+  // interpyy, interpxx and the energies only read the state; each products part reads and
   // writes fields no kernel beside it touches; difvisxx reads parts 0 and 2;
   // k_dt needs the CFL maxima of parts 0 and 2; genflu needs dt, writes plane
   // 1 of u, v, w after difvisxx has read it and reads plane xout before the
@@ -556,21 +555,25 @@ static int rhsp_issue(otbl_ctx *c, int m, int setstep) {
   c->stream = side;
   e = launch_interpy(c);
   if (e == cudaSuccess) e = cudaEventRecord(c->ev[1], side);
+  if (e == cudaSuccess && m == 1) e = launch_energies(c);
   c->stream = main_s;
   if (check(c, e, "launch_interpy") != OTBL_OK) return OTBL_ERR_CUDA;
   LAUNCH(c, launch_interpx(c));
-  LAUNCH(c, launch_products(c, setstep, 0));
+  const bool merged = products_merged(c);
+  if (!merged) LAUNCH(c, launch_products(c, setstep, 0));
   OTBL_CUDA_TRY(c, cudaStreamWaitEvent(main_s, c->ev[1], 0));
-  LAUNCH(c, launch_products(c, setstep, 2));
+  LAUNCH(c, launch_products(c, setstep, merged ? 3 : 2));
   OTBL_CUDA_TRY(c, cudaEventRecord(c->ev[0], main_s));
   // part 1 needs only interpyy, but started beside parts 0 and 2 it measured
   // no faster (42.8 against 42.7 ms per FP64 RK3 step), so it follows them
-  OTBL_CUDA_TRY(c, cudaStreamWaitEvent(side_lo, c->ev[0], 0));
-  c->stream = side_lo;
-  e = launch_products(c, setstep, 1);
-  if (e == cudaSuccess) e = cudaEventRecord(c->ev[4], side_lo);
-  c->stream = main_s;
-  if (check(c, e, "products part 1") != OTBL_OK) return OTBL_ERR_CUDA;
+  if (!merged) {
+    OTBL_CUDA_TRY(c, cudaStreamWaitEvent(side_lo, c->ev[0], 0));
+    c->stream = side_lo;
+    e = launch_products(c, setstep, 1);
+    if (e == cudaSuccess) e = cudaEventRecord(c->ev[4], side_lo);
+    c->stream = main_s;
+    if (check(c, e, "products part 1") != OTBL_OK) return OTBL_ERR_CUDA;
+  }
   OTBL_CUDA_TRY(c, cudaStreamWaitEvent(side, c->ev[0], 0));
   c->stream = side;
   e = launch_dt(c, m, setstep);
@@ -601,6 +604,10 @@ static int rhsp_issue(otbl_ctx *c, int m, int setstep) {
     return OTBL_OK;
   }
   OTBL_CUDA_TRY(c, cudaStreamWaitEvent(main_s, c->ev[3], 0));
+  if (merged) {
+    LAUNCH(c, launch_final(c, 1 | 2 | 4));
+    return OTBL_OK;
+  }
   LAUNCH(c, launch_final(c, 1));
   OTBL_CUDA_TRY(c, cudaStreamWaitEvent(main_s, c->ev[4], 0));
   LAUNCH(c, launch_final(c, 2 | 4));

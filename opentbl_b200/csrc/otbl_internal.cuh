@@ -42,7 +42,7 @@ struct DState {
   double var1, var2, var3, var4, rkk, varstep;  // RK3 factors of the substep
   double umax, wmax, vmax;
   double ener[15];  // energies of rhsp.F90:116 (module statistics, mod.F90:264)
-  unsigned long long umax_bits, wmax_bits;      // atomicMax targets (>= 0)
+  unsigned long long umax_bits, wmax_bits;      // atomicMax targets (>= 0), zeroed by k_dt when consumed
   int err;        // OTBL_ERR_NAN when the dt reduction saw a non-finite value
   int dt_frozen;  // fixed-dt mode: dt taken
   int pad[2];
@@ -225,7 +225,9 @@ cudaError_t launch_interpx(otbl_ctx *c);
 cudaError_t launch_interpy(otbl_ctx *c);
 // part 0: uu, uw and the u, w CFL maxima; part 2: uv and the v maxima;
 // part 1: vw, vv, ww
+// part 3: all of them (products_merged)
 cudaError_t launch_products(otbl_ctx *c, int setstep, int part);
+bool products_merged(const otbl_ctx *c);
 cudaError_t launch_difvisx(otbl_ctx *c);
 cudaError_t launch_dt(otbl_ctx *c, int m, int setstep);
 // genflu's two kernels: the tables (needs dt, reads plane xout) and the new
@@ -251,7 +253,6 @@ void build_stream_maps(otbl_ctx *c);
 cudaError_t prepare_stream(otbl_ctx *c);
 cudaError_t launch_outflow(otbl_ctx *c);
 cudaError_t launch_pois(otbl_ctx *c, int m);
-cudaError_t launch_reset_max(otbl_ctx *c);
 cudaError_t launch_boun_all(otbl_ctx *c);
 cudaError_t launch_tiempo(otbl_ctx *c);
 cudaError_t launch_energies(otbl_ctx *c);
