@@ -587,18 +587,18 @@ __global__ void __launch_bounds__(256) k_genflu_tab(DCoef c, GenArgs a) {
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
     if (t == 0) {
-    *a.timec = timec;
-    *a.utauout = sqrt(fabs((um[2] - um[1]) / (y[2] - y[1]) / re));
-    *a.dout = y[jtop];
-    const double rthout = s * re / uinf;
-    *a.rthout = rthout;
-    const double gamma2 = rthin / rthout;
-    const double gamma1 = pow(gamma2, 0.125);
-    *a.gamma2 = gamma2;
-    *a.gamma1 = gamma1;
-    s_g1 = gamma1;
-    s_g2 = gamma2;
-    a.tab[3 * N1] = 1.0 / gamma1;  // ggg
+      *a.timec = timec;
+      *a.utauout = sqrt(fabs((um[2] - um[1]) / (y[2] - y[1]) / re));
+      *a.dout = y[jtop];
+      const double rthout = s * re / uinf;
+      *a.rthout = rthout;
+      const double gamma2 = rthin / rthout;
+      const double gamma1 = pow(gamma2, 0.125);
+      *a.gamma2 = gamma2;
+      *a.gamma1 = gamma1;
+      s_g1 = gamma1;
+      s_g2 = gamma2;
+      a.tab[3 * N1] = 1.0 / gamma1;  // ggg
     }
   }
   // rescaled grids: kk = 0 (u rows, cell centres) and kk = 1 (v rows)

@@ -332,6 +332,7 @@ extern "C" int otbl_ctx_rebind(otbl_ctx *c, const otbl_config *cfg, const double
     return OTBL_ERR_CONFIG;
   cudaSetDevice(c->device);
   OTBL_CUDA_TRY(c, cudaStreamSynchronize(c->stream));
+  drop_step_graph(c);
   otbl_coef_offsets o;
   otbl_coef_layout(cfg->nx, cfg->ny, cfg->nz, &o);
   const size_t ncoef = o.off[OTBL_C_COUNT];
@@ -368,6 +369,8 @@ extern "C" void otbl_ctx_destroy(otbl_ctx *c) {
   for (cudaEvent_t e : c->prof_pool) cudaEventDestroy(e);
   if (c->side) cudaStreamSynchronize(c->side);
   if (c->side_lo) cudaStreamSynchronize(c->side_lo);
+  if (c->step_exec) cudaGraphExecDestroy(c->step_exec);
+  if (c->stale_exec) cudaGraphExecDestroy(c->stale_exec);
   for (void *p : c->allocs) cudaFree(p);
   for (cudaEvent_t e : c->ev)
     if (e) cudaEventDestroy(e);
@@ -636,14 +639,79 @@ extern "C" int otbl_substep(otbl_ctx *c, int m, int setstep) {
   return otbl_pois(c, m);
 }
 
+static int step_direct(otbl_ctx *c) {
+  for (int m = 1; m <= 3; ++m) {
+    const int r = otbl_substep(c, m, m == 1);
+    if (r != OTBL_OK) return r;
+  }
+  LAUNCH(c, launch_tiempo(c));
+  return OTBL_OK;
+}
+
+// One RK3 step as a CUDA graph. A step of a small box is some 40 launches and
+// 40 event calls, 220 us of host time, more than its kernels take when a few
+// boxes share the GPU; the replay is one call. It holds the pointers, sizes
+// and options of the step's launches, so whatever changes them drops it
+// (otbl_bind_state, otbl_ctx_rebind, the tuning calls), and it is captured
+// only after three plain steps since then, so that a short run, or one that
+// rebinds every step, never pays for the capture (1-2 ms). Boxes above 4
+// million points are bound by their kernels. Not used while the context's
+// stream is being captured or its kernels are timed.
+static bool step_graph(otbl_ctx *c) {
+  const double pts = (double)c->cfg.nx * c->cfg.ny * c->cfg.nz;
+  if (pts > 4e6 || c->prof_on) return false;
+  cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(c->stream, &cs) != cudaSuccess || cs != cudaStreamCaptureStatusNone) return false;
+  if (c->step_exec) return true;
+  if (c->direct_steps < 3) return false;
+  if (c->stale_exec) {
+    if (cudaStreamQuery(c->stream) != cudaSuccess) return false;
+    cudaGraphExecDestroy(c->stale_exec);
+    c->stale_exec = nullptr;
+  }
+  c->direct_steps = -1000;  // after a failed capture, not again soon
+  const long long l0 = c->launches;
+  if (cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeThreadLocal) != cudaSuccess) {
+    cudaGetLastError();
+    return false;
+  }
+  const int st = step_direct(c);
+  cudaGraph_t g = nullptr;
+  const cudaError_t e = cudaStreamEndCapture(c->stream, &g);
+  c->step_kernels = c->launches - l0;
+  c->launches = l0;
+  if (st == OTBL_OK && e == cudaSuccess && g)
+    if (cudaGraphInstantiate(&c->step_exec, g, cudaGraphInstantiateFlagUseNodePriority) != cudaSuccess)
+      c->step_exec = nullptr;
+  if (g) cudaGraphDestroy(g);
+  if (!c->step_exec) {
+    cudaGetLastError();
+    c->err.clear();
+    return false;
+  }
+  return true;
+}
+
+namespace otbl {
+void drop_step_graph(otbl_ctx *c) {
+  c->direct_steps = 0;
+  if (c->step_exec) c->stale_exec = c->step_exec;  // built only once the last stale one was destroyed
+  c->step_exec = nullptr;
+}
+}  // namespace otbl
+
 extern "C" int otbl_advance(otbl_ctx *c, int nsteps) {
   if (!c || nsteps < 0) return OTBL_ERR_ARG;
+  cudaSetDevice(c->device);
   for (int s = 0; s < nsteps; ++s) {
-    for (int m = 1; m <= 3; ++m) {
-      const int r = otbl_substep(c, m, m == 1);
-      if (r != OTBL_OK) return r;
+    if (step_graph(c)) {
+      OTBL_CUDA_TRY(c, cudaGraphLaunch(c->step_exec, c->stream));
+      c->launches += c->step_kernels;
+      continue;
     }
-    LAUNCH(c, launch_tiempo(c));
+    const int r = step_direct(c);
+    if (r != OTBL_OK) return r;
+    ++c->direct_steps;
   }
   return OTBL_OK;
 }
@@ -676,6 +744,7 @@ static int bind_fields(otbl_ctx *c, double *const *ptr, const bool *use) {
     changed = true;
   }
   if (!changed) return OTBL_OK;
+  drop_step_graph(c);
   for (int id = 0; id < OTBL_F_COUNT; ++id)
     if (use[id]) c->f[id] = ptr[id] ? ptr[id] : c->f_own[id];
   if (!getenv("OTBL_NO_TMA")) {

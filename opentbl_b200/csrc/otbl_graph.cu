@@ -191,6 +191,7 @@ extern "C" int otbl_autotune(otbl_ctx *c, int *choice) {
     cudaEventDestroy(e0);
     return OTBL_ERR_CUDA;
   }
+  drop_step_graph(c);
   const long long l0 = c->launches;
   int st = OTBL_OK;
   for (int k = 0; k < 3 && st == OTBL_OK; ++k) {
@@ -238,6 +239,7 @@ extern "C" int otbl_set_tuning(otbl_ctx *c, const int *bs) {
   if (!c || !bs) return OTBL_ERR_ARG;
   for (int k = 0; k < 3; ++k)
     if (bs[k] != 32 && bs[k] != 64 && bs[k] != 128) return OTBL_ERR_ARG;
+  drop_step_graph(c);
   for (int k = 0; k < 3; ++k) c->tune_bs[k] = bs[k];
   return OTBL_OK;
 }

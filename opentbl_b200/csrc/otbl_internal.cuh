@@ -172,6 +172,11 @@ struct otbl_ctx {
   size_t bytes;
   long long launches;
   std::string err;
+  // one RK3 step as a CUDA graph, replayed by otbl_advance on small boxes
+  // (step_graph in otbl_capi.cu); `stale` waits to be destroyed once idle
+  cudaGraphExec_t step_exec = nullptr, stale_exec = nullptr;
+  long long step_kernels = 0;
+  int direct_steps = 0;  // since the last change of what a step launches
   // optional per-kernel timing: a CUDA event pair around every launch
   bool prof_on = false;
   struct ProfRec {
@@ -191,6 +196,8 @@ enum ProfKind {
 extern const char *const kProfNames[PK_COUNT];
 void prof_begin(otbl_ctx *c, int kind);
 void prof_end(otbl_ctx *c);
+// forgets the step graph: what a step launches has changed
+void drop_step_graph(otbl_ctx *c);
 }  // namespace otbl
 
 // Mixed path: the Poisson solve (x-DCTs, y-systems, phi) of a spanwise mode

@@ -153,8 +153,10 @@ class Server:
         self.idle = {}
         self.used = 0
         self.tuning = {}  # CTA sizes picked by the autotuner, per grid size
-        self.creator = ThreadPoolExecutor(max_workers=1)
-        self.pending = None  # (request, future of its new slot)
+        # the slots of the next two requests are prepared side by side: a small
+        # box runs its steps in less time than one preparation takes
+        self.creator = ThreadPoolExecutor(max_workers=2)
+        self.pending = deque()  # (request, future of its slot, new), in queue order
         self.stats = {"created": 0, "reused": 0, "evicted": 0, "graph_launches": 0,
                       "direct_steps": 0, "peak_bytes": 0, "peak_active": 0,
                       "create_s": 0.0, "rebind_s": 0.0, "capture_s": 0.0}
@@ -197,32 +199,34 @@ class Server:
         self.stats["capture_s"] += time.perf_counter() - t
         return slot
 
-    def _acquire(self, req: Request, init: dict):
-        """A slot for the request at the head of the queue, prepared in the
-        background: an idle slot of its grid size re-bound, or a new one
-        (None until it is ready, or while memory is short)."""
+    def _start(self, req: Request, init: dict) -> bool:
+        """Begins preparing a slot for `req` in the background: an idle slot
+        of its grid size re-bound, or a new one (False while memory is
+        short)."""
         key = size_key(req.cfg)
-        if self.pending is not None:
-            preq, fut, created = self.pending
-            if preq is not req or not fut.done():
-                return None
-            self.pending = None
-            self.stats["created" if created else "reused"] += 1
-            return fut.result()
         lst = self.idle.get(key)
         if lst:
             s = lst.pop()
-            self.pending = (req, self.creator.submit(self._prepare, req, init, s, s.nbytes, key), False)
-            return None
+            self.pending.append((req, self.creator.submit(self._prepare, req, init, s, s.nbytes, key), False))
+            return True
         need = self._bytes(req.cfg, init)
         while self.used + need > self.budget and self._evict_one():
             pass
         if self.used + need > self.budget:
-            return None
+            return False
         self.used += need
         self.stats["peak_bytes"] = max(self.stats["peak_bytes"], self.used)
-        self.pending = (req, self.creator.submit(self._prepare, req, init, None, need, key), True)
-        return None
+        self.pending.append((req, self.creator.submit(self._prepare, req, init, None, need, key), True))
+        return True
+
+    def _acquire(self):
+        """The prepared slot of the request at the head of the queue (None
+        until it is ready)."""
+        if not self.pending or not self.pending[0][1].done():
+            return None
+        _, fut, created = self.pending.popleft()
+        self.stats["created" if created else "reused"] += 1
+        return fut.result()
 
     def _issue(self, s: _Slot):
         """Next chunk of the slot's request: a graph launch of `chunk` steps,
@@ -263,7 +267,7 @@ class Server:
         queue = deque()
         active = []
         results = []
-        head = None  # the queue head and its initial state
+        head = None  # the next request to prepare a slot for and its initial state
         t0 = time.perf_counter()
         while pending or queue or active:
             now = time.perf_counter() - t0
@@ -272,14 +276,17 @@ class Server:
             did = False
             # admission, first come first served
             while queue and len(active) < self.max_active:
-                req = queue[0]
-                if head is None or head[0] is not req:
-                    head = (req, self.templates.get(req.cfg))
-                init = head[1]
-                s = self._acquire(req, init)
+                ahead = min(2, self.max_active - len(active), len(queue))
+                while len(self.pending) < ahead:
+                    req = queue[len(self.pending)]
+                    if head is None or head[0] is not req:
+                        head = (req, self.templates.get(req.cfg))
+                    if not self._start(*head):
+                        break
+                s = self._acquire()
                 if s is None:
                     break
-                queue.popleft()
+                req = queue.popleft()
                 s.req = req
                 s.remaining = req.steps
                 s.admitted = time.perf_counter() - t0
