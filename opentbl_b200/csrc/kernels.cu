@@ -1387,40 +1387,55 @@ __global__ void __launch_bounds__(128, M >= 128 ? 3 : 5) k_fourxz_r(ZTab z, doub
   }
 }
 
-// cosftx on pencils c(nx, nlines), elements 2..nx; two real lines per CTA
-__global__ void __launch_bounds__(256) k_cosftx(XTab x, double *cp, int nx, int nlines, int iopt) {
-  extern __shared__ double2 xsm[];
-  const int n = x.n;
-  const int l0 = blockIdx.x * 2;
-  double *la = cp + (size_t)l0 * nx + 1;
-  double *lb = (l0 + 1 < nlines) ? cp + (size_t)(l0 + 1) * nx + 1 : nullptr;
+// cosftx on pencils c(nx, nlines), elements 2..nx; MB pairs of real lines per
+// CTA, each pair one complex line, transformed together as in k_pois_fwd (one
+// pair per CTA waited at the CTA barriers of its passes)
+// NN: the length n when it is a power of two from 256 to 1024, else 0
+template <int MB, int NT, int NN>
+__global__ void __launch_bounds__(NT, NN > 0 && NT >= 512 ? 2 : 1) k_cosftx(XTab x, double *cp, int nx, int nlines,
+                                                                           int iopt) {
+  extern __shared__ __align__(16) unsigned char xsm_raw[];
+  double2 *xsm = reinterpret_cast<double2 *>(xsm_raw);
+  constexpr int G = NT / MB;
+  const int n = NN > 0 ? NN : x.n, ld = xline_ld<double2>(n, MB), l = threadIdx.x / G, t = threadIdx.x % G;
+  const int l0 = (blockIdx.x * MB + l) * 2;
+  double *la = l0 < nlines ? cp + (size_t)l0 * nx + 1 : nullptr;
+  double *lb = l0 + 1 < nlines ? la + nx : nullptr;
+  double2 *line = xsm + l * ld;
   if (iopt < 0) {
-    for (int tt = threadIdx.x; tt < n; tt += 256) {
+    for (int tt = t; tt < n; tt += G) {
       const int dst = (tt & 1) ? n - 1 - (tt >> 1) : (tt >> 1);
-      xsm[dst] = make_double2(la[tt], lb ? lb[tt] : 0.0);
+      line[xpad<double2>(dst)] = make_double2(la ? la[tt] : 0.0, lb ? lb[tt] : 0.0);
     }
     __syncthreads();
-    block_fft<-1, 1>(xsm, n, x.tw);
+    if constexpr (NN > 0)
+      block_fft_lines_n<-1, NT, NN>(line, x.tw, t, G);
+    else
+      block_fft_lines<-1, NT>(line, n, x.tw, t, G);
     const double dnf = 1.0 / (double)n;
-    for (int kk = threadIdx.x; kk < n; kk += 256) {
-      const double2 V = xsm[kk], Vm = xsm[kk == 0 ? 0 : n - kk];
+    for (int kk = t; kk < n; kk += G) {
+      const double2 V = line[xpad<double2>(kk)], Vm = line[xpad<double2>(kk == 0 ? 0 : n - kk)];
       const double2 wq = __ldg(x.tw2 + kk);
       const double2 y = cadd(cmul(wq, V), cmul(cconj(wq), Vm));
-      la[kk] = dnf * y.x;
+      if (la) la[kk] = dnf * y.x;
       if (lb) lb[kk] = dnf * y.y;
     }
   } else {
-    for (int kk = threadIdx.x; kk < n; kk += 256) {
-      const double2 Y = make_double2(la[kk], lb ? lb[kk] : 0.0);
-      const double2 Ym = kk > 0 ? make_double2(la[n - kk], lb ? lb[n - kk] : 0.0) : make_double2(0.0, 0.0);
+    for (int kk = t; kk < n; kk += G) {
+      const double2 Y = make_double2(la ? la[kk] : 0.0, lb ? lb[kk] : 0.0);
+      const double2 Ym =
+          kk > 0 ? make_double2(la ? la[n - kk] : 0.0, lb ? lb[n - kk] : 0.0) : make_double2(0.0, 0.0);
       const double2 d = make_double2(Y.x + Ym.y, Y.y - Ym.x);
-      xsm[kk] = cmul(cconj(__ldg(x.tw2 + kk)), d);
+      line[xpad<double2>(kk)] = cmul(cconj(__ldg(x.tw2 + kk)), d);
     }
     __syncthreads();
-    block_fft<1, 1>(xsm, n, x.tw);
-    for (int tt = threadIdx.x; tt < n; tt += 256) {
-      const double2 V = xsm[(tt & 1) ? n - 1 - (tt >> 1) : (tt >> 1)];
-      la[tt] = 0.5 * V.x;
+    if constexpr (NN > 0)
+      block_fft_lines_n<1, NT, NN>(line, x.tw, t, G);
+    else
+      block_fft_lines<1, NT>(line, n, x.tw, t, G);
+    for (int tt = t; tt < n; tt += G) {
+      const double2 V = line[xpad<double2>((tt & 1) ? n - 1 - (tt >> 1) : (tt >> 1))];
+      if (la) la[tt] = 0.5 * V.x;
       if (lb) lb[tt] = 0.5 * V.y;
     }
   }
@@ -1997,9 +2012,28 @@ cudaError_t launch_fourxz(otbl_ctx *c, double *fou, double *phys, int iopt, int 
 }
 
 cudaError_t launch_cosftx(otbl_ctx *c, double *cp, int nlines, int iopt) {
-  const int n = c->cfg.nx - 1;
-  const size_t smem = (size_t)n * sizeof(double2);
-  k_cosftx<<<(nlines + 1) / 2, 256, smem, c->stream>>>(xtab(c), cp, c->cfg.nx, nlines, iopt);
+  const int n = c->cfg.nx - 1, MB = pois_mb(n);
+  const size_t smem = (size_t)MB * xline_ld<double2>(n, MB) * sizeof(double2);
+  auto go = [&](auto mb, auto nn) {
+    constexpr int B = decltype(mb)::value, NN = decltype(nn)::value;
+    auto k = n * B >= 2048 ? k_cosftx<B, 512, NN> : k_cosftx<B, 256, NN>;
+    if (smem > 48 * 1024) cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    k<<<(nlines + 2 * B - 1) / (2 * B), n * B >= 2048 ? 512 : 256, smem, c->stream>>>(xtab(c), cp, c->cfg.nx, nlines,
+                                                                                     iopt);
+  };
+  using std::integral_constant;
+  switch (n) {
+    case 256: go(integral_constant<int, pois_mb(256)>{}, integral_constant<int, 256>{}); break;
+    case 512: go(integral_constant<int, pois_mb(512)>{}, integral_constant<int, 512>{}); break;
+    case 1024: go(integral_constant<int, pois_mb(1024)>{}, integral_constant<int, 1024>{}); break;
+    default:
+      switch (MB) {
+        case 8: go(integral_constant<int, 8>{}, integral_constant<int, 0>{}); break;
+        case 4: go(integral_constant<int, 4>{}, integral_constant<int, 0>{}); break;
+        case 2: go(integral_constant<int, 2>{}, integral_constant<int, 0>{}); break;
+        default: go(integral_constant<int, 1>{}, integral_constant<int, 0>{});
+      }
+  }
   c->launches += 1;
   return cudaGetLastError();
 }
