@@ -337,14 +337,14 @@ void otbl_graph_destroy(otbl_graph *g);
 /* OTBL_OK when every call issued on the context has finished, OTBL_BUSY
  * while work is in flight (never blocks) */
 int otbl_query(otbl_ctx *ctx);
-/* Autotuner (no counterpart in the reference): times CTA sizes of 32, 64
- * and 128 threads for the x-interpolation, d/dx and y-interpolation line
- * kernels on this context's box and precision and keeps the fastest. Those
- * kernels write only work arrays, so the state is unchanged; the arithmetic
- * does not depend on the CTA size. choice (3 ints, may be NULL) receives the
- * sizes picked. Call before otbl_graph_create. Synchronizes. */
+/* Autotuner (no counterpart in the reference): times full, half
+ * and quarter CTA tiles (128, 64, 32) for the x-interpolation, d/dx and
+ * y-interpolation line kernels on this context's box and precision and keeps
+ * the fastest. Those kernels write only work arrays, so the state is
+ * unchanged; the arithmetic does not depend on the tile. choice (3 ints, may
+ * be NULL) receives the tiles picked. Call before otbl_graph_create. Synchronizes. */
 int otbl_autotune(otbl_ctx *ctx, int *choice);
-/* sets the three CTA sizes (each 32, 64 or 128) without timing, e.g. those
+/* sets the three tiles (each 32, 64 or 128) without timing, e.g. those
  * otbl_autotune picked for another context of the same box size */
 int otbl_set_tuning(otbl_ctx *ctx, const int *bs);
 /* failure detection of the device-side waits (no counterpart in the

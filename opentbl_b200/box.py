@@ -167,7 +167,7 @@ class Box:
         self._check(self.L.otbl_sync(self.h), "otbl_sync")
 
     def autotune(self) -> tuple:
-        """CTA sizes for k_interpx, k_difvisx, k_interpy picked by timing."""
+        """CTA tiles for interpxx, difvisxx, interpyy picked by timing."""
         ch = (ctypes.c_int * 3)()
         self._check(self.L.otbl_autotune(self.h, ch), "otbl_autotune")
         return tuple(ch)

@@ -1,6 +1,6 @@
 """Builds the in-tree extension opentbl_b200/libotbl.so for sm_100a.
 
-One nvcc invocation compiles the CUDA kernels (csrc/kernels.cu), the C ABI
+nvcc compiles the CUDA kernels (csrc/kernels.cu, csrc/k_*.cu), the C ABI
 (csrc/otbl_capi.cu) and the host-side coefficient setup (csrc/coef.cpp) into
 a shared library with the CUDA runtime linked statically, so the library has
 no dependency on torch and can be bound from C, Fortran (iso_c_binding) or

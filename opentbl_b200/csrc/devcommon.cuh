@@ -20,13 +20,6 @@ __device__ __forceinline__ double nmax(double m, double v) {
   return (m != m) ? m : ((v != v) ? v : fmax(m, v));
 }
 
-// Asynchronous 8-byte global -> shared copy (cp.async, zero-filled when
-// !valid: the source size operand is 0 and nothing is read from `g`).
-__device__ __forceinline__ void cp_async8(double *s, const double *g, bool valid) {
-  const unsigned sa = (unsigned)__cvta_generic_to_shared(s);
-  const int sz = valid ? 8 : 0;
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;\n" ::"r"(sa), "l"(g), "r"(sz) : "memory");
-}
 // Waits for every cp.async this thread issued (the caller then syncs the CTA).
 __device__ __forceinline__ void cp_async_wait_all() {
   asm volatile("cp.async.commit_group;\ncp.async.wait_group 0;\n" ::: "memory");

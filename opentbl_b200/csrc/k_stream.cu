@@ -9,7 +9,7 @@
 // hide their latency. Below the limits of stream_* the chunked solves win (by
 // 1.1 to 8, the more the fewer the lines).
 //   k_xline_t            interpxx, difvisxx
-//   k_interpy_t          interpyy (FP64)
+//   k_interpy_t          interpyy (most boxes with nz >= 128)
 //   k_final_ta, tb, s2   the tail of rhsp (rhsp.F90:291-484)
 #include <cudaTypedefs.h>
 
@@ -323,7 +323,8 @@ cudaError_t launch_xlines_stream(otbl_ctx *c, bool dv) {
 // ---------------------------------------------------------------------------
 struct StreamYArgs {
   const double *in[3];
-  double *out[3], *ck[3];
+  void *out[3];
+  double *ck[3];
   int which[3];
 };
 constexpr int KYT = 8;  // rows per segment
@@ -332,9 +333,9 @@ constexpr int KYT = 8;  // rows per segment
 // field; thread 0 loads, for the next segment of KYT rows, a box of 128 kr x
 // KYT+2 rows of the input into a two-stage shared-memory ring on mbarriers
 // (bounded waits); the segments run forward (0..nseg-1), then backward.
-__global__ void __launch_bounds__(128) k_interpy_t(DCoef c, StreamYArgs a, int *err,
+template <typename T>
+__global__ void __launch_bounds__(128) k_interpy_t(DCoefT<T> c, StreamYArgs a, int *err,
                                                    const __grid_constant__ YMaps maps) {
-  using T = double;
   constexpr int K = KYT, TB = 128, R = K + 2;
   constexpr int RC = K * 8 * (int)sizeof(T);  // the segment's coefficient rows
   constexpr int STG = R * TB * 8 + RC;
@@ -366,8 +367,8 @@ __global__ void __launch_bounds__(128) k_interpy_t(DCoef c, StreamYArgs a, int *
   const size_t S = nz1;
   const int col = (i - 1) * nz1 + krc;
   const double *g = pick3(a.in, f) + (size_t)(i - 1) * jin * nz1 + krc;
-  T *o = pick3(a.out, f) + (size_t)(i - 1) * ny * nz1 + krc;
-  T *ck = pick3(a.ck, f) + col;
+  T *o = static_cast<T *>(pick3(a.out, f)) + (size_t)(i - 1) * ny * nz1 + krc;
+  T *ck = reinterpret_cast<T *>(pick3(a.ck, f)) + col;
   const T *ib = c.inby;
   auto G = [&](int r) { return (T)__ldg(g + (size_t)min(max(r, 0), jin - 1) * S); };
   T b0 = T(0), bN;
@@ -431,8 +432,8 @@ __global__ void __launch_bounds__(128) k_interpy_t(DCoef c, StreamYArgs a, int *
 // 1: v-type input, v): interpyy's right-hand-side weights econ[2r],
 // econ[2r+1] and LU coefficients iny[3r..3r+2]; the rest 0. k_interpy_t's
 // ring stages a segment's rows with its field box.
-__global__ void __launch_bounds__(128) k_y_rows(DCoef c, double *tab) {
-  using T = double;
+template <typename T>
+__global__ void __launch_bounds__(128) k_y_rows(DCoefT<T> c, T *tab) {
   const int ny = c.ny;
   const int e = blockIdx.x * blockDim.x + threadIdx.x;
   if (e >= 2 * ny) return;
@@ -477,7 +478,6 @@ static bool encode_table(CUtensorMap *m, const void *base, size_t esz, int width
 
 static bool build_y_maps(otbl_ctx *c) {
   const int K = KYT;
-  if (c->mixed) return c->ymaps_ok = false;  // FP32: the chunked solve wins at every size
   const int nx = c->cfg.nx, ny = c->cfg.ny, nz1 = c->dc.nz1;
   const double *in[3] = {c->f[OTBL_F_U], c->f[OTBL_F_W], c->f[OTBL_F_V]};
   const int rows[3] = {ny + 1, ny + 1, ny};
@@ -485,34 +485,51 @@ static bool build_y_maps(otbl_ctx *c) {
   const int which[3] = {0, 0, 1};
   for (int f = 0; f < 3 && ok; ++f) {
     ok = encode_field(&c->ymi.g[f], in[f], 8, nx, rows[f], nz1, K + 2, 1);
-    ok = ok && encode_table(&c->ymi.r[f], c->w.yrowc + (size_t)which[f] * ny * 8, 8, 8, ny, K);
+    const size_t ew = c->mixed ? sizeof(float) : sizeof(double);
+    const char *tab = reinterpret_cast<const char *>(c->w.yrowc) + (size_t)which[f] * ny * 8 * ew;
+    ok = ok && encode_table(&c->ymi.r[f], tab, ew, 8, ny, K);
   }
   c->ymaps_ok = ok;
   return ok;
 }
 
-// Streamed interpyy against the chunked one, us per FP64 substep on B200:
-// 1025x193x512 (174 thousand modes) 827 : 957, 1025x48x512 179 : 214,
-// 721x96x256 (61 thousand) 163 : 167, 513x129x256 (44 thousand) 176 : 161,
-// 257x97x128 (11 thousand) 39 : 33; FP32 659 : 653 at 1025x193x512, 165 : 159,
-// 156 : 112 and 37 : 23.
-bool stream_interpy(const otbl_ctx *c) { return c->ymaps_ok && c->cfg.nx * (c->dc.nz1 / 2) > 50000; }
+// Streamed interpyy against the chunked one, us per substep alone: FP64
+// 1025x193x512 827 : 957, 513x129x256 176 : 161, 257x97x128 39 : 33; FP32 659 :
+// 653, 156 : 112, 37 : 23. But it runs beside interpxx, so what counts is how
+// much of the GPU it takes: three boxes at once, us per RK3 step, 257x97x128
+// 1234 : 1277, 81x150x128 876 : 898, 33x100x512 934 : 968, 513x129x256 6885 :
+// 6963; with nz = 64, whose 42 columns fill a third of a CTA, 385x97x64 1009 :
+// 967.
+// FP32 gains only where the blocks of 128 columns are nearly full: 33x100x512
+// 619 : 664, 1025x193x512 28563 : 29047, but 257x97x128 1062 : 1061 and slower alone.
+bool stream_interpy(const otbl_ctx *c) {
+  const int nz1 = c->dc.nz1, filled = 100 * nz1 / ((nz1 + 127) / 128 * 128);
+  return c->ymaps_ok && (c->mixed ? filled > 85 : nz1 >= 84);
+}
 
-cudaError_t launch_interpy_stream(otbl_ctx *c) {
+template <typename T>
+static void interpy_t_launch(otbl_ctx *c, const DCoefT<T> &dc) {
   StreamYArgs a;
   const double *ins[3] = {c->f[OTBL_F_U], c->f[OTBL_F_W], c->f[OTBL_F_V]};
   void *outs[3] = {c->w.uy, c->w.wy, c->w.vy};
-  double *cks[3] = {c->w.s1, c->w.s2, c->w.s3};  // FP64 interpxx beside it uses none
+  double *cks[3] = {c->w.t1, c->w.t2, c->w.t3};  // interpxx beside it uses s1..s3
   for (int f = 0; f < 3; ++f) {
     a.in[f] = ins[f];
-    a.out[f] = static_cast<double *>(outs[f]);
+    a.out[f] = outs[f];
     a.ck[f] = cks[f];
     a.which[f] = f == 2;
   }
   const dim3 gt((c->dc.nz1 + 127) / 128, c->cfg.nx, 3);
-  const int sm = 2 * ((KYT + 2) * 128 * 8 + KYT * 8 * 8) + 128;
-  cudaFuncSetAttribute(k_interpy_t, cudaFuncAttributeMaxDynamicSharedMemorySize, sm);
-  k_interpy_t<<<gt, 128, sm, c->stream>>>(c->dc, a, &c->st->err, c->ymi);
+  const int sm = 2 * ((KYT + 2) * 128 * 8 + KYT * 8 * (int)sizeof(T)) + 128;
+  cudaFuncSetAttribute(k_interpy_t<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm);
+  k_interpy_t<T><<<gt, 128, sm, c->stream>>>(dc, a, &c->st->err, c->ymi);
+}
+
+cudaError_t launch_interpy_stream(otbl_ctx *c) {
+  if (c->mixed)
+    interpy_t_launch<float>(c, c->dcf);
+  else
+    interpy_t_launch<double>(c, c->dc);
   return cudaGetLastError();
 }
 
@@ -1028,11 +1045,16 @@ cudaError_t launch_tail_rows(otbl_ctx *c) {
 // : 3120, mixed 1925 : 2029; 257x193x512 (44 thousand) 1048 : 1195, mixed 833
 // : 821; 513x129x256 (44 thousand) 874 : 795; 1025x48x512 mixed 746 : 609;
 // 513x65x128 (22 thousand) 309 : 171, mixed 221 : 135; 257x97x128 270 : 154,
-// mixed 262 : 109.
+// mixed 262 : 109. The chunked FP64 tail fills the GPU with fewer warps: of
+// three boxes at once it takes more time where the streamed one's blocks of
+// 128 columns are well filled (nz = 512: 340 of 384; 33x100x512 903 : 968 us
+// per step), about as much at two thirds (nz = 128, 256) and less at one third.
 bool stream_tail(const otbl_ctx *c) {
   const int modes = (c->cfg.nx - 1) * (c->dc.nz1 / 2), ny = c->cfg.ny;
   if (!c->fmaps_ok || ny > 447) return false;
-  return c->mixed ? modes > 50000 && ny > 110 : modes > 50000 || (modes > 30000 && ny > 150);
+  if (c->mixed) return modes > 50000 && ny > 110;
+  const int nz1 = c->dc.nz1, filled = 100 * nz1 / ((nz1 + 127) / 128 * 128);
+  return modes > 50000 || (modes > 30000 && ny > 150) || filled > 85;
 }
 
 template <typename W>
@@ -1103,11 +1125,13 @@ void build_stream_maps(otbl_ctx *c) {
 // the per-plane and per-row coefficient tables of the rings
 cudaError_t prepare_stream(otbl_ctx *c) {
   const int n = 4 * c->cfg.nx, m = 2 * c->cfg.ny;
-  if (c->mixed)
+  if (c->mixed) {
     k_x_rows<float><<<(n + 127) / 128, 128, 0, c->stream>>>(c->dcf, static_cast<float *>(c->w.xrowc));
-  else
+    k_y_rows<float><<<(m + 127) / 128, 128, 0, c->stream>>>(c->dcf, reinterpret_cast<float *>(c->w.yrowc));
+  } else {
     k_x_rows<double><<<(n + 127) / 128, 128, 0, c->stream>>>(c->dc, static_cast<double *>(c->w.xrowc));
-  k_y_rows<<<(m + 127) / 128, 128, 0, c->stream>>>(c->dc, c->w.yrowc);
+    k_y_rows<double><<<(m + 127) / 128, 128, 0, c->stream>>>(c->dc, c->w.yrowc);
+  }
   c->launches += 2;
   return cudaGetLastError();
 }

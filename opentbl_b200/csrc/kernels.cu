@@ -1,24 +1,25 @@
 // CUDA kernels of the RK3 substep (sm_100a, FP64).
 //
 // Stage map (reference routine -> kernel):
-//   interpxx  lip.f90:248   k_interpx     x-lines (one thread per line), mid-point interp.
-//   interpyy  lip.f90:359   k_interpy     y-lines in Fourier space
+//   interpxx  lip.f90:248   k_xlines.cu   x-lines, mid-point interpolation
+//   interpyy  lip.f90:359   k_ylines.cu   y-lines in Fourier space
 //   fourxz    ffts.f90:27   k_products    z-lines: 9 c2r + 6 r2c per (i,j)
 //                                          line, the six nonlinear products
 //                                          and the CFL maxima (rhsp.F90:120-171,
 //                                          367-415)
-//   difvisxx  lip.f90:52    k_difvisx     x-lines (one thread per line), d/dx + d2/dx2
+//   difvisxx  lip.f90:52    k_xlines.cu   x-lines, d/dx + d2/dx2
 //   dt        rhsp.F90:214  k_dt          dt, RK3 factors, implzy LU factors
 //   genflu    genflu.F90:3  k_genflu_tab  integral quantities, rescaling tables
 //                           k_genflu_cols inflow plane + boun of plane 1
-//   rhsp tail rhsp.F90:291-484 k_final_s1 y-lines: pressure gradient, RHS
+//   rhsp tail rhsp.F90:291-484 k_ylines.cu y-lines: pressure gradient, RHS
 //                                          assembly (differzy), boun, vistyy,
 //                                          RK3 combination, implzy
 //   outflow_correction boun.f90:63  k_outflow
 //   pois      pois.f90:11   k_pois_fwd    divergence + DCT-II along x
-//                           k_pois_solve  tridiagonal in y per (x-mode, kz)
+//                           k_pois_solve  (k_ylines.cu) tridiagonal in y per (x-mode, kz)
 //                           k_pois_bwd    DCT-III along x
 //                           k_project     pressure/velocity update
+// (k_stream.cu holds the line operators of the largest boxes.)
 // The reference's transposes (change.f90) are not executed on the substep:
 // x-lines are read straight from the plane layout (threads over the
 // contiguous (j, kr) index, a walk over i with the plane stride), and the
@@ -1556,7 +1557,7 @@ static bool products_in_registers(int M) { return M >= 16 && M <= 256 && !getenv
 // one launch for the three parts: below 12 thousand rows a part takes one wave
 // of CTAs or less (129x65x64: 22 us in three launches)
 bool products_merged(const otbl_ctx *c) {
-  return c->cfg.nx > 2 && c->cfg.nx * c->cfg.ny < 12000 && products_in_registers(c->cfg.nz / 2);
+  return !stream_tail(c) && c->cfg.nx > 2 && c->cfg.nx * c->cfg.ny < 12000 && products_in_registers(c->cfg.nz / 2);
 }
 
 template <typename T>

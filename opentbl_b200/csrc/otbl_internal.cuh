@@ -68,7 +68,7 @@ struct Work {
   // streamed kernels of the largest boxes (k_stream.cu): per-plane and per-row
   // coefficients of their rings, implzy's top-down factors
   void *xrowc;                 // [2][2][nx][16] (T)
-  double *yrowc, *rowc;        // [2][ny][8], [2][ny+2][16]
+  double *yrowc, *rowc;        // [2][ny][8] (T), [2][ny+2][16]
   double *fac_u, *fac_v;
   void *ytab;                  // k_interpy's and k_tail's coefficient tables (T)
   double *tdtab;               // implzy's tables (k_tail), its factors for the current dt
@@ -130,8 +130,8 @@ struct otbl_ctx {
   cudaEvent_t ev[6] = {nullptr, nullptr, nullptr, nullptr, nullptr, nullptr};
   otbl::DCoef dc;
   otbl::DCoefT<float> dcf;  // FP32 coefficients (mixed path)
-  // threads per CTA of the line kernels that otbl_autotune times:
-  // [0] interpxx, [1] difvisxx (half the CTA's threads), [2] k_interpy; the
+  // CTA tiles (128 full, 64, 32) of the chunked line kernels that
+  // otbl_autotune times: [0] interpxx, [1] difvisxx, [2] interpyy; the
   // choice changes the schedule, never the arithmetic
   int tune_bs[3] = {128, 128, 128};
   int pois_klo = 0;  // mixed path: spanwise modes k < pois_klo solve in FP64 (kPoisCond)
