@@ -41,8 +41,21 @@ def test_one_substep(nx, ny, dy):
     assert max(e.values()) <= 1e-10, e
 
 
-def test_mixed_one_substep():
-    cfg = replace(config.TINY, nx=151, ny=50, lx=54.0, precision=1, name="lines-mixed")
+def test_wide_one_substep():
+    """nz1 = 340 fills the streamed kernels' blocks of 128 columns: interpyy and
+    the tail are streamed on a small box too."""
+    cfg = replace(config.TINY, nx=17, ny=50, nz=512, name="lines-wide")
+    init, coef = setup(cfg)
+    g, o = Box(cfg, init, coef), oracle_box(cfg, init)
+    g.substep(1, True)
+    o.substep(1, 1)
+    e = {n: rel_l2(g.field(n), o.field(n)) for n in STATE}
+    assert max(e.values()) <= 1e-11, e
+
+
+@pytest.mark.parametrize("nx,ny,nz", [(151, 50, 32), (17, 50, 512)], ids=str)
+def test_mixed_one_substep(nx, ny, nz):
+    cfg = replace(config.TINY, nx=nx, ny=ny, nz=nz, lx=12.0 * max(nx, 33) / 33, precision=1, name="lines-mixed")
     init, coef = setup(cfg)
     g, o = Box(cfg, init, coef), oracle_box(replace(cfg, precision=0), init)
     g.substep(1, True)
