@@ -314,6 +314,9 @@ int otbl_genflu_arrays(otbl_ctx *ctx, double *u, double *v, double *w);
 
 /* kernel launches issued by this context since creation */
 long long otbl_launch_count(const otbl_ctx *ctx);
+/* RK3 steps that otbl_advance replayed from the context's captured step
+ * (small boxes) instead of launching their kernels one by one */
+long long otbl_step_replays(const otbl_ctx *ctx);
 
 /* ---- CUDA graphs of RK3 steps, ensembles (no counterpart in the reference,
  *      which advances one box per MPI job) ----

@@ -144,6 +144,11 @@ class Box:
         return int(self.L.otbl_launch_count(self.h))
 
     @property
+    def replays(self) -> int:
+        """Steps of advance() that were replays of the captured step."""
+        return int(self.L.otbl_step_replays(self.h))
+
+    @property
     def device_bytes(self) -> int:
         return int(self.L.otbl_device_bytes(self.h))
 

@@ -386,6 +386,8 @@ extern "C" size_t otbl_device_bytes(const otbl_ctx *c) { return c ? c->bytes : 0
 
 extern "C" long long otbl_launch_count(const otbl_ctx *c) { return c ? c->launches : 0; }
 
+extern "C" long long otbl_step_replays(const otbl_ctx *c) { return c ? c->step_replays : 0; }
+
 extern "C" int otbl_set_field(otbl_ctx *c, int id, const double *host) {
   if (!c || !host || id < 0 || id >= OTBL_F_COUNT) return OTBL_ERR_ARG;
   cudaSetDevice(c->device);
@@ -656,12 +658,11 @@ static int step_direct(otbl_ctx *c) {
 // only after three plain steps since then, so that a short run, or one that
 // rebinds every step, never pays for the capture (1-2 ms). Boxes above 4
 // million points are bound by their kernels. Not used while the context's
-// stream is being captured or its kernels are timed.
+// stream is being captured (whose steps are recorded, not run, and are not
+// counted as plain ones) or its kernels are timed.
 static bool step_graph(otbl_ctx *c) {
   const double pts = (double)c->cfg.nx * c->cfg.ny * c->cfg.nz;
   if (pts > 4e6 || c->prof_on) return false;
-  cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
-  if (cudaStreamIsCapturing(c->stream, &cs) != cudaSuccess || cs != cudaStreamCaptureStatusNone) return false;
   if (c->step_exec) return true;
   if (c->direct_steps < 3) return false;
   if (c->stale_exec) {
@@ -703,15 +704,18 @@ void drop_step_graph(otbl_ctx *c) {
 extern "C" int otbl_advance(otbl_ctx *c, int nsteps) {
   if (!c || nsteps < 0) return OTBL_ERR_ARG;
   cudaSetDevice(c->device);
+  cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+  const bool captured = cudaStreamIsCapturing(c->stream, &cs) != cudaSuccess || cs != cudaStreamCaptureStatusNone;
   for (int s = 0; s < nsteps; ++s) {
-    if (step_graph(c)) {
+    if (!captured && step_graph(c)) {
       OTBL_CUDA_TRY(c, cudaGraphLaunch(c->step_exec, c->stream));
       c->launches += c->step_kernels;
+      ++c->step_replays;
       continue;
     }
     const int r = step_direct(c);
     if (r != OTBL_OK) return r;
-    ++c->direct_steps;
+    if (!captured) ++c->direct_steps;
   }
   return OTBL_OK;
 }

@@ -175,7 +175,7 @@ struct otbl_ctx {
   // one RK3 step as a CUDA graph, replayed by otbl_advance on small boxes
   // (step_graph in otbl_capi.cu); `stale` waits to be destroyed once idle
   cudaGraphExec_t step_exec = nullptr, stale_exec = nullptr;
-  long long step_kernels = 0;
+  long long step_kernels = 0, step_replays = 0;
   int direct_steps = 0;  // since the last change of what a step launches
   // optional per-kernel timing: a CUDA event pair around every launch
   bool prof_on = false;

@@ -103,6 +103,7 @@ def _bind(L):
         "otbl_boun_arrays": ([P, P, P, P], I),
         "otbl_genflu_arrays": ([P, P, P, P], I),
         "otbl_launch_count": ([P], ctypes.c_longlong),
+        "otbl_step_replays": ([P], ctypes.c_longlong),
         "otbl_graph_create": ([ctypes.POINTER(P), I, I, ctypes.POINTER(P)], I),
         "otbl_graph_launch": ([P], I),
         "otbl_graph_sync": ([P], I),

@@ -3,9 +3,12 @@ ones (otbl_capi.cu step_graph); whatever changes a step's launches drops it.
 The same box advanced in one call, step by step, over a rebind of its state
 arrays and over a change of the CTA sizes ends bit for bit where plain
 otbl_substep calls end."""
+import numpy as np
 import pytest
 
 from opentbl_b200 import Box, config
+from opentbl_b200.config import replace
+from opentbl_b200.ensemble import Graph
 
 from helpers import setup
 
@@ -16,7 +19,6 @@ STATE = ("u", "v", "w", "p", "rhsupa", "rhsvpa", "rhswpa")
 
 def test_replay_is_the_step():
     torch = pytest.importorskip("torch")
-    import numpy as np
 
     cfg = config.SMALL
     init, coef = setup(cfg)
@@ -46,3 +48,41 @@ def test_replay_is_the_step():
         # plain substeps (which do not advance it) agree too
         np.testing.assert_array_equal(once.field(n), plain.field(n))
         np.testing.assert_array_equal(split.field(n), plain.field(n))
+
+
+def test_captured_steps_are_not_plain_steps():
+    """A graph of four steps records them without running them, so the next
+    three plain steps build no step graph; the fourth replays one."""
+    cfg = config.TINY
+    b = Box(cfg, *setup(cfg))
+    g = Graph([b], 4)
+    g.launch()
+    g.sync()
+    b.advance(3)
+    b.sync()
+    assert b.replays == 0
+    b.advance(2)
+    b.sync()
+    assert b.replays == 2
+    g.close()
+
+
+def test_replay_after_rebind():
+    """The step captured for one box is not replayed for the box that the
+    context is re-bound to."""
+    a = config.TINY
+    c = replace(a, lx=14.0, lz=5.0, re_theta=350.0)
+    b, fresh = Box(a, *setup(a)), Box(c, *setup(c))
+    b.advance(5)
+    b.sync()
+    assert b.replays == 2
+    b.rebind(c, *setup(c))
+    b.advance(3)
+    b.sync()  # the old step graph is destroyed once the stream is idle
+    b.advance(2)
+    assert b.replays == 4
+    fresh.advance(5)
+    for x in (b, fresh):
+        x.sync()
+    for n in STATE:
+        np.testing.assert_array_equal(b.field(n), fresh.field(n))
