@@ -406,7 +406,7 @@ cudaError_t launch_statsp(otbl_ctx *c) {
   int K, C, L, NT;
   size_t sm;
   auto go = [&](auto kern, dim3 g, auto... args) {
-    if (sm > 48 * 1024) cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+    allow_smem(kern, sm);
     kern<<<g, NT, sm, s>>>(c->dc, op, args..., C, L);
     c->launches += 1;
   };
@@ -424,7 +424,7 @@ cudaError_t launch_statsp(otbl_ctx *c) {
   z.nz = nz;
   z.nz2 = c->dc.nz2;
   const size_t smem = (size_t)4 * 3 * z.M * sizeof(double2);
-  cudaFuncSetAttribute(k_stats_acc, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  allow_smem(k_stats_acc, smem);
   for (int i0 = 1; i0 <= nx; i0 += G) {
     const int g = std::min(G, nx - i0 + 1);
     StatsBufs bf;

@@ -294,7 +294,7 @@ static void xline_t_launch(otbl_ctx *c, const DCoefT<T> &dc) {
   }
   const int gb = (4 * (K + 1) * 32 * (int)sizeof(TG) + 127) / 128 * 128;
   const int smem = 2 * (gb + (DV ? 4 * (K + 2) * 32 * 8 : 0) + K * 16 * (int)sizeof(T)) + 128;
-  cudaFuncSetAttribute(k_xline_t<T, DV>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+  allow_smem(k_xline_t<T, DV>, smem);
   k_xline_t<T, DV><<<dim3((npu + 127) / 128, 3), 128, smem, c->stream>>>(dc, a, &c->st->err, DV ? c->xmd : c->xmi);
 }
 
@@ -521,7 +521,7 @@ static void interpy_t_launch(otbl_ctx *c, const DCoefT<T> &dc) {
   }
   const dim3 gt((c->dc.nz1 + 127) / 128, c->cfg.nx, 3);
   const int sm = 2 * ((KYT + 2) * 128 * 8 + KYT * 8 * (int)sizeof(T)) + 128;
-  cudaFuncSetAttribute(k_interpy_t<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm);
+  allow_smem(k_interpy_t<T>, sm);
   k_interpy_t<T><<<gt, 128, sm, c->stream>>>(dc, a, &c->st->err, c->ymi);
 }
 
@@ -1090,9 +1090,9 @@ static int final_t(otbl_ctx *c, const DCoefT<W> &cw, unsigned comps, cudaEvent_t
     constexpr int K = decltype(C)::value;
     constexpr int sma = 2 * ((10 * 128 * (int)sizeof(W) + 127) / 128 * 128 + 10 * 128 * 8 + 8 * 128) + 128;
     constexpr int smb = FinalBox<W, K>::smem;
-    cudaFuncSetAttribute(k_final_ta<K, W>, cudaFuncAttributeMaxDynamicSharedMemorySize, sma);
+    allow_smem(k_final_ta<K, W>, sma);
     k_final_ta<K, W><<<gt, 128, sma, c->stream>>>(c->dc, cw, fs, &c->st->err, c->fmaps[K]);
-    cudaFuncSetAttribute(k_final_tb<K, W>, cudaFuncAttributeMaxDynamicSharedMemorySize, smb);
+    allow_smem(k_final_tb<K, W>, smb);
     k_final_tb<K, W><<<gt, 128, smb, c->stream>>>(c->dc, cw, fs, &c->st->err, c->fmaps[K]);
     if (before_vel) {  // the first velocity write waits for this event
       cudaStreamWaitEvent(c->stream, before_vel, 0);

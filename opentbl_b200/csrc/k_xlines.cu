@@ -300,7 +300,7 @@ static cudaError_t xline_launch(otbl_ctx *c, const DCoefT<T> &dc, XArgs &a) {
   }
   const int NT = ((C << lg) + 31) / 32 * 32;
   auto go = [&](auto kern) {
-    if (smem > 48 * 1024) cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    allow_smem(kern, smem);
     const int regs = K > 9 ? 256 : 128;  // per thread, by the launch bounds
     const int per = std::max(1, std::min((int)(233472 / (smem + 1024)), 65536 / (regs * NT)));
     kern<<<std::min(ntile, per * sm_count()), NT, smem, c->stream>>>(dc, a);

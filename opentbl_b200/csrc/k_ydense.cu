@@ -621,7 +621,7 @@ cudaError_t launch_interpy_dense(otbl_ctx *c) {
   }
   const int grid = std::min(3 * a.tiles, nsm);
   const size_t smem = ydense_smem(a.nt, a.sf);
-  cudaFuncSetAttribute(k_ydense, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  allow_smem(k_ydense, smem);
   k_ydense<<<grid, YD_THREADS, smem, s>>>(nx, ny, nz1, a, &c->st->err, c->yd_maps);
   c->launches += 1;
   return cudaGetLastError();

@@ -781,7 +781,7 @@ static void tail_t(otbl_ctx *c, const DCoefT<W> &cw, unsigned comps) {
   const size_t sm = (size_t)4 * NT * 16 + (gt ? 0 : (size_t)5 * z.K * NT * sizeof(V2<W>)) + tabs;
   const int per = std::max(1, std::min((int)(233472 / (sm + 1024)), gt ? 1 : (sizeof(W) == 8 ? 256 : 384) / NT));
   auto go = [&](auto kern) {
-    if (sm > 48 * 1024) cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+    allow_smem(kern, sm);
     kern<<<dim3(y_grid(ntile, per, n), n), NT, sm, c->stream>>>(c->dc, cw, a);
   };
   if (z.K == 7)

@@ -28,6 +28,8 @@
 #include <cfloat>
 #include <cudaTypedefs.h>
 #include <mutex>
+#include <set>
+#include <utility>
 #include <algorithm>
 #include <type_traits>
 
@@ -808,7 +810,7 @@ __global__ void __launch_bounds__(128) k_genflu_cols(DCoef c, GenArgs a) {
 
 cudaError_t genflu_tab_launch(otbl_ctx *c, const GenArgs &a) {
   const size_t smem = genflu_smem_bytes(c->cfg.ny);
-  if (smem > 48 * 1024) cudaFuncSetAttribute(k_genflu_tab, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  allow_smem(k_genflu_tab, smem);
   k_genflu_tab<<<1, 256, smem, c->stream>>>(c->dc, a);
   c->launches += 1;
   return cudaGetLastError();
@@ -1614,7 +1616,7 @@ static cudaError_t products_t(otbl_ctx *c, int setstep, int part, const ZTabT<T>
   } else {
     const size_t smem = (size_t)4 * 3 * M * sizeof(V2<T>);
     auto k = part == 0 ? k_products<T, 0> : (part == 1 ? k_products<T, 1> : k_products<T, 2>);
-    cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    allow_smem(k, smem);
     k<<<g, 128, smem, c->stream>>>(c->dc, z, a);
   }
   return cudaGetLastError();
@@ -1644,7 +1646,7 @@ cudaError_t launch_dt(otbl_ctx *c, int m, int setstep) {
   prof_begin(c, PK_DT);
   const bool st = stream_tail(c);
   const size_t smem = (size_t)(st ? 12 : 8) * (c->cfg.ny + 1) * sizeof(double);
-  if (smem > 40 * 1024) cudaFuncSetAttribute(k_dt, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  allow_smem(k_dt, smem);
   k_dt<<<1, 256, smem, c->stream>>>(c->dc, c->st, c->w.vm_bits, implzy_tab(c, 0), implzy_tab(c, 1),
                                     st ? c->w.fac_u : nullptr, st ? c->w.fac_v : nullptr, m, setstep,
                                     c->cfg.dt_mode, c->cfg.dt_fixed);
@@ -1818,6 +1820,24 @@ int sm_count() {
   return nsm[dev];
 }
 
+cudaError_t allow_smem_ptr(const void *kern, size_t bytes) {
+  if (bytes <= 32 * 1024) return cudaSuccess;  // 48 KB, static arrays included, need no leave
+  static std::mutex mu;
+  static std::set<std::pair<int, const void *>> &raised = *new std::set<std::pair<int, const void *>>;
+  int dev = 0, most = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e != cudaSuccess) return e;
+  std::lock_guard<std::mutex> lock(mu);
+  if (raised.count({dev, kern})) return cudaSuccess;
+  cudaFuncAttributes a;
+  e = cudaFuncGetAttributes(&a, kern);
+  if (e == cudaSuccess) e = cudaDeviceGetAttribute(&most, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
+  if (e == cudaSuccess)
+    e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, most - (int)a.sharedSizeBytes);
+  if (e == cudaSuccess) raised.insert({dev, kern});
+  return e;
+}
+
 // The TMA-fed x-DCT pass when its descriptors exist and n is 256, 512, 1024
 // or 2048; false leaves the pass to pois_xdct's one-shot kernels
 // (OTBL_POIS_ONESHOT=1 forces them).
@@ -1845,7 +1865,7 @@ static bool pois_xdct_t(otbl_ctx *c, bool fwd, T *phi, int kbeg, int kend) {
       const int S = std::min(6, (int)((smax - xs - 64) / ch));
       if (S < 2) return false;
       const size_t smem = (size_t)S * ch + xs + 8 * (size_t)S;
-      cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+      allow_smem(kern, smem);
       kern<<<std::min(ntile, sm_count()), 512, smem, c->stream>>>(c->dc, xt, c->pmaps, phi, kbeg, kend, S, err);
       return true;
     };
@@ -1863,7 +1883,7 @@ static bool pois_xdct_t(otbl_ctx *c, bool fwd, T *phi, int kbeg, int kend) {
   if (smem > (size_t)smax) return false;
   constexpr int MINB = F64 ? 1 : 2;
   auto go = [&](auto kern) {
-    cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    allow_smem(kern, smem);
     const int per = smem * 2 + 2048 <= 233472 ? MINB : 1;  // CTAs per SM that fit
     kern<<<std::min(ntile, per * sm_count()), 512, smem, c->stream>>>(c->dc, xt, c->pmaps, phi, kbeg, kend, err);
     return true;
@@ -1900,10 +1920,10 @@ static void pois_xdct(otbl_ctx *c, bool fwd, T *phi, int kbeg, int kend) {
     xt = xtabf(c);
   auto go = [&](auto kf, auto kb) {
     if (fwd) {
-      cudaFuncSetAttribute(kf, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+      allow_smem(kf, smem);
       kf<<<gx, NT, smem, c->stream>>>(c->dc, xt, c->f[OTBL_F_U], c->f[OTBL_F_V], c->f[OTBL_F_W], phi, kbeg, kend);
     } else {
-      cudaFuncSetAttribute(kb, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+      allow_smem(kb, smem);
       kb<<<gx, NT, smem, c->stream>>>(c->dc, xt, phi, kbeg, kend);
     }
   };
@@ -2018,7 +2038,7 @@ cudaError_t launch_cosftx(otbl_ctx *c, double *cp, int nlines, int iopt) {
   auto go = [&](auto mb, auto nn) {
     constexpr int B = decltype(mb)::value, NN = decltype(nn)::value;
     auto k = n * B >= 2048 ? k_cosftx<B, 512, NN> : k_cosftx<B, 256, NN>;
-    if (smem > 48 * 1024) cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    allow_smem(k, smem);
     k<<<(nlines + 2 * B - 1) / (2 * B), n * B >= 2048 ? 512 : 256, smem, c->stream>>>(xtab(c), cp, c->cfg.nx, nlines,
                                                                                      iopt);
   };

@@ -264,6 +264,16 @@ cudaError_t launch_boun_all(otbl_ctx *c);
 cudaError_t launch_tiempo(otbl_ctx *c);
 cudaError_t launch_energies(otbl_ctx *c);
 int sm_count();  // SMs of the current device
+// Lets kern be launched with `bytes` of dynamic shared memory. The limit is a
+// property of the kernel that every context and host thread shares, so it is
+// raised once per kernel and device to all that a CTA may have, never set to
+// what one launch needs: another thread's smaller box would lower it between
+// this launch's setting and the launch, which is then refused.
+cudaError_t allow_smem_ptr(const void *kern, size_t bytes);
+template <typename... A>
+cudaError_t allow_smem(void (*kern)(A...), size_t bytes) {
+  return allow_smem_ptr(reinterpret_cast<const void *>(kern), bytes);
+}
 // the driver's cuTensorMapEncodeTiled (as void *), nullptr if unavailable
 void *tensor_map_encoder();
 // fill the coefficient tables (at creation and on new coefficients)
