@@ -328,7 +328,8 @@ long long otbl_step_replays(const otbl_ctx *ctx);
  * driven through their own entry points while a launch is in flight
  * (otbl_graph_sync or a finished otbl_graph_query orders them again). The
  * graph holds the members' device buffers: destroy it before them.
- * Per-kernel profiling must be off while capturing. */
+ * Per-kernel profiling must be off while capturing. When it fails,
+ * otbl_last_error of the members says why. */
 typedef struct otbl_graph otbl_graph;
 int otbl_graph_create(otbl_ctx *const *ctxs, int n, int nsteps, otbl_graph **out);
 int otbl_graph_launch(otbl_graph *g);

@@ -53,46 +53,51 @@ static void graph_free(otbl_graph *g) {
   if (!g) return;
   if (g->exec) cudaGraphExecDestroy(g->exec);
   if (g->graph) cudaGraphDestroy(g->graph);
-  for (cudaEvent_t e : g->events) cudaEventDestroy(e);
+  for (cudaEvent_t e : g->events)
+    if (e) cudaEventDestroy(e);
   if (g->stream) cudaStreamDestroy(g->stream);
   delete g;
+}
+
+// gives up a graph: every member's otbl_last_error says why
+static int graph_fail(otbl_graph *g, const std::string &why) {
+  for (otbl_ctx *c : g->members) c->err = "otbl_graph_create: " + why;
+  cudaGetLastError();
+  graph_free(g);
+  return OTBL_ERR_CUDA;
 }
 
 extern "C" int otbl_graph_create(otbl_ctx *const *ctxs, int n, int nsteps, otbl_graph **out) {
   if (!ctxs || n < 1 || nsteps < 1 || !out) return OTBL_ERR_ARG;
   *out = nullptr;
   const int dev = ctxs[0] ? ctxs[0]->device : -1;
+  auto refuse = [&](const char *why) {
+    for (int k = 0; k < n; ++k)
+      if (ctxs[k]) ctxs[k]->err = std::string("otbl_graph_create: ") + why;
+    return OTBL_ERR_ARG;
+  };
   for (int k = 0; k < n; ++k) {
-    if (!ctxs[k] || ctxs[k]->device != dev) return OTBL_ERR_ARG;
-    if (ctxs[k]->prof_on) return OTBL_ERR_ARG;  // per-launch events cannot be captured
+    if (!ctxs[k]) return OTBL_ERR_ARG;
+    if (ctxs[k]->device != dev) return refuse("the members are on different devices");
+    if (ctxs[k]->prof_on) return refuse("per-launch timing is on, its events cannot be captured");
     for (int q = 0; q < k; ++q)
-      if (ctxs[q] == ctxs[k]) return OTBL_ERR_ARG;
+      if (ctxs[q] == ctxs[k]) return refuse("a context is a member twice");
   }
-  if (cudaSetDevice(dev) != cudaSuccess) return OTBL_ERR_CUDA;
   otbl_graph *g = new otbl_graph();
   g->device = dev;
   g->members.assign(ctxs, ctxs + n);
+  cudaError_t e = cudaSetDevice(dev);
   // finish outstanding work of the members before capturing
   for (otbl_ctx *c : g->members)
-    if (cudaStreamSynchronize(c->stream) != cudaSuccess) {
-      graph_free(g);
-      return OTBL_ERR_CUDA;
-    }
-  if (cudaStreamCreateWithFlags(&g->stream, cudaStreamNonBlocking) != cudaSuccess) {
-    graph_free(g);
-    return OTBL_ERR_CUDA;
-  }
+    if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
+  if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&g->stream, cudaStreamNonBlocking);
   g->events.resize(n + 1, nullptr);
-  for (auto &e : g->events)
-    if (cudaEventCreateWithFlags(&e, cudaEventDisableTiming) != cudaSuccess) {
-      graph_free(g);
-      return OTBL_ERR_CUDA;
-    }
+  for (auto &ev : g->events)
+    if (e == cudaSuccess) e = cudaEventCreateWithFlags(&ev, cudaEventDisableTiming);
+  if (e == cudaSuccess) e = cudaStreamBeginCapture(g->stream, cudaStreamCaptureModeRelaxed);
+  if (e != cudaSuccess) return graph_fail(g, cudaGetErrorString(e));
   int st = OTBL_OK;
-  if (cudaStreamBeginCapture(g->stream, cudaStreamCaptureModeRelaxed) != cudaSuccess) {
-    graph_free(g);
-    return OTBL_ERR_CUDA;
-  }
+  std::string why;  // of the first launch that was refused
   cudaEventRecord(g->events[n], g->stream);
   g->kernels.assign(n, 0);
   for (int k = 0; k < n && st == OTBL_OK; ++k) {
@@ -100,25 +105,22 @@ extern "C" int otbl_graph_create(otbl_ctx *const *ctxs, int n, int nsteps, otbl_
     cudaStreamWaitEvent(c->stream, g->events[n], 0);  // fork
     const long long l0 = c->launches;
     st = otbl_advance(c, nsteps);
+    if (st != OTBL_OK) why = "member " + std::to_string(k) + ": " + c->err;
     g->kernels[k] = c->launches - l0;
     c->launches = l0;  // counted again at every launch of the graph
     cudaEventRecord(g->events[k], c->stream);
     cudaStreamWaitEvent(g->stream, g->events[k], 0);  // join
   }
   cudaGraph_t graph = nullptr;
-  const cudaError_t ec = cudaStreamEndCapture(g->stream, &graph);
+  e = cudaStreamEndCapture(g->stream, &graph);
   g->graph = graph;
-  if (st != OTBL_OK || ec != cudaSuccess) {
-    cudaGetLastError();
-    graph_free(g);
-    return st != OTBL_OK ? st : OTBL_ERR_CUDA;
+  if (st != OTBL_OK) {
+    graph_fail(g, why);
+    return st;
   }
   // keep the priorities of the streams the kernels were captured from
-  if (cudaGraphInstantiate(&g->exec, g->graph, cudaGraphInstantiateFlagUseNodePriority) != cudaSuccess) {
-    cudaGetLastError();
-    graph_free(g);
-    return OTBL_ERR_CUDA;
-  }
+  if (e == cudaSuccess) e = cudaGraphInstantiate(&g->exec, g->graph, cudaGraphInstantiateFlagUseNodePriority);
+  if (e != cudaSuccess) return graph_fail(g, cudaGetErrorString(e));
   for (long long k : g->kernels) g->total_kernels += k;
   *out = g;
   return OTBL_OK;

@@ -28,7 +28,8 @@ class Graph:
         h = ctypes.c_void_p()
         st = self.L.otbl_graph_create(arr, len(self.boxes), nsteps, ctypes.byref(h))
         if st != native.OTBL_OK:
-            raise native.OtblError(f"otbl_graph_create: {native.ERRORS.get(st, st)}")
+            why = self.L.otbl_last_error(self.boxes[0].h).decode() if self.boxes else ""
+            raise native.OtblError(f"otbl_graph_create: {native.ERRORS.get(st, st)} {why}")
         self.h = h
 
     @property

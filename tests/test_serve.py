@@ -115,6 +115,23 @@ def test_graph_ensemble_equals_boxes_alone():
 
 
 @pytest.mark.gpu
+def test_graph_refusals_say_why():
+    cfg = config.TINY
+    init = synth.make_initial(cfg)
+    a, b = Box(cfg, init), Box(cfg, init)
+    with pytest.raises(native.OtblError, match="a member twice"):
+        ensemble.Graph([a, a], 1)
+    b.profile(True)
+    with pytest.raises(native.OtblError, match="per-launch timing is on"):
+        ensemble.Graph([a, b], 1)
+    b.profile(False)
+    g = ensemble.Graph([a, b], 1)
+    g.launch()
+    g.sync()
+    g.close()
+
+
+@pytest.mark.gpu
 def test_serving_mix_equals_alone():
     """Six requests on three grid sizes (slots are created, re-bound and
     reused), arriving while others run: each result equals the same request
