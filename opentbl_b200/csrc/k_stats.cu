@@ -88,12 +88,12 @@ template <typename OP, int K>
 __device__ __forceinline__ void stats_solve(const double *__restrict__ c8, const double2 *tile, int n, int C, int L,
                                             int q, int lane, int xr, double2 (&y)[K], double2 *ex, double *px) {
   const int t = threadIdx.x, NT = blockDim.x, s = q * K;
-  double l[K], d[K], e[K], pl = 1.0, pe = 1.0;
+  double l[K], d[K], u[K], pl = 1.0, pu = 1.0;
 #pragma unroll
   for (int b = 0; b < K; ++b) {
     const int r = s + b;
     y[b] = make_double2(0.0, 0.0);
-    l[b] = d[b] = e[b] = 0.0;
+    l[b] = d[b] = u[b] = 0.0;
     if (r < n) {
       const Win w = OP::win(r, n);
       const double *cw = c8 + (size_t)w.wr * 8, *cr = c8 + (size_t)r * 8;
@@ -109,24 +109,21 @@ __device__ __forceinline__ void stats_solve(const double *__restrict__ c8, const
       } else {
         d[b] = __ldg(cr + 6);
         if (r > OP::first) l[b] = -__ldg(cr + 5);
-        if (r < n - 1) e[b] = -__ldg(cr + 7) * d[b];
+        if (r < n - 1) u[b] = __ldg(cr + 7);
       }
     }
     pl *= l[b];
   }
 #pragma unroll
-  for (int b = 0; b < K; ++b) pe *= e[b];
-  forward_local<K, 1, double>(y, l);
-  ex[t] = y[K - 1];
+  for (int b = 0; b < K; ++b) pu *= -u[b] * d[b];
+  ex[t] = forward_end<K, 1, double>(y, l);
   px[t] = pl;
-  px[NT + t] = pe;
+  px[NT + t] = pu;
   __syncthreads();
-  if (q > 0) forward_fix<K, 1, double>(y, l, chunk_carry<double>(ex + t - L, -L, px + t - L, -L, q));
-  backward_local<K, 1, double>(y, d, e);
-  ex[NT + t] = y[0];
+  forward_from<K, 1, double>(y, l, chunk_carry<double>(ex + t - L, -L, px + t - L, -L, q));
+  ex[NT + t] = backward_end<K, 1, double>(y, d, u);
   __syncthreads();
-  if (q < C - 1)
-    backward_fix<K, 1, double>(y, e, chunk_carry<double>(ex + NT + t + L, L, px + NT + t + L, L, C - 1 - q));
+  backward_from<K, 1, double>(y, d, u, chunk_carry<double>(ex + NT + t + L, L, px + NT + t + L, L, C - 1 - q));
 }
 
 struct StatsOps {

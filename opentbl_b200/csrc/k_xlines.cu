@@ -27,8 +27,8 @@ struct XArgs {
   int C, lgL;
 };
 
-// coefficients of a table: interpxx w0, w1, l, d, e; difvisxx the same for
-// the convective system, then f1, f2, f3, l, d, e of the viscous one; after
+// coefficients of a table: interpxx w0, w1, l, d, u; difvisxx the same for
+// the convective system, then f1, f2, f3, l, d, u of the viscous one; after
 // the C chunks' values, the chunk products P, Q of each system
 constexpr int xcoefs(bool dv) { return dv ? 11 : 5; }
 // Tables of lines longer than 1152 planes (K > 9) stay in global memory:
@@ -256,13 +256,13 @@ static cudaError_t x_tables(otbl_ctx *c) {
         put(0, i, econ[2 * i]);
         put(1, i, econ[2 * i + 1]);
       }
-      auto lde = [&](int at) { return [&put, at](int i, int r, T v) { put(at + i, r, v); }; };
-      chunk_factors<T>(lde(2), K, nx, icon, 0, P, P + C);
+      auto ldu = [&](int at) { return [&put, at](int i, int r, T v) { put(at + i, r, v); }; };
+      chunk_factors<T>(ldu(2), K, nx, icon, 0, P, P + C);
       if (dv) {
         const T *ev = A(wh ? OTBL_C_COFVXV : OTBL_C_COFVXU);
         for (int i = 1; i < nx - 1; ++i)
           for (int k = 0; k < 3; ++k) put(5 + k, i, ev[3 * i + k]);
-        chunk_factors<T>(lde(8), K, nx, A(wh ? OTBL_C_VIXV : OTBL_C_VIXU), 0, P + 2 * C, P + 3 * C);
+        chunk_factors<T>(ldu(8), K, nx, A(wh ? OTBL_C_VIXV : OTBL_C_VIXU), 0, P + 2 * C, P + 3 * C);
       }
       all.insert(all.end(), tab.begin(), tab.end());
     }

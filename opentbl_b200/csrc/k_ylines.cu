@@ -71,7 +71,7 @@ struct YPlace {
 struct InterpyArgs {
   const double *in[3];
   void *out[3];
-  const void *tab[2];  // wA, wB, l, d, e, then P, Q, per which
+  const void *tab[2];  // wA, wB, l, d, u, then P, Q, per which
   int which[3];
   int C, L;
 };
@@ -173,8 +173,8 @@ struct TailArgs {
   W *rhsupa, *rhsvpa, *rhswpa;       // old on entry, new on exit
   const W *cu, *cv, *cw;             // difvisxx outputs
   const W *uv, *uw, *vw, *vv, *ww;
-  const W *tw[2];                    // differzy wA, wB, l, d, e; vistyy f1, f2, f3, l, d, e; P, Q of each
-  const double *td[2];               // vyi (3), l, d, e of implzy, idyy; P, Q; A_2, C_{jee-1}
+  const W *tw[2];                    // differzy wA, wB, l, d, u; vistyy f1, f2, f3, l, d, u; P, Q of each
+  const double *td[2];               // vyi (3), l, d, u of implzy, idyy; P, Q; A_2, C_{jee-1}
   const DState *st;
   int comp[3];
   int C[2], L[2], nw[2], nd[2];      // chunks, lanes, elements of the tables
@@ -343,26 +343,20 @@ __device__ __forceinline__ void tail_body(const DCoef &c, const DCoefT<W> &cw, c
     {
       VW *e0 = reinterpret_cast<VW *>(ex), *e1 = reinterpret_cast<VW *>(ex + NT);
       const W *ld = tw + 2 * K, *lv = tw + 8 * K;
-      forward_local<K, 1, W>(yd, ld);
-      forward_local<K, 1, W>(yv, lv);
-      e0[t] = yd[K - 1];
-      e1[t] = yv[K - 1];
+      e0[t] = forward_end<K, 1, W>(yd, ld);
+      e1[t] = forward_end<K, 1, W>(yv, lv);
       __syncthreads();
-      if (q > 0) {
-        forward_fix<K, 1, W>(yd, ld, chunk_carry<W>(e0 + t - L, -L, PW + q - 1, -1, q));
-        forward_fix<K, 1, W>(yv, lv, chunk_carry<W>(e1 + t - L, -L, PW + 2 * C + q - 1, -1, q));
-      }
+      forward_from<K, 1, W>(yd, ld, chunk_carry<W>(e0 + t - L, -L, PW + q - 1, -1, q));
+      forward_from<K, 1, W>(yv, lv, chunk_carry<W>(e1 + t - L, -L, PW + 2 * C + q - 1, -1, q));
       e0 = reinterpret_cast<VW *>(ex + 2 * NT);
       e1 = reinterpret_cast<VW *>(ex + 3 * NT);
-      backward_local<K, 1, W>(yd, ld + K, ld + 2 * K);
-      backward_local<K, 1, W>(yv, lv + K, lv + 2 * K);
-      e0[t] = yd[0];
-      e1[t] = yv[0];
+      e0[t] = backward_end<K, 1, W>(yd, ld + K, ld + 2 * K);
+      e1[t] = backward_end<K, 1, W>(yv, lv + K, lv + 2 * K);
       __syncthreads();
-      if (q < C - 1) {
-        backward_fix<K, 1, W>(yd, ld + 2 * K, chunk_carry<W>(e0 + t + L, L, PW + C + q + 1, 1, C - 1 - q));
-        backward_fix<K, 1, W>(yv, lv + 2 * K, chunk_carry<W>(e1 + t + L, L, PW + 3 * C + q + 1, 1, C - 1 - q));
-      }
+      backward_from<K, 1, W>(yd, ld + K, ld + 2 * K,
+                             chunk_carry<W>(e0 + t + L, L, PW + C + q + 1, 1, C - 1 - q));
+      backward_from<K, 1, W>(yv, lv + K, lv + 2 * K,
+                             chunk_carry<W>(e1 + t + L, L, PW + 3 * C + q + 1, 1, C - 1 - q));
     }
     cp_async_wait<0>();  // the thread's own slots
     // ---- RHS assembly (rhsp.F90:164-169, 181-204, 351-418, 423-445), RK3
@@ -553,22 +547,20 @@ __global__ void __launch_bounds__(256, 2) k_pois_solve(DCoefT<T> c, T *phi, cons
     pr *= l[b];
     dp = d[b];
   }
-  forward_local<K, 1, T>(y, l);
-  e0[t] = y[K - 1];
+  e0[t] = forward_end<K, 1, T>(y, l);
   p0[t] = pr;
   __syncthreads();
-  if (q > 0) forward_fix<K, 1, T>(y, l, chunk_carry<T>(e0 + t - w.L, -w.L, p0 + t - w.L, -w.L, q));
+  forward_from<K, 1, T>(y, l, chunk_carry<T>(e0 + t - w.L, -w.L, p0 + t - w.L, -w.L, q));
   pr = T(1);
 #pragma unroll
-  for (int b = 0; b < K; ++b) {  // l holds e from here on
-    l[b] = s + b < ny1 - 1 ? -__ldg(ayp + 3 * b + 2) * d[b] : T(0);
-    pr *= l[b];
+  for (int b = 0; b < K; ++b) {  // l holds u from here on
+    l[b] = s + b < ny1 - 1 ? __ldg(ayp + 3 * b + 2) : T(0);
+    pr *= -l[b] * d[b];
   }
-  backward_local<K, 1, T>(y, d, l);
-  e1[t] = y[0];
+  e1[t] = backward_end<K, 1, T>(y, d, l);
   p1[t] = pr;
   __syncthreads();
-  if (q < C - 1) backward_fix<K, 1, T>(y, l, chunk_carry<T>(e1 + t + w.L, w.L, p1 + t + w.L, w.L, C - 1 - q));
+  backward_from<K, 1, T>(y, d, l, chunk_carry<T>(e1 + t + w.L, w.L, p1 + t + w.L, w.L, C - 1 - q));
   if (!w.active) return;
 #pragma unroll
   for (int b = 0; b < K; ++b)
@@ -580,7 +572,7 @@ __global__ void __launch_bounds__(256, 2) k_pois_solve(DCoefT<T> c, T *phi, cons
 // ---------------------------------------------------------------------------
 // Work::ytab in T: interpyy (u-type, v-type), then differzy and vistyy
 // (u-type, v-type); Work::tdtab in FP64: implzy (u-type, v-type), whose l, d,
-// e and products k_dt writes for the substep's dt
+// u and products k_dt writes for the substep's dt
 struct YSizes {
   int K, C[2], Ci;            // rows per chunk; chunks of the tail (u-, v-type) and of interpyy
   size_t in, tw[2], td[2];    // elements of each table
@@ -638,7 +630,7 @@ static cudaError_t y_tables(otbl_ctx *c) {
   }
   const int S = kTailW * K;
   auto put = [&](int i, int r, T v) { tab[(size_t)(r / K) * S + i * K + r % K] = v; };
-  auto lde = [&](int at) { return [&put, at](int i, int r, T v) { put(at + i, r, v); }; };
+  auto ldu = [&](int at) { return [&put, at](int i, int r, T v) { put(at + i, r, v); }; };
   for (int wh = 0; wh < 2; tab += z.tw[wh], ++wh) {
     const int jee = wh ? ny : ny + 1, C = z.C[wh];
     const T *e = A(wh ? OTBL_C_COFCYV : OTBL_C_COFCYU), *ev = A(wh ? OTBL_C_COFVYV : OTBL_C_COFVYU);
@@ -648,8 +640,8 @@ static cudaError_t y_tables(otbl_ctx *c) {
       for (int k = 0; k < 3; ++k) put(5 + k, r, ev[3 * r + k]);
     }
     T *P = tab + (size_t)C * S;
-    chunk_factors<T>(lde(2), K, jee, A(wh ? OTBL_C_DCYV : OTBL_C_DCYU), 0, P, P + C);
-    chunk_factors<T>(lde(8), K, jee, A(wh ? OTBL_C_VIYV : OTBL_C_VIYU), 0, P + 2 * C, P + 3 * C);
+    chunk_factors<T>(ldu(2), K, jee, A(wh ? OTBL_C_DCYV : OTBL_C_DCYU), 0, P, P + C);
+    chunk_factors<T>(ldu(8), K, jee, A(wh ? OTBL_C_VIYV : OTBL_C_VIYU), 0, P + 2 * C, P + 3 * C);
   }
   std::vector<double> dt(z.td[0] + z.td[1], 0.0);
   for (int wh = 0; wh < 2; ++wh) {

@@ -283,8 +283,8 @@ __global__ void __launch_bounds__(128, prod_min_ctas<M, T>()) k_products_all(DCo
 // Factors of (A + var1*B) for implzy (lip.f90:545-568): with A_r, B_r, C_r the
 // sub-, main and super-diagonal of row r (0-based, the unknowns r = 1..jee-2),
 // pivot_r = B_r - A_r C_{r-1} / pivot_{r-1}, l_r = -A_r / pivot_{r-1}, d_r =
-// 1 / pivot_r, e_r = -C_r d_r; the boundary rows pass their value through (l =
-// e = 0, d = 1). The pivots are the ratios of the continuants t_r = B_r
+// 1 / pivot_r, u_r = C_r; the boundary rows pass their value through (l = u =
+// 0, d = 1). The pivots are the ratios of the continuants t_r = B_r
 // t_{r-1} - A_r C_{r-1} t_{r-2}, which leaves no division on the serial
 // chain (one multiply-add a row instead of a division and two; computed
 // ratios satisfy the pivot recurrence to one rounding, so it loses nothing).
@@ -423,7 +423,7 @@ __global__ void __launch_bounds__(256) k_dt(DCoef c, DState *st, unsigned long l
       const ImplzyRow w = implzy_row(c, which, r, rkk);
       d = den[e] / num[e];
       if (r > 1) l = -w.A * (den[e - 1] / num[e - 1]);
-      if (r < jee - 2) u = -w.C * d;
+      if (r < jee - 2) u = w.C;
       if (fac_u) {
         double *fac = which == 0 ? fac_u : fac_v;
         const double *tp = top + e;
@@ -437,8 +437,8 @@ __global__ void __launch_bounds__(256) k_dt(DCoef c, DState *st, unsigned long l
       if (r == jee - 2) tb.P[2 * tb.C + 1] = w.C;
     }
     bs[e] = l;  // free since the chain
-    ac[e] = u;
-    double *row = tb.lde + (size_t)(r / tb.K) * tb.S + r % tb.K;
+    ac[e] = -u * d;
+    double *row = tb.ldu + (size_t)(r / tb.K) * tb.S + r % tb.K;
     row[0] = l;
     row[tb.K] = d;
     row[2 * tb.K] = u;

@@ -77,11 +77,11 @@ struct Work {
   float *pois_dinvf;           // the same rounded to FP32 (mixed path, modes >= kPoisLow)
 };
 
-// where k_dt writes implzy's factors of one velocity type: l, d, e (row r at
-// lde[(r / K) S + i K + r mod K], i = 0, 1, 2), the products P, Q of the C
+// where k_dt writes implzy's factors of one velocity type: l, d, u (row r at
+// ldu[(r / K) S + i K + r mod K], i = 0, 1, 2), the products P, Q of the C
 // chunks and the two boundary couplings
 struct ImplzyTab {
-  double *lde, *P;
+  double *ldu, *P;
   int K, S, C;
 };
 
