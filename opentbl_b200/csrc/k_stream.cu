@@ -31,6 +31,7 @@ struct XStream {
   void *out[3];
   double *ck[3];         // checkpoint scratch of each line set
   int which[3], np[3];
+  CflReset reset;        // interpxx
 };
 
 // planes per segment, interpxx and difvisxx, measured at 1025x193x512: FP64
@@ -65,6 +66,7 @@ __global__ void __launch_bounds__(128) k_xline_t(DCoefT<T> c, XStream a, int *er
   uint64_t *bar = reinterpret_cast<uint64_t *>(smraw + 2 * STG);
   const int f = blockIdx.y, np = pick3(a.np, f);
   const int t = threadIdx.x, mp0 = blockIdx.x * TB;
+  if (!DV && blockIdx.x == 0 && f == 0) a.reset(c.ny);
   if (mp0 >= np) return;  // the whole CTA lies past this field's lines
   const int mp = mp0 + t;
   const bool active = mp < np;
@@ -275,7 +277,7 @@ static bool build_x_maps(otbl_ctx *c) {
 }
 
 template <typename T, bool DV>
-static void xline_t_launch(otbl_ctx *c, const DCoefT<T> &dc) {
+static void xline_t_launch(otbl_ctx *c, const DCoefT<T> &dc, int reset) {
   constexpr int K = xseg<T, DV>();
   using TG = typename std::conditional<DV, T, double>::type;
   const int nz1 = c->dc.nz1, ny = c->cfg.ny, npu = nz1 * (ny + 1), npv = nz1 * ny;
@@ -292,6 +294,7 @@ static void xline_t_launch(otbl_ctx *c, const DCoefT<T> &dc) {
     a.which[f] = f == 0 ? 0 : 1;
     a.np[f] = f == 1 ? npv : npu;
   }
+  if (reset) a.reset = {c->st, c->w.vm_bits};
   const int gb = (4 * (K + 1) * 32 * (int)sizeof(TG) + 127) / 128 * 128;
   const int smem = 2 * (gb + (DV ? 4 * (K + 2) * 32 * 8 : 0) + K * 16 * (int)sizeof(T)) + 128;
   allow_smem(k_xline_t<T, DV>, smem);
@@ -310,11 +313,11 @@ bool stream_xlines(const otbl_ctx *c, bool dv) {
   return c->mixed ? mb > (dv ? 420 : 300) : (dv && mb > 500);
 }
 
-cudaError_t launch_xlines_stream(otbl_ctx *c, bool dv) {
+cudaError_t launch_xlines_stream(otbl_ctx *c, bool dv, int reset) {
   if (c->mixed)
-    dv ? xline_t_launch<float, true>(c, c->dcf) : xline_t_launch<float, false>(c, c->dcf);
+    dv ? xline_t_launch<float, true>(c, c->dcf, 0) : xline_t_launch<float, false>(c, c->dcf, reset);
   else
-    dv ? xline_t_launch<double, true>(c, c->dc) : xline_t_launch<double, false>(c, c->dc);
+    dv ? xline_t_launch<double, true>(c, c->dc, 0) : xline_t_launch<double, false>(c, c->dc, reset);
   return cudaGetLastError();
 }
 

@@ -25,6 +25,7 @@ struct XArgs {
   int tiles[3];          // CTA tiles of each field
   const void *tab;       // coefficient tables (T): u-type, then v-type
   int C, lgL;
+  CflReset reset;        // interpxx
 };
 
 // coefficients of a table: interpxx w0, w1, l, d, u; difvisxx the same for
@@ -101,6 +102,7 @@ __global__ void __launch_bounds__(K > 9 ? 256 : 512, 1) k_xline(DCoefT<T> c, XAr
   };
   stage_u(blockIdx.x);
   stage_g(blockIdx.x);
+  if (!DV && blockIdx.x == 0) a.reset(c.ny);
   const T rex = c.S[OTBL_S_REX], idx = c.S[OTBL_S_IDX], uinf = c.S[OTBL_S_UINF];
   int have = -1;  // the table in shared memory
   for (int tile = blockIdx.x; tile < ntile; tile += gridDim.x) {
@@ -326,7 +328,7 @@ static cudaError_t xline_launch(otbl_ctx *c, const DCoefT<T> &dc, XArgs &a) {
 }
 
 template <bool DV>
-static cudaError_t xlines(otbl_ctx *c, const void *const (&in)[3], void *const (&out)[3]) {
+static cudaError_t xlines(otbl_ctx *c, const void *const (&in)[3], void *const (&out)[3], int reset) {
   const int nz1 = c->dc.nz1, ny = c->cfg.ny;
   const double *st[3] = {c->f[OTBL_F_U], c->f[OTBL_F_V], c->f[OTBL_F_W]};
   XArgs a;
@@ -336,8 +338,9 @@ static cudaError_t xlines(otbl_ctx *c, const void *const (&in)[3], void *const (
     a.out[f] = out[f];
     a.np[f] = nz1 * (f == 1 ? ny : ny + 1);
   }
+  if (reset) a.reset = {c->st, c->w.vm_bits};
   prof_begin(c, DV ? PK_DIFVISX : PK_INTERPX);
-  const cudaError_t e = stream_xlines(c, DV) ? launch_xlines_stream(c, DV)
+  const cudaError_t e = stream_xlines(c, DV) ? launch_xlines_stream(c, DV, reset)
                         : c->mixed           ? xline_launch<float, DV>(c, c->dcf, a)
                                              : xline_launch<double, DV>(c, c->dc, a);
   prof_end(c);
@@ -345,12 +348,12 @@ static cudaError_t xlines(otbl_ctx *c, const void *const (&in)[3], void *const (
   return e;
 }
 
-cudaError_t launch_interpx(otbl_ctx *c) {
-  return xlines<false>(c, {c->f[OTBL_F_U], c->f[OTBL_F_V], c->f[OTBL_F_W]}, {c->w.ux, c->w.vx, c->w.wx});
+cudaError_t launch_interpx(otbl_ctx *c, int reset) {
+  return xlines<false>(c, {c->f[OTBL_F_U], c->f[OTBL_F_V], c->f[OTBL_F_W]}, {c->w.ux, c->w.vx, c->w.wx}, reset);
 }
 
 cudaError_t launch_difvisx(otbl_ctx *c) {
-  return xlines<true>(c, {c->w.uu, c->w.uv, c->w.uw}, {c->w.cu, c->w.cv, c->w.cw});
+  return xlines<true>(c, {c->w.uu, c->w.uv, c->w.uw}, {c->w.cu, c->w.cv, c->w.cw}, 0);
 }
 
 }  // namespace otbl

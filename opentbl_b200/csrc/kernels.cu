@@ -306,7 +306,7 @@ __device__ __forceinline__ ImplzyRow implzy_row(const DCoef &c, int which, int r
 // fac[3j+2] = -C_j / B'_{j+1} (0 for j = jee-1); descending y_j = r_j +
 // fac[3j+2] y_{j+1}, ascending x_j = (y_j - fac[3j] x_{j-1}) fac[3j+1];
 // fac[3(jee+1)] = A_2, fac[3(jee+1)+1] = C_{jee-1}.
-__global__ void __launch_bounds__(256) k_dt(DCoef c, DState *st, unsigned long long *vm_bits, ImplzyTab tu,
+__global__ void __launch_bounds__(256) k_dt(DCoef c, DState *st, const unsigned long long *vm_bits, ImplzyTab tu,
                                             ImplzyTab tv, double *fac_u, double *fac_v, int m, int setstep, int dt_mode, double dt_fixed) {
   extern __shared__ double dsm[];
   __shared__ double s_dt3[8], s_vmax[8], s_rkk;
@@ -319,7 +319,6 @@ __global__ void __launch_bounds__(256) k_dt(DCoef c, DState *st, unsigned long l
       const double vm = __longlong_as_double((long long)vm_bits[j]);
       dt3 = fmin(dt3, c.dymin[j - 1] / fmax(poco, vm));
       vmax = nmax(vmax, vm);
-      vm_bits[j] = 0ull;
     }
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) {
@@ -355,7 +354,6 @@ __global__ void __launch_bounds__(256) k_dt(DCoef c, DState *st, unsigned long l
         st->dt_frozen = 1;
       }
     }
-    if (setstep) st->umax_bits = st->wmax_bits = 0ull;  // consumed: the next reduction starts from 0
     const double dt = st->dt;
     if (!(dt > 0.0) || !isfinite(dt)) atomicCAS(&st->err, 0, OTBL_ERR_NAN);
     const int q = m - 1;

@@ -563,7 +563,7 @@ static int rhsp_issue(otbl_ctx *c, int m, int setstep) {
   if (e == cudaSuccess && m == 1) e = launch_energies(c);
   c->stream = main_s;
   if (check(c, e, "launch_interpy") != OTBL_OK) return OTBL_ERR_CUDA;
-  LAUNCH(c, launch_interpx(c));
+  LAUNCH(c, launch_interpx(c, setstep));
   const bool merged = products_merged(c);
   if (!merged) LAUNCH(c, launch_products(c, setstep, 0));
   OTBL_CUDA_TRY(c, cudaStreamWaitEvent(main_s, c->ev[1], 0));

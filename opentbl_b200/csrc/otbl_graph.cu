@@ -202,7 +202,7 @@ extern "C" int otbl_autotune(otbl_ctx *c, int *choice) {
     for (int bs : cand) {
       c->tune_bs[k] = bs;
       auto run = [&]() {
-        return k == 0 ? launch_interpx(c) : (k == 1 ? launch_difvisx(c) : launch_interpy(c));
+        return k == 0 ? launch_interpx(c, 0) : (k == 1 ? launch_difvisx(c) : launch_interpy(c));
       };
       if (run() != cudaSuccess) {
         st = OTBL_ERR_CUDA;

@@ -42,7 +42,7 @@ struct DState {
   double var1, var2, var3, var4, rkk, varstep;  // RK3 factors of the substep
   double umax, wmax, vmax;
   double ener[15];  // energies of rhsp.F90:116 (module statistics, mod.F90:264)
-  unsigned long long umax_bits, wmax_bits;      // atomicMax targets (>= 0), zeroed by k_dt when consumed
+  unsigned long long umax_bits, wmax_bits;      // atomicMax targets (>= 0)
   int err;        // OTBL_ERR_NAN when the dt reduction saw a non-finite value
   int dt_frozen;  // fixed-dt mode: dt taken
   int pad[2];
@@ -227,8 +227,22 @@ constexpr double kPoisCond = 1024.0;
   } while (0)
 
 namespace otbl {
+// The CFL maxima start at 0 in every substep that takes a dt: block 0 of
+// interpxx, the first kernel on the context stream, clears them (in k_dt,
+// after their use, they outlived a step whose k_dt was never launched).
+struct CflReset {
+  DState *st = nullptr;  // null: nothing to do
+  unsigned long long *vm = nullptr;
+  __device__ void operator()(int ny) const {
+    if (!st) return;
+    for (int j = threadIdx.x; j <= ny; j += blockDim.x) vm[j] = 0ull;
+    if (threadIdx.x == 0) st->umax_bits = st->wmax_bits = 0ull;
+  }
+};
 // kernel launch wrappers (kernels.cu); each returns cudaGetLastError()
-cudaError_t launch_interpx(otbl_ctx *c);
+// interpxx; with reset it also sets the CFL maxima to 0, which the products
+// after it raise
+cudaError_t launch_interpx(otbl_ctx *c, int reset);
 cudaError_t launch_interpy(otbl_ctx *c);
 // part 0: uu, uw and the u, w CFL maxima; part 2: uv and the v maxima;
 // part 1: vw, vv, ww
@@ -251,7 +265,7 @@ cudaError_t launch_final(otbl_ctx *c, unsigned comps);
 bool stream_xlines(const otbl_ctx *c, bool dv);
 bool stream_interpy(const otbl_ctx *c);
 bool stream_tail(const otbl_ctx *c);
-cudaError_t launch_xlines_stream(otbl_ctx *c, bool dv);
+cudaError_t launch_xlines_stream(otbl_ctx *c, bool dv, int reset);
 cudaError_t launch_interpy_stream(otbl_ctx *c);
 cudaError_t launch_tail_rows(otbl_ctx *c);
 cudaError_t launch_final_stream(otbl_ctx *c, unsigned comps, cudaEvent_t before_vel = nullptr,
