@@ -247,6 +247,59 @@ __global__ void __launch_bounds__(256) k_stats_y(DCoef c, StatsOps op, const dou
   }
 }
 
+// The same for columns of more than 256 chunks (rows above 8448), which no CTA
+// holds: a thread per mode, serial sweeps, the forward one's values kept in
+// the output.
+template <typename OP, typename F>
+__device__ __forceinline__ void stats_serial(const double *__restrict__ c8, F in, int n, double2 *out, int so) {
+  double2 x = make_double2(0.0, 0.0);
+  for (int r = 0; r < n; ++r) {
+    const Win w = OP::win(r, n);
+    double2 y = make_double2(0.0, 0.0);
+    for (int m = 0; m < w.cnt; ++m) fma2(y, c8[(size_t)w.wr * 8 + m], in(w.o + m));
+    if (r > OP::first) fma2(y, -c8[(size_t)r * 8 + 5], x);
+    out[(size_t)r * so] = x = y;
+  }
+  for (int r = n - 1; r >= OP::first; --r) {
+    double2 y = out[(size_t)r * so];
+    const double *cr = c8 + (size_t)r * 8;
+    if (r < n - 1) fma2(y, -cr[7], x);
+    x = make_double2(y.x * cr[6], y.y * cr[6]);
+    out[(size_t)r * so] = x;
+  }
+}
+
+template <typename TP>
+__global__ void __launch_bounds__(128) k_stats_y_tall(DCoef c, StatsOps op, const double *__restrict__ ux,
+                                                      const double *__restrict__ w, const double *__restrict__ dwdx,
+                                                      const double *__restrict__ dudx, const TP *__restrict__ p,
+                                                      const double *__restrict__ v, StatsBufs bf, int i0, int G) {
+  const int ny = c.ny, nk = c.nz1 >> 1, f = blockIdx.y, m = blockIdx.x * 128 + threadIdx.x;
+  if (m >= G * nk) return;
+  const int il = m / nk, k = m - il * nk, rows = f < 4 ? ny + 1 : ny;
+  const double *src = f == 0 ? ux : (f == 1 ? w : (f == 2 ? dwdx : (f == 3 ? dudx : v)));
+  const size_t at = (size_t)(i0 - 1 + il) * rows * nk + k;
+  auto in = [&](int r) { return __ldg(reinterpret_cast<const double2 *>(src) + at + (size_t)r * nk); };
+  auto inp = [&](int r) {
+    const V2<TP> x = __ldg(reinterpret_cast<const V2<TP> *>(p) + at + (size_t)r * nk);
+    return make_double2((double)x.x, (double)x.y);
+  };
+  auto buf = [&](int b) {
+    double *base = b < 4 ? (b < 2 ? (b == 0 ? bf.b[0] : bf.b[1]) : (b == 2 ? bf.b[2] : bf.b[3]))
+                         : (b < 6 ? (b == 4 ? bf.b[4] : bf.b[5]) : (b == 6 ? bf.b[6] : bf.b[7]));
+    return reinterpret_cast<double2 *>(base) + (size_t)il * ny * nk + k;
+  };
+  if (f < 4) {
+    double2 *o = buf(f);
+    stats_serial<OpIntY<0>>(op.fiy, in, ny, o, nk);
+    if (f < 2) stats_serial<OpDifY>(op.fdvdy, [&](int r) { return o[(size_t)r * nk]; }, ny, buf(5 + f), nk);
+  } else if (f == 4) {
+    stats_serial<OpIntY<1>>(op.fiyp, inp, ny, buf(4), nk);
+  } else {
+    stats_serial<OpDifY>(op.fdvdy, in, ny, buf(7), nk);
+  }
+}
+
 __device__ __forceinline__ double warp_sum(double x) {
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
@@ -429,12 +482,20 @@ cudaError_t launch_statsp(otbl_ctx *c) {
     const bool sy = shape(ny, K, C, L, NT, sm);
     const dim3 gy((g * (nz1 / 2) + L - 1) / L, 6);
     const double *cx = ux, *cw = c->f[OTBL_F_W], *cdw = dwdx, *cdu = dudx, *cv = c->f[OTBL_F_V];
-    if (c->f32[OTBL_F_P])
-      go(sy ? k_stats_y<float, 9> : k_stats_y<float, 33>, gy, cx, cw, cdw, cdu,
-         reinterpret_cast<const float *>(c->f[OTBL_F_P]), cv, bf, i0, g);
-    else
-      go(sy ? k_stats_y<double, 9> : k_stats_y<double, 33>, gy, cx, cw, cdw, cdu, (const double *)c->f[OTBL_F_P], cv,
-         bf, i0, g);
+    const float *pf = reinterpret_cast<const float *>(c->f[OTBL_F_P]);
+    const double *pd = c->f[OTBL_F_P];
+    if (C > 256) {
+      const dim3 gt((g * (nz1 / 2) + 127) / 128, 6);
+      if (c->f32[OTBL_F_P])
+        k_stats_y_tall<float><<<gt, 128, 0, s>>>(c->dc, op, cx, cw, cdw, cdu, pf, cv, bf, i0, g);
+      else
+        k_stats_y_tall<double><<<gt, 128, 0, s>>>(c->dc, op, cx, cw, cdw, cdu, pd, cv, bf, i0, g);
+      c->launches += 1;
+    } else if (c->f32[OTBL_F_P]) {
+      go(sy ? k_stats_y<float, 9> : k_stats_y<float, 33>, gy, cx, cw, cdw, cdu, pf, cv, bf, i0, g);
+    } else {
+      go(sy ? k_stats_y<double, 9> : k_stats_y<double, 33>, gy, cx, cw, cdw, cdu, pd, cv, bf, i0, g);
+    }
     k_stats_acc<<<(g * ny + 3) / 4, 128, smem, s>>>(c->dc, z, bf, c->f[OTBL_F_V], dvdx, c->stats, i0, g);
     c->launches += 1;
   }

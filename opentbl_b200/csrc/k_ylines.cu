@@ -34,7 +34,8 @@ __device__ __forceinline__ V ld_row(const V *p, bool ok) {
 }
 
 // Rows per chunk: 7 rows keep the tail's three solves in 168 registers; boxes
-// taller than 447 rows take longer chunks.
+// taller than 447 rows take longer chunks, above 3840 rows (256 chunks of 15)
+// the serial kernels *_tall.
 static int y_chunk(int ny) { return ny < 7 * 64 ? 7 : 15; }
 constexpr bool y_table_global(int K) { return K > 7; }
 // The tail's tables: coefficient i of row s + b of chunk q at tab[q S + i K +
@@ -567,6 +568,70 @@ __global__ void __launch_bounds__(256, 2) k_pois_solve(DCoefT<T> c, T *phi, cons
     if (s + b < ny1) x[(size_t)b * nk] = y[b];
 }
 
+// interpyy and the solve of columns of more than 256 chunks (rows above 3840),
+// which no CTA holds: a thread per mode, serial sweeps, the forward one's
+// values kept in the output. Only there for their range (the boxes of a step
+// end at genflu's 3227 rows).
+template <typename T>
+__global__ void __launch_bounds__(128) k_interpy_tall(DCoefT<T> c, InterpyArgs a) {
+  using V = V2<T>;
+  const int f = blockIdx.y, ny = c.ny, nk = c.nz1 >> 1, m = blockIdx.x * 128 + threadIdx.x;
+  if (m >= c.nx * nk) return;
+  const int i = m / nk, k = m - i * nk, which = pick3(a.which, f), jin = which == 0 ? ny + 1 : ny;
+  const double2 *in = reinterpret_cast<const double2 *>(pick3(a.in, f)) + (size_t)i * jin * nk + k;
+  V *o = static_cast<V *>(pick3(a.out, f)) + (size_t)i * ny * nk + k;
+  const T *lu = which == 0 ? c.inyu : c.inyv, *e = which == 0 ? c.cofiuy : c.cofivy;
+  auto g = [&](int r) {
+    const double2 v = __ldg(in + (size_t)r * nk);
+    return cmake<V>((T)v.x, (T)v.y);
+  };
+  const int off = which == 0 ? 0 : -1;
+  V x = cmake<V>(T(0), T(0));
+  for (int r = 0; r < ny; ++r) {
+    V y = cmake<V>(T(0), T(0));
+    if (r > 0 && r < ny - 1) {
+      fma2(y, e[2 * r], g(r + off));
+      fma2(y, e[2 * r + 1], g(r + off + 1));
+    } else if (r > 0 || which == 1) {
+      for (int q = 1; q <= 4; ++q)
+        fma2(y, M4(c.inby, (r == 0 ? 3 : (which == 0 ? 1 : 4)), q), g(r == 0 ? q - 1 : jin - q));
+    }
+    if (r > 0) fma2(y, lu[3 * r], x);
+    o[(size_t)r * nk] = x = y;
+  }
+  for (int r = ny - 1; r >= 0; --r) {
+    V y = o[(size_t)r * nk];
+    if (r < ny - 1) fma2(y, -lu[3 * r + 2], x);
+    x = cmake<V>(lu[3 * r + 1] * y.x, lu[3 * r + 1] * y.y);
+    o[(size_t)r * nk] = x;
+  }
+}
+
+template <typename T>
+__global__ void __launch_bounds__(128) k_pois_solve_tall(DCoefT<T> c, T *phi, const T *__restrict__ dinv, int k0,
+                                                         int nkm) {
+  using V = V2<T>;
+  const int ny = c.ny, ny1 = ny - 1, nk = c.nz1 >> 1, m = blockIdx.x * 128 + threadIdx.x;
+  if (m >= (c.nx - 1) * nkm) return;
+  const int i = m / nkm + 2, k = k0 + m - (i - 2) * nkm;
+  V *p = reinterpret_cast<V *>(phi) + (size_t)(i - 1) * ny * nk + k;
+  const T *dv = dinv + (size_t)(i - 1) * ny * nk + k, *ayp = c.ayp;
+  if (i == 2 && k == 0) p[(size_t)(ny1 - 1) * nk] = cmake<V>(T(0), T(0));
+  V x = p[0];
+  for (int r = 1; r < ny1; ++r) {
+    V y = p[(size_t)r * nk];
+    fma2(y, -ayp[3 * r] * dv[(size_t)(r - 1) * nk], x);
+    p[(size_t)r * nk] = x = y;
+  }
+  for (int r = ny1 - 1; r >= 0; --r) {
+    V y = p[(size_t)r * nk];
+    const T d = dv[(size_t)r * nk];
+    if (r < ny1 - 1) fma2(y, -ayp[3 * r + 2], x);
+    x = cmake<V>(d * y.x, d * y.y);
+    p[(size_t)r * nk] = x;
+  }
+}
+
 // ---------------------------------------------------------------------------
 // tables and launch wrappers
 // ---------------------------------------------------------------------------
@@ -618,6 +683,7 @@ static cudaError_t y_tables(otbl_ctx *c) {
   std::vector<T> all(2 * z.in + z.tw[0] + z.tw[1], T(0));
   T *tab = all.data();
   for (int wh = 0; wh < 2; ++wh, tab += z.in) {
+    if (z.Ci > z.QS) continue;  // k_interpy_tall reads the coefficients
     const T *e = A(wh ? OTBL_C_COFIVY : OTBL_C_COFIUY);
     auto put = [&](int i, int r, T v) { tab[(size_t)(i * K + r % K) * z.QS + r / K] = v; };
     for (int r = 1; r < ny - 1; ++r) {
@@ -675,6 +741,10 @@ static void interpy_t(otbl_ctx *c, const DCoefT<T> &dc, InterpyArgs &a) {
   const YSizes z = y_sizes(c->cfg.ny);
   for (int wh = 0; wh < 2; ++wh) a.tab[wh] = static_cast<const T *>(c->w.ytab) + wh * z.in;
   a.C = z.Ci;
+  if (a.C > 256) {
+    k_interpy_tall<T><<<dim3((c->cfg.nx * (c->dc.nz1 / 2) + 127) / 128, 3), 128, 0, c->stream>>>(dc, a);
+    return;
+  }
   // as wide as the threads allow, or narrower when the autotuner found that
   // faster (tune_bs 128, 64, 32)
   a.L = std::max(1, y_lanes(a.C, 256) * c->tune_bs[2] / 128);
@@ -812,7 +882,9 @@ static void pois_solve_t(otbl_ctx *c, const DCoefT<T> &dc, T *phi, const T *dinv
   const int C = (c->cfg.ny - 1 + K - 1) / K, L = std::max(1, std::min(32, 224 / C)), NT = y_threads(C, L);
   const int ncm = (c->cfg.nx - 1) * nkm, nb = (ncm + L - 1) / L;
   const size_t sm = (size_t)2 * NT * (sizeof(V2<T>) + sizeof(T));
-  if (K == 7)
+  if (C > 256)
+    k_pois_solve_tall<T><<<(ncm + 127) / 128, 128, 0, c->stream>>>(dc, phi, dinv, k0, nkm);
+  else if (K == 7)
     k_pois_solve<T, 7><<<nb, NT, sm, c->stream>>>(dc, phi, dinv, k0, nkm, C, L);
   else
     k_pois_solve<T, 15><<<nb, NT, sm, c->stream>>>(dc, phi, dinv, k0, nkm, C, L);
