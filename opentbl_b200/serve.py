@@ -156,7 +156,7 @@ class Server:
         # the slots of the next two requests are prepared side by side: a small
         # box runs its steps in less time than one preparation takes
         self.creator = ThreadPoolExecutor(max_workers=2)
-        self.pending = deque()  # (request, future of its slot, new), in queue order
+        self.pending = deque()  # (request, future of its slot, new, bytes), in queue order
         self.stats = {"created": 0, "reused": 0, "evicted": 0, "graph_launches": 0,
                       "direct_steps": 0, "peak_bytes": 0, "peak_active": 0,
                       "create_s": 0.0, "rebind_s": 0.0, "capture_s": 0.0}
@@ -181,22 +181,28 @@ class Server:
         (or given the CTA sizes already picked for its grid size), or the
         idle `slot` re-bound to req; then the CUDA graph of its chunk."""
         t = time.perf_counter()
-        if slot is None:
-            box = Box(req.cfg, init, device=self.device)
-            if self.autotune:
-                if key in self.tuning:
-                    box.set_tuning(self.tuning[key])
-                else:
-                    self.tuning[key] = box.autotune()
-            slot = _Slot(box, need)
-            self.stats["create_s"] += time.perf_counter() - t
-        else:
-            slot.box.rebind(req.cfg, init)
-            self.stats["rebind_s"] += time.perf_counter() - t
-        t = time.perf_counter()
-        slot.chunk = min(self.chunk, req.steps)
-        slot.graph = Graph([slot.box], slot.chunk) if req.steps >= slot.chunk else None
-        self.stats["capture_s"] += time.perf_counter() - t
+        box = slot.box if slot is not None else None
+        try:
+            if box is None:
+                box = Box(req.cfg, init, device=self.device)
+                if self.autotune:
+                    if key in self.tuning:
+                        box.set_tuning(self.tuning[key])
+                    else:
+                        self.tuning[key] = box.autotune()
+                slot = _Slot(box, need)
+                self.stats["create_s"] += time.perf_counter() - t
+            else:
+                box.rebind(req.cfg, init)
+                self.stats["rebind_s"] += time.perf_counter() - t
+            t = time.perf_counter()
+            slot.chunk = min(self.chunk, req.steps)
+            slot.graph = Graph([box], slot.chunk) if req.steps >= slot.chunk else None
+            self.stats["capture_s"] += time.perf_counter() - t
+        except BaseException:
+            if box is not None:
+                box.close()
+            raise
         return slot
 
     def _start(self, req: Request, init: dict) -> bool:
@@ -207,7 +213,7 @@ class Server:
         lst = self.idle.get(key)
         if lst:
             s = lst.pop()
-            self.pending.append((req, self.creator.submit(self._prepare, req, init, s, s.nbytes, key), False))
+            self.pending.append((req, self.creator.submit(self._prepare, req, init, s, s.nbytes, key), False, s.nbytes))
             return True
         need = self._bytes(req.cfg, init)
         while self.used + need > self.budget and self._evict_one():
@@ -216,17 +222,44 @@ class Server:
             return False
         self.used += need
         self.stats["peak_bytes"] = max(self.stats["peak_bytes"], self.used)
-        self.pending.append((req, self.creator.submit(self._prepare, req, init, None, need, key), True))
+        self.pending.append((req, self.creator.submit(self._prepare, req, init, None, need, key), True, need))
         return True
 
-    def _acquire(self):
-        """The prepared slot of the request at the head of the queue (None
-        until it is ready)."""
-        if not self.pending or not self.pending[0][1].done():
+    def _acquire(self, req: Request):
+        """The slot prepared for `req`, the head of the queue (None until it
+        is ready). A preparation that failed closed its box: its bytes are
+        free again."""
+        if not self.pending or self.pending[0][0] is not req or not self.pending[0][1].done():
             return None
-        _, fut, created = self.pending.popleft()
+        _, fut, created, need = self.pending.popleft()
+        try:
+            s = fut.result()
+        except BaseException:
+            self.used -= need
+            raise
         self.stats["created" if created else "reused"] += 1
-        return fut.result()
+        return s
+
+    def _drain(self, active):
+        """Ends what a run left behind (it ended by an exception): slots in
+        preparation become idle ones, those of running requests are closed."""
+        while self.pending:
+            _, fut, _, need = self.pending.popleft()
+            try:
+                s = fut.result()
+            except Exception:
+                self.used -= need
+                continue
+            if s.graph is not None:
+                s.graph.close()
+                s.graph = None
+            self.idle.setdefault(s.key, []).append(s)
+        for s in active:
+            if s.graph is not None:
+                s.graph.close()
+                s.graph = None
+            s.box.close()
+            self.used -= s.nbytes
 
     def _issue(self, s: _Slot):
         """Next chunk of the slot's request: a graph launch of `chunk` steps,
@@ -263,9 +296,15 @@ class Server:
 
     # ---- the loop ----
     def run(self, requests: list[Request], poll: float = 2e-4) -> list[Result]:
+        active = []
+        try:
+            return self._run(requests, poll, active)
+        finally:
+            self._drain(active)
+
+    def _run(self, requests, poll, active):
         pending = deque(sorted(requests, key=lambda r: r.arrival))
         queue = deque()
-        active = []
         results = []
         head = None  # the next request to prepare a slot for and its initial state
         t0 = time.perf_counter()
@@ -283,14 +322,14 @@ class Server:
                         head = (req, self.templates.get(req.cfg))
                     if not self._start(*head):
                         break
-                s = self._acquire()
+                s = self._acquire(queue[0])
                 if s is None:
                     break
                 req = queue.popleft()
+                active.append(s)
                 s.req = req
                 s.remaining = req.steps
                 s.admitted = time.perf_counter() - t0
-                active.append(s)
                 self._issue(s)
                 did = True
             self.stats["peak_active"] = max(self.stats["peak_active"], len(active))
@@ -301,8 +340,8 @@ class Server:
                 if s.remaining > 0:
                     self._issue(s)
                 else:
-                    active.remove(s)
                     results.append(self._finish(s, time.perf_counter() - t0))
+                    active.remove(s)
                 did = True
             if not did:
                 if not active and not queue and pending:

@@ -70,6 +70,94 @@ def test_admission_evicts_idle_slots_of_other_sizes():
     assert all(b.box.closed for b in boxes)
 
 
+class _FakeRun(_FakeBox):
+    """Host stand-in for Box in a whole run: `field` tells whose box it is."""
+    open = 0
+    fail = ()  # Re_theta whose preparation fails, whose result fails
+
+    def __init__(self, cfg, init, device=0):
+        super().__init__(cfg)
+        self.check()
+        type(self).open += 1
+
+    def check(self):
+        if self.cfg.re_theta == self.fail[0]:
+            raise native.OtblError("preparation fails")
+
+    def rebind(self, cfg, init):
+        self.cfg = cfg
+        self.check()
+
+    def close(self):
+        type(self).open -= not self.closed
+        super().close()
+
+    def autotune(self):
+        return (128, 128, 128)
+
+    def set_tuning(self, bs):
+        pass
+
+    def advance(self, n):
+        pass
+
+    def busy(self):
+        return False
+
+    def sync(self):
+        if self.cfg.re_theta == self.fail[1]:
+            raise native.OtblError("result fails")
+
+    def inflow(self):
+        return None, dict(dt=0.0, utauout=0.0, rthout=0.0)
+
+    def field(self, n):
+        return self.cfg.re_theta
+
+
+class _FakeGraph:
+    def __init__(self, boxes, steps):
+        pass
+
+    def launch(self):
+        pass
+
+    def busy(self):
+        return False
+
+    def sync(self):
+        pass
+
+    def close(self):
+        pass
+
+
+class _FakeTemplates:
+    def get(self, cfg):
+        return dict(re=1000.0, xout=10)
+
+
+@pytest.mark.parametrize("fail", [(301.0, None), (None, 301.0), (303.0, None), (None, 304.0)], ids=str)
+def test_server_survives_a_failed_run(monkeypatch, fail):
+    """One of six requests fails, in preparation or at its end: run raises, no
+    box and no byte is lost, and the next run of the same server gives each
+    request its own box."""
+    monkeypatch.setattr(serve, "Box", type("B", (_FakeRun,), dict(fail=fail)))
+    monkeypatch.setattr(serve, "Graph", _FakeGraph)
+    reqs = [serve.Request(k, replace(config.TINY, nx=(33, 41)[k % 2], re_theta=300.0 + k), 4, 0.0) for k in range(6)]
+    srv = serve.Server(chunk=2, max_active=3, keep_fields=True, templates=_FakeTemplates())
+    with pytest.raises(native.OtblError, match="fails"):
+        srv.run(reqs)
+    idle = [s for lst in srv.idle.values() for s in lst]
+    assert not srv.pending
+    assert srv.used == sum(s.nbytes for s in idle) and serve.Box.open == len(idle)
+    good = [r for r in reversed(reqs) if r.cfg.re_theta not in fail]
+    res = srv.run(good)
+    assert {r.rid: r.fields["u"] for r in res} == {r.rid: r.cfg.re_theta for r in good}
+    srv.close()
+    assert serve.Box.open == 0
+
+
 @pytest.mark.gpu
 @pytest.mark.parametrize("precision", [0, 1])
 def test_ctx_bytes_is_what_a_context_allocates(precision):
