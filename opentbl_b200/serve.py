@@ -9,8 +9,8 @@ in chunks of RK3 steps, each chunk one CUDA graph launch, so the kernels of
 all admitted requests overlap on the device. Slots are kept when their
 request finishes and re-bound (otbl_ctx_rebind) to the next request of the
 same grid size and precision; idle slots of other sizes are released when
-memory is needed. A slot is prepared for its request on a background host
-thread (a new context: device allocation, coefficient upload, autotuning;
+memory is needed. A slot is prepared for its request on one of two background
+host threads (a new context: device allocation, coefficient upload, autotuning;
 or an idle one re-bound: the request's coefficients and initial fields
 uploaded on the slot's stream; then the capture of its chunk's CUDA graph),
 so the loop keeps feeding the running requests meanwhile. The host loop
@@ -26,6 +26,7 @@ for bit).
 from __future__ import annotations
 
 import dataclasses
+import threading
 import time
 from collections import deque
 from concurrent.futures import ThreadPoolExecutor
@@ -132,6 +133,7 @@ class _Slot:
         self.graph = None
         self.chunk = 0
         self.admitted = 0.0
+        self.took = {}  # seconds its last preparation spent, by kind
 
     @property
     def key(self):
@@ -152,7 +154,10 @@ class Server:
         self.L = native.lib()
         self.idle = {}
         self.used = 0
-        self.tuning = {}  # CTA sizes picked by the autotuner, per grid size
+        self.tuning = {}  # CTA tiles picked by the autotuner, per grid size
+        # one autotuner at a time: two would time each other's launches, and the
+        # second request of a size takes what the first one's found
+        self.tune_lock = threading.Lock()
         # the slots of the next two requests are prepared side by side: a small
         # box runs its steps in less time than one preparation takes
         self.creator = ThreadPoolExecutor(max_workers=2)
@@ -177,8 +182,8 @@ class Server:
         return False
 
     def _prepare(self, req: Request, init: dict, slot: "_Slot | None", need: int, key):
-        """Runs on the preparation thread: a new context for req, autotuned
-        (or given the CTA sizes already picked for its grid size), or the
+        """Runs on a preparation thread: a new context for req, autotuned (or
+        given the CTA tiles already picked for its grid size), or the
         idle `slot` re-bound to req; then the CUDA graph of its chunk."""
         t = time.perf_counter()
         box = slot.box if slot is not None else None
@@ -186,19 +191,20 @@ class Server:
             if box is None:
                 box = Box(req.cfg, init, device=self.device)
                 if self.autotune:
-                    if key in self.tuning:
-                        box.set_tuning(self.tuning[key])
-                    else:
-                        self.tuning[key] = box.autotune()
+                    with self.tune_lock:
+                        if key not in self.tuning:
+                            self.tuning[key] = box.autotune()
+                        else:
+                            box.set_tuning(self.tuning[key])
                 slot = _Slot(box, need)
-                self.stats["create_s"] += time.perf_counter() - t
+                what = "create_s"
             else:
                 box.rebind(req.cfg, init)
-                self.stats["rebind_s"] += time.perf_counter() - t
-            t = time.perf_counter()
+                what = "rebind_s"
+            t, took = time.perf_counter(), time.perf_counter() - t
             slot.chunk = min(self.chunk, req.steps)
             slot.graph = Graph([box], slot.chunk) if req.steps >= slot.chunk else None
-            self.stats["capture_s"] += time.perf_counter() - t
+            slot.took = {what: took, "capture_s": time.perf_counter() - t}
         except BaseException:
             if box is not None:
                 box.close()
@@ -238,6 +244,8 @@ class Server:
             self.used -= need
             raise
         self.stats["created" if created else "reused"] += 1
+        for what, took in s.took.items():  # added up here: the preparation has two threads
+            self.stats[what] += took
         return s
 
     def _drain(self, active):

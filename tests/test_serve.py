@@ -2,6 +2,8 @@
 loop. CPU tests cover request generation and the host logic of admission;
 GPU tests check that a graph-launched ensemble and the serving mix give the
 same bits as each box advanced alone."""
+import time
+
 import numpy as np
 import pytest
 
@@ -156,6 +158,32 @@ def test_server_survives_a_failed_run(monkeypatch, fail):
     assert {r.rid: r.fields["u"] for r in res} == {r.rid: r.cfg.re_theta for r in good}
     srv.close()
     assert serve.Box.open == 0
+
+
+def test_one_autotuner_per_size(monkeypatch):
+    """Slots of the same size prepared side by side: the first is autotuned,
+    the others take its tiles."""
+    class Slow(_FakeRun):
+        fail = (None, None)
+        calls = []
+
+        def autotune(self):
+            self.calls.append("autotune")
+            time.sleep(0.05)
+            return (64, 32, 128)
+
+        def set_tuning(self, bs):
+            assert bs == (64, 32, 128)
+            self.calls.append("set")
+
+    monkeypatch.setattr(serve, "Box", Slow)
+    monkeypatch.setattr(serve, "Graph", _FakeGraph)
+    reqs = [serve.Request(k, replace(config.TINY, re_theta=300.0 + k), 4, 0.0) for k in range(2)]
+    srv = serve.Server(chunk=2, max_active=2, templates=_FakeTemplates())
+    srv.run(reqs)
+    assert Slow.calls == ["autotune", "set"]
+    assert srv.stats["create_s"] >= 0.05
+    srv.close()
 
 
 @pytest.mark.gpu
