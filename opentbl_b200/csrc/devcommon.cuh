@@ -4,7 +4,6 @@
 
 // Fortran-shaped accessors into the packed coefficient buffer
 #define A3(a, r, i) (a)[((i)-1) * 3 + (r)-1]
-#define A2(a, r, i) (a)[((i)-1) * 2 + (r)-1]
 #define M4(a, r, cc) (a)[((cc)-1) * 4 + (r)-1]
 #define M5(a, r, cc) (a)[((cc)-1) * 5 + (r)-1]
 #define M2(a, r, cc) (a)[((cc)-1) * 2 + (r)-1]
@@ -18,11 +17,6 @@ __device__ __forceinline__ float rnd(float x, int) { return x; }
 // NaN-propagating maximum of non-negative values
 __device__ __forceinline__ double nmax(double m, double v) {
   return (m != m) ? m : ((v != v) ? v : fmax(m, v));
-}
-
-// Waits for every cp.async this thread issued (the caller then syncs the CTA).
-__device__ __forceinline__ void cp_async_wait_all() {
-  asm volatile("cp.async.commit_group;\ncp.async.wait_group 0;\n" ::: "memory");
 }
 
 // a[f] of a kernel-parameter array with f uniform across the grid's y index,

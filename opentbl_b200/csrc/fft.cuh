@@ -54,14 +54,6 @@ __device__ __forceinline__ V cmul_i(V a, int s) {
   r.y = s > 0 ? a.x : -a.x;
   return r;
 }
-// a*(x, y) for a real scalar
-template <typename V, typename S>
-__device__ __forceinline__ V cscale(S a, V v) {
-  V r;
-  r.x = a * v.x;
-  r.y = a * v.y;
-  return r;
-}
 template <typename V>
 __device__ __forceinline__ V cmake(decltype(V{}.x) x, decltype(V{}.x) y) {
   V r;
@@ -194,8 +186,8 @@ __device__ __forceinline__ void dft_small(V *v) {
 //   item j (0 <= j < M/R), k = j mod Ns:
 //   v[r] = buf[j + r*M/R] * W_{Ns*R}^{r*k};  v = DFT_R(v);
 //   buf[(j/Ns)*Ns*R + k + r*Ns] = v[r]
-// MAXIT bounds the items per thread. SYNC is __syncwarp or __syncthreads.
-template <int R, int SIGN, int MAXIT, bool BLOCK, typename V>
+// MAXIT bounds the items per thread of the warp.
+template <int R, int SIGN, int MAXIT, typename V>
 __device__ __forceinline__ void stockham_pass(V *buf, int M, int Ns, const V *__restrict__ tw, int t, int G) {
   const int nit = M / R;
   const int stride_tw = M / (Ns * R);
@@ -208,10 +200,7 @@ __device__ __forceinline__ void stockham_pass(V *buf, int M, int Ns, const V *__
       for (int r = 0; r < R; ++r) v[it][r] = buf[j + r * nit];
     }
   }
-  if (BLOCK)
-    __syncthreads();
-  else
-    __syncwarp();
+  __syncwarp();
 #pragma unroll
   for (int it = 0; it < MAXIT; ++it) {
     const int j = t + it * G;
@@ -231,10 +220,7 @@ __device__ __forceinline__ void stockham_pass(V *buf, int M, int Ns, const V *__
       for (int r = 0; r < R; ++r) buf[base + r * Ns] = v[it][r];
     }
   }
-  if (BLOCK)
-    __syncthreads();
-  else
-    __syncwarp();
+  __syncwarp();
 }
 
 // Warp FFT of a power-of-two length M <= 512 in shared memory (in place).
@@ -242,38 +228,17 @@ template <int SIGN, typename V>
 __device__ __forceinline__ void warp_fft(V *buf, int M, const V *__restrict__ tw, int lane) {
   int Ns = 1;
   while (Ns * 8 <= M) {
-    stockham_pass<8, SIGN, 2, false>(buf, M, Ns, tw, lane, 32);
+    stockham_pass<8, SIGN, 2>(buf, M, Ns, tw, lane, 32);
     Ns *= 8;
   }
   if (Ns * 4 <= M) {
-    stockham_pass<4, SIGN, 4, false>(buf, M, Ns, tw, lane, 32);
+    stockham_pass<4, SIGN, 4>(buf, M, Ns, tw, lane, 32);
     Ns *= 4;
   }
   if (Ns * 2 <= M) {
-    stockham_pass<2, SIGN, 8, false>(buf, M, Ns, tw, lane, 32);
+    stockham_pass<2, SIGN, 8>(buf, M, Ns, tw, lane, 32);
     Ns *= 2;
   }
-}
-
-// CTA FFT of length n = 2^a 3^b 5^c (n <= 4096) in shared memory; NB lines
-// stored back to back (line l at buf + l*n) are transformed in turn by the
-// 256 threads of the CTA. The twiddle table has n entries.
-template <int R, int SIGN, int NB, typename V>
-__device__ __forceinline__ void block_pass(V *buf, int n, int Ns, const V *__restrict__ tw) {
-  constexpr int MAXIT = (4096 / R + 255) / 256;
-#pragma unroll 1
-  for (int l = 0; l < NB; ++l)
-    stockham_pass<R, SIGN, MAXIT, true>(buf + l * n, n, Ns, tw, threadIdx.x, 256);
-}
-
-template <int SIGN, int NB, typename V>
-__device__ __forceinline__ void block_fft(V *buf, int n, const V *__restrict__ tw) {
-  int Ns = 1, rem = n;
-  while (rem % 8 == 0) { block_pass<8, SIGN, NB>(buf, n, Ns, tw); Ns *= 8; rem /= 8; }
-  while (rem % 4 == 0) { block_pass<4, SIGN, NB>(buf, n, Ns, tw); Ns *= 4; rem /= 4; }
-  while (rem % 2 == 0) { block_pass<2, SIGN, NB>(buf, n, Ns, tw); Ns *= 2; rem /= 2; }
-  while (rem % 3 == 0) { block_pass<3, SIGN, NB>(buf, n, Ns, tw); Ns *= 3; rem /= 3; }
-  while (rem % 5 == 0) { block_pass<5, SIGN, NB>(buf, n, Ns, tw); Ns *= 5; rem /= 5; }
 }
 
 // Shared-memory index of element i of a line for the line FFTs below.
@@ -350,8 +315,7 @@ __device__ __forceinline__ void stockham_pass_pad(V *buf, int M, int Ns, const V
 }
 
 // FFT of length n = 2^a 3^b 5^c of this thread's padded line (n * lines per
-// CTA <= 4096), the radix order of block_fft (8s, 4s, 2s, 3s, 5s), so the
-// arithmetic is block_fft's operation for operation.
+// CTA <= 4096), radices in the order 8s, 4s, 2s, 3s, 5s.
 // NT: threads of the CTA (n * lines <= 4096, so a thread has at most
 // 4096 / (NT R) items of a radix-R pass)
 template <int SIGN, int NT = 256, typename V>

@@ -34,9 +34,8 @@ struct XStream {
   CflReset reset;        // interpxx
 };
 
-// planes per segment, interpxx and difvisxx, measured at 1025x193x512: FP64
-// RK3 step 42.2 ms at 8 planes for interpxx, 42.5 at 4; difvisxx 6 against 4
-// and 8: 42.5, 42.7, 42.7 (FP32 8 against 12: 30.8, 30.9)
+// planes per segment, measured at 1025x193x512: FP64 difvisxx 6 against 4 and
+// 8, 42.5, 42.7, 42.7 ms per RK3 step; FP32 8 against 12, 30.8, 30.9
 template <typename T, bool DV>
 constexpr int xseg() {
   return DV && sizeof(T) == 8 ? 6 : 8;
@@ -49,7 +48,7 @@ constexpr int xseg() {
 // serial sweeps from shared memory. The sequence of segments is the forward
 // sweep (0..nseg-1) then the backward one (nseg-1..0). DV: difvisxx (inputs:
 // the product, FP32 on the mixed path, and the FP64 velocity) or interpxx
-// (input: the FP64 velocity).
+// (input: the FP64 velocity; mixed path only).
 // ---------------------------------------------------------------------------
 template <typename T, bool DV>
 __global__ void __launch_bounds__(128) k_xline_t(DCoefT<T> c, XStream a, int *err, const __grid_constant__ XMaps maps) {
@@ -193,18 +192,19 @@ __global__ void __launch_bounds__(128) k_xline_t(DCoefT<T> c, XStream a, int *er
   }
 }
 
-// One row of 16 T per plane i of each table (dv, which), dv 0 interpxx and
-// 1 difvisxx, which 0 u-type and 1 v-type coefficients: the right-hand-side
-// weights econ[2i], econ[2i+1] and the LU coefficients icon[3i..3i+2], then
-// for difvisxx the viscous operator's econv[3i..3i+2] and iconv[3i..3i+2].
-// k_xline_t's ring stages a segment's rows with its line boxes. Entries a
-// plane does not use are 0.
+// One row of 16 T per plane i of each table (dv, which), dv 0 interpxx (mixed
+// path) and 1 difvisxx, which 0 u-type and 1 v-type coefficients: the
+// right-hand-side weights econ[2i], econ[2i+1] and the LU coefficients
+// icon[3i..3i+2], then for difvisxx the viscous operator's econv[3i..3i+2] and
+// iconv[3i..3i+2]. k_xline_t's ring stages a segment's rows with its line
+// boxes. Entries a plane does not use are 0.
 template <typename T>
 __global__ void __launch_bounds__(128) k_x_rows(DCoefT<T> c, T *tab) {
   const int nx = c.nx;
+  constexpr int dv0 = sizeof(T) == 8;  // the first table's
   const int e = blockIdx.x * blockDim.x + threadIdx.x;
-  if (e >= 4 * nx) return;
-  const int dv = e / (2 * nx), which = (e / nx) & 1, i = e % nx;
+  if (e >= (4 - 2 * dv0) * nx) return;
+  const int dv = e / (2 * nx) + dv0, which = (e / nx) & 1, i = e % nx;
   T *q = tab + (size_t)e * 16;
   for (int k = 0; k < 16; ++k) q[k] = T(0);
   const T *icon = dv ? (which == 0 ? c.dcxu : c.dcxv) : (which == 0 ? c.inxu : c.inxv);
@@ -253,7 +253,7 @@ static bool encode_lines(CUtensorMap *m, const void *base, size_t esz, int nx, i
 }
 
 static bool build_x_maps(otbl_ctx *c) {
-  const int KI = c->mixed ? xseg<float, false>() : xseg<double, false>();
+  const int KI = xseg<float, false>();
   const int KD = c->mixed ? xseg<float, true>() : xseg<double, true>();
   const int nx = c->cfg.nx, nz1 = c->dc.nz1, ny = c->cfg.ny;
   const int np[3] = {nz1 * (ny + 1), nz1 * ny, nz1 * (ny + 1)};
@@ -263,11 +263,13 @@ static bool build_x_maps(otbl_ctx *c) {
   bool ok = true;
   const int which[3] = {0, 1, 1};  // u-type or v-type operator of each field
   const char *tab = static_cast<const char *>(c->w.xrowc);
-  auto table = [&](int dv, int wh) { return tab + (size_t)(2 * dv + wh) * nx * 16 * ew; };
+  auto table = [&](int dv, int wh) { return tab + (size_t)(2 * (dv - !c->mixed) + wh) * nx * 16 * ew; };
   for (int f = 0; f < 3 && ok; ++f) {
-    ok = ok && encode_lines(&c->xmi.g[f], st[f], 8, nx, np[f], KI + 1);
-    c->xmi.u[f] = c->xmi.g[f];  // unused by interpxx
-    ok = ok && encode_xrows(&c->xmi.r[f], table(0, which[f]), ew, nx, KI);
+    if (c->mixed) {
+      ok = ok && encode_lines(&c->xmi.g[f], st[f], 8, nx, np[f], KI + 1);
+      c->xmi.u[f] = c->xmi.g[f];  // unused by interpxx
+      ok = ok && encode_xrows(&c->xmi.r[f], table(0, which[f]), ew, nx, KI);
+    }
     ok = ok && encode_lines(&c->xmd.g[f], pr[f], ew, nx, np[f], KD + 1);
     ok = ok && encode_lines(&c->xmd.u[f], st[f], 8, nx, np[f], KD + 2);
     ok = ok && encode_xrows(&c->xmd.r[f], table(1, which[f]), ew, nx, KD);
@@ -317,7 +319,7 @@ cudaError_t launch_xlines_stream(otbl_ctx *c, bool dv, int reset) {
   if (c->mixed)
     dv ? xline_t_launch<float, true>(c, c->dcf, 0) : xline_t_launch<float, false>(c, c->dcf, reset);
   else
-    dv ? xline_t_launch<double, true>(c, c->dc, 0) : xline_t_launch<double, false>(c, c->dc, reset);
+    xline_t_launch<double, true>(c, c->dc, 0);
   return cudaGetLastError();
 }
 
@@ -1127,7 +1129,7 @@ void build_stream_maps(otbl_ctx *c) {
 
 // the per-plane and per-row coefficient tables of the rings
 cudaError_t prepare_stream(otbl_ctx *c) {
-  const int n = 4 * c->cfg.nx, m = 2 * c->cfg.ny;
+  const int n = (c->mixed ? 4 : 2) * c->cfg.nx, m = 2 * c->cfg.ny;
   if (c->mixed) {
     k_x_rows<float><<<(n + 127) / 128, 128, 0, c->stream>>>(c->dcf, static_cast<float *>(c->w.xrowc));
     k_y_rows<float><<<(m + 127) / 128, 128, 0, c->stream>>>(c->dcf, reinterpret_cast<float *>(c->w.yrowc));

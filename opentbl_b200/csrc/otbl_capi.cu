@@ -267,7 +267,7 @@ extern "C" int otbl_ctx_create(const otbl_config *cfg, const double *coef, int d
     char *xt = nullptr;
     TRY(dalloc(c, &xt, xline_table_bytes(nx, c->mixed)));
     w.xtab = xt;
-    TRY(dalloc(c, &xt, 64 * (size_t)nx * (c->mixed ? sizeof(float) : sizeof(double))));
+    TRY(dalloc(c, &xt, xrow_bytes(nx, c->mixed)));
     w.xrowc = xt;
     TRY(dalloc(c, &xt, ytab_bytes(ny, c->mixed)));
     w.ytab = xt;
@@ -318,7 +318,7 @@ extern "C" size_t otbl_ctx_bytes(const otbl_config *cfg) {
   b += (size_t)nx * ny * (nz1 / 2) * (sizeof(double) + (mixed ? sizeof(float) : 0));  // Poisson pivots
   if (cfg->options & OTBL_OPT_YDENSE) b += ydense_bytes(ny);     // dense interpyy operators
   b += xline_table_bytes(nx, mixed) + ytab_bytes(ny, mixed) + tdtab_doubles(ny) * sizeof(double);  // coefficient tables
-  b += 64 * (size_t)nx * (mixed ? sizeof(float) : sizeof(double));                 // streamed kernels' rows, factors
+  b += xrow_bytes(nx, mixed);                                      // streamed kernels' rows, factors
   b += (16 * (size_t)ny + 32 * (size_t)(ny + 2) + 6 * (size_t)(ny + 4)) * sizeof(double);
   return b;
 }

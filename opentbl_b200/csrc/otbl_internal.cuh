@@ -67,7 +67,7 @@ struct Work {
   void *xtab;                  // k_xline's coefficient tables (T): interpxx u, v, difvisxx u, v
   // streamed kernels of the largest boxes (k_stream.cu): per-plane and per-row
   // coefficients of their rings, implzy's top-down factors
-  void *xrowc;                 // [2][2][nx][16] (T)
+  void *xrowc;                 // [2][2][nx][16] (T), FP64 [1][2][nx][16]: interpxx is not streamed
   double *yrowc, *rowc;        // [2][ny][8] (T), [2][ny+2][16]
   double *fac_u, *fac_v;
   void *ytab;                  // k_interpy's and k_tail's coefficient tables (T)
@@ -271,6 +271,9 @@ cudaError_t launch_tail_rows(otbl_ctx *c);
 cudaError_t launch_final_stream(otbl_ctx *c, unsigned comps, cudaEvent_t before_vel = nullptr,
                                 bool second_scratch = false);
 void build_stream_maps(otbl_ctx *c);
+constexpr size_t xrow_bytes(int nx, bool mixed) {
+  return 16 * (size_t)nx * (mixed ? 4 * sizeof(float) : 2 * sizeof(double));
+}
 cudaError_t prepare_stream(otbl_ctx *c);
 cudaError_t launch_outflow(otbl_ctx *c);
 cudaError_t launch_pois(otbl_ctx *c, int m);
