@@ -1045,21 +1045,34 @@ cudaError_t launch_tail_rows(otbl_ctx *c) {
   return cudaGetLastError();
 }
 
-// Streamed tail against the chunked one, us per substep on B200: 1025x193x512
-// (174 thousand modes) FP64 3492 : 4800, mixed 2616 : 3300; 1025x140x512 2561
-// : 3120, mixed 1925 : 2029; 257x193x512 (44 thousand) 1048 : 1195, mixed 833
-// : 821; 513x129x256 (44 thousand) 874 : 795; 1025x48x512 mixed 746 : 609;
-// 513x65x128 (22 thousand) 309 : 171, mixed 221 : 135; 257x97x128 270 : 154,
-// mixed 262 : 109. The chunked FP64 tail fills the GPU with fewer warps: of
-// three boxes at once it takes more time where the streamed one's blocks of
-// 128 columns are well filled (nz = 512: 340 of 384; 33x100x512 903 : 968 us
-// per step), about as much at two thirds (nz = 128, 256) and less at one third.
+// Streamed tail : chunked tail on B200. Kernels alone, us per substep:
+// 1025x193x512 (174 thousand modes) FP64 3470 : 4863, mixed 2625 : 3368;
+// 1025x140x512 2557 : 3168, mixed 1916 : 2171; 257x193x512 (44 thousand) 1053 :
+// 1226, mixed 838 : 870; 513x129x256 (44 thousand) 882 : 827; 1025x48x512 mixed
+// 754 : 611; 513x65x128 (22 thousand) 311 : 182, mixed 222 : 146; 257x97x128
+// 277 : 163, mixed 264 : 116. But the chunked tail's CTAs fill an SM's
+// registers, so that no other kernel runs beside it: steps of one box, and of
+// three boxes issued in turn, us per step (/ start of the chunked kernels'
+// predecessors for three):
+//   mixed 65x150x512 2048 : 2105, 1558 : 1778 / 1574; 97x133x512 2440 : 2319,
+//   2076 : 2392 / 2010; 193x150x512 4500 : 4781, 4379 : 5448 / 4209; 321x97x512
+//   4582 : 4475, 4571 : 5160 / 4413; 33x100x512 (5 thousand modes) 1006 : 793,
+//   646 : 627 / 722
+//   FP64 65x92x256 1102 : 1024, 782 : 855 / 778; 193x73x256 1802 : 1742, 1681 :
+//   1793 / 1646; 193x150x256 3452 : 3620, 3214 : 3654 / 3313; 513x129x256 6662 :
+//   7120, 6532 : 7019 / 7116; 33x60x256 580 : 374, 337 : 292 / 388; 1025x60x256
+//   6571 : 6225, 6475 : 6385 / 7174; 33x100x512 1240 : 1123, 909 : 962 / 1042
+//   FP64 nz = 128 (one block of 84 columns): 513x97x128 2627 : 2467, 2287 :
+//   2411 / 3177; 769x65x128 2541 : 2438, 2431 : 2363 / 3281
+// So a box whose rows take several blocks of 128 columns is streamed unless it
+// is low (FP64, nz = 256) or has few modes, and one whose columns fill less
+// than a block only when it is large.
 bool stream_tail(const otbl_ctx *c) {
   const int modes = (c->cfg.nx - 1) * (c->dc.nz1 / 2), ny = c->cfg.ny;
   if (!c->fmaps_ok || ny > 447) return false;
-  if (c->mixed) return modes > 50000 && ny > 110;
   const int nz1 = c->dc.nz1, filled = 100 * nz1 / ((nz1 + 127) / 128 * 128);
-  return modes > 50000 || (modes > 30000 && ny > 150) || filled > 85;
+  if (c->mixed) return (modes > 50000 && ny > 110) || (filled > 85 && modes > 10000);
+  return modes > 50000 || (modes > 30000 && ny > 150) || filled > 85 || (nz1 > 128 && modes > 5000 && ny > 70);
 }
 
 template <typename W>

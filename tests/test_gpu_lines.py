@@ -42,10 +42,11 @@ def test_one_substep(nx, ny, dy):
     assert max(e.values()) <= 1e-10, e
 
 
-def test_wide_one_substep():
-    """nz1 = 340 fills the streamed kernels' blocks of 128 columns: interpyy and
-    the tail are streamed on a small box too."""
-    cfg = replace(config.TINY, nx=17, ny=50, nz=512, name="lines-wide")
+@pytest.mark.parametrize("nx,ny,nz", [(17, 50, 512), (65, 71, 256)], ids=str)
+def test_wide_one_substep(nx, ny, nz):
+    """Rows of several blocks of 128 columns: interpyy and the tail are streamed
+    on small boxes too."""
+    cfg = replace(config.TINY, nx=nx, ny=ny, nz=nz, lx=12.0 * max(nx, 33) / 33, name="lines-wide")
     init, coef = setup(cfg)
     g, o = Box(cfg, init, coef), oracle_box(cfg, init)
     g.substep(1, True)
@@ -54,7 +55,7 @@ def test_wide_one_substep():
     assert max(e.values()) <= 1e-11, e
 
 
-@pytest.mark.parametrize("nx,ny,nz", [(151, 50, 32), (17, 50, 512)], ids=str)
+@pytest.mark.parametrize("nx,ny,nz", [(151, 50, 32), (17, 50, 512), (65, 50, 512)], ids=str)
 def test_mixed_one_substep(nx, ny, nz):
     cfg = replace(config.TINY, nx=nx, ny=ny, nz=nz, lx=12.0 * max(nx, 33) / 33, precision=1, name="lines-mixed")
     init, coef = setup(cfg)
