@@ -1,15 +1,17 @@
-// The line operators of the largest boxes, one thread per line fed by TMA
-// rings: the serial Thomas sweeps of lip.f90, forward with a checkpoint every
-// few rows, then backward segment by segment, each recomputed from its
-// checkpoint. They move 1.5-1.8x the algorithmic bytes, but with hundreds of
-// thousands of lines they do it at 4.8-5.9 TB/s of DRAM traffic, and the
-// chunked solves of k_xlines.cu and k_ylines.cu, which read each input once,
-// are slower there: a CTA cannot hold whole lines of many neighbouring
-// columns, so their rows are 64-byte pieces of planes of 0.5 MB, and few warps
-// hide their latency. Below the limits of stream_* the chunked solves win (by
-// 1.1 to 8, the more the fewer the lines).
-//   k_xline_t            interpxx, difvisxx
-//   k_interpy_t          interpyy (most boxes with nz >= 128)
+// The line operators as streams, one thread per line fed by TMA rings: the
+// serial Thomas sweeps of lip.f90, forward with a checkpoint every few rows,
+// then backward segment by segment, each recomputed from its checkpoint. They
+// move 1.5-1.8x the algorithmic bytes, but with hundreds of thousands of lines
+// they do it at 4.8-5.9 TB/s of DRAM traffic, and the chunked solves of
+// k_xlines.cu and k_ylines.cu, which read each input once, are slower there: a
+// CTA cannot hold whole lines of many neighbouring columns, so their rows are
+// 64-byte pieces of planes of 0.5 MB, and few warps hide their latency. With
+// fewer lines the chunked kernels are the faster ones alone (by 1.1 to 2.5), but
+// they fill an SM and leave no room for kernels beside them, so the y-lines of
+// well-filled column blocks are streamed on small boxes too. The rules stream_*
+// say where, each with both sides measured.
+//   k_xline_t            difvisxx, interpxx (mixed path)
+//   k_interpy_t          interpyy
 //   k_final_ta, tb, s2   the tail of rhsp (rhsp.F90:291-484)
 #include <cudaTypedefs.h>
 
@@ -303,12 +305,12 @@ static void xline_t_launch(otbl_ctx *c, const DCoefT<T> &dc, int reset) {
   k_xline_t<T, DV><<<dim3((npu + 127) / 128, 3), 128, smem, c->stream>>>(dc, a, &c->st->err, DV ? c->xmd : c->xmi);
 }
 
-// Streamed interpxx and difvisxx against the chunked ones, us per substep on
-// B200: 1025x193x512 (fields of 541 MB) FP64 1195 : 1050 and 1838 : 2260,
-// mixed 712 : 915 and 1134 : 1366; 865x193x512 (456 MB) 1000 : 890 and 1554 :
-// 1370, mixed 596 : 746 and 952 : 1149; 1025x140x512 (393 MB) 645 : 707 and
-// 1522 : 1550, mixed 483 : 578 and 1011 : 893; 1025x96x512 (270 MB) 520 : 420
-// and 1011 : 945, mixed 389 : 316 and 564 : 510.
+// Streamed : chunked on B200, us per substep: difvisxx FP64 1025x193x512
+// (fields of 541 MB) 1835 : 2253, 865x193x512 (456 MB) 1554 : 1388, 1025x140x512
+// (393 MB) 1526 : 1550; mixed the same boxes 1125 : 1361, 975 : 1151, 1038 :
+// 889, 1025x96x512 (270 MB) 574 : 516; interpxx mixed 710 : 888, 593 : 783, 485
+// : 563, 393 : 313. FP64 interpxx was the slower one streamed at three of
+// these four (1195 : 1050, 1000 : 890, 645 : 707, 520 : 420) and is not built.
 bool stream_xlines(const otbl_ctx *c, bool dv) {
   const double mb = (double)otbl_field_len(c->cfg.nx, c->cfg.ny, c->cfg.nz, 1) * 8e-6;
   if (!c->xmaps_ok) return false;
@@ -498,15 +500,17 @@ static bool build_y_maps(otbl_ctx *c) {
   return ok;
 }
 
-// Streamed interpyy against the chunked one, us per substep alone: FP64
-// 1025x193x512 827 : 957, 513x129x256 176 : 161, 257x97x128 39 : 33; FP32 659 :
-// 653, 156 : 112, 37 : 23. But it runs beside interpxx, so what counts is how
-// much of the GPU it takes: three boxes at once, us per RK3 step, 257x97x128
-// 1234 : 1277, 81x150x128 876 : 898, 33x100x512 934 : 968, 513x129x256 6885 :
-// 6963; with nz = 64, whose 42 columns fill a third of a CTA, 385x97x64 1009 :
-// 967.
-// FP32 gains only where the blocks of 128 columns are nearly full: 33x100x512
-// 619 : 664, 1025x193x512 28563 : 29047, but 257x97x128 1062 : 1061 and slower alone.
+// Streamed : chunked on B200, us. Alone per substep: FP64 1025x193x512 821 :
+// 959, 513x129x256 177 : 164, 257x97x128 41 : 35; FP32 660 : 654, 163 : 115, 40 :
+// 26. But it runs beside interpxx, so what counts is how much of the GPU it
+// takes: steps of one box, and of three boxes issued in turn,
+//   FP64 257x97x128 1294 : 1310, 1268 : 1312; 513x129x256 7112 : 7125, 7046 :
+//   7197; 81x150x128 1006 : 985, 892 : 911; 33x100x512 1245 : 1248, 909 : 926;
+//   1025x193x512 one box 38177 : 38672; nz = 64, whose 42 columns fill a third
+//   of a CTA, 385x97x64 1105 : 1086, 1043 : 982
+//   FP32, which gains only where the blocks of 128 columns are nearly full:
+//   33x100x512 796 : 781, 626 : 676; 257x97x128 1094 : 1081, 1094 : 1085;
+//   513x129x256 5149 : 5060, 5894 : 5832; 1025x193x512 26693 : 26700
 bool stream_interpy(const otbl_ctx *c) {
   const int nz1 = c->dc.nz1, filled = 100 * nz1 / ((nz1 + 127) / 128 * 128);
   return c->ymaps_ok && (c->mixed ? filled > 85 : nz1 >= 84);
@@ -1045,15 +1049,14 @@ cudaError_t launch_tail_rows(otbl_ctx *c) {
   return cudaGetLastError();
 }
 
-// Streamed tail : chunked tail on B200. Kernels alone, us per substep:
+// Streamed : chunked on B200, us. The kernels alone per substep:
 // 1025x193x512 (174 thousand modes) FP64 3470 : 4863, mixed 2625 : 3368;
 // 1025x140x512 2557 : 3168, mixed 1916 : 2171; 257x193x512 (44 thousand) 1053 :
 // 1226, mixed 838 : 870; 513x129x256 (44 thousand) 882 : 827; 1025x48x512 mixed
 // 754 : 611; 513x65x128 (22 thousand) 311 : 182, mixed 222 : 146; 257x97x128
 // 277 : 163, mixed 264 : 116. But the chunked tail's CTAs fill an SM's
 // registers, so that no other kernel runs beside it: steps of one box, and of
-// three boxes issued in turn, us per step (/ start of the chunked kernels'
-// predecessors for three):
+// three boxes issued in turn (/ three with the tail that both replaced):
 //   mixed 65x150x512 2048 : 2105, 1558 : 1778 / 1574; 97x133x512 2440 : 2319,
 //   2076 : 2392 / 2010; 193x150x512 4500 : 4781, 4379 : 5448 / 4209; 321x97x512
 //   4582 : 4475, 4571 : 5160 / 4413; 33x100x512 (5 thousand modes) 1006 : 793,
@@ -1061,7 +1064,7 @@ cudaError_t launch_tail_rows(otbl_ctx *c) {
 //   FP64 65x92x256 1102 : 1024, 782 : 855 / 778; 193x73x256 1802 : 1742, 1681 :
 //   1793 / 1646; 193x150x256 3452 : 3620, 3214 : 3654 / 3313; 513x129x256 6662 :
 //   7120, 6532 : 7019 / 7116; 33x60x256 580 : 374, 337 : 292 / 388; 1025x60x256
-//   6571 : 6225, 6475 : 6385 / 7174; 33x100x512 1240 : 1123, 909 : 962 / 1042
+//   6571 : 6225, 6475 : 6385 / 7174; 33x100x512 1240 : 1123, 909 : 962 / 916
 //   FP64 nz = 128 (one block of 84 columns): 513x97x128 2627 : 2467, 2287 :
 //   2411 / 3177; 769x65x128 2541 : 2438, 2431 : 2363 / 3281
 // So a box whose rows take several blocks of 128 columns is streamed unless it
