@@ -1,8 +1,8 @@
 """otbl_advance replays small boxes' steps from a CUDA graph after three plain
 ones (otbl_capi.cu step_graph); whatever changes a step's launches drops it.
-The same box advanced in one call, step by step, over a rebind of its state
-arrays and over a change of the CTA sizes ends bit for bit where plain
-otbl_substep calls end."""
+The same box advanced in one call, and step by step over changes of the CTA tiles
+and a rebind of its state arrays, ends bit for bit where plain otbl_substep calls
+end."""
 import numpy as np
 import pytest
 
@@ -20,7 +20,8 @@ STATE = ("u", "v", "w", "p", "rhsupa", "rhsvpa", "rhswpa")
 def test_replay_is_the_step():
     torch = pytest.importorskip("torch")
 
-    cfg = config.SMALL
+    # the last chunks hold 3 planes, 3 (v) and 4 (u, w) rows
+    cfg = replace(config.SMALL, nx=73, ny=59)
     init, coef = setup(cfg)
     plain, once, split = (Box(cfg, init, coef) for _ in range(3))
     for _ in range(12):
@@ -31,14 +32,18 @@ def test_replay_is_the_step():
     per = (once.launches - l0) / 3
     once.advance(9)
     assert once.launches - l0 == 12 * per  # replayed kernels are counted too
+    assert once.replays == 9
     split.advance(5)
+    assert split.replays == 2
+    for tile in (64, 32):  # half and quarter tiles: plain steps, not the old graph
+        split.set_tuning((tile,) * 3)
+        split.advance(2)
+    assert split.replays == 2
+    split.set_tuning((128,) * 3)
     split.sync()
     own = {n: torch.from_numpy(split.field(n)).cuda() for n in STATE}
     torch.cuda.synchronize()
     split.bind_state({n: t.data_ptr() for n, t in own.items()})
-    split.advance(4)
-    split.set_tuning((64, 64, 64))
-    split.set_tuning((128, 128, 128))
     for _ in range(3):
         split.advance(1)
     for b in (plain, once, split):
