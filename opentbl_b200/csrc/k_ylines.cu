@@ -33,9 +33,10 @@ __device__ __forceinline__ V ld_row(const V *p, bool ok) {
   return ok ? ld_stream(p) : cmake<V>(0, 0);
 }
 
-// Rows per chunk: 7 rows keep the tail's three solves in 168 registers; boxes
-// taller than 447 rows take longer chunks, above 3840 rows (256 chunks of 15)
-// the serial kernels *_tall.
+// Rows per chunk: 7 rows keep the tail's three solves in 168 registers on the
+// mixed path (24 bytes spilled) and 255 in FP64 (48 bytes); boxes taller than
+// 447 rows take longer chunks, above 3840 rows (256 chunks of 15) the serial
+// kernels *_tall.
 static int y_chunk(int ny) { return ny < 7 * 64 ? 7 : 15; }
 constexpr bool y_table_global(int K) { return K > 7; }
 // The tail's tables: coefficient i of row s + b of chunk q at tab[q S + i K +

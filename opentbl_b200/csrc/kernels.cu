@@ -19,7 +19,7 @@
 //                           k_pois_solve  (k_ylines.cu) tridiagonal in y per (x-mode, kz)
 //                           k_pois_bwd    DCT-III along x
 //                           k_project     pressure/velocity update
-// (k_stream.cu holds the line operators of the largest boxes.)
+// (k_stream.cu holds the line operators of the largest and the widest boxes.)
 // The reference's transposes (change.f90) are not executed on the substep:
 // x-lines are read straight from the plane layout (threads over the
 // contiguous (j, kr) index, a walk over i with the plane stride), and the

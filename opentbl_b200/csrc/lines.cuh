@@ -21,7 +21,7 @@
 //
 // Against one thread per line with checkpoints every few rows (read the
 // inputs twice, 1.5-1.8x the algorithmic bytes, a serial chain as long as the
-// line) this reads each input once and the chain is K rows and two barriers.
+// line) this reads each input once and the chain is 2 K rows and two barriers.
 //
 // Where they exceed a few KB, the coefficients are staged in shared memory,
 // coefficient i of row s + b of chunk q at tab[q S + i K + b], S the number of

@@ -546,11 +546,12 @@ static int rhsp_issue(otbl_ctx *c, int m, int setstep) {
   //            genflu's plane 1
   //   side_lo: [products 2] products 1 (vw, vv, ww)
   // Small boxes (products_merged): all products and all tails in one launch
-  // each on main. With the streamed tail (the largest boxes): main: [k_dt] u tail ([genflu]
-  // before its velocity write), [products 1] v tail, [w tail]; side: [products
-  // 1] w tail on line scratch of its own.
-  // interpyy, interpxx and the energies only read the state; each products part reads and
-  // writes fields no kernel beside it touches; difvisxx reads parts 0 and 2;
+  // each on main. With the streamed tail (stream_tail): main: [k_dt] u tail
+  // ([genflu] before its velocity write), [products 1] v tail, [w tail]; side:
+  // [products 1] w tail on line scratch of its own.
+  // interpyy, interpxx and the energies only read the state (interpxx also
+  // clears the CFL maxima, before the products raise them); each products part
+  // reads and writes fields no kernel beside it touches; difvisxx reads parts 0 and 2;
   // k_dt needs the CFL maxima of parts 0 and 2; genflu needs dt, writes plane
   // 1 of u, v, w after difvisxx has read it and reads plane xout before the
   // tails rewrite it.

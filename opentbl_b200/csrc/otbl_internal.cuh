@@ -65,7 +65,7 @@ struct Work {
   float *twxf, *twx2f;         // the same rounded to FP32 (mixed path)
   unsigned long long *vm_bits; // vm(j) maxima, j = 1..ny
   void *xtab;                  // k_xline's coefficient tables (T): interpxx u, v, difvisxx u, v
-  // streamed kernels of the largest boxes (k_stream.cu): per-plane and per-row
+  // streamed kernels (k_stream.cu): per-plane and per-row
   // coefficients of their rings, implzy's top-down factors
   void *xrowc;                 // [2][2][nx][16] (T), FP64 [1][2][nx][16]: interpxx is not streamed
   double *yrowc, *rowc;        // [2][ny][8] (T), [2][ny+2][16]
@@ -258,7 +258,7 @@ cudaError_t launch_genflu_cols(otbl_ctx *c, int tail);
 // the rhsp tail of the velocity components in the bit mask comps (1 u, 2 v,
 // 4 w), one launch
 cudaError_t launch_final(otbl_ctx *c, unsigned comps);
-// the streamed forms for the largest boxes (k_stream.cu) and where they are
+// the streamed forms (k_stream.cu) and where they are
 // the faster ones; the streamed tail works on line scratch s1..s3
 // (second_scratch: t1..t3), needs launch_tail_rows after k_dt, and its first
 // velocity write waits for before_vel when it is not null
